@@ -405,14 +405,18 @@ constexpr uint32_t kStripBlocksPerSm = 6;
 constexpr int kStageGateThreads = 128;
 constexpr int kStageWordsPerThread = 2;
 
-mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run) {
+mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
+                        const std::function<uint64_t(uint64_t)> &extra_words) {
     const uint64_t nn = std::max<uint64_t>(e->graph.n_nodes(), 1);
     // two chunk buffers, together at most ~48 GB by default
     uint64_t words = run.layered_max_words ? run.layered_max_words : (24ull << 30) / (nn * sizeof(uint64_t));
     words = std::max<uint64_t>(256, std::min<uint64_t>(words, 1ull << 20));
     words = (words + 255) / 256 * 256;
     e->stage_words = words;
-    for (int i = 0; i < 2; ++i) MCG_CUDA(work_alloc(e, (void **)&e->d_stage[i], nn * words * sizeof(uint64_t)));
+    const uint64_t extra = extra_words ? extra_words(words) : 0;
+    MCG_CUDA(work_alloc(e, (void **)&e->d_stage[0], (nn * words + extra) * sizeof(uint64_t)));
+    MCG_CUDA(work_alloc(e, (void **)&e->d_stage[1], nn * words * sizeof(uint64_t)));
+    if (extra) e->d_stage_extra = e->d_stage[0] + nn * words;
     MCG_CUDA(cudaMalloc((void **)&e->d_event_table,
                         std::max<uint64_t>(e->graph.n_be, 1) * mcg::dev::kEventTableStride * sizeof(uint2)));
     // Cap the resident sampler blocks per SM through their shared-memory
@@ -698,9 +702,8 @@ mcg_status run_staged(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t 
 }  // namespace internal
 }  // namespace mcg
 
-extern "C" {
-
-mcg_status mcg_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in, mcg_engine **out) {
+mcg_status mcg::internal::create_with_extra(const mcg_graph_desc *graph, const mcg_run_desc *run_in,
+                                            const std::function<uint64_t(uint64_t)> &extra_words, mcg_engine **out) {
     mcg::clear_error();
     if (!graph || !out) return mcg::fail(MCG_ERR_INVALID, "graph and out must not be NULL");
     *out = nullptr;
@@ -770,7 +773,7 @@ mcg_status mcg_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in, m
         if (st != MCG_OK) break;
         // the fused program is compiled here only for the fused mode (on request otherwise)
         if (e->mode == MCG_MODE_FUSED) st = setup_fused(e, run);
-        else if (e->mode == MCG_MODE_STAGED) st = setup_staged(e, run);
+        else if (e->mode == MCG_MODE_STAGED) st = setup_staged(e, run, extra_words);
         else if (e->mode == MCG_MODE_STRIP) st = setup_strip(e, run);
     } while (false);
     if (st != MCG_OK) {
@@ -780,6 +783,12 @@ mcg_status mcg_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in, m
     }
     *out = e;
     return MCG_OK;
+}
+
+extern "C" {
+
+mcg_status mcg_create(const mcg_graph_desc *graph, const mcg_run_desc *run, mcg_engine **out) {
+    return mcg::internal::create_with_extra(graph, run, {}, out);
 }
 
 mcg_status mcg_engine_launch_shape(mcg_engine *e, uint32_t *mode, uint32_t *ctas_per_sm) {

@@ -71,6 +71,7 @@ struct mcg_engine {
     std::function<mcg_status(cudaStream_t, uint64_t *, uint64_t, uint64_t)> sample_hook;
     uint32_t sampler_smem = 0;          // dynamic smem that caps sampler blocks per SM
     uint64_t stage_words = 0;           // words per chunk the stage buffers hold
+    uint64_t *d_stage_extra = nullptr;  // extra words the creator asked for, behind the first stage buffer
     cudaStream_t s_a = nullptr, s_b = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_a[2] = {nullptr, nullptr}, ev_b[2] = {nullptr, nullptr};
     cudaEvent_t ev_join_a = nullptr, ev_join_b = nullptr;
@@ -100,6 +101,12 @@ struct mcg_engine {
 
 namespace mcg {
 namespace internal {
+
+// mcg_create for an engine whose first stage buffer carries `extra_words(words
+// per chunk)` 64-bit words behind it (d_stage_extra; staged mode only): room
+// that comes and goes with the kept work buffers instead of an allocation.
+mcg_status create_with_extra(const mcg_graph_desc *graph, const mcg_run_desc *run,
+                             const std::function<uint64_t(uint64_t)> &extra_words, mcg_engine **out);
 
 // Staged pass over [word_begin, word_begin + count) for n_it passes (engine.cu).
 mcg_status run_staged(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count);

@@ -30,7 +30,7 @@ namespace {
         }                                                                                       \
     } while (0)
 
-constexpr int kWeightThreads = 256;
+constexpr int kWeightThreads = 128;  // four warps: four neighbouring words are one 32-byte sector of a row
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -54,76 +54,9 @@ __device__ void atomic_max_double(double *addr, double v) {
     }
 }
 
-// One warp per sample column: lane l owns samples l and l + 32 of the word.
-// For samples where the top fires: log w = C + sum_i a_i x_i (FP64).
-// sums = {sum w, sum w^2, hits, max log w}.  With ce != nullptr also
-// ce[i] += sum over hits of w x_i.  Shared memory: a[n_be] (+ ce[n_be]).
-__global__ void __launch_bounds__(kWeightThreads) k_is_weights(const uint64_t *__restrict__ buf, uint64_t W,
-                                                               uint32_t n_be, uint32_t root_row,
-                                                               const double *__restrict__ a, double C,
-                                                               double *__restrict__ sums, double *__restrict__ ce) {
-    extern __shared__ double smem_d[];
-    double *s_a = smem_d;
-    double *s_ce = smem_d + n_be;
-    for (uint32_t i = threadIdx.x; i < n_be; i += blockDim.x) {
-        s_a[i] = a[i];
-        if (ce) s_ce[i] = 0.0;
-    }
-    __syncthreads();
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    double lsum = 0.0, lsum2 = 0.0, lhits = 0.0, lmax = -INFINITY;
-    for (uint64_t w = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < W; w += warps) {
-        const uint64_t top = buf[(uint64_t)root_row * W + w];
-        if (top == 0) continue;  // uniform across the warp
-        const bool f0 = (top >> lane) & 1ull, f1 = (top >> (lane + 32)) & 1ull;
-        double s0 = 0.0, s1 = 0.0;
-        for (uint32_t i = 0; i < n_be; ++i) {
-            const uint64_t x = buf[(uint64_t)i * W + w];
-            if ((x >> lane) & 1ull) s0 += s_a[i];
-            if ((x >> (lane + 32)) & 1ull) s1 += s_a[i];
-        }
-        const double lw0 = C + s0, lw1 = C + s1;
-        const double w0 = f0 ? exp(lw0) : 0.0, w1 = f1 ? exp(lw1) : 0.0;
-        lsum += w0 + w1;
-        lsum2 += w0 * w0 + w1 * w1;
-        lhits += (double)f0 + (double)f1;
-        if (f0) lmax = fmax(lmax, lw0);
-        if (f1) lmax = fmax(lmax, lw1);
-        if (ce) {
-            for (uint32_t i = 0; i < n_be; ++i) {
-                const uint64_t x = buf[(uint64_t)i * W + w];
-                double c = (((x >> lane) & 1ull) ? w0 : 0.0) + (((x >> (lane + 32)) & 1ull) ? w1 : 0.0);
-                c = warp_sum(c);
-                if (lane == 0 && c != 0.0) atomicAdd(&s_ce[i], c);
-            }
-        }
-    }
-    lsum = warp_sum(lsum);
-    lsum2 = warp_sum(lsum2);
-    lhits = warp_sum(lhits);
-    lmax = warp_max(lmax);
-    if (lane == 0) {
-        if (lsum != 0.0) atomicAdd(&sums[0], lsum);
-        if (lsum2 != 0.0) atomicAdd(&sums[1], lsum2);
-        if (lhits != 0.0) atomicAdd(&sums[2], lhits);
-        if (lmax > -INFINITY) atomic_max_double(&sums[3], lmax);
-    }
-    if (ce) {
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n_be; i += blockDim.x)
-            if (s_ce[i] != 0.0) atomicAdd(&ce[i], s_ce[i]);
-    }
-}
-
-// Batched form: many independent trees in one graph, tree k owning basic
-// events [be_begin[k], be_begin[k + 1]) and tallied root root_row[k].
-// Work items are (tree, strip of 256 words), taken from a queue (a counter
-// zeroed before the launch) so that trees of very different size balance.
-// One thread per word: the buffer rows are read coalesced, and because
-// x_i & top is almost always zero under a proposal, the FP64 log-ratios of
-// a sample are only touched where event i fired in a sample where the
-// tree's top event fired.
+// Likelihood ratios: many independent trees in one graph (or one tree), tree
+// k owning basic events [be_begin[k], be_begin[k + 1]) and tallied root
+// root_row[k].  One warp per (tree, word), see k_is_weights.
 // A pass may draw its words from several proposals (components c = 0 ..
 // n_comp - 1, component 0 the main one, c taking a share pi_c of the
 // words).  Every sample is then weighted by the balance heuristic of
@@ -131,8 +64,6 @@ __global__ void __launch_bounds__(kWeightThreads) k_is_weights(const uint64_t *_
 //     w = p(x) / sum_c pi_c q_c(x),
 //     log w = -logsumexp_c(ln pi_c - log(p / q_c)(x)),
 // which is unbiased and keeps w <= p / (pi_c q_c) for every c.
-// acc[c][b] (per-thread, local memory) holds log(p / q_c) - C_c of sample
-// b, acc[0][b] later its weight.
 constexpr int kMaxComponents = 8;
 
 // ---------------------------------------------------------------------------
@@ -202,56 +133,47 @@ struct CutArgs {
     const uint32_t *z_begin;       // per tree: its shared events are z_event[z_begin[k] .. z_begin[k + 1])
     const uint32_t *z_event;
     const uint64_t *z_thr;         // per shared event: z_i = 1 with probability z_thr / 2^32
-    const uint32_t *z_index;       // per basic event: its entry in z_event (shared events only)
     const uint32_t *z_occ_begin;   // per shared event: its occurrences z_occ[z_occ_begin[j] .. z_occ_begin[j + 1])
     const uint32_t *z_occ;
     uint64_t seed;
     unsigned int *error;
 };
 
-// No memo: every entered gate is evaluated.
-struct NoMemo {
-    __device__ bool get(uint32_t, double &) { return false; }
-    __device__ void put(uint32_t, double) {}
-};
-
 // Values of gates already evaluated for one sample: open addressing over
 // kMemoSlots node ids with at most kMemoProbes probes, so a full table costs
 // a few loads per lookup (a sample that sets many shared events evaluates
-// hundreds of gates); values that find no slot are simply not kept.  The
-// slots are cleared on first use, so samples that never evaluate a gate pay
-// nothing.
+// hundreds of gates); values that find no slot are simply not kept.  A bit
+// per slot says that it holds a value, so a new sample clears 32 bytes: the
+// table is per-thread memory, and clearing its keys moved 2.2 GB of it
+// through DRAM for 629,000 samples (1.5 ms of the kernel's 1.6).
 constexpr int kMemoBits = 8;
 constexpr int kMemoSlots = 1 << kMemoBits;
 constexpr int kMemoProbes = 8;
 struct GateMemo {
     uint32_t key[kMemoSlots];
     double val[kMemoSlots];
-    bool ready = false;
-    __device__ void clear() { ready = false; }
-    __device__ void prepare() {
-        if (ready) return;
+    uint32_t used[kMemoSlots / 32];
+    __device__ void clear() {
 #pragma unroll
-        for (int i = 0; i < kMemoSlots; ++i) key[i] = kNoNode;
-        ready = true;
+        for (int i = 0; i < kMemoSlots / 32; ++i) used[i] = 0;
     }
+    __device__ bool holds(uint32_t h) const { return (used[h >> 5] >> (h & 31u)) & 1u; }
     __device__ bool get(uint32_t node, double &v) {
-        prepare();
         uint32_t h = (node * 2654435761u) >> (32 - kMemoBits);
         for (int i = 0; i < kMemoProbes; ++i, h = (h + 1) & (kMemoSlots - 1)) {
+            if (!holds(h)) return false;
             if (key[h] == node) {
                 v = val[h];
                 return true;
             }
-            if (key[h] == kNoNode) return false;
         }
         return false;
     }
     __device__ void put(uint32_t node, double v) {
-        prepare();
         uint32_t h = (node * 2654435761u) >> (32 - kMemoBits);
         for (int i = 0; i < kMemoProbes; ++i, h = (h + 1) & (kMemoSlots - 1)) {
-            if (key[h] == kNoNode || key[h] == node) {
+            if (!holds(h) || key[h] == node) {
+                used[h >> 5] |= 1u << (h & 31u);
                 key[h] = node;
                 val[h] = v;
                 return;
@@ -267,11 +189,11 @@ struct GateMemo {
 // -1 when the tree is deeper than the frames hold.  The frame being worked
 // on (node, next input, accumulator, gate record) stays in registers; only
 // the suspended ancestors and the ATLEAST k-subset sums are in local memory.
-template <class Leaf, class Enter, class Other, class Memo = NoMemo>
+template <class Leaf, class Enter, class Other>
 __device__ double tree_eval(uint32_t root, const uint4 *gate, const uint32_t *inputs, uint32_t n_be, Leaf leaf,
-                            Enter enter, Other other, Memo *memo = nullptr) {
+                            Enter enter, Other other, GateMemo &memo) {
     double known;
-    if (memo && memo->get(root, known)) return known;
+    if (memo.get(root, known)) return known;
     struct Suspended {
         uint32_t node, j;
         double acc;
@@ -310,7 +232,7 @@ __device__ double tree_eval(uint32_t root, const uint4 *gate, const uint32_t *in
                 deliver(other(x));
                 continue;
             }
-            if (memo && memo->get(x, known)) {
+            if (memo.get(x, known)) {
                 deliver(known);
                 continue;
             }
@@ -327,7 +249,7 @@ __device__ double tree_eval(uint32_t root, const uint4 *gate, const uint32_t *in
             continue;
         }
         const double v = op == MCG_ATLEAST ? dp[sp][kk] : acc;
-        if (memo) memo->put(node, v);
+        memo.put(node, v);
         if (sp == 0) return v;
         --sp;
         node = st[sp].node;
@@ -340,9 +262,58 @@ __device__ double tree_eval(uint32_t root, const uint4 *gate, const uint32_t *in
     }
 }
 
-// One thread per (tree, word, sample): draws the tree's shared events, then
-// descends from the tree's top on the conditioned tree and ORs the sample's
-// bit into the words of the chosen cut set's private events.
+// The stream of sample b of word w of tree k.
+__device__ __forceinline__ uint64_t cut_base(const CutArgs &a, uint32_t k, uint64_t w, uint32_t b) {
+    uint64_t base = mix64(a.seed ^ ((uint64_t)k << 32));
+    base = mix64(base ^ (a.word_begin + w));
+    return mix64(base ^ (uint64_t)b);
+}
+
+// Draws the shared events, kDrawEvents of them and kDrawWords words per
+// block: a warp takes a word, lane l its samples l and l + 32, and the two
+// ballots of a draw are the event's word.  Every shared event of the tree
+// draws from the stream zbase of the sample.  Bound by the two 64-bit hashes
+// per lane and draw; drawn inside k_cut_force, one sample per thread, the
+// trees with the most shared events held their SMs long after the others
+// were done.
+constexpr uint32_t kDrawEvents = 32, kDrawWords = 32;
+__global__ void __launch_bounds__(256) k_cut_draw(const __grid_constant__ CutArgs a, uint32_t n_z) {
+    __shared__ uint64_t s_word[kDrawEvents][kDrawWords + 1];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t j0 = blockIdx.x * kDrawEvents, j1 = min(n_z, j0 + kDrawEvents);
+    const uint64_t w0 = (uint64_t)blockIdx.y * kDrawWords;  // at most 2^20 words a chunk
+    uint32_t k0 = 0, hi = a.n_inst;  // the tree of j0: z_begin[k0] <= j0 < z_begin[k0 + 1]
+    while (hi - k0 > 1) {
+        const uint32_t mid = (k0 + hi) / 2;
+        if (a.z_begin[mid] <= j0) k0 = mid;
+        else hi = mid;
+    }
+    for (uint32_t i = warp; i < kDrawWords && w0 + i < a.W; i += 8) {
+        uint32_t k = k0, first = 0, end = 0;
+        uint64_t zbase[2] = {0, 0};
+        for (uint32_t j = j0; j < j1; ++j) {
+            if (j >= end) {  // the first event, or the first of the next tree that has any
+                while (a.z_begin[k + 1] <= j) ++k;
+                first = a.z_begin[k];
+                end = a.z_begin[k + 1];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) zbase[h] = mix64(cut_base(a, k, w0 + i, lane + 32u * h) ^ 0x2545F4914F6CDD1Dull);
+            }
+            const uint64_t add = (uint64_t)(j - first + 1) * 0x9E3779B97F4A7C15ull, thr = a.z_thr[j];
+            const uint32_t lo = __ballot_sync(0xFFFFFFFFu, (mix64(zbase[0] + add) >> 32) < thr);
+            const uint32_t up = __ballot_sync(0xFFFFFFFFu, (mix64(zbase[1] + add) >> 32) < thr);
+            if (lane == 0) s_word[j - j0][i] = ((uint64_t)up << 32) | lo;
+        }
+    }
+    __syncthreads();
+    for (uint32_t j = j0 + warp; j < j1; j += 8)
+        if (w0 + lane < a.W) a.buf[(uint64_t)a.z_event[j] * a.W + w0 + lane] = s_word[j - j0][lane];
+}
+
+// One thread per (tree, word, sample): collects the sample's shared events
+// (drawn by k_cut_draw), then descends from the tree's top on the conditioned
+// tree and ORs the sample's bit into the words of the chosen cut set's
+// private events.
 __global__ void __launch_bounds__(256) k_cut_force(CutArgs a) {
     const uint64_t item = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (item >= (uint64_t)a.n_inst * a.W * 64) return;
@@ -351,36 +322,38 @@ __global__ void __launch_bounds__(256) k_cut_force(CutArgs a) {
     const uint64_t w = wi % a.W;
     const uint32_t k = (uint32_t)(wi / a.W);
     if (!a.tree_ok[k]) return;  // a tree the component cannot draw: nominal samples
-    uint64_t base = mix64(a.seed ^ ((uint64_t)k << 32));
-    base = mix64(base ^ (a.word_begin + w));
-    base = mix64(base ^ (uint64_t)b);
+    const uint64_t base = cut_base(a, k, w, b);
     uint32_t draw = 0;
     const unsigned long long bit = 1ull << b;
     const uint32_t n_be = a.n_be;
-    // z: every shared event of the tree from its own draw of the stream zbase
-    const uint32_t z0 = a.z_begin[k], z1 = a.z_begin[k + 1];
-    const uint64_t zbase = mix64(base ^ 0x2545F4914F6CDD1Dull);
-    auto z_of = [&](uint32_t j) -> bool {  // entry j of z_event
-        return (mix64(zbase + (uint64_t)(j - z0 + 1) * 0x9E3779B97F4A7C15ull) >> 32) < a.z_thr[j];
-    };
+    // the occurrences of the tree's shared events that the sample sets, in
+    // the events' order: a warp holds 32 samples of one word, so its lanes
+    // read 32 events' words at once and pass on the ones set in any sample
     uint32_t occ[kZOcc];
     int n_occ = 0;
     bool prune = true;
-    for (uint32_t j = z0; j < z1; ++j) {
-        if (!z_of(j)) continue;
-        atomicOr(reinterpret_cast<unsigned long long *>(a.buf + (uint64_t)a.z_event[j] * a.W + w), bit);
-        for (uint32_t o = a.z_occ_begin[j]; prune && o < a.z_occ_begin[j + 1]; ++o) {
-            if (n_occ == kZOcc) {
-                prune = false;
-                break;
+    const uint32_t lane = threadIdx.x & 31u, half = b & 32u;
+    const uint32_t z0 = a.z_begin[k], z1 = a.z_begin[k + 1];
+    for (uint32_t j0 = z0; j0 < z1; j0 += 32) {
+        uint32_t x = 0;
+        if (j0 + lane < z1) x = (uint32_t)(a.buf[(uint64_t)a.z_event[j0 + lane] * a.W + w] >> half);
+        for (uint32_t m = __ballot_sync(0xFFFFFFFFu, x != 0); m; m &= m - 1) {
+            const int src = __ffs((int)m) - 1;
+            if (!((__shfl_sync(0xFFFFFFFFu, x, src) >> lane) & 1u)) continue;
+            const uint32_t j = j0 + (uint32_t)src;
+            for (uint32_t o = a.z_occ_begin[j]; prune && o < a.z_occ_begin[j + 1]; ++o) {
+                if (n_occ == kZOcc) {
+                    prune = false;
+                    break;
+                }
+                const uint32_t v = a.z_occ[o];
+                int q = n_occ++;
+                while (q > 0 && occ[q - 1] > v) {
+                    occ[q] = occ[q - 1];
+                    --q;
+                }
+                occ[q] = v;
             }
-            const uint32_t v = a.z_occ[o];
-            int q = n_occ++;
-            while (q > 0 && occ[q - 1] > v) {
-                occ[q] = occ[q - 1];
-                --q;
-            }
-            occ[q] = v;
         }
     }
     // a gate whose subtree holds a z_i = 1 leaf (every gate with shared leaves
@@ -393,14 +366,16 @@ __global__ void __launch_bounds__(256) k_cut_force(CutArgs a) {
             if (occ[q] >= r.x) return occ[q] < r.y;
         return false;
     };
-    auto leaf = [&](uint32_t x) -> double { return a.shared[x] ? (z_of(a.z_index[x]) ? 1.0 : 0.0) : a.S[x]; };
+    auto leaf = [&](uint32_t x) -> double {
+        return a.shared[x] ? (double)((a.buf[(uint64_t)x * a.W + w] >> b) & 1ull) : a.S[x];
+    };
     auto s0 = [&](uint32_t x) -> double { return a.S[x]; };
     GateMemo memo;
     memo.clear();
     auto sz = [&](uint32_t x) -> double {  // S_z of any node
         if (x < n_be) return leaf(x);
         if (!affected(x)) return a.S[x];
-        const double v = tree_eval(x, a.gate, a.inputs, n_be, leaf, affected, s0, &memo);
+        const double v = tree_eval(x, a.gate, a.inputs, n_be, leaf, affected, s0, memo);
         if (v < 0.0) atomicOr(a.error, 4u);
         return v;
     };
@@ -485,23 +460,12 @@ inline uint64_t mix64_host(uint64_t z) {
     return z ^ (z >> 31);
 }
 
-// N(x) of sample b of the word whose rows start at col (row stride W), for
-// the tree rooted at the fired gate `root`; only fired children are visited.
-// Returns -1 when the tree is deeper than the frames hold.
-__device__ double cut_count(const uint64_t *col, uint64_t W, uint32_t root, int b, const uint4 *gate,
-                            const uint32_t *inputs, uint32_t n_be) {
-    auto fired = [&](uint32_t x) -> bool { return (col[(uint64_t)x * W] >> b) & 1ull; };
-    return tree_eval(
-        root, gate, inputs, n_be, [&](uint32_t x) { return fired(x) ? 1.0 : 0.0; }, fired,
-        [&](uint32_t) { return 0.0; });
-}
-
 struct IsBatchArgs {
     const uint64_t *buf;
-    uint64_t W;
+    uint64_t W;                    // row stride of buf
+    uint64_t w_begin, w_count;     // the words of this launch
     uint32_t n_inst;
-    uint32_t strips;               // ceil(W / (kWeightThreads / split))
-    uint32_t split;                // threads per word: 1, 2, 4 or 8
+    uint32_t words_per_warp;       // words a warp takes
     uint32_t n_comp;               // 1 .. kMaxComponents
     uint32_t n_be;                 // stride of a[] and C[] between components
     const uint32_t *be_begin;      // n_inst + 1
@@ -521,125 +485,411 @@ struct IsBatchArgs {
     uint32_t n_be_nodes;           // basic events of the joined graph (node ids below are events)
     unsigned int *error;
     double *sums;                  // per tree: sum w, sum w^2, hits, max log w
+    double *weights;               // [n_inst][w_count][64]: the hits' weights for k_is_ce, or null
     double *ce;                    // per event, or null
-    unsigned long long *queue;
 };
 
-__global__ void __launch_bounds__(kWeightThreads) k_is_weights_batch(IsBatchArgs p) {
-    __shared__ unsigned long long s_item;
-    double acc[kMaxComponents][64];
+constexpr int kWeightWarps = kWeightThreads / 32;
+
+// The suspended frames of a warp's walk (the same for all of its lanes).
+struct WalkFrame {
+    uint64_t mask;     // samples of the word that the frame is evaluated for
+    uint32_t node, j;  // gate, next input
+};
+
+// Values of the recursion of tree_eval for all samples of one word at once:
+// lane l evaluates samples l and l + 32 (v[0], v[1]), the warp walks the
+// union of the gates its samples enter, so there is no divergence and the
+// inputs of a gate are read by 32 lanes at once.  mask holds the samples to
+// evaluate; a lane outside a frame's mask carries values nobody reads.
+//   COUNT: N(x), entered through fired gates, a leaf gives its own bit; only
+//          inputs that fired in some sample of the mask are visited (the
+//          others add 0, and multiply an AND that did not fire).
+//   else:  S_z, entered through gates whose companion fired, every other
+//          input gives S_0 (a shared leaf its bit).
+// The order of the inputs, and with it every rounding, is tree_eval's.
+// Returns false when the tree is deeper than the frames hold.
+template <bool COUNT>
+__device__ bool word_eval(const IsBatchArgs &p, const uint64_t *col, uint32_t root, uint64_t root_mask,
+                          WalkFrame *stack, double (&v)[2]) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nc = p.n_comp;
-    const uint64_t items = (uint64_t)p.n_inst * p.strips;
-    for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(p.queue, 1ull);
-        __syncthreads();
-        const uint64_t item = s_item;
-        __syncthreads();
-        if (item >= items) break;
-        const uint32_t k = (uint32_t)(item / p.strips);
-        // p.split threads share a word, thread q taking its samples [q * 64 / split, (q + 1) * 64 / split)
-        const uint32_t q = threadIdx.x % p.split, per = 64u / p.split;
-        const uint64_t w = (item % p.strips) * (kWeightThreads / p.split) + threadIdx.x / p.split;
-        const bool valid = w < p.W;
-        const uint64_t mine = per == 64u ? ~0ull : ((1ull << per) - 1ull) << (q * per);
-        const uint64_t top = valid ? p.buf[(uint64_t)p.root_row[k] * p.W + w] & mine : 0ull;
-        if (!__syncthreads_or(top != 0ull)) continue;
-        for (uint64_t m = top; m; m &= m - 1) {
-            const int b = __ffsll((long long)m) - 1;
-            for (uint32_t c = 0; c < nc; ++c) acc[c][b] = 0.0;
+    const uint32_t nbn = p.n_be_nodes;
+    double st_acc[kCountDepth][2];               // suspended accumulators
+    double dp[kCountDepth][kCutMaxK + 1][2];     // the k-subset sums of an ATLEAST frame at each depth
+    int sp = 0;
+    uint32_t node = root, j = 0;
+    uint64_t mask = root_mask;
+    uint4 g = p.cut_gate[root - nbn];
+    uint32_t op = g.x & 0xFFu, kk = (g.x >> 8) & 0xFFu;
+    double acc[2];
+    auto start = [&]() {
+        acc[0] = acc[1] = op == MCG_AND ? 1.0 : 0.0;
+        if (op == MCG_ATLEAST) {
+            dp[sp][0][0] = dp[sp][0][1] = 1.0;
+            for (uint32_t r = 1; r <= kk && r <= (uint32_t)kCutMaxK; ++r) dp[sp][r][0] = dp[sp][r][1] = 0.0;
         }
-        const uint32_t b0 = p.be_begin[k], b1 = p.be_begin[k + 1];
-        const uint64_t *col = p.buf + w;
-        uint32_t i = b0;
-        for (; i + 4 <= b1; i += 4) {
+    };
+    auto deliver = [&](double x0, double x1) {
+        if (op == MCG_AND) {
+            acc[0] *= x0;
+            acc[1] *= x1;
+        } else if (op == MCG_ATLEAST) {
+            for (int r = (int)kk; r >= 1; --r) {
+                dp[sp][r][0] += dp[sp][r - 1][0] * x0;
+                dp[sp][r][1] += dp[sp][r - 1][1] * x1;
+            }
+        } else {
+            acc[0] += x0;
+            acc[1] += x1;
+        }
+    };
+    auto bit = [&](uint64_t x, int h) -> bool { return (x >> (lane + 32u * h)) & 1ull; };
+    // the inputs [base, base + 32) of the current gate, one per lane: node id,
+    // the word that says in which samples it is entered (a leaf: fired), S_0
+    uint32_t base = 0xFFFFFFFFu, cid = 0, live = 0;
+    uint64_t cword = 0;
+    double cval = 0.0;
+    uint4 cgate = make_uint4(0u, 0u, 0u, 0u);  // a gate input's record, for the walk into it
+    auto load = [&](uint32_t b) {
+        base = b;
+        cword = 0;
+        cval = 0.0;
+        cid = b + lane < g.z ? p.inputs[g.y + b + lane] : kNoNode;
+        if (cid != kNoNode) {
+            if (cid >= nbn) cgate = p.cut_gate[cid - nbn];
+            if (COUNT) {
+                cword = col[(uint64_t)cid * p.W] & mask;
+            } else if (cid < nbn) {
+                if (p.shared[cid]) cword = col[(uint64_t)cid * p.W] & mask;
+                else cval = p.cut_S[cid];
+            } else {
+                const uint32_t c = p.companion[cid - nbn];
+                if (c != kNoNode) cword = col[(uint64_t)c * p.W] & mask;
+                cval = p.cut_S[cid];
+            }
+        }
+        live = __ballot_sync(0xFFFFFFFFu, COUNT ? cword != 0 : cid != kNoNode);
+    };
+    start();
+    load(0);
+    for (;;) {
+        const uint32_t rest = j - base < 32u ? live & (0xFFFFFFFFu << (j - base)) : 0u;
+        if (rest) {
+            const int s = __ffs((int)rest) - 1;
+            j = base + (uint32_t)s + 1u;
+            const uint32_t x = __shfl_sync(0xFFFFFFFFu, cid, s);
+            const uint64_t xw = __shfl_sync(0xFFFFFFFFu, cword, s);
+            if (COUNT) {
+                if (x < nbn) {
+                    deliver(bit(xw, 0) ? 1.0 : 0.0, bit(xw, 1) ? 1.0 : 0.0);
+                    continue;
+                }
+            } else {
+                const double c = __shfl_sync(0xFFFFFFFFu, cval, s);
+                if (x < nbn || xw == 0) {
+                    // a shared leaf has S_0 = 0, so its bit is all of its value
+                    deliver(x < nbn && bit(xw, 0) ? 1.0 : c, x < nbn && bit(xw, 1) ? 1.0 : c);
+                    continue;
+                }
+            }
+            if (sp + 1 == kCountDepth) return false;
+            if (lane == 0) stack[sp] = WalkFrame{mask, node, j};
+            st_acc[sp][0] = acc[0];
+            st_acc[sp][1] = acc[1];
+            ++sp;
+            node = x;
+            j = 0;
+            mask = xw;
+            g.x = __shfl_sync(0xFFFFFFFFu, cgate.x, s);
+            g.y = __shfl_sync(0xFFFFFFFFu, cgate.y, s);
+            g.z = __shfl_sync(0xFFFFFFFFu, cgate.z, s);
+            op = g.x & 0xFFu;
+            kk = (g.x >> 8) & 0xFFu;
+            start();
+            load(0);
+            continue;
+        }
+        if (base + 32u < g.z) {
+            j = base + 32u;
+            load(j);
+            continue;
+        }
+        double r[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) r[h] = op == MCG_ATLEAST ? dp[sp][kk][h] : acc[h];
+        if (sp == 0) {
+            v[0] = r[0];
+            v[1] = r[1];
+            return true;
+        }
+        // back to the parent: samples that did not enter this gate get its other value
+        const double c = COUNT ? 0.0 : p.cut_S[node];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) r[h] = bit(mask, h) ? r[h] : c;
+        --sp;
+        __syncwarp();
+        const WalkFrame f = stack[sp];
+        __syncwarp();
+        node = f.node;
+        j = f.j;
+        mask = f.mask;
+        acc[0] = st_acc[sp][0];
+        acc[1] = st_acc[sp][1];
+        g = p.cut_gate[node - nbn];
+        op = g.x & 0xFFu;
+        kk = (g.x >> 8) & 0xFFu;
+        deliver(r[0], r[1]);
+        // more inputs of the parent are read again (from L1: the walk has just been there)
+        if (j < g.z) load(j / 32u * 32u);
+        else base = (g.z + 31u) / 32u * 32u, live = 0;
+    }
+}
+
+// One warp per (tree, word): lane l owns samples l and l + 32.  The events'
+// words are read 128 rows at a time (row-major, so the warps of a block, which
+// take neighbouring words, share their sectors), and only events that fired in
+// a sample in which the tree's top event fired touch the FP64 sums, in the
+// events' order.  Then the cut-set terms (word_eval), the balance heuristic
+// and the weights of the two samples, and the sums of the warp's words reduced
+// once per block.  Bound by the walks' instructions (issue slots 45 % busy, the
+// rest latency).  16 trees of 55 to 9,956 events with shared events, 2,048
+// words, 1.2 million hits: 1.9 ms with k_is_ce's 0.3 ms behind it, where one
+// thread per word (or eight), with the 64 samples' sums in local memory, a
+// walk per sample and the cross-entropy sums in the same kernel, took 20 ms.
+// A word's samples over two or four warps: 1.9 and 2.7 ms (their walks visit
+// nearly the same gates), so a word stays with one warp.
+template <int NC>
+__global__ void __launch_bounds__(kWeightThreads, NC <= 2 ? 8 : 4) k_is_weights(const __grid_constant__ IsBatchArgs p) {
+    __shared__ WalkFrame s_stack[kWeightWarps][kCountDepth];
+    __shared__ double s_sum[kWeightWarps][4];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t per_block = (uint64_t)kWeightWarps * p.words_per_warp;
+    const uint64_t blocks_per_tree = (p.w_count + per_block - 1) / per_block;
+    const uint32_t k = (uint32_t)(blockIdx.x / blocks_per_tree);
+    const uint64_t first = (blockIdx.x % blocks_per_tree) * per_block;
+    const uint32_t b0 = p.be_begin[k], b1 = p.be_begin[k + 1], root = p.root_row[k];
+    const bool cut = p.cut_comp >= 0, cut_ok = cut && p.cut_tree_ok[k];
+    double lsum = 0.0, lsum2 = 0.0, lhits = 0.0, lmax = -INFINITY;
+    for (uint32_t i = 0; i < p.words_per_warp; ++i) {
+        const uint64_t wl = first + (uint64_t)i * kWeightWarps + warp;  // the block's warps take neighbouring words
+        if (wl >= p.w_count) break;
+        const uint64_t *col = p.buf + p.w_begin + wl;
+        const uint64_t top = col[(uint64_t)root * p.W];
+        if (top == 0) continue;  // uniform across the warp
+        double s[NC][2];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) s[c][0] = s[c][1] = 0.0;
+        for (uint32_t e0 = b0; e0 < b1; e0 += 128) {
             uint64_t x[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) x[j] = valid ? col[(uint64_t)(i + j) * p.W] : 0ull;
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t e = e0 + 32u * u + lane;
+                x[u] = e < b1 ? col[(uint64_t)e * p.W] & top : 0ull;
+            }
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                for (uint64_t m = x[j] & top; m; m &= m - 1) {
-                    const int b = __ffsll((long long)m) - 1;
-                    for (uint32_t c = 0; c < nc; ++c) acc[c][b] += p.a[(uint64_t)c * p.n_be + i + j];
+            for (int u = 0; u < 4; ++u) {
+                uint32_t m = __ballot_sync(0xFFFFFFFFu, x[u] != 0);
+                if (!m) continue;
+                double av[NC];
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    av[c] = x[u] && c < (int)p.n_comp ? p.a[(uint64_t)c * p.n_be + e0 + 32u * u + lane] : 0.0;
+                for (; m; m &= m - 1) {
+                    const int src = __ffs((int)m) - 1;
+                    const uint64_t xe = __shfl_sync(0xFFFFFFFFu, x[u], src);
+                    const bool f0 = (xe >> lane) & 1ull, f1 = (xe >> (lane + 32u)) & 1ull;
+#pragma unroll
+                    for (int c = 0; c < NC; ++c) {
+                        const double a = __shfl_sync(0xFFFFFFFFu, av[c], src);
+                        if (f0) s[c][0] += a;
+                        if (f1) s[c][1] += a;
+                    }
                 }
             }
         }
-        for (; i < b1; ++i) {
-            for (uint64_t m = (valid ? col[(uint64_t)i * p.W] : 0ull) & top; m; m &= m - 1) {
-                const int b = __ffsll((long long)m) - 1;
-                for (uint32_t c = 0; c < nc; ++c) acc[c][b] += p.a[(uint64_t)c * p.n_be + i];
+        double n_cut[2] = {1.0, 1.0}, log_sz[2] = {0.0, 0.0};
+        if (cut_ok) {
+            log_sz[0] = log_sz[1] = p.cut_logS[k];
+            if (root < p.n_be_nodes) {  // the top is an event: one cut set (a shared one's S_z is 1)
+                if (p.shared[root]) log_sz[0] = log_sz[1] = 0.0;
+            } else {
+                if (!word_eval<true>(p, col, root, top, s_stack[warp], n_cut)) n_cut[0] = n_cut[1] = -1.0;
+                const uint32_t comp = p.companion[root - p.n_be_nodes];
+                const uint64_t ent = comp != kNoNode ? col[(uint64_t)comp * p.W] & top : 0ull;
+                if (ent) {  // samples with a shared leaf z_i = 1 below the top: S_z(top)
+                    double sz[2] = {0.0, 0.0};
+                    if (!word_eval<false>(p, col, root, ent, s_stack[warp], sz)) sz[0] = sz[1] = -1.0;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                        if ((ent >> (lane + 32u * h)) & 1ull) {
+                            if (!(sz[h] > 0.0)) atomicOr(p.error, 2u);
+                            log_sz[h] = log(fmax(sz[h], 1e-300));
+                        }
+                }
             }
         }
-        double lsum = 0.0, lsum2 = 0.0, lhits = 0.0, lmax = -INFINITY;
-        for (uint64_t m = top; m; m &= m - 1) {
-            const int b = __ffsll((long long)m) - 1;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (!((top >> (lane + 32u * h)) & 1ull)) continue;
             double lw_cut = 0.0;
-            if (p.cut_comp >= 0 && !p.cut_tree_ok[k]) {
-                lw_cut = p.C[(uint64_t)p.cut_comp * p.n_inst + k] + acc[p.cut_comp][b];  // nominal: 0
-            } else if (p.cut_comp >= 0) {
-                const uint32_t root = p.root_row[k], nbn = p.n_be_nodes;
-                const double n_cut = cut_count(col, p.W, root, b, p.cut_gate, p.inputs, nbn);
-                if (!(n_cut >= 1.0)) atomicOr(p.error, 2u);  // too deep, or a failure without a cut set
-                double log_sz = p.cut_logS[k];
-                auto fired = [&](uint32_t x) -> bool { return (col[(uint64_t)x * p.W] >> b) & 1ull; };
-                auto entered = [&](uint32_t x) -> bool {
-                    const uint32_t c = p.companion[x - nbn];
-                    return c != kNoNode && fired(c);
-                };
-                if (entered(root)) {  // a shared leaf with z_i = 1 below the top: S_z(top)
-                    const double sz = tree_eval(
-                        root, p.cut_gate, p.inputs, nbn,
-                        [&](uint32_t x) { return p.shared[x] ? (fired(x) ? 1.0 : 0.0) : p.cut_S[x]; }, entered,
-                        [&](uint32_t x) { return p.cut_S[x]; });
-                    if (!(sz > 0.0)) atomicOr(p.error, 2u);
-                    log_sz = log(fmax(sz, 1e-300));
+            if (cut) {
+                double s_cut = 0.0;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) s_cut = c == p.cut_comp ? s[c][h] : s_cut;
+                lw_cut = p.C[(uint64_t)p.cut_comp * p.n_inst + k] + s_cut;
+                if (cut_ok) {
+                    if (!(n_cut[h] >= 1.0)) atomicOr(p.error, 2u);  // too deep, or a failure without a cut set
+                    lw_cut += log_sz[h];
+                    if (n_cut[h] > 1.0) lw_cut -= log(n_cut[h]);
                 }
-                lw_cut = p.C[(uint64_t)p.cut_comp * p.n_inst + k] + acc[p.cut_comp][b] + log_sz -
-                         log(fmax(n_cut, 1.0));
             }
-            double lw = p.cut_comp == 0 ? lw_cut : p.C[k] + acc[0][b];
-            if (nc > 1) {
+            double lw = p.cut_comp == 0 ? lw_cut : p.C[k] + s[0][h];
+            if (NC > 1 && p.n_comp > 1) {
                 // -logsumexp_c(ln pi_c - log(p/q_c))
-                double u[kMaxComponents], hi = -INFINITY;
-                for (uint32_t c = 0; c < nc; ++c) {
-                    const double lwc = (int)c == p.cut_comp ? lw_cut : p.C[(uint64_t)c * p.n_inst + k] + acc[c][b];
-                    u[c] = p.log_pi[c] - lwc;
-                    hi = fmax(hi, u[c]);
+                double u[NC], hi = -INFINITY;
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    u[c] = -INFINITY;
+                    if (c < (int)p.n_comp) {
+                        u[c] = p.log_pi[c] -
+                               (c == p.cut_comp ? lw_cut : p.C[(uint64_t)c * p.n_inst + k] + s[c][h]);
+                        hi = fmax(hi, u[c]);
+                    }
                 }
-                double s = 0.0;
-                for (uint32_t c = 0; c < nc; ++c) s += exp(u[c] - hi);
-                lw = -(hi + log(s));
+                double sum = 0.0;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (c < (int)p.n_comp) sum += u[c] == hi ? 1.0 : exp(u[c] - hi);
+                lw = -(hi + log(sum));
             }
             const double wv = exp(lw);
-            acc[0][b] = wv;
+            if (p.weights) p.weights[((uint64_t)k * p.w_count + wl) * 64u + lane + 32u * h] = wv;
             lsum += wv;
             lsum2 += wv * wv;
             lhits += 1.0;
             lmax = fmax(lmax, lw);
         }
-        if (p.ce) {
-            for (uint32_t e = b0; e < b1; ++e) {
-                uint64_t m = (valid ? col[(uint64_t)e * p.W] : 0ull) & top;
-                double c = 0.0;
-                for (; m; m &= m - 1) c += acc[0][__ffsll((long long)m) - 1];
-                if (__any_sync(0xFFFFFFFFu, c != 0.0)) {
-                    c = warp_sum(c);
-                    if (lane == 0 && c != 0.0) atomicAdd(&p.ce[e], c);
-                }
-            }
+    }
+    lsum = warp_sum(lsum);
+    lsum2 = warp_sum(lsum2);
+    lhits = warp_sum(lhits);
+    lmax = warp_max(lmax);
+    if (lane == 0) {
+        s_sum[warp][0] = lsum;
+        s_sum[warp][1] = lsum2;
+        s_sum[warp][2] = lhits;
+        s_sum[warp][3] = lmax;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t[4] = {0.0, 0.0, 0.0, -INFINITY};
+        for (int q = 0; q < kWeightWarps; ++q) {
+            t[0] += s_sum[q][0];
+            t[1] += s_sum[q][1];
+            t[2] += s_sum[q][2];
+            t[3] = fmax(t[3], s_sum[q][3]);
         }
-        lsum = warp_sum(lsum);
-        lsum2 = warp_sum(lsum2);
-        lhits = warp_sum(lhits);
-        lmax = warp_max(lmax);
-        if (lane == 0 && lhits != 0.0) {
+        if (t[2] != 0.0) {
             double *out = p.sums + 4ull * k;
-            atomicAdd(&out[0], lsum);
-            atomicAdd(&out[1], lsum2);
-            atomicAdd(&out[2], lhits);
-            atomic_max_double(&out[3], lmax);
+            atomicAdd(&out[0], t[0]);
+            atomicAdd(&out[1], t[1]);
+            atomicAdd(&out[2], t[2]);
+            atomic_max_double(&out[3], t[3]);
         }
     }
+}
+
+// Cross-entropy numerators, sum over hits of w x_i: one warp per event and
+// share of the words, reading the weights k_is_weights left of the samples
+// where the event and the top event fired, and one reduction per warp (inside
+// the weights kernel it was one per event and 32 words, with an FP64 atomic
+// each: 5.4 ms of the 20).  Shares of at most 256 words: the events whose
+// proposal is near 1/2 read every word and would be a long tail (0.31 ms on
+// the set above; 0.75 ms with 1,024 words).
+__global__ void __launch_bounds__(kWeightThreads) k_is_ce(const __grid_constant__ IsBatchArgs p, uint32_t n_events) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t e = blockIdx.x * kWeightWarps + (threadIdx.x >> 5);
+    if (e >= n_events) return;
+    uint32_t lo = 0, hi = p.n_inst;  // the tree: be_begin[lo] <= e < be_begin[lo + 1]
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) / 2;
+        if (p.be_begin[mid] <= e) lo = mid;
+        else hi = mid;
+    }
+    const uint64_t *row = p.buf + (uint64_t)e * p.W + p.w_begin;
+    const uint64_t *top = p.buf + (uint64_t)p.root_row[lo] * p.W + p.w_begin;
+    const double *weights = p.weights + (uint64_t)lo * p.w_count * 64u;
+    double c = 0.0;
+    const uint64_t step = 128ull * gridDim.y;
+    for (uint64_t w0 = 128ull * blockIdx.y; w0 < p.w_count; w0 += step) {
+        uint64_t x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t w = w0 + 32u * u + lane;
+            x[u] = w < p.w_count ? row[w] : 0ull;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t w = w0 + 32u * u + lane;
+            if (x[u]) x[u] &= top[w];
+            // a word with few samples is its lane's; a dense one (an event whose proposal is near 1/2) is read by
+            // all lanes together, two weights each
+            const bool dense = __popcll(x[u]) > 3;
+            uint32_t m = __ballot_sync(0xFFFFFFFFu, dense);
+            if (!dense)
+                for (uint64_t b = x[u]; b; b &= b - 1)
+                    c += weights[w * 64u + (uint32_t)__ffsll((long long)b) - 1u];
+            for (; m; m &= m - 1) {
+                const int src = __ffs((int)m) - 1;
+                const uint64_t xe = __shfl_sync(0xFFFFFFFFu, x[u], src);
+                const double *ww = weights + (w0 + 32u * u + (uint32_t)src) * 64u + lane;
+                if ((xe >> lane) & 1ull) c += ww[0];
+                if ((xe >> (lane + 32u)) & 1ull) c += ww[32];
+            }
+        }
+    }
+    if (!__any_sync(0xFFFFFFFFu, c != 0.0)) return;
+    c = warp_sum(c);
+    if (lane == 0) {
+        if (gridDim.y == 1) p.ce[e] += c;
+        else atomicAdd(&p.ce[e], c);
+    }
+}
+
+// Size of the buffer between the two kernels (behind the engine's first stage
+// buffer), for chunks of `words` words: 64 weights per tree and word, at most
+// 1 GiB; longer chunks are taken in several launches.
+uint64_t hit_weight_words(uint32_t n_inst, uint64_t words) {
+    const uint64_t most = std::max<uint64_t>(32, (1ull << 27) / (64ull * n_inst));
+    return 64ull * n_inst * std::min<uint64_t>(words, most);
+}
+
+// Queues both kernels for one chunk of W words.
+cudaError_t launch_weights(IsBatchArgs p, uint32_t n_events, uint64_t weight_words, int sms, cudaStream_t s) {
+    const uint64_t W = p.W;
+    for (uint64_t at = 0; at < W; at += p.w_count) {
+        p.w_begin = at;
+        p.w_count = p.ce ? std::min<uint64_t>(W - at, weight_words) : W - at;
+        // a warp takes one word, and several where a launch has far more words than the chip runs at once: fewer
+        // atomics on a tree's four sums
+        const uint64_t words = (uint64_t)p.n_inst * p.w_count;
+        p.words_per_warp = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(16, words / ((uint64_t)sms * 64 * 4)));
+        const uint64_t per_block = (uint64_t)kWeightWarps * p.words_per_warp;
+        const uint32_t blocks = (uint32_t)(p.n_inst * ((p.w_count + per_block - 1) / per_block));
+        if (p.n_comp == 1) k_is_weights<1><<<blocks, kWeightThreads, 0, s>>>(p);
+        else if (p.n_comp == 2) k_is_weights<2><<<blocks, kWeightThreads, 0, s>>>(p);
+        else if (p.n_comp <= 4) k_is_weights<4><<<blocks, kWeightThreads, 0, s>>>(p);
+        else k_is_weights<kMaxComponents><<<blocks, kWeightThreads, 0, s>>>(p);
+        if (p.ce && n_events) {
+            const uint32_t eb = (n_events + kWeightWarps - 1) / kWeightWarps;
+            uint32_t split = 1;
+            while (p.w_count / split > 256) split *= 2;
+            k_is_ce<<<dim3(eb, split), kWeightThreads, 0, s>>>(p, n_events);
+        }
+        const cudaError_t err = cudaGetLastError();
+        if (err != cudaSuccess) return err;
+    }
+    return cudaSuccess;
 }
 
 // Proposal table and log-ratio terms at the quantised probabilities, for the
@@ -676,8 +926,8 @@ struct mcg_is {
     double *d_a = nullptr;       // per-event log-ratio increments
     double *d_sums = nullptr;    // 4 doubles
     double *d_ce = nullptr;      // per-event CE numerators
-    uint32_t root_row = 0;
-    uint32_t weight_smem = 0;
+    double *d_C = nullptr;       // the constant of the log-ratio
+    uint32_t *d_tree = nullptr;  // the one tree of k_is_weights: its events [0, n_be), its root row
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -705,27 +955,26 @@ mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in
     run.mode = MCG_MODE_STAGED;
     default_chunk(*graph, run);
     auto is = std::make_unique<mcg_is>();
-    mcg_status st = mcg_create(graph, &run, &is->engine);
+    mcg_status st = mcg::internal::create_with_extra(
+        graph, &run, [](uint64_t words) { return hit_weight_words(1, words); }, &is->engine);
     if (st != MCG_OK) return st;
     mcg_engine *e = is->engine;
     const uint32_t nb = e->graph.n_be;
-    is->root_row = e->graph.tally_nodes[0];
-    is->weight_smem = (uint32_t)(2ull * std::max<uint32_t>(nb, 1) * sizeof(double));
     cudaDeviceProp prop;
     MCG_CUDA(cudaGetDeviceProperties(&prop, e->device));
-    if (is->weight_smem > prop.sharedMemPerBlockOptin) {
+    if (2ull * std::max<uint32_t>(nb, 1) * sizeof(double) > prop.sharedMemPerBlockOptin) {
+        // the documented limit of this entry point (larger trees: mcg_is_batch_create with one tree)
         mcg_destroy(e);
         return mcg::fail(MCG_ERR_INVALID, "too many basic events for the weights kernel's shared memory");
-    }
-    st = mcg::set_smem_limit(k_is_weights, is->weight_smem);
-    if (st != MCG_OK) {
-        mcg_destroy(e);
-        return st;
     }
     MCG_CUDA(cudaMalloc((void **)&is->d_be_q, std::max<uint32_t>(nb, 1) * sizeof(uint4)));
     MCG_CUDA(cudaMalloc((void **)&is->d_a, std::max<uint32_t>(nb, 1) * sizeof(double)));
     MCG_CUDA(cudaMalloc((void **)&is->d_ce, std::max<uint32_t>(nb, 1) * sizeof(double)));
     MCG_CUDA(cudaMalloc((void **)&is->d_sums, 4 * sizeof(double)));
+    MCG_CUDA(cudaMalloc((void **)&is->d_C, sizeof(double)));
+    MCG_CUDA(cudaMalloc((void **)&is->d_tree, 3 * sizeof(uint32_t)));
+    const uint32_t tree[3] = {0u, nb, e->graph.tally_nodes[0]};
+    MCG_CUDA(cudaMemcpy(is->d_tree, tree, sizeof(tree), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaEventCreate(&is->ev0));
     MCG_CUDA(cudaEventCreate(&is->ev1));
     *out = is.release();
@@ -743,6 +992,8 @@ mcg_status mcg_is_destroy(mcg_is *is) {
     cudaFree(is->d_a);
     cudaFree(is->d_ce);
     cudaFree(is->d_sums);
+    cudaFree(is->d_C);
+    cudaFree(is->d_tree);
     if (is->ev0) cudaEventDestroy(is->ev0);
     if (is->ev1) cudaEventDestroy(is->ev1);
     if (is->engine) mcg_destroy(is->engine);
@@ -769,21 +1020,30 @@ mcg_status mcg_is_run(mcg_is *is, const uint64_t *q_thr, uint32_t iteration, uin
     MCG_CUDA(cudaMemcpyAsync(is->d_a, a.data(), nb * sizeof(double), cudaMemcpyHostToDevice, e->stream));
     const double init[4] = {0.0, 0.0, 0.0, -std::numeric_limits<double>::infinity()};
     MCG_CUDA(cudaMemcpyAsync(is->d_sums, init, sizeof(init), cudaMemcpyHostToDevice, e->stream));
+    MCG_CUDA(cudaMemcpyAsync(is->d_C, &C, sizeof(C), cudaMemcpyHostToDevice, e->stream));
     MCG_CUDA(cudaMemsetAsync(is->d_ce, 0, std::max<uint32_t>(nb, 1) * sizeof(double), e->stream));
     const bool want_ce = ce_num != nullptr;
     e->d_be_sample = is->d_be_q;
     e->table_iteration = 0xFFFFFFFFu;  // the sampler table follows the proposal
-    const uint32_t root_row = is->root_row;
-    const uint32_t smem = want_ce ? is->weight_smem : is->weight_smem / 2;
-    double *d_a = is->d_a, *d_sums = is->d_sums, *d_ce = want_ce ? is->d_ce : nullptr;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
+    IsBatchArgs args{};
+    args.n_inst = args.n_comp = 1;
+    args.n_be = args.n_be_nodes = nb;
+    args.be_begin = is->d_tree;
+    args.root_row = is->d_tree + 2;
+    args.a = is->d_a;
+    args.C = is->d_C;
+    args.cut_comp = -1;
+    args.sums = is->d_sums;
+    args.weights = want_ce ? reinterpret_cast<double *>(e->d_stage_extra) : nullptr;
+    args.ce = want_ce ? is->d_ce : nullptr;
+    const uint64_t weight_words = hit_weight_words(1, e->stage_words) / 64u;
     e->chunk_hook = [=](cudaStream_t s, const uint64_t *buf, uint64_t W) -> mcg_status {
-        const uint64_t warps = (W + 0) / 1;
-        const uint32_t blocks = (uint32_t)std::min<uint64_t>((warps + 7) / 8, (uint64_t)sms * 8);
-        k_is_weights<<<std::max<uint32_t>(blocks, 1), kWeightThreads, smem, s>>>(buf, W, nb, root_row, d_a, C,
-                                                                                 d_sums, d_ce);
-        const cudaError_t err = cudaGetLastError();
+        IsBatchArgs p = args;
+        p.buf = buf;
+        p.W = W;
+        const cudaError_t err = launch_weights(p, nb, weight_words, sms, s);
         if (err != cudaSuccess) return mcg::fail(MCG_ERR_CUDA, std::string("k_is_weights: ") + cudaGetErrorString(err));
         return MCG_OK;
     };
@@ -833,7 +1093,6 @@ struct mcg_is_batch {
     double *d_ce = nullptr;
     uint32_t *d_be_begin = nullptr;
     uint32_t *d_root = nullptr;
-    unsigned long long *d_queue = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     std::vector<uint4> beq;
     std::vector<double> a, C, init;
@@ -855,7 +1114,7 @@ struct mcg_is_batch {
     std::vector<uint64_t> z_thr, cut_q;  // per run: their proposal thresholds; the component's table
     unsigned char *d_shared = nullptr;
     uint2 *d_gate_occ = nullptr;
-    uint32_t *d_companion = nullptr, *d_z_begin = nullptr, *d_z_event = nullptr, *d_z_index = nullptr;
+    uint32_t *d_companion = nullptr, *d_z_begin = nullptr, *d_z_event = nullptr;
     uint32_t *d_z_occ_begin = nullptr, *d_z_occ = nullptr;
     uint64_t *d_z_thr = nullptr;
 };
@@ -876,14 +1135,13 @@ void release_batch(mcg_is_batch *b) {
     cudaFree(b->d_ce);
     cudaFree(b->d_be_begin);
     cudaFree(b->d_root);
-    cudaFree(b->d_queue);
     cudaFree(b->d_cut_gate);
     cudaFree(b->d_cut_S);
     cudaFree(b->d_cut_tab);
     cudaFree(b->d_cut_logS);
     cudaFree(b->d_cut_error);
     for (void *q : {(void *)b->d_tree_ok, (void *)b->d_shared, (void *)b->d_gate_occ, (void *)b->d_companion, (void *)b->d_z_begin,
-                    (void *)b->d_z_event, (void *)b->d_z_index, (void *)b->d_z_occ_begin, (void *)b->d_z_occ,
+                    (void *)b->d_z_event, (void *)b->d_z_occ_begin, (void *)b->d_z_occ,
                     (void *)b->d_z_thr})
         cudaFree(q);
     if (b->ev0) cudaEventDestroy(b->ev0);
@@ -1028,7 +1286,9 @@ mcg_status mcg_is_batch_create(const mcg_graph_desc *graph, uint32_t n_inst, con
     b->companions = add_companions(*graph, n_inst, be_begin, aug);
     b->companion = aug.companion;
     b->tree_gates_ok = aug.tree_ok;
-    mcg_status st = mcg_create(b->companions ? &aug.desc : graph, &run, &b->engine);
+    mcg_status st = mcg::internal::create_with_extra(
+        b->companions ? &aug.desc : graph, &run,
+        [n_inst](uint64_t words) { return hit_weight_words(n_inst, words); }, &b->engine);
     if (st != MCG_OK) return st;
     const mcg::Graph &g = b->engine->graph;
     const std::string bad = check_partition(g, b->be_begin);
@@ -1039,7 +1299,6 @@ mcg_status mcg_is_batch_create(const mcg_graph_desc *graph, uint32_t n_inst, con
     MCG_CUDA(cudaMalloc((void **)&b->d_sums, 4ull * n_inst * sizeof(double)));
     MCG_CUDA(cudaMalloc((void **)&b->d_be_begin, (n_inst + 1ull) * sizeof(uint32_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_root, n_inst * sizeof(uint32_t)));
-    MCG_CUDA(cudaMalloc((void **)&b->d_queue, sizeof(unsigned long long)));
     MCG_CUDA(cudaMemcpy(b->d_be_begin, be_begin, (n_inst + 1ull) * sizeof(uint32_t), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_root, g.tally_nodes.data(), n_inst * sizeof(uint32_t), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaEventCreate(&b->ev0));
@@ -1207,13 +1466,12 @@ mcg_status build_cut_tables(mcg_is_batch *b) {
     bool any = false;
     for (uint32_t t = 0; t < b->n_inst; ++t) any |= ok[t] != 0;
     if (!any) return mcg::fail(MCG_ERR_INVALID, why.empty() ? std::string("cut-set sampling: no tree qualifies") : why);
-    std::vector<uint32_t> z_begin(b->n_inst + 1, 0), z_index(nb, 0), z_occ_begin{0}, z_occ;
+    std::vector<uint32_t> z_begin(b->n_inst + 1, 0), z_occ_begin{0}, z_occ;
     b->z_event.clear();
     for (uint32_t t = 0; t < b->n_inst; ++t) {
         z_begin[t] = (uint32_t)b->z_event.size();
         for (uint32_t i = b->be_begin[t]; i < b->be_begin[t + 1]; ++i) {
             if (!b->shared[i] || !ok[t]) continue;
-            z_index[i] = (uint32_t)b->z_event.size();
             b->z_event.push_back(i);
             z_occ.insert(z_occ.end(), occ_of[i].begin(), occ_of[i].end());
             z_occ_begin.push_back((uint32_t)z_occ.size());
@@ -1237,7 +1495,6 @@ mcg_status build_cut_tables(mcg_is_batch *b) {
     MCG_CUDA(cudaMalloc((void **)&b->d_companion, comp.size() * sizeof(uint32_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_z_begin, z_begin.size() * sizeof(uint32_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_z_event, nz * sizeof(uint32_t)));
-    MCG_CUDA(cudaMalloc((void **)&b->d_z_index, std::max<uint32_t>(nb, 1) * sizeof(uint32_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_z_occ_begin, z_occ_begin.size() * sizeof(uint32_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_z_occ, z_occ.size() * sizeof(uint32_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_z_thr, nz * sizeof(uint64_t)));
@@ -1245,10 +1502,7 @@ mcg_status build_cut_tables(mcg_is_batch *b) {
     MCG_CUDA(cudaMemcpy(b->d_cut_S, S.data(), nn * sizeof(double), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_cut_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_cut_logS, logS.data(), b->n_inst * sizeof(double), cudaMemcpyHostToDevice));
-    if (nb) {
-        MCG_CUDA(cudaMemcpy(b->d_shared, b->shared.data(), nb, cudaMemcpyHostToDevice));
-        MCG_CUDA(cudaMemcpy(b->d_z_index, z_index.data(), nb * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    }
+    if (nb) MCG_CUDA(cudaMemcpy(b->d_shared, b->shared.data(), nb, cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_gate_occ, occ_range.data(), occ_range.size() * sizeof(uint2), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_companion, comp.data(), comp.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_z_begin, z_begin.data(), z_begin.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -1398,7 +1652,8 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
         args.log_pi[c] = nc > 1 ? std::log((double)comp_words[c] / (double)word_count) : 0.0;
     args.sums = b->d_sums;
     args.ce = ce_num ? b->d_ce : nullptr;
-    args.queue = b->d_queue;
+    args.weights = ce_num ? reinterpret_cast<double *>(e->d_stage_extra) : nullptr;
+    const uint64_t weight_words = hit_weight_words(n_inst, e->stage_words) / (64ull * n_inst);
     args.cut_comp = cut_comp;
     args.cut_logS = b->d_cut_logS;
     args.cut_gate = b->d_cut_gate;
@@ -1414,21 +1669,9 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
         IsBatchArgs p = args;
         p.buf = buf;
         p.W = W;
-        // one thread per word, or more where that leaves most SMs idle (a
-        // few trees in a short pass: each sample's cut-set terms are costly)
-        p.split = 1;
-        while (p.split < 8 && (uint64_t)n_inst * ((W * p.split + kWeightThreads - 1) / kWeightThreads) < 4ull * sms)
-            p.split *= 2;
-        p.strips = (uint32_t)((W * p.split + kWeightThreads - 1) / kWeightThreads);
-        const uint64_t items = (uint64_t)n_inst * p.strips;
-        const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(items, (uint64_t)sms * 8));
-        cudaError_t err = cudaMemsetAsync(p.queue, 0, sizeof(unsigned long long), s);
-        if (err == cudaSuccess) {
-            k_is_weights_batch<<<blocks, kWeightThreads, 0, s>>>(p);
-            err = cudaGetLastError();
-        }
+        const cudaError_t err = launch_weights(p, (uint32_t)nb, weight_words, sms, s);
         if (err != cudaSuccess)
-            return mcg::fail(MCG_ERR_CUDA, std::string("k_is_weights_batch: ") + cudaGetErrorString(err));
+            return mcg::fail(MCG_ERR_CUDA, std::string("k_is_weights: ") + cudaGetErrorString(err));
         return MCG_OK;
     };
     MCG_CUDA(cudaEventRecord(b->ev0, e->stream));
@@ -1453,17 +1696,21 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
             ca.z_begin = b->d_z_begin;
             ca.z_event = b->d_z_event;
             ca.z_thr = b->d_z_thr;
-            ca.z_index = b->d_z_index;
             ca.z_occ_begin = b->d_z_occ_begin;
             ca.z_occ = b->d_z_occ;
             ca.seed = mix64_host(((uint64_t)iteration << 32) ^ 0x5bd1e995u);
             ca.error = b->d_cut_error;
+            const uint32_t n_z = (uint32_t)b->z_event.size();
             e->sample_hook = [=](cudaStream_t s, uint64_t *buf, uint64_t W, uint64_t wb) -> mcg_status {
                 CutArgs x = ca;
                 x.buf = buf;
                 x.W = W;
                 x.word_begin = wb;
                 const uint64_t threads = (uint64_t)x.n_inst * W * 64;
+                if (n_z) {
+                    const dim3 grid((n_z + kDrawEvents - 1) / kDrawEvents, (uint32_t)((W + kDrawWords - 1) / kDrawWords));
+                    k_cut_draw<<<grid, 256, 0, s>>>(x, n_z);
+                }
                 k_cut_force<<<(uint32_t)((threads + 255) / 256), 256, 0, s>>>(x);
                 const cudaError_t err = cudaGetLastError();
                 if (err != cudaSuccess) return mcg::fail(MCG_ERR_CUDA, std::string("k_cut_force: ") + cudaGetErrorString(err));
