@@ -8,10 +8,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <limits>
 #include <memory>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "engine_internal.hpp"
@@ -132,7 +130,7 @@ struct CutArgs {
     const uint2 *gate_occ;         // per gate: [lo, hi) of the shared-leaf occurrences below it
     const uint32_t *z_begin;       // per tree: its shared events are z_event[z_begin[k] .. z_begin[k + 1])
     const uint32_t *z_event;
-    const uint64_t *z_thr;         // per shared event: z_i = 1 with probability z_thr / 2^32
+    const uint64_t *q;             // per basic event: a shared event z_i = 1 with probability q / 2^32
     const uint32_t *z_occ_begin;   // per shared event: its occurrences z_occ[z_occ_begin[j] .. z_occ_begin[j + 1])
     const uint32_t *z_occ;
     uint64_t seed;
@@ -299,7 +297,7 @@ __global__ void __launch_bounds__(256) k_cut_draw(const __grid_constant__ CutArg
 #pragma unroll
                 for (int h = 0; h < 2; ++h) zbase[h] = mix64(cut_base(a, k, w0 + i, lane + 32u * h) ^ 0x2545F4914F6CDD1Dull);
             }
-            const uint64_t add = (uint64_t)(j - first + 1) * 0x9E3779B97F4A7C15ull, thr = a.z_thr[j];
+            const uint64_t add = (uint64_t)(j - first + 1) * 0x9E3779B97F4A7C15ull, thr = a.q[a.z_event[j]];
             const uint32_t lo = __ballot_sync(0xFFFFFFFFu, (mix64(zbase[0] + add) >> 32) < thr);
             const uint32_t up = __ballot_sync(0xFFFFFFFFu, (mix64(zbase[1] + add) >> 32) < thr);
             if (lane == 0) s_word[j - j0][i] = ((uint64_t)up << 32) | lo;
@@ -892,40 +890,93 @@ cudaError_t launch_weights(IsBatchArgs p, uint32_t n_events, uint64_t weight_wor
     return cudaSuccess;
 }
 
-// Proposal table and log-ratio terms at the quantised probabilities, for the
-// events [b0, b1): beq[i] (the sampler's layout), a[i], and the sum of the
-// constant terms over the range.  Returns false with `why` set on a bad q.
-bool ratio_terms(const mcg::Graph &g, const uint64_t *q_thr, uint32_t b0, uint32_t b1, uint4 *beq, double *a,
-                 double &C, std::string &why) {
-    const double two32 = 4294967296.0;
-    C = 0.0;
-    for (uint32_t i = b0; i < b1; ++i) {
+// Inputs of a run from its proposal thresholds, one block per (tree,
+// component): the sampler's table beq, the log-ratio terms at the quantised
+// probabilities
+//     a_i = ln(p_i / q_i) - l_i,  l_i = ln((1 - p_i) / (1 - q_i)),
+// and the tree's constant C = sum_i l_i (threads take events at a fixed
+// stride and are summed in a fixed order: the same thresholds give the same
+// C).  Component 0's blocks also reset the tree's sums.  On the device
+// because four logarithms per event and component took the host 2 ms for two
+// components of 30,000 events, and the terms 24 bytes per event of upload
+// where the thresholds are 8.
+struct RatioArgs {
+    const uint4 *be;               // nominal table {pdag + 1, event + 1, thr lo, thr hi}
+    const uint64_t *q;             // [n_comp][n_be]
+    const uint32_t *be_begin;      // n_inst + 1
+    uint32_t n_be, n_inst;
+    int cut_comp;                  // its shared events are drawn by k_cut_draw: the sampler leaves them 0
+    const unsigned char *drawn;    // per basic event: such an event (cut_comp >= 0)
+    uint4 *beq;                    // [n_comp][n_be]
+    double *a, *C;                 // [n_comp][n_be], [n_comp][n_inst]
+    double *sums, *ce;             // ce may be null
+};
+
+constexpr int kRatioThreads = 256;
+__global__ void __launch_bounds__(kRatioThreads) k_ratio_terms(RatioArgs r) {
+    __shared__ double s_part[kRatioThreads / 32];
+    const uint32_t k = blockIdx.x, c = blockIdx.y;
+    const uint32_t b1 = r.be_begin[k + 1];
+    const uint64_t row = (uint64_t)c * r.n_be;
+    constexpr double kTwo32 = 4294967296.0;
+    double l = 0.0;
+    for (uint32_t i = r.be_begin[k] + threadIdx.x; i < b1; i += kRatioThreads) {
+        const uint4 n = r.be[i];
+        const uint64_t tp = ((uint64_t)n.w << 32) | n.z, tq = r.q[row + i];
+        const bool zero = (int)c == r.cut_comp && r.drawn[i];
+        r.beq[row + i] = make_uint4(n.x, n.y, zero ? 0u : (uint32_t)tq, zero ? 0u : (uint32_t)(tq >> 32));
+        double a = 0.0;
+        if (tp != 0 && tp < (1ull << 32)) {
+            const double p = (double)tp / kTwo32, q = (double)tq / kTwo32;
+            const double l1 = log1p(-p) - log1p(-q);
+            a = log(p) - log(q) - l1;
+            l += l1;
+        }
+        r.a[row + i] = a;
+        if (c == 0 && r.ce) r.ce[i] = 0.0;
+    }
+    l = warp_sum(l);
+    if ((threadIdx.x & 31u) == 0) s_part[threadIdx.x >> 5] = l;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < kRatioThreads / 32; ++w) t += s_part[w];
+        r.C[(uint64_t)c * r.n_inst + k] = t;
+        if (c == 0) {
+            double *out = r.sums + 4ull * k;
+            out[0] = out[1] = out[2] = 0.0;
+            out[3] = -INFINITY;
+        }
+    }
+}
+
+// A proposal threshold must lie in [1, 2^32 - 1], or equal a constant nominal
+// one; returns the first event where it does not, or n_be.
+uint32_t bad_threshold(const mcg::Graph &g, const uint64_t *q_thr) {
+    for (uint32_t i = 0; i < g.n_be; ++i) {
         const uint64_t tp = g.be_threshold[i], tq = q_thr[i];
         const bool fixed = tp == 0 || tp >= (1ull << 32);
-        if (fixed ? tq != tp : (tq == 0 || tq >= (1ull << 32))) {
-            why = "proposal threshold " + std::to_string(i) +
-                  " must lie in [1, 2^32 - 1] (or equal a constant nominal one)";
-            return false;
-        }
-        beq[i] = make_uint4((uint32_t)g.be_pdag_idx[i] + 1u, g.be_event_idx[i] + 1u, (uint32_t)tq, (uint32_t)(tq >> 32));
-        a[i] = 0.0;
-        if (fixed) continue;
-        const double p = (double)tp / two32, q = (double)tq / two32;
-        const double l1 = std::log1p(-p) - std::log1p(-q);
-        a[i] = std::log(p) - std::log(q) - l1;
-        C += l1;
+        if (fixed ? tq != tp : (tq == 0 || tq >= (1ull << 32))) return i;
     }
-    return true;
+    return g.n_be;
+}
+
+mcg_status check_thresholds(const mcg::Graph &g, const uint64_t *q_thr) {
+    const uint32_t i = bad_threshold(g, q_thr);
+    if (i == g.n_be) return MCG_OK;
+    return mcg::fail(MCG_ERR_INVALID, "proposal threshold " + std::to_string(i) +
+                                          " must lie in [1, 2^32 - 1] (or equal a constant nominal one)");
 }
 
 }  // namespace
 
 struct mcg_is {
     mcg_engine *engine = nullptr;
-    uint4 *d_be_q = nullptr;     // proposal thresholds in the sampler's table layout
+    uint64_t *d_q = nullptr;     // proposal thresholds
+    uint4 *d_be_q = nullptr;     // in the sampler's table layout
     double *d_a = nullptr;       // per-event log-ratio increments
-    double *d_sums = nullptr;    // 4 doubles
-    double *d_ce = nullptr;      // per-event CE numerators
+    double *d_sums = nullptr;    // 4 doubles, and behind them
+    double *d_ce = nullptr;      // the per-event CE numerators: read back in one copy
     double *d_C = nullptr;       // the constant of the log-ratio
     uint32_t *d_tree = nullptr;  // the one tree of k_is_weights: its events [0, n_be), its root row
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -969,8 +1020,9 @@ mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in
     }
     MCG_CUDA(cudaMalloc((void **)&is->d_be_q, std::max<uint32_t>(nb, 1) * sizeof(uint4)));
     MCG_CUDA(cudaMalloc((void **)&is->d_a, std::max<uint32_t>(nb, 1) * sizeof(double)));
-    MCG_CUDA(cudaMalloc((void **)&is->d_ce, std::max<uint32_t>(nb, 1) * sizeof(double)));
-    MCG_CUDA(cudaMalloc((void **)&is->d_sums, 4 * sizeof(double)));
+    MCG_CUDA(cudaMalloc((void **)&is->d_q, std::max<uint32_t>(nb, 1) * sizeof(uint64_t)));
+    MCG_CUDA(cudaMalloc((void **)&is->d_sums, (4ull + nb) * sizeof(double)));
+    is->d_ce = is->d_sums + 4;
     MCG_CUDA(cudaMalloc((void **)&is->d_C, sizeof(double)));
     MCG_CUDA(cudaMalloc((void **)&is->d_tree, 3 * sizeof(uint32_t)));
     const uint32_t tree[3] = {0u, nb, e->graph.tally_nodes[0]};
@@ -989,8 +1041,8 @@ mcg_status mcg_is_destroy(mcg_is *is) {
         cudaStreamSynchronize(is->engine->stream);
     }
     cudaFree(is->d_be_q);
+    cudaFree(is->d_q);
     cudaFree(is->d_a);
-    cudaFree(is->d_ce);
     cudaFree(is->d_sums);
     cudaFree(is->d_C);
     cudaFree(is->d_tree);
@@ -1009,25 +1061,30 @@ mcg_status mcg_is_run(mcg_is *is, const uint64_t *q_thr, uint32_t iteration, uin
     const mcg::Graph &g = e->graph;
     const uint32_t nb = g.n_be;
     if (word_begin + word_count > (1ull << 32)) return mcg::fail(MCG_ERR_INVALID, "word range exceeds the counter");
-    // Log-ratio terms at the quantised probabilities.
-    std::vector<double> a(nb, 0.0);
-    double C = 0.0;
-    std::vector<uint4> beq(nb);
-    std::string why;
-    if (!ratio_terms(g, q_thr, 0, nb, beq.data(), a.data(), C, why)) return mcg::fail(MCG_ERR_INVALID, why);
+    const mcg_status bad = check_thresholds(g, q_thr);
+    if (bad != MCG_OK) return bad;
     MCG_CUDA(cudaSetDevice(e->device));
-    MCG_CUDA(cudaMemcpyAsync(is->d_be_q, beq.data(), nb * sizeof(uint4), cudaMemcpyHostToDevice, e->stream));
-    MCG_CUDA(cudaMemcpyAsync(is->d_a, a.data(), nb * sizeof(double), cudaMemcpyHostToDevice, e->stream));
-    const double init[4] = {0.0, 0.0, 0.0, -std::numeric_limits<double>::infinity()};
-    MCG_CUDA(cudaMemcpyAsync(is->d_sums, init, sizeof(init), cudaMemcpyHostToDevice, e->stream));
-    MCG_CUDA(cudaMemcpyAsync(is->d_C, &C, sizeof(C), cudaMemcpyHostToDevice, e->stream));
-    MCG_CUDA(cudaMemsetAsync(is->d_ce, 0, std::max<uint32_t>(nb, 1) * sizeof(double), e->stream));
+    MCG_CUDA(cudaMemcpyAsync(is->d_q, q_thr, nb * sizeof(uint64_t), cudaMemcpyHostToDevice, e->stream));
     const bool want_ce = ce_num != nullptr;
     e->d_be_sample = is->d_be_q;
     e->table_iteration = 0xFFFFFFFFu;  // the sampler table follows the proposal
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
     IsBatchArgs args{};
+    RatioArgs ra{};
+    ra.be = e->d_be;
+    ra.q = is->d_q;
+    ra.be_begin = is->d_tree;
+    ra.n_be = nb;
+    ra.n_inst = 1;
+    ra.cut_comp = -1;
+    ra.beq = is->d_be_q;
+    ra.a = is->d_a;
+    ra.C = is->d_C;
+    ra.sums = is->d_sums;
+    ra.ce = want_ce ? is->d_ce : nullptr;
+    k_ratio_terms<<<1, kRatioThreads, 0, e->stream>>>(ra);
+    MCG_CUDA(cudaGetLastError());
     args.n_inst = args.n_comp = 1;
     args.n_be = args.n_be_nodes = nb;
     args.be_begin = is->d_tree;
@@ -1054,10 +1111,10 @@ mcg_status mcg_is_run(mcg_is *is, const uint64_t *q_thr, uint32_t iteration, uin
     e->table_iteration = 0xFFFFFFFFu;
     if (st != MCG_OK) return st;
     MCG_CUDA(cudaEventRecord(is->ev1, e->stream));
-    double sums[4];
-    MCG_CUDA(cudaMemcpyAsync(sums, is->d_sums, sizeof(sums), cudaMemcpyDeviceToHost, e->stream));
-    if (want_ce) MCG_CUDA(cudaMemcpyAsync(ce_num, is->d_ce, nb * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
+    std::vector<double> sums(4ull + (want_ce ? nb : 0));
+    MCG_CUDA(cudaMemcpyAsync(sums.data(), is->d_sums, sums.size() * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
     MCG_CUDA(cudaStreamSynchronize(e->stream));
+    if (want_ce) std::copy(sums.begin() + 4, sums.end(), ce_num);
     float ms = 0;
     MCG_CUDA(cudaEventElapsedTime(&ms, is->ev0, is->ev1));
     std::memset(result, 0, sizeof(*result));
@@ -1086,6 +1143,7 @@ struct mcg_is_batch {
     uint32_t n_inst = 0;
     uint32_t n_comp_cap = 0;             // components the device arrays hold
     std::vector<uint32_t> be_begin;
+    uint64_t *d_q = nullptr;             // [n_comp][n_be] proposal thresholds
     uint4 *d_be_q = nullptr;             // [n_comp][n_be] sampler tables
     double *d_a = nullptr;               // [n_comp][n_be]
     double *d_C = nullptr;               // [n_comp][n_inst]
@@ -1094,8 +1152,6 @@ struct mcg_is_batch {
     uint32_t *d_be_begin = nullptr;
     uint32_t *d_root = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    std::vector<uint4> beq;
-    std::vector<double> a, C, init;
     // cut-set component (built on first use)
     bool cut_ready = false;
     uint4 *d_cut_gate = nullptr;
@@ -1111,12 +1167,11 @@ struct mcg_is_batch {
     std::vector<unsigned char> tree_ok;  // per tree: the cut-set component draws it (else its samples stay nominal)
     unsigned char *d_tree_ok = nullptr;
     std::vector<uint32_t> z_event;       // shared events, tree by tree
-    std::vector<uint64_t> z_thr, cut_q;  // per run: their proposal thresholds; the component's table
-    unsigned char *d_shared = nullptr;
+    std::vector<uint64_t> cut_q;         // per run: the component's thresholds
+    unsigned char *d_shared = nullptr, *d_drawn = nullptr;
     uint2 *d_gate_occ = nullptr;
     uint32_t *d_companion = nullptr, *d_z_begin = nullptr, *d_z_event = nullptr;
     uint32_t *d_z_occ_begin = nullptr, *d_z_occ = nullptr;
-    uint64_t *d_z_thr = nullptr;
 };
 
 namespace {
@@ -1128,6 +1183,7 @@ void release_batch(mcg_is_batch *b) {
         cudaSetDevice(b->engine->device);
         cudaStreamSynchronize(b->engine->stream);
     }
+    cudaFree(b->d_q);
     cudaFree(b->d_be_q);
     cudaFree(b->d_a);
     cudaFree(b->d_C);
@@ -1142,7 +1198,7 @@ void release_batch(mcg_is_batch *b) {
     cudaFree(b->d_cut_error);
     for (void *q : {(void *)b->d_tree_ok, (void *)b->d_shared, (void *)b->d_gate_occ, (void *)b->d_companion, (void *)b->d_z_begin,
                     (void *)b->d_z_event, (void *)b->d_z_occ_begin, (void *)b->d_z_occ,
-                    (void *)b->d_z_thr})
+                    (void *)b->d_drawn})
         cudaFree(q);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
@@ -1303,11 +1359,6 @@ mcg_status mcg_is_batch_create(const mcg_graph_desc *graph, uint32_t n_inst, con
     MCG_CUDA(cudaMemcpy(b->d_root, g.tally_nodes.data(), n_inst * sizeof(uint32_t), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaEventCreate(&b->ev0));
     MCG_CUDA(cudaEventCreate(&b->ev1));
-    b->init.resize(4ull * n_inst);
-    for (uint32_t k = 0; k < n_inst; ++k) {
-        b->init[4ull * k] = b->init[4ull * k + 1] = b->init[4ull * k + 2] = 0.0;
-        b->init[4ull * k + 3] = -std::numeric_limits<double>::infinity();
-    }
     *out = b.release();
     return MCG_OK;
 }
@@ -1497,7 +1548,10 @@ mcg_status build_cut_tables(mcg_is_batch *b) {
     MCG_CUDA(cudaMalloc((void **)&b->d_z_event, nz * sizeof(uint32_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_z_occ_begin, z_occ_begin.size() * sizeof(uint32_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_z_occ, z_occ.size() * sizeof(uint32_t)));
-    MCG_CUDA(cudaMalloc((void **)&b->d_z_thr, nz * sizeof(uint64_t)));
+    std::vector<unsigned char> drawn(std::max<uint32_t>(nb, 1), 0);
+    for (uint32_t i : b->z_event) drawn[i] = 1;
+    MCG_CUDA(cudaMalloc((void **)&b->d_drawn, drawn.size()));
+    MCG_CUDA(cudaMemcpy(b->d_drawn, drawn.data(), drawn.size(), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_cut_gate, gate.data(), gate.size() * sizeof(uint4), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_cut_S, S.data(), nn * sizeof(double), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemcpy(b->d_cut_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -1520,12 +1574,15 @@ mcg_status build_cut_tables(mcg_is_batch *b) {
 mcg_status ensure_components(mcg_is_batch *b, uint32_t n_comp) {
     if (n_comp <= b->n_comp_cap) return MCG_OK;
     const uint64_t nb = std::max<uint32_t>(b->engine->graph.n_be, 1);
+    cudaFree(b->d_q);
     cudaFree(b->d_be_q);
     cudaFree(b->d_a);
     cudaFree(b->d_C);
+    b->d_q = nullptr;
     b->d_be_q = nullptr;
     b->d_a = b->d_C = nullptr;
     b->n_comp_cap = 0;
+    MCG_CUDA(cudaMalloc((void **)&b->d_q, n_comp * nb * sizeof(uint64_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_be_q, n_comp * nb * sizeof(uint4)));
     MCG_CUDA(cudaMalloc((void **)&b->d_a, n_comp * nb * sizeof(double)));
     MCG_CUDA(cudaMalloc((void **)&b->d_C, (uint64_t)n_comp * b->n_inst * sizeof(double)));
@@ -1581,12 +1638,9 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
             if (cs != MCG_OK) return cs;
         }
         b->cut_q.assign(g.be_threshold.begin(), g.be_threshold.end());
-        b->z_thr.resize(b->z_event.size());
-        for (size_t j = 0; j < b->z_event.size(); ++j) {
-            const uint32_t i = b->z_event[j];
+        for (uint32_t i : b->z_event) {
             const uint64_t tp = g.be_threshold[i];
             if (q_cutset && tp != 0 && tp < (1ull << 32)) b->cut_q[i] = q_cutset[i];
-            b->z_thr[j] = b->cut_q[i];
         }
         cut_comp = (int)comp_q.size();
         comp_q.push_back(b->cut_q.data());
@@ -1597,47 +1651,27 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
     MCG_CUDA(cudaSetDevice(e->device));
     mcg_status st = ensure_components(b, nc);
     if (st != MCG_OK) return st;
-    b->beq.resize(nc * std::max<uint64_t>(nb, 1));
-    b->a.resize(nc * std::max<uint64_t>(nb, 1));
-    b->C.resize((uint64_t)nc * n_inst);
-    // log-ratio terms of every (component, tree), split over the host threads
-    const uint64_t jobs = (uint64_t)nc * n_inst;
-    const unsigned n_thr = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(
-        std::max(1u, std::thread::hardware_concurrency()), std::min<uint64_t>(jobs, nb / 65536 + 1)));
-    std::vector<std::string> why(n_thr);
-    std::vector<char> bad(n_thr, 0);
-    auto work = [&](unsigned t) {
-        for (uint64_t j = t; j < jobs; j += n_thr) {
-            const uint32_t c = (uint32_t)(j / n_inst), k = (uint32_t)(j % n_inst);
-            if (!ratio_terms(g, comp_q[c], b->be_begin[k], b->be_begin[k + 1], b->beq.data() + c * nb,
-                             b->a.data() + c * nb, b->C[(uint64_t)c * n_inst + k], why[t])) {
-                bad[t] = 1;
-                return;
-            }
-        }
-    };
-    std::vector<std::thread> pool;
-    for (unsigned t = 1; t < n_thr; ++t) pool.emplace_back(work, t);
-    work(0);
-    for (auto &th : pool) th.join();
-    for (unsigned t = 0; t < n_thr; ++t)
-        if (bad[t]) return mcg::fail(MCG_ERR_INVALID, why[t]);
-    if (cut_comp >= 0) {  // the forcing kernel draws the shared events itself: the sampler leaves them 0
-        uint4 *cq = b->beq.data() + (uint64_t)cut_comp * nb;
-        for (uint32_t i : b->z_event) cq[i].z = cq[i].w = 0u;
-        if (!b->z_thr.empty())
-            MCG_CUDA(cudaMemcpyAsync(b->d_z_thr, b->z_thr.data(), b->z_thr.size() * sizeof(uint64_t),
-                                     cudaMemcpyHostToDevice, e->stream));
+    for (uint32_t c = 0; c < nc; ++c) {
+        st = check_thresholds(g, comp_q[c]);
+        if (st != MCG_OK) return st;
     }
-    if (nb) {
-        MCG_CUDA(cudaMemcpyAsync(b->d_be_q, b->beq.data(), nc * nb * sizeof(uint4), cudaMemcpyHostToDevice, e->stream));
-        MCG_CUDA(cudaMemcpyAsync(b->d_a, b->a.data(), nc * nb * sizeof(double), cudaMemcpyHostToDevice, e->stream));
-        MCG_CUDA(cudaMemsetAsync(b->d_ce, 0, nb * sizeof(double), e->stream));
-    }
-    MCG_CUDA(cudaMemcpyAsync(b->d_C, b->C.data(), (uint64_t)nc * n_inst * sizeof(double), cudaMemcpyHostToDevice,
-                             e->stream));
-    MCG_CUDA(cudaMemcpyAsync(b->d_sums, b->init.data(), 4ull * n_inst * sizeof(double), cudaMemcpyHostToDevice,
-                             e->stream));
+    for (uint32_t c = 0; c < nc && nb; ++c)
+        MCG_CUDA(cudaMemcpyAsync(b->d_q + c * nb, comp_q[c], nb * sizeof(uint64_t), cudaMemcpyHostToDevice, e->stream));
+    RatioArgs ra{};
+    ra.be = e->d_be;
+    ra.q = b->d_q;
+    ra.be_begin = b->d_be_begin;
+    ra.n_be = (uint32_t)nb;
+    ra.n_inst = n_inst;
+    ra.cut_comp = cut_comp;
+    ra.drawn = b->d_drawn;
+    ra.beq = b->d_be_q;
+    ra.a = b->d_a;
+    ra.C = b->d_C;
+    ra.sums = b->d_sums;
+    ra.ce = ce_num ? b->d_ce : nullptr;
+    k_ratio_terms<<<dim3(n_inst, nc), kRatioThreads, 0, e->stream>>>(ra);
+    MCG_CUDA(cudaGetLastError());
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device);
     IsBatchArgs args{};
@@ -1695,7 +1729,7 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
             ca.gate_occ = b->d_gate_occ;
             ca.z_begin = b->d_z_begin;
             ca.z_event = b->d_z_event;
-            ca.z_thr = b->d_z_thr;
+            ca.q = b->d_q + (uint64_t)cut_comp * nb;
             ca.z_occ_begin = b->d_z_occ_begin;
             ca.z_occ = b->d_z_occ;
             ca.seed = mix64_host(((uint64_t)iteration << 32) ^ 0x5bd1e995u);
