@@ -55,7 +55,10 @@ enum mcg_mode {
                              threads sample every event of their word and then evaluate every gate
                              for it from scratch rows of their own (n_nodes x 32 words per warp);
                              sampling and gate work of different blocks overlap on every SM */
-    MCG_MODE_FUSED = 4    /* one persistent kernel per launch chunk: sample, gates, tallies fused */
+    MCG_MODE_FUSED = 4    /* one persistent kernel per launch chunk: sample, gates, tallies fused; in its
+                             default shape a tree whose node words fit in shared memory (about 880
+                             nodes) is evaluated in tiles of 32 words per block, others (and other
+                             shapes) by an interpreter of the compiled program */
 };
 
 /* Flattened PDAG handed to the engine.  All arrays are host memory, copied

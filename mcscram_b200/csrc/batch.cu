@@ -17,7 +17,6 @@
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMulForm = 1;
 constexpr int kPackForm = 1;
 // Instances of one tree that differ only in thresholds (uncertainty draws)
 // share their Philox calls kShare at a time (k_fused_batch_k) unless a tree
@@ -40,22 +39,22 @@ using BatchKernel = void (*)(mcg::dev::BatchArgs);
 BatchKernel batch_kernel(uint32_t ctas_per_sm, uint32_t share, bool atleast) {
     if (share == kShare && atleast) {
         switch (ctas_per_sm) {
-            case 2: return mcg::dev::k_fused_batch_k<kThreads, 2, kMulForm, kPackForm, kShare, true>;
-            case 3: return mcg::dev::k_fused_batch_k<kThreads, 3, kMulForm, kPackForm, kShare, true>;
-            default: return mcg::dev::k_fused_batch_k<kThreads, 4, kMulForm, kPackForm, kShare, true>;
+            case 2: return mcg::dev::k_fused_batch_k<kThreads, 2, kPackForm, kShare, true>;
+            case 3: return mcg::dev::k_fused_batch_k<kThreads, 3, kPackForm, kShare, true>;
+            default: return mcg::dev::k_fused_batch_k<kThreads, 4, kPackForm, kShare, true>;
         }
     }
     if (share == kShare) {
         switch (ctas_per_sm) {
-            case 2: return mcg::dev::k_fused_batch_k<kThreads, 2, kMulForm, kPackForm, kShare, false>;
-            case 3: return mcg::dev::k_fused_batch_k<kThreads, 3, kMulForm, kPackForm, kShare, false>;
-            default: return mcg::dev::k_fused_batch_k<kThreads, 4, kMulForm, kPackForm, kShare, false>;
+            case 2: return mcg::dev::k_fused_batch_k<kThreads, 2, kPackForm, kShare, false>;
+            case 3: return mcg::dev::k_fused_batch_k<kThreads, 3, kPackForm, kShare, false>;
+            default: return mcg::dev::k_fused_batch_k<kThreads, 4, kPackForm, kShare, false>;
         }
     }
     switch (ctas_per_sm) {
-        case 2: return mcg::dev::k_fused_batch<kThreads, 2, kMulForm, kPackForm>;
-        case 3: return mcg::dev::k_fused_batch<kThreads, 3, kMulForm, kPackForm>;
-        default: return mcg::dev::k_fused_batch<kThreads, 4, kMulForm, kPackForm>;
+        case 2: return mcg::dev::k_fused_batch<kThreads, 2, kPackForm>;
+        case 3: return mcg::dev::k_fused_batch<kThreads, 3, kPackForm>;
+        default: return mcg::dev::k_fused_batch<kThreads, 4, kPackForm>;
     }
 }
 

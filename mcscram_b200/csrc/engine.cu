@@ -27,9 +27,7 @@
 
 namespace {
 
-// Sampler code form: separate high/low multiplies and the carry-chain bit
-// packing measured fastest of the four forms on B200 (register-only sampler).
-constexpr int kMulForm = 1;
+// Bit packing of the sampler: the carry chain measured faster than compares on B200 (register-only sampler).
 constexpr int kPackForm = 1;
 using mcg::internal::kDefaultChunkWords;
 using mcg::internal::kFusedThreads;
@@ -327,7 +325,7 @@ mcg_status layered_eval(mcg_engine *e, uint32_t iteration, uint64_t word_begin, 
     }
     const uint32_t t3 = (iteration + 1u) << 6;
     if (g.n_be > 0) {
-        mcg::dev::k_layer_be<kMulForm, kPackForm><<<rows_grid(W, g.n_be, 256), 256, 0, e->stream>>>(
+        mcg::dev::k_layer_be<kPackForm><<<rows_grid(W, g.n_be, 256), 256, 0, e->stream>>>(
             e->d_be, g.n_be, W, word_begin, t3, e->d_buf);
         ++e->launches;
     }
@@ -347,10 +345,10 @@ using FusedKernel = void (*)(mcg::dev::FusedArgs);
 // Register budget follows the CTAs wanted per SM (65536 / (256 * n) per thread).
 FusedKernel fused_kernel(uint32_t ctas_per_sm) {
     switch (ctas_per_sm) {
-        case 1: return mcg::dev::k_fused<kFusedThreads, 1, kMulForm, kPackForm>;
-        case 3: return mcg::dev::k_fused<kFusedThreads, 3, kMulForm, kPackForm>;
-        case 4: return mcg::dev::k_fused<kFusedThreads, 4, kMulForm, kPackForm>;
-        default: return mcg::dev::k_fused<kFusedThreads, 2, kMulForm, kPackForm>;
+        case 1: return mcg::dev::k_fused<kFusedThreads, 1, kPackForm>;
+        case 3: return mcg::dev::k_fused<kFusedThreads, 3, kPackForm>;
+        case 4: return mcg::dev::k_fused<kFusedThreads, 4, kPackForm>;
+        default: return mcg::dev::k_fused<kFusedThreads, 2, kPackForm>;
     }
 }
 
@@ -385,7 +383,182 @@ mcg_status compile_fused(mcg_engine *e, const mcg_run_desc &run) {
     return MCG_OK;
 }
 
+using TileKernel = void (*)(const mcg::dev::TileArgs);
+TileKernel tile_kernel(uint32_t threads) {
+    switch (threads) {
+        case 256: return mcg::dev::k_tile<256, kPackForm>;
+        case 512: return mcg::dev::k_tile<512, kPackForm>;
+        default: return mcg::dev::k_tile<1024, kPackForm>;
+    }
+}
+
+// The nodes some tally depends on, as slots of the tile kernel: events in
+// their order, then gates layer by layer.  NOT and NULL gates read their last
+// input only.
+struct TilePlan {
+    std::vector<uint32_t> event;                 // slot -> event
+    std::vector<uint4> gates;
+    std::vector<uint32_t> in, layer{0}, tally_list;
+    std::vector<uint2> be_tally;
+    uint32_t slots() const { return (uint32_t)(event.size() + gates.size()) + 1u; }  // and the empty input
+    bool fits = true;  // the records' fields
+};
+
+TilePlan plan_tile(const mcg::Graph &g) {
+    TilePlan t;
+    const uint32_t nb = g.n_be;
+    auto first_input = [&](uint32_t i) {
+        const bool last_only = (g.gate_op[i] == MCG_NOT || g.gate_op[i] == MCG_NULL) && g.gate_in_count[i] > 0;
+        return last_only ? g.gate_in_count[i] - 1 : 0u;
+    };
+    std::vector<uint32_t> slot(g.n_nodes(), 0), depth(g.n_gates, 0);
+    std::vector<char> needed(g.n_nodes(), 0);
+    for (uint32_t v : g.tally_nodes) needed[v] = 1;
+    for (uint32_t i = g.n_gates; i-- > 0;) {
+        if (!needed[nb + i]) continue;
+        for (uint32_t j = first_input(i); j < g.gate_in_count[i]; ++j) needed[g.inputs[g.gate_in_begin[i] + j]] = 1;
+    }
+    std::vector<std::vector<uint32_t>> layers, tallies(g.n_nodes());
+    for (uint32_t i = 0; i < g.n_gates; ++i) {
+        if (!needed[nb + i]) continue;
+        for (uint32_t j = first_input(i); j < g.gate_in_count[i]; ++j) {
+            const uint32_t c = g.inputs[g.gate_in_begin[i] + j];
+            if (c >= nb) depth[i] = std::max(depth[i], depth[c - nb] + 1);
+        }
+        if (layers.size() <= depth[i]) layers.resize(depth[i] + 1);
+        layers[depth[i]].push_back(i);
+    }
+    for (uint32_t k = 0; k < (uint32_t)g.tally_nodes.size(); ++k) tallies[g.tally_nodes[k]].push_back(k);
+    for (uint32_t e = 0; e < nb; ++e) {
+        if (!needed[e]) continue;
+        slot[e] = (uint32_t)t.event.size();
+        t.event.push_back(e);
+        for (uint32_t k : tallies[e]) t.be_tally.push_back(make_uint2(slot[e], k));
+    }
+    constexpr uint32_t kSlotBytes = mcg::dev::kTileLanes * sizeof(uint64_t);
+    uint32_t next = (uint32_t)t.event.size(), n_gates = 0;
+    for (const auto &layer : layers) n_gates += (uint32_t)layer.size();
+    const uint32_t empty = (next + n_gates) * kSlotBytes;
+    for (const auto &layer : layers) {
+        for (uint32_t i : layer) slot[nb + i] = next++;
+        for (uint32_t i : layer) {
+            const uint8_t op = g.gate_op[i];
+            const uint32_t n = g.gate_in_count[i], from = first_input(i);
+            const bool and_type = op == MCG_AND || op == MCG_NAND;  // AND = ~OR(~x), NAND = OR(~x)
+            const bool inverted = op == MCG_AND || op == MCG_NOR || op == MCG_NOT;
+            const uint32_t kind = op == MCG_ATLEAST ? mcg::dev::kTileAtleast
+                                  : op == MCG_XOR   ? mcg::dev::kTileXor
+                                                    : mcg::dev::kTileOr;
+            uint32_t nbits = 0;
+            while (nbits < 8 && (n >> nbits) != 0) ++nbits;
+            const std::vector<uint32_t> &mine = tallies[nb + i];
+            if (mine.size() > 0xFFFu) t.fits = false;
+            t.gates.push_back(make_uint4(kind | (inverted ? 4u : 0u) | ((g.gate_k[i] & 0xFFu) << 8) |
+                                             (std::max(nbits, 1u) << 16) | ((uint32_t)mine.size() << 20),
+                                         (uint32_t)t.in.size(), (n - from + 1) / 2,
+                                         mine.size() == 1 ? mine[0] : (uint32_t)t.tally_list.size()));
+            if (mine.size() > 1) t.tally_list.insert(t.tally_list.end(), mine.begin(), mine.end());
+            for (uint32_t j = from; j < n; ++j) {
+                const bool negated = j >= n - g.gate_neg_count[i];
+                t.in.push_back(slot[g.inputs[g.gate_in_begin[i] + j]] * kSlotBytes | (uint32_t)(negated != and_type));
+            }
+            if ((n - from) % 2) t.in.push_back(empty);
+        }
+        t.layer.push_back((uint32_t)t.gates.size());
+    }
+    return t;
+}
+
+template <typename T>
+mcg_status upload_tile(mcg_engine *e, const T **dptr, const std::vector<T> &v) {
+    T *p = nullptr;
+    MCG_CUDA(upload(&p, v));
+    if (p) e->tile_tables.push_back(p);
+    *dptr = p;
+    return MCG_OK;
+}
+
+// Fused mode's default shape where every needed node has room for 32 words in
+// shared memory (about 880 nodes on a B200): e->tile, or not.
+mcg_status setup_tile(mcg_engine *e) {
+    const mcg::Graph &g = e->graph;
+    int optin = 0, per_sm = 0, reserved = 0, sms = 0;
+    MCG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
+    MCG_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, e->device));
+    MCG_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, e->device));
+    MCG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
+    const TilePlan t = plan_tile(g);
+    const uint64_t words = (uint64_t)t.slots() * mcg::dev::kTileLanes * sizeof(uint64_t);
+    if (!t.fits) return MCG_OK;
+    // the most, and so the smallest, blocks that share an SM's 1,024 threads
+    // and its shared memory; the tally counters go to shared memory where
+    // they fit as well
+    uint32_t threads = 0;
+    uint64_t room = 0;
+    for (uint32_t nt : {256u, 512u, 1024u}) {
+        const uint64_t own = (nt / 32u) * (mcg::dev::kEventTableStride + 1) * sizeof(uint2);
+        const uint64_t most = std::min<uint64_t>(optin, per_sm / (1024u / nt) - reserved);
+        if (words + own > most) continue;
+        threads = nt;
+        room = most - own;
+        break;
+    }
+    if (!threads) return MCG_OK;
+    const uint64_t counters = g.tally_nodes.size() * sizeof(unsigned long long);
+    mcg::dev::TileArgs &a = e->tile_args;
+    a = mcg::dev::TileArgs{};
+    a.tally_in_smem = words + counters <= room ? 1u : 0u;
+    e->tile_smem = (uint32_t)(words + (a.tally_in_smem ? counters : 0));
+    mcg_status st = mcg::set_smem_limit(tile_kernel(threads), e->tile_smem);
+    if (st != MCG_OK) return st;
+    std::vector<uint4> be(t.event.size());
+    for (size_t i = 0; i < be.size(); ++i) {
+        const uint32_t v = t.event[i];
+        be[i] = make_uint4((uint32_t)g.be_pdag_idx[v] + 1u, g.be_event_idx[v] + 1u, (uint32_t)g.be_threshold[v],
+                           (uint32_t)(g.be_threshold[v] >> 32));
+    }
+    if ((st = upload_tile(e, &a.be, be)) != MCG_OK || (st = upload_tile(e, &a.gates, t.gates)) != MCG_OK ||
+        (st = upload_tile(e, &a.in, t.in)) != MCG_OK || (st = upload_tile(e, &a.layer, t.layer)) != MCG_OK ||
+        (st = upload_tile(e, &a.tally_list, t.tally_list)) != MCG_OK ||
+        (st = upload_tile(e, &a.be_tally, t.be_tally)) != MCG_OK)
+        return st;
+    a.n_be = (uint32_t)t.event.size();
+    a.n_slots = t.slots();
+    a.n_layers = (uint32_t)t.layer.size() - 1;
+    a.n_be_tally = (uint32_t)t.be_tally.size();
+    a.n_tally = (uint32_t)g.tally_nodes.size();
+    e->tile_threads = threads;
+    e->tile_grid = (uint32_t)sms * (1024u / threads);
+    e->tile = true;
+    return MCG_OK;
+}
+
+mcg_status launch_tile(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {
+    mcg::dev::TileArgs a = e->tile_args;
+    a.iteration_first = it_first;
+    a.n_iterations = n_it;
+    a.word_begin = word_begin;
+    a.word_count = count;
+    a.ones = e->d_tally;
+    const uint64_t tiles = (count + mcg::dev::kTileLanes - 1) / mcg::dev::kTileLanes;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(e->tile_grid, std::max<uint64_t>(tiles, 1));
+    tile_kernel(e->tile_threads)<<<grid, e->tile_threads, e->tile_smem, e->stream>>>(a);
+    ++e->launches;
+    MCG_CUDA(cudaGetLastError());
+    return MCG_OK;
+}
+
 mcg_status setup_fused(mcg_engine *e, const mcg_run_desc &run) {
+    // the default shape (no slot count, block size or residency of its own)
+    if (!run.smem_slots && !run.block_threads && (!run.ctas_per_sm || run.ctas_per_sm == 4)) {
+        const mcg_status ts = setup_tile(e);
+        if (ts != MCG_OK) return ts;
+        if (e->tile) {
+            e->ctas_per_sm = 4;
+            e->chunk_words = run.chunk_words ? run.chunk_words : kDefaultChunkWords;
+            return MCG_OK;
+        }
+    }
     mcg_status st = compile_fused(e, run);
     if (st != MCG_OK) return st;
     st = mcg::set_smem_limit(fused_kernel(e->ctas_per_sm), e->smem_bytes);
@@ -426,7 +599,7 @@ mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
     const uint32_t blocks = run.sampler_blocks_per_sm ? run.sampler_blocks_per_sm : 8u;
     if (blocks < 1 || blocks > 8) return mcg::fail(MCG_ERR_INVALID, "sampler_blocks_per_sm must be 1..8");
     e->sampler_smem = blocks >= 8 ? 0u : (uint32_t)(prop.sharedMemPerMultiprocessor / blocks - 2048);
-    const mcg_status lim = mcg::set_smem_limit(mcg::dev::k_stage_be<kMulForm, kPackForm, kStageEventsPerThread>,
+    const mcg_status lim = mcg::set_smem_limit(mcg::dev::k_stage_be<kPackForm, kStageEventsPerThread>,
                                                e->sampler_smem);
     if (lim != MCG_OK) return lim;
     // The gate phase of chunk k runs while chunk k+1 is sampled: giving its
@@ -447,9 +620,9 @@ mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
 using StripKernel = void (*)(mcg::dev::StripArgs);
 StripKernel strip_kernel(uint32_t blocks_per_sm) {
     switch (blocks_per_sm) {
-        case 4: return mcg::dev::k_strip<kMulForm, kPackForm, 4>;
-        case 5: return mcg::dev::k_strip<kMulForm, kPackForm, 5>;
-        default: return mcg::dev::k_strip<kMulForm, kPackForm, 6>;
+        case 4: return mcg::dev::k_strip<kPackForm, 4>;
+        case 5: return mcg::dev::k_strip<kPackForm, 5>;
+        default: return mcg::dev::k_strip<kPackForm, 6>;
     }
 }
 
@@ -510,7 +683,7 @@ mcg_status run_strip(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t w
         const uint32_t iteration = it_first + it;
         if (g.n_be > 0 && e->table_iteration != iteration) {
             const uint64_t n = (uint64_t)g.n_be * mcg::dev::kEventTableStride;
-            mcg::dev::k_event_table<kMulForm><<<(uint32_t)((n + 255) / 256), 256, 0, e->stream>>>(
+            mcg::dev::k_event_table<<<(uint32_t)((n + 255) / 256), 256, 0, e->stream>>>(
                 e->d_be, g.n_be, (iteration + 1u) << 6, e->d_event_table);
             ++e->launches;
             e->table_iteration = iteration;
@@ -550,7 +723,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
     if (g.n_be > 0 && e->table_iteration != iteration) {
         // s_a is in order: earlier sampler launches finish before the table changes
         const uint64_t n = (uint64_t)g.n_be * mcg::dev::kEventTableStride;
-        mcg::dev::k_event_table<kMulForm><<<(uint32_t)((n + 255) / 256), 256, 0, e->s_a>>>(be_tab, g.n_be, t3,
+        mcg::dev::k_event_table<<<(uint32_t)((n + 255) / 256), 256, 0, e->s_a>>>(be_tab, g.n_be, t3,
                                                                                            e->d_event_table);
         ++e->launches;
         e->table_iteration = iteration;
@@ -570,7 +743,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
             ++e->prof_used;
             MCG_CUDA(cudaEventRecord(p0, e->s_a));
         }
-        mcg::dev::k_stage_be<kMulForm, kPackForm, kStageEventsPerThread>
+        mcg::dev::k_stage_be<kPackForm, kStageEventsPerThread>
             <<<rows_grid(W, groups, 256), 256, e->sampler_smem, e->s_a>>>(be_tab, e->d_event_table, g.n_be, W,
                                                                           word_begin, buf);
         ++e->launches;
@@ -660,6 +833,7 @@ void release(mcg_engine *e) {
     work_free(e, e->d_stage[0]);
     work_free(e, e->d_stage[1]);
     work_free(e, e->d_strip_scratch);
+    for (void *p : e->tile_tables) cudaFree(p);
     cudaFree(e->d_ops);
     cudaFree(e->d_tally);
     cudaFree(e->d_be);
@@ -829,7 +1003,8 @@ mcg_status mcg_run(mcg_engine *e, uint32_t iteration_first, uint32_t n_iteration
     } else if (e->mode == MCG_MODE_FUSED) {
         for (uint64_t off = 0; off < word_count; off += e->chunk_words) {
             const uint64_t n = std::min<uint64_t>(e->chunk_words, word_count - off);
-            const mcg_status st = launch_fused(e, iteration_first, n_iterations, word_begin + off, n);
+            const mcg_status st = (e->tile ? launch_tile : launch_fused)(e, iteration_first, n_iterations,
+                                                                         word_begin + off, n);
             if (st != MCG_OK) return st;
         }
     } else {
@@ -1023,13 +1198,13 @@ mcg_status mcg_sampler_peak(int32_t device, uint64_t n_events, uint64_t n_words,
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     const uint64_t nt = n_events * mcg::dev::kEventTableStride;
-    mcg::dev::k_peak_table<kMulForm><<<(uint32_t)((nt + 255) / 256), 256>>>((uint32_t)n_events, 2u << 6, table);
+    mcg::dev::k_peak_table<<<(uint32_t)((nt + 255) / 256), 256>>>((uint32_t)n_events, 2u << 6, table);
     const uint32_t blocks = (uint32_t)((n_words + 255) / 256);
     // warm-up
-    mcg::dev::k_sampler_peak<kMulForm, kPackForm><<<blocks, 256>>>((uint32_t)n_events, n_words, table, sink);
+    mcg::dev::k_sampler_peak<kPackForm><<<blocks, 256>>>((uint32_t)n_events, n_words, table, sink);
     cudaEventRecord(a);
     for (uint32_t r = 0; r < repeats; ++r)
-        mcg::dev::k_sampler_peak<kMulForm, kPackForm><<<blocks, 256>>>((uint32_t)n_events, n_words, table, sink);
+        mcg::dev::k_sampler_peak<kPackForm><<<blocks, 256>>>((uint32_t)n_events, n_words, table, sink);
     cudaEventRecord(b);
     cudaError_t err = cudaEventSynchronize(b);
     float ms = 0;
@@ -1055,9 +1230,9 @@ mcg_status mcg_sampler_peak_shared(int32_t device, uint64_t n_events, uint64_t n
     auto launch = [&] {
         const uint32_t blocks = (uint32_t)((n_words + 255) / 256);
         if (instances == 4)
-            mcg::dev::k_sampler_peak_shared<kMulForm, kPackForm, 4><<<blocks, 256>>>((uint32_t)n_events, n_words, sink);
+            mcg::dev::k_sampler_peak_shared<kPackForm, 4><<<blocks, 256>>>((uint32_t)n_events, n_words, sink);
         else
-            mcg::dev::k_sampler_peak_shared<kMulForm, kPackForm, 1><<<blocks, 256>>>((uint32_t)n_events, n_words, sink);
+            mcg::dev::k_sampler_peak_shared<kPackForm, 1><<<blocks, 256>>>((uint32_t)n_events, n_words, sink);
     };
     cudaEvent_t a, b;
     cudaEventCreate(&a);
@@ -1101,6 +1276,6 @@ mcg_status mcg_profile_sampler_read(mcg_engine *e, uint64_t *launches, double *t
     return MCG_OK;
 }
 
-const char *mcg_version(void) { return "mcg 0.1 (sm_100a)"; }
+const char *mcg_version(void) { return "mcg 0.2 (sm_100a)"; }
 
 }  // extern "C"

@@ -10,6 +10,7 @@
 #include "graph.hpp"
 #include "mcg.h"
 #include "program.hpp"
+#include "tile.hpp"
 
 namespace mcg {
 namespace internal {
@@ -37,6 +38,12 @@ struct mcg_engine {
     uint32_t smem_bytes = 0;
     bool tally_in_smem = false;
     uint64_t chunk_words = mcg::internal::kDefaultChunkWords;
+
+    // tile kernel (fused mode, small trees): its tables and launch shape
+    bool tile = false;
+    mcg::dev::TileArgs tile_args{};        // device pointers and sizes; the pass is filled in per launch
+    std::vector<void *> tile_tables;
+    uint32_t tile_threads = 0, tile_smem = 0, tile_grid = 0;
 
     // tallies
     unsigned long long *d_tally = nullptr;

@@ -1,5 +1,8 @@
 // kernels.cuh -- sm_100a kernels of the Monte Carlo engine.
 //
+//  k_tile        fused mode, trees that fit in shared memory: a block evaluates
+//                32 words of every node at a time, its warps share out events
+//                and gates; one launch per pass.
 //  k_fused       persistent interpreter: each thread owns one sample word per
 //                slab and walks the compiled node program (program_format.h):
 //                Philox sampling in registers, gates in an accumulator,
@@ -17,6 +20,7 @@
 #include "mcg.h"
 #include "philox.cuh"
 #include "program_format.h"
+#include "tile.hpp"
 
 namespace mcg {
 namespace dev {
@@ -102,7 +106,7 @@ __device__ __forceinline__ void store_slot(uint32_t ref, uint64_t v, uint64_t *m
 // basic-event ops carry an index into thr (a per-instance uint64 threshold
 // table) instead of the threshold itself.  tally(index, count) is called by
 // lane 0 of each warp with the warp's popcount sum for a TALLY op.
-template <int NT, int MF, int PF, bool THR_TABLE, class Tally>
+template <int NT, int PF, bool THR_TABLE, class Tally>
 __device__ __forceinline__ void interpret(const uint4 *__restrict__ ops, const WordCtx &ctx, uint32_t t3, bool valid,
                                           uint64_t *my_slots, uint64_t *my_scratch, uint64_t stride,
                                           const uint64_t *__restrict__ thr, Tally &&tally) {
@@ -125,9 +129,9 @@ __device__ __forceinline__ void interpret(const uint4 *__restrict__ ops, const W
                 const uint64_t t = thr[op.z];
                 if (t >= (1ull << 32)) v = kAllOnes;
                 else if (t == 0) v = 0;
-                else v = be_word<MF, PF>(op.y, op.w, ctx, t3, (uint32_t)t);
+                else v = be_word<PF>(op.y, op.w, ctx, t3, (uint32_t)t);
             } else {
-                v = be_word<MF, PF>(op.y, op.w, ctx, t3, op.z);
+                v = be_word<PF>(op.y, op.w, ctx, t3, op.z);
             }
         } else if (code == kOpInSlot) {
             v = load_slot(op.y, my_slots, my_scratch, NT, stride);
@@ -181,7 +185,7 @@ struct FusedArgs {
     uint64_t word_count;
 };
 
-template <int NT, int MINB, int MF, int PF>
+template <int NT, int MINB, int PF>
 __global__ void __launch_bounds__(NT, MINB) k_fused(FusedArgs a) {
     extern __shared__ __align__(16) uint64_t smem[];
     const uint32_t tid = threadIdx.x;
@@ -201,8 +205,8 @@ __global__ void __launch_bounds__(NT, MINB) k_fused(FusedArgs a) {
         const uint32_t t3 = (a.iteration_first + it + 1u) << 6;
         for (uint64_t base = 0; base < a.word_count; base += total_threads) {
             const uint64_t j = base + gtid;
-            const WordCtx ctx = make_word_ctx<MF>((uint32_t)(a.word_begin + j));
-            interpret<NT, MF, PF, false>(a.ops, ctx, t3, j < a.word_count, my_slots, my_scratch, a.scratch_stride,
+            const WordCtx ctx = make_word_ctx((uint32_t)(a.word_begin + j));
+            interpret<NT, PF, false>(a.ops, ctx, t3, j < a.word_count, my_slots, my_scratch, a.scratch_stride,
                                          nullptr, add);
         }
     }
@@ -240,7 +244,7 @@ struct BatchArgs {
     uint32_t n_groups;
 };
 
-template <int NT, int MINB, int MF, int PF>
+template <int NT, int MINB, int PF>
 __global__ void __launch_bounds__(NT, MINB) k_fused_batch(BatchArgs a) {
     extern __shared__ __align__(16) uint64_t smem[];
     __shared__ unsigned int s_item;
@@ -258,10 +262,10 @@ __global__ void __launch_bounds__(NT, MINB) k_fused_batch(BatchArgs a) {
         if (item >= n_items) break;
         const uint32_t inst = item / a.slabs_per_instance;
         const uint64_t j = (uint64_t)(item % a.slabs_per_instance) * NT + tid;
-        const WordCtx ctx = make_word_ctx<MF>((uint32_t)j);
+        const WordCtx ctx = make_word_ctx((uint32_t)j);
         unsigned long long *ones = a.inst_ones + inst;
         auto add = [ones](uint32_t, uint32_t c) { atomicAdd(ones, (unsigned long long)c); };
-        interpret<NT, MF, PF, true>(a.ops + a.tree_op_offset[a.inst_tree[inst]], ctx, t3, j < a.words_per_instance,
+        interpret<NT, PF, true>(a.ops + a.tree_op_offset[a.inst_tree[inst]], ctx, t3, j < a.words_per_instance,
                                     my_slots, my_scratch, a.scratch_stride, a.thr + a.inst_thr_offset[inst], add);
     }
 }
@@ -290,7 +294,7 @@ __device__ __forceinline__ void store_slot_k(uint32_t ref, int k, uint64_t v, ui
 // bit slices per instance; without it the program must have no ATLEAST gate
 // (the batch runs wider ones one instance at a time).  tally(k, count) is
 // called by lane 0 with instance k's warp popcount sum.
-template <int NT, int MF, int PF, int K, bool ATL, class Tally>
+template <int NT, int PF, int K, bool ATL, class Tally>
 __device__ __forceinline__ void interpret_k(const uint4 *__restrict__ ops, const WordCtx &ctx, uint32_t t3,
                                             bool valid, uint64_t *my_slots, uint64_t *my_scratch, uint64_t stride,
                                             const uint64_t *const *thr, Tally &&tally) {
@@ -324,7 +328,7 @@ __device__ __forceinline__ void interpret_k(const uint4 *__restrict__ ops, const
                     t32[k] = 1u;
                 }
             }
-            if ((ones | zeros) != (1u << K) - 1u) be_words<MF, PF, K>(op.y, op.w, ctx, t3, t32, v);
+            if ((ones | zeros) != (1u << K) - 1u) be_words<PF, K>(op.y, op.w, ctx, t3, t32, v);
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 if ((ones >> k) & 1u) v[k] = kAllOnes;
@@ -407,7 +411,7 @@ __device__ __forceinline__ void interpret_k(const uint4 *__restrict__ ops, const
 // Batched instances K at a time: a work item is (group, slab), a group up to
 // K consecutive instances of one tree; missing members of a short group
 // repeat its first instance's thresholds and add nothing to any tally.
-template <int NT, int MINB, int MF, int PF, int K, bool ATL>
+template <int NT, int MINB, int PF, int K, bool ATL>
 __global__ void __launch_bounds__(NT, MINB) k_fused_batch_k(BatchArgs a) {
     extern __shared__ __align__(16) uint64_t smem[];
     __shared__ unsigned int s_item;
@@ -429,12 +433,12 @@ __global__ void __launch_bounds__(NT, MINB) k_fused_batch_k(BatchArgs a) {
         const uint64_t *thr[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) thr[k] = a.thr + a.inst_thr_offset[first + ((uint32_t)k < n ? (uint32_t)k : 0u)];
-        const WordCtx ctx = make_word_ctx<MF>((uint32_t)j);
+        const WordCtx ctx = make_word_ctx((uint32_t)j);
         unsigned long long *ones = a.inst_ones + first;
         auto add = [ones, n](uint32_t k, uint32_t c) {
             if (k < n) atomicAdd(ones + k, (unsigned long long)c);
         };
-        interpret_k<NT, MF, PF, K, ATL>(a.ops + a.tree_op_offset[a.inst_tree[first]], ctx, t3, j < a.words_per_instance,
+        interpret_k<NT, PF, K, ATL>(a.ops + a.tree_op_offset[a.inst_tree[first]], ctx, t3, j < a.words_per_instance,
                                    my_slots, my_scratch, a.scratch_stride, thr, add);
     }
 }
@@ -443,7 +447,7 @@ __global__ void __launch_bounds__(NT, MINB) k_fused_batch_k(BatchArgs a) {
 // Reference dataflow (layered).  Node words live in buf[node * W + w].
 
 // Basic events: be[e] = {pdag_idx+1, event_idx+1, thr_lo, thr_hi}.
-template <int MF, int PF>
+template <int PF>
 __global__ void __launch_bounds__(256) k_layer_be(const uint4 *__restrict__ be, uint32_t n_be, uint64_t W,
                                                   uint64_t word_begin, uint32_t t3, uint64_t *__restrict__ buf) {
     const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(256) k_layer_be(const uint4 *__restrict__ be, 
     uint64_t v;
     if (thr == 0) v = 0;
     else if (thr >= (1ull << 32)) v = kAllOnes;
-    else v = be_word<MF, PF>(r.x, r.y, make_word_ctx<MF>((uint32_t)(word_begin + w)), t3, (uint32_t)thr);
+    else v = be_word<PF>(r.x, r.y, make_word_ctx((uint32_t)(word_begin + w)), t3, (uint32_t)thr);
     buf[(uint64_t)e * W + w] = v;
 }
 
@@ -529,27 +533,26 @@ static __global__ void __launch_bounds__(256) k_layer_tally(const uint32_t *__re
 // n_be + g, with tallies fused.
 
 // Per-pass event table (philox.cuh): thread (e, g) fills entry g of event e.
-template <int MF>
-__global__ void __launch_bounds__(256) k_event_table(const uint4 *__restrict__ be, uint32_t n_be, uint32_t t3,
+static __global__ void __launch_bounds__(256) k_event_table(const uint4 *__restrict__ be, uint32_t n_be, uint32_t t3,
                                                      uint2 *__restrict__ table) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (uint64_t)n_be * kEventTableStride) return;
     const uint32_t e = (uint32_t)(i / kEventTableStride);
     const int g = (int)(i % kEventTableStride);
-    event_table_entry<MF>(be[e].x, t3, g, table[i]);
+    event_table_entry(be[e].x, t3, g, table[i]);
 }
 
 // Phase A: thread (w, group) samples word w of events [group * EPT, +EPT)
 // using the pass's event table.  Launched with dynamic shared memory that
 // only caps the blocks per SM, leaving room for gate-phase blocks.
-template <int MF, int PF, int EPT>
+template <int PF, int EPT>
 __global__ void __launch_bounds__(256, 6) k_stage_be(const uint4 *__restrict__ be, const uint2 *__restrict__ table,
                                                   uint32_t n_be, uint64_t W, uint64_t word_begin,
                                                   uint64_t *__restrict__ buf) {
     const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t e0 = (blockIdx.y + gridDim.y * blockIdx.z) * EPT;
     if (w >= W || e0 >= n_be) return;
-    const WordCtx ctx = make_word_ctx<MF>((uint32_t)(word_begin + w));
+    const WordCtx ctx = make_word_ctx((uint32_t)(word_begin + w));
 #pragma unroll 1
     for (uint32_t i = 0; i < EPT; ++i) {
         const uint32_t e = e0 + i;
@@ -558,7 +561,7 @@ __global__ void __launch_bounds__(256, 6) k_stage_be(const uint4 *__restrict__ b
         uint64_t v;
         if (r.w != 0) v = kAllOnes;           // threshold 2^32
         else if (r.z == 0) v = 0;             // threshold 0
-        else v = be_word_tab<MF, PF>(r.y, ctx, table + (uint64_t)e * kEventTableStride, r.z);
+        else v = be_word_tab<PF>(r.y, ctx, GlobalTable{table + (uint64_t)e * kEventTableStride}, r.z);
         buf[(uint64_t)e * W + w] = v;
     }
 }
@@ -812,7 +815,7 @@ static __device__ __noinline__ uint64_t strip_gate(const StripArgs &a, const uin
     return (op == MCG_NAND || op == MCG_NOR || op == MCG_NOT) ? ~acc : acc;
 }
 
-template <int MF, int PF, int MINB>
+template <int PF, int MINB>
 __global__ void __launch_bounds__(kStripThreads, MINB) k_strip(StripArgs a) {
     extern __shared__ unsigned long long s_ones[];
     __shared__ unsigned long long s_strip;
@@ -830,14 +833,14 @@ __global__ void __launch_bounds__(kStripThreads, MINB) k_strip(StripArgs a) {
         if (strip >= n_strips) break;
         const uint64_t wl = strip * kStripThreads + threadIdx.x;
         const bool valid = wl < a.word_count;
-        const WordCtx ctx = make_word_ctx<MF>((uint32_t)(a.word_begin + wl));
+        const WordCtx ctx = make_word_ctx((uint32_t)(a.word_begin + wl));
 #pragma unroll 1
         for (uint32_t e = 0; e < a.n_be; ++e) {
             const uint4 r = a.be[e];
             uint64_t v;
             if (r.w != 0) v = kAllOnes;
             else if (r.z == 0) v = 0;
-            else v = be_word_tab<MF, PF>(r.y, ctx, a.table + (uint64_t)e * kEventTableStride, r.z);
+            else v = be_word_tab<PF>(r.y, ctx, GlobalTable{a.table + (uint64_t)e * kEventTableStride}, r.z);
             col[(uint64_t)e * kStripLanes] = v;
         }
         for (uint32_t j = 0; j < a.n_be_tally; ++j) {
@@ -896,20 +899,159 @@ __global__ void __launch_bounds__(kStripThreads, MINB) k_strip(StripArgs a) {
             if (s_ones[i]) atomicAdd(&a.ones[i], s_ones[i]);
 }
 
+// Tile kernel (fused mode, trees whose node words fit in shared memory): a
+// block evaluates 32 sample words (lane = word) of every needed node at a
+// time, the whole pass in one launch.  Its warps share the events out, then
+// the gates of each layer.  Nothing but the counters leaves the SM, an event's
+// table entries are made by the warp that samples it (17 lanes, one product
+// each: 1.5 % of the sampling), and a pass spreads over events x words, so
+// that 4,096 words of a small tree already keep every SM busy where the
+// interpreter had 16 blocks.  1,024 threads per SM in all (64 registers each),
+// in as many blocks as the tile's size allows: one block's layers run under
+// the sampling of another.  Bound by the sampler's multiplies (0.86 of the
+// register-only sampler; the rest is gate work and the last, partly filled
+// round of events).  262,221 words of the 200-event tree: 1.98 ms, the
+// interpreter 2.67 ms; 4,096 words of a 60-event tree: 23 us of kernel where
+// the staged pipeline ran nine launches.
+// An input record's word: x, or its complement.
+__device__ __forceinline__ uint64_t tile_in(const uint64_t *col, uint32_t rec) {
+    const uint64_t x = *reinterpret_cast<const uint64_t *>(reinterpret_cast<const unsigned char *>(col) + (rec & ~1u));
+    return x ^ (uint64_t)(-(int64_t)(rec & 1u));
+}
+
+// An event's table entries in shared memory, two to a 16-byte load.
+struct SharedTable {
+    const uint4 *tab;
+    __device__ __forceinline__ uint2 operator()(int g) const {
+        const uint4 q = tab[g >> 1];
+        return g & 1 ? make_uint2(q.z, q.w) : make_uint2(q.x, q.y);
+    }
+};
+
+template <int NT, int PF>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_tile(const __grid_constant__ TileArgs a) {
+    constexpr uint32_t kWarps = NT / 32;
+    extern __shared__ __align__(16) uint64_t smem[];
+    __shared__ uint4 s_tab[kWarps][(kEventTableStride + 1) / 2];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint64_t *col = smem + lane;
+    unsigned long long *s_ones = reinterpret_cast<unsigned long long *>(smem + (size_t)a.n_slots * kTileLanes);
+    if (a.tally_in_smem)
+        for (uint32_t i = threadIdx.x; i < a.n_tally; i += NT) s_ones[i] = 0;
+    if (warp == 0) col[(a.n_slots - 1) * kTileLanes] = 0;  // the empty input
+    __syncthreads();
+    // one warp per tallied node and tile: the shared counters need no atomics
+    auto add = [&](uint32_t t, uint32_t c) {
+        if (a.tally_in_smem) s_ones[t] += c;
+        else atomicAdd(&a.ones[t], (unsigned long long)c);
+    };
+    const uint64_t tiles = (a.word_count + kTileLanes - 1) / kTileLanes;
+    for (uint32_t it = 0; it < a.n_iterations; ++it) {
+        const uint32_t t3 = (a.iteration_first + it + 1u) << 6;
+        for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+            const uint64_t wl = tile * kTileLanes + lane;
+            const bool valid = wl < a.word_count;
+            const WordCtx ctx = make_word_ctx((uint32_t)(a.word_begin + wl));
+#pragma unroll 1
+            for (uint32_t e = warp; e < a.n_be; e += kWarps) {
+                const uint4 r = a.be[e];
+                uint64_t v;
+                if (r.w != 0) {
+                    v = kAllOnes;
+                } else if (r.z == 0) {
+                    v = 0;
+                } else {
+                    __syncwarp();  // the last event's entries have been read
+                    if (lane < (uint32_t)kEventTableStride)
+                        event_table_entry(r.x, t3, (int)lane, reinterpret_cast<uint2 *>(s_tab[warp])[lane]);
+                    __syncwarp();
+                    v = be_word_tab<PF>(r.y, ctx, SharedTable{s_tab[warp]}, r.z);
+                }
+                col[e * kTileLanes] = v;
+            }
+            __syncthreads();
+            for (uint32_t j = warp; j < a.n_be_tally; j += kWarps) {
+                const uint2 t = a.be_tally[j];
+                const uint32_t c =
+                    __reduce_add_sync(0xFFFFFFFFu, valid ? (uint32_t)__popcll(col[t.x * kTileLanes]) : 0u);
+                if (lane == 0 && c) add(t.y, c);
+            }
+            for (uint32_t l = 0; l < a.n_layers; ++l) {
+                const uint32_t end = a.layer[l + 1];
+                for (uint32_t i = a.layer[l] + warp; i < end; i += kWarps) {
+                    const uint4 m = a.gates[i];
+                    const uint32_t kind = m.x & 3u;
+                    const uint2 *in = reinterpret_cast<const uint2 *>(a.in + m.y);
+                    uint64_t r = 0;
+                    if (kind == kTileOr) {
+#pragma unroll 2
+                        for (uint32_t j = 0; j < m.z; ++j) {
+                            const uint2 s = in[j];
+                            r |= tile_in(col, s.x) | tile_in(col, s.y);
+                        }
+                    } else if (kind == kTileXor) {
+                        for (uint32_t j = 0; j < m.z; ++j) {
+                            const uint2 s = in[j];
+                            r ^= tile_in(col, s.x) ^ tile_in(col, s.y);
+                        }
+                    } else {
+                        const uint32_t kk = (m.x >> 8) & 0xFFu, nbits = (m.x >> 16) & 0xFu;
+                        if (nbits <= 4) {  // at most 15 inputs
+                            SlicedCount4 cnt;
+                            for (uint32_t j = 0; j < m.z; ++j) {
+                                const uint2 s = in[j];
+                                cnt.add(tile_in(col, s.x));
+                                cnt.add(tile_in(col, s.y));
+                            }
+                            r = kk > 15 ? 0ull : cnt.ge(kk);
+                        } else {
+                            SlicedCount cnt;
+                            cnt.clear();
+                            for (uint32_t j = 0; j < m.z; ++j) {
+                                const uint2 s = in[j];
+                                cnt.add(tile_in(col, s.x), nbits);
+                                cnt.add(tile_in(col, s.y), nbits);
+                            }
+                            r = cnt.ge(kk);
+                        }
+                    }
+                    if (m.x & 4u) r = ~r;
+                    col[(a.n_be + i) * kTileLanes] = r;
+                    const uint32_t nt = m.x >> 20;  // tallies of the gate: one (its index), or a list
+                    if (nt) {
+                        const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, valid ? (uint32_t)__popcll(r) : 0u);
+                        if (lane == 0 && c) {
+                            if (nt == 1) add(m.w, c);
+                            else
+                                for (uint32_t j = 0; j < nt; ++j) add(a.tally_list[m.w + j], c);
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+            if (a.n_layers == 0) __syncthreads();  // the words are free again
+        }
+    }
+    __syncthreads();
+    if (a.tally_in_smem)
+        for (uint32_t i = threadIdx.x; i < a.n_tally; i += NT)
+            if (s_ones[i]) atomicAdd(&a.ones[i], s_ones[i]);
+}
+
 // Register-only sampler: thread w generates words (e, w) for n_events events
 // (event e: pdag_idx + 1 = e + 3, event_idx + 1 = e + 1, table row e) and
 // xors them together; one store per thread keeps the work alive.  Same
 // sampler code as the product's sampling kernel.
-template <int MF, int PF>
+template <int PF>
 __global__ void __launch_bounds__(256) k_sampler_peak(uint32_t n_events, uint64_t n_words,
                                                       const uint2 *__restrict__ table, uint64_t *__restrict__ sink) {
     const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= n_words) return;
-    const WordCtx ctx = make_word_ctx<MF>((uint32_t)w);
+    const WordCtx ctx = make_word_ctx((uint32_t)w);
     uint64_t x = 0;
     for (uint32_t e = 0; e < n_events; ++e) {
         const uint32_t thr = 0x01000000u + (e * 0x9E3779B9u >> 8);  // spread of probabilities
-        x ^= be_word_tab<MF, PF>(e + 1u, ctx, table + (uint64_t)e * kEventTableStride, thr);
+        x ^= be_word_tab<PF>(e + 1u, ctx, GlobalTable{table + (uint64_t)e * kEventTableStride}, thr);
     }
     sink[w] = x;
 }
@@ -917,19 +1059,19 @@ __global__ void __launch_bounds__(256) k_sampler_peak(uint32_t n_events, uint64_
 // Register-only sampler of the shared batch path: thread w generates words
 // (e, w) of K instances per Philox evaluation (be_words, the sampler the
 // batch interpreters call) and xors them together.
-template <int MF, int PF, int K>
+template <int PF, int K>
 __global__ void __launch_bounds__(256) k_sampler_peak_shared(uint32_t n_events, uint64_t n_words,
                                                              uint64_t *__restrict__ sink) {
     const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= n_words) return;
-    const WordCtx ctx = make_word_ctx<MF>((uint32_t)w);
+    const WordCtx ctx = make_word_ctx((uint32_t)w);
     uint64_t x = 0;
     for (uint32_t e = 0; e < n_events; ++e) {
         uint32_t thr[K];
         uint64_t out[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) thr[k] = 0x01000000u + ((e * 0x9E3779B9u + (uint32_t)k * 0x7F4A7C15u) >> 8);
-        be_words<MF, PF, K>(e + 3u, e + 1u, ctx, 2u << 6, thr, out);
+        be_words<PF, K>(e + 3u, e + 1u, ctx, 2u << 6, thr, out);
 #pragma unroll
         for (int k = 0; k < K; ++k) x ^= out[k];
     }
@@ -937,12 +1079,11 @@ __global__ void __launch_bounds__(256) k_sampler_peak_shared(uint32_t n_events, 
 }
 
 // Event table for k_sampler_peak's synthetic events.
-template <int MF>
-__global__ void __launch_bounds__(256) k_peak_table(uint32_t n_events, uint32_t t3, uint2 *__restrict__ table) {
+static __global__ void __launch_bounds__(256) k_peak_table(uint32_t n_events, uint32_t t3, uint2 *__restrict__ table) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (uint64_t)n_events * kEventTableStride) return;
     const uint32_t e = (uint32_t)(i / kEventTableStride);
-    event_table_entry<MF>(e + 3u, t3, (int)(i % kEventTableStride), table[i]);
+    event_table_entry(e + 3u, t3, (int)(i % kEventTableStride), table[i]);
 }
 
 }  // namespace dev

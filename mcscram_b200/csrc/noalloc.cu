@@ -64,7 +64,7 @@ mcg_status setup_device(int dev, DeviceSetup *&out) {
         // what one of the two CTAs per SM may use; the kernel's limit itself
         // is the device maximum, as engines with this kernel set it too
         const size_t cap = std::min<size_t>((size_t)optin, (size_t)per_sm / kCtasPerSm) - 1024;
-        const mcg_status lim = mcg::set_smem_limit(mcg::dev::k_fused<kThreads, kCtasPerSm, 1, 1>, cap);
+        const mcg_status lim = mcg::set_smem_limit(mcg::dev::k_fused<kThreads, kCtasPerSm, 1>, cap);
         if (lim != MCG_OK) return lim;
         s.scratch = static_cast<uint64_t *>(p);
         s.sms = sms;
@@ -127,7 +127,7 @@ extern "C" mcg_status mcg_run_fused_noalloc(const void *d_ops, uint64_t n_ops, u
         a.n_iterations = n_iterations;
         a.word_begin = word_begin + off;
         a.word_count = count;
-        mcg::dev::k_fused<kThreads, kCtasPerSm, 1, 1><<<grid, kThreads, smem, cs>>>(a);
+        mcg::dev::k_fused<kThreads, kCtasPerSm, 1><<<grid, kThreads, smem, cs>>>(a);
         err = cudaGetLastError();
         if (err != cudaSuccess) return mcg::fail(MCG_ERR_CUDA, std::string("k_fused launch: ") + cudaGetErrorString(err));
     }

@@ -33,25 +33,24 @@ struct RoundKey {
     static constexpr uint32_t k1 = kKey1 + (uint32_t)R * kW1;
 };
 
-// 32x32 -> 64-bit product split into halves.
-template <int MulForm>
+// 32x32 -> 64-bit product split into halves.  One wide multiply whose halves
+// are named: written as a 64-bit product the compiler carries the halves
+// through 64-bit operations (0.82 of the rate in the strip kernel), written as
+// a high and a low multiply it adds 30 register moves per word on the multiply
+// pipe (30.1 against 30.8 G words/s register-only, 198.0 against 194.3 ms for
+// 2^20 words of the 5,000-event tree).
 __device__ __forceinline__ void mul_hilo(uint32_t a, uint32_t b, uint32_t &hi, uint32_t &lo) {
-    if constexpr (MulForm == 0) {
-        const uint64_t p = (uint64_t)a * (uint64_t)b;
-        hi = (uint32_t)(p >> 32);
-        lo = (uint32_t)p;
-    } else {
-        hi = __umulhi(a, b);
-        lo = a * b;
-    }
+    asm("{\n\t.reg .u64 p;\n\tmul.wide.u32 p, %2, %3;\n\tmov.b64 {%1, %0}, p;\n\t}"
+        : "=r"(hi), "=r"(lo)
+        : "r"(a), "r"(b));
 }
 
 // Standard round r on the full state (rounds 4..10 of every call).
-template <int R, int MulForm>
+template <int R>
 __device__ __forceinline__ void philox_round(uint32_t &x0, uint32_t &x1, uint32_t &x2, uint32_t &x3) {
     uint32_t ha, la, hb, lb;
-    mul_hilo<MulForm>(kM0, x0, ha, la);
-    mul_hilo<MulForm>(kM1, x2, hb, lb);
+    mul_hilo(kM0, x0, ha, la);
+    mul_hilo(kM1, x2, hb, lb);
     x0 = hb ^ x1 ^ RoundKey<R>::k0;
     x1 = lb;
     x2 = ha ^ x3 ^ RoundKey<R>::k1;
@@ -63,10 +62,9 @@ struct WordCtx {
     uint32_t hb, lb;
 };
 
-template <int MulForm>
 __device__ __forceinline__ WordCtx make_word_ctx(uint32_t sample_idx) {
     WordCtx c;
-    mul_hilo<MulForm>(kM1, sample_idx + 1u, c.hb, c.lb);
+    mul_hilo(kM1, sample_idx + 1u, c.hb, c.lb);
     return c;
 }
 
@@ -95,24 +93,24 @@ __device__ __forceinline__ uint32_t shift_in_ge(uint32_t acc, uint32_t o, uint32
 // the word be_word gives for that threshold.  Instances that share a counter
 // stream but not their thresholds (draws of one tree) pay for the 16 Philox
 // calls once.
-template <int MulForm, int PackForm, int K>
+template <int PackForm, int K>
 __device__ __forceinline__ void be_words(uint32_t x0, uint32_t x1, const WordCtx &ctx, uint32_t t3,
                                          const uint32_t (&thr)[K], uint64_t (&out)[K]) {
     // Round 1, shared by the 16 calls.
     uint32_t ha, la;
-    mul_hilo<MulForm>(kM0, x0, ha, la);
+    mul_hilo(kM0, x0, ha, la);
     const uint32_t a0 = ctx.hb ^ x1 ^ RoundKey<0>::k0;
     const uint32_t a1 = ctx.lb;
     const uint32_t a2base = ha ^ t3 ^ RoundKey<0>::k1;  // x3 = t3 + g == t3 ^ g (g < 64)
     const uint32_t a3 = la;
     // Round 2: the M0 product is shared.
     uint32_t hc, lc;
-    mul_hilo<MulForm>(kM0, a0, hc, lc);
+    mul_hilo(kM0, a0, hc, lc);
     const uint32_t b2 = hc ^ a3 ^ RoundKey<1>::k1;
     const uint32_t b3 = lc;
     // Round 3: the M1 product is shared.
     uint32_t hf, lf;
-    mul_hilo<MulForm>(kM1, b2, hf, lf);
+    mul_hilo(kM1, b2, hf, lf);
     const uint32_t c1 = lf;
 
     uint32_t lo[K], hi[K];
@@ -122,23 +120,23 @@ __device__ __forceinline__ void be_words(uint32_t x0, uint32_t x1, const WordCtx
     for (int g = 0; g < 16; ++g) {
         // Round 2, per call.
         uint32_t hd, ld;
-        mul_hilo<MulForm>(kM1, a2base ^ (uint32_t)g, hd, ld);
+        mul_hilo(kM1, a2base ^ (uint32_t)g, hd, ld);
         const uint32_t b0 = hd ^ a1 ^ RoundKey<1>::k0;
         const uint32_t b1 = ld;
         // Round 3, per call.
         uint32_t he, le;
-        mul_hilo<MulForm>(kM0, b0, he, le);
+        mul_hilo(kM0, b0, he, le);
         uint32_t x0r = hf ^ b1 ^ RoundKey<2>::k0;
         uint32_t x1r = c1;
         uint32_t x2r = he ^ b3 ^ RoundKey<2>::k1;
         uint32_t x3r = le;
-        philox_round<3, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<4, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<5, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<6, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<7, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<8, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<9, MulForm>(x0r, x1r, x2r, x3r);
+        philox_round<3>(x0r, x1r, x2r, x3r);
+        philox_round<4>(x0r, x1r, x2r, x3r);
+        philox_round<5>(x0r, x1r, x2r, x3r);
+        philox_round<6>(x0r, x1r, x2r, x3r);
+        philox_round<7>(x0r, x1r, x2r, x3r);
+        philox_round<8>(x0r, x1r, x2r, x3r);
+        philox_round<9>(x0r, x1r, x2r, x3r);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             if constexpr (PackForm == 0) {
@@ -178,12 +176,12 @@ __device__ __forceinline__ void be_words(uint32_t x0, uint32_t x1, const WordCtx
     }
 }
 
-template <int MulForm, int PackForm>
+template <int PackForm>
 __device__ __forceinline__ uint64_t be_word(uint32_t x0, uint32_t x1, const WordCtx &ctx, uint32_t t3,
                                             uint32_t thr) {
     const uint32_t t[1] = {thr};
     uint64_t w[1];
-    be_words<MulForm, PackForm, 1>(x0, x1, ctx, t3, t, w);
+    be_words<PackForm, 1>(x0, x1, ctx, t3, t, w);
     return w[0];
 }
 
@@ -196,53 +194,52 @@ __device__ __forceinline__ uint64_t be_word(uint32_t x0, uint32_t x1, const Word
 // g = 0..15, [16] = {lo(M0 * x0), hi(M0 * x0)}.
 constexpr int kEventTableStride = 17;
 
-template <int MulForm>
 __device__ __forceinline__ void event_table_entry(uint32_t x0, uint32_t t3, int g, uint2 &out) {
     uint32_t ha, la;
-    mul_hilo<MulForm>(kM0, x0, ha, la);
+    mul_hilo(kM0, x0, ha, la);
     if (g < 16) {
         const uint32_t a2 = ha ^ t3 ^ RoundKey<0>::k1 ^ (uint32_t)g;
         uint32_t hd, ld;
-        mul_hilo<MulForm>(kM1, a2, hd, ld);
+        mul_hilo(kM1, a2, hd, ld);
         out = make_uint2(hd, ld);
     } else {
         out = make_uint2(la, ha);
     }
 }
 
-// be_word with the per-pass event table (same result as be_word).
-template <int MulForm, int PackForm>
-__device__ __forceinline__ uint64_t be_word_tab(uint32_t x1, const WordCtx &ctx, const uint2 *__restrict__ tab,
-                                                uint32_t thr) {
+// be_word with the per-pass event table (same result as be_word); tab(g) gives
+// entry g.
+template <int PackForm, class Table>
+__device__ __forceinline__ uint64_t be_word_tab(uint32_t x1, const WordCtx &ctx, Table &&tab, uint32_t thr) {
     const uint32_t a0 = ctx.hb ^ x1 ^ RoundKey<0>::k0;
     const uint32_t a1 = ctx.lb;
-    const uint32_t a3 = __ldg(&tab[16].x);
+    const uint32_t a3 = tab(16).x;
     uint32_t hc, lc;
-    mul_hilo<MulForm>(kM0, a0, hc, lc);
+    mul_hilo(kM0, a0, hc, lc);
     const uint32_t b2 = hc ^ a3 ^ RoundKey<1>::k1;
     const uint32_t b3 = lc;
     uint32_t hf, lf;
-    mul_hilo<MulForm>(kM1, b2, hf, lf);
+    mul_hilo(kM1, b2, hf, lf);
     const uint32_t c1 = lf;
     uint32_t lo = 0, hi = 0;
 #pragma unroll
     for (int g = 0; g < 16; ++g) {
-        const uint2 d = __ldg(&tab[g]);
+        const uint2 d = tab(g);
         const uint32_t b0 = d.x ^ a1 ^ RoundKey<1>::k0;
         const uint32_t b1 = d.y;
         uint32_t he, le;
-        mul_hilo<MulForm>(kM0, b0, he, le);
+        mul_hilo(kM0, b0, he, le);
         uint32_t x0r = hf ^ b1 ^ RoundKey<2>::k0;
         uint32_t x1r = c1;
         uint32_t x2r = he ^ b3 ^ RoundKey<2>::k1;
         uint32_t x3r = le;
-        philox_round<3, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<4, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<5, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<6, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<7, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<8, MulForm>(x0r, x1r, x2r, x3r);
-        philox_round<9, MulForm>(x0r, x1r, x2r, x3r);
+        philox_round<3>(x0r, x1r, x2r, x3r);
+        philox_round<4>(x0r, x1r, x2r, x3r);
+        philox_round<5>(x0r, x1r, x2r, x3r);
+        philox_round<6>(x0r, x1r, x2r, x3r);
+        philox_round<7>(x0r, x1r, x2r, x3r);
+        philox_round<8>(x0r, x1r, x2r, x3r);
+        philox_round<9>(x0r, x1r, x2r, x3r);
         if constexpr (PackForm == 0) {
             const uint32_t nib = nibble_lt(x0r, x1r, x2r, x3r, thr);
             if (g < 8) lo |= nib << (4 * g);
@@ -271,6 +268,12 @@ __device__ __forceinline__ uint64_t be_word_tab(uint32_t x1, const WordCtx &ctx,
         return ((uint64_t)(~rev_nibbles(hi)) << 32) | (uint64_t)(~rev_nibbles(lo));
     }
 }
+
+// Entry access for a table in global memory.
+struct GlobalTable {
+    const uint2 *__restrict__ tab;
+    __device__ __forceinline__ uint2 operator()(int g) const { return __ldg(tab + g); }
+};
 
 }  // namespace dev
 }  // namespace mcg

@@ -1,0 +1,74 @@
+"""The fused mode's tile kernel (trees whose node words fit in shared memory)
+against the oracle: tile and block edges of a pass, every connective with
+negated tails, constant events, single-event and event-only tallies, trees at
+each block size, and the first size that no longer fits."""
+import numpy as np
+import pytest
+
+from mcscram_b200 import graph as G
+from mcscram_b200 import synth
+from mcscram_b200.graph import AND, ATLEAST, NAND, NOR, NOT, NULL, OR, XOR
+
+
+def _every_connective(rng, n_be=40, n_gates=60):
+    """Random gates of all connectives with negated tails, empty gates, wide
+    gates and shared inputs; thresholds 0 and 2^32 among the events."""
+    ops, ks, begin, count, neg, inputs = [], [], [], [], [], []
+    for j in range(n_gates):
+        op = int(rng.choice([AND, OR, ATLEAST, XOR, NOT, NAND, NOR, NULL]))
+        n = int(rng.choice([0, 1, 2, 3, 5, 9, 16, 33])) if j else 3
+        ops.append(op)
+        ks.append(int(rng.integers(0, n + 2)))
+        begin.append(len(inputs))
+        count.append(n)
+        neg.append(int(rng.integers(0, n + 1)))
+        inputs += [int(x) for x in rng.integers(0, n_be + j, n)]
+    thr = rng.integers(1, 1 << 32, n_be).astype(np.uint64)
+    thr[0], thr[1] = 0, 1 << 32
+    return G.FlatGraph(be_pdag_idx=np.arange(2, 2 + n_be), be_event_idx=rng.permutation(n_be), be_threshold=thr,
+                       gate_op=ops, gate_k=ks, gate_in_begin=begin, gate_in_count=count, gate_neg_count=neg,
+                       inputs=inputs, tally_nodes=np.arange(n_be + n_gates))
+
+
+def _popcounts(words):
+    return np.array([int(np.unpackbits(r.view(np.uint8)).sum()) for r in words], dtype=np.uint64)
+
+
+def _check(capi, oracle_mod, g, words, begin=0, passes=1, first=1):
+    with capi.Engine(g, mode=capi.MODE_FUSED) as e:
+        e.run(first, passes, begin, words)
+        ones, total = e.tallies()
+    want = sum(_popcounts(oracle_mod.eval_words(g, first + i, begin, words)[g.tally_nodes]) for i in range(passes))
+    assert total == passes * words * 64
+    assert np.array_equal(ones, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("seed", range(4))
+def test_every_connective(capi, oracle_mod, gpu, seed):
+    _check(capi, oracle_mod, _every_connective(np.random.default_rng(seed)), 45, passes=2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("words,begin", [(1, 0), (31, 5), (32, 0), (33, 7), (1000, 123), (20000, 0),
+                                         (40, (1 << 32) - 40)])
+def test_pass_edges(capi, oracle_mod, gpu, words, begin):
+    g = synth.config1()
+    _check(capi, oracle_mod, g.with_tallies(np.arange(g.n_nodes)), words, begin, passes=1 if words > 5000 else 3, first=7)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_be,n_gates", [(6, 3), (130, 70), (160, 80), (280, 150), (560, 300), (620, 320)])
+def test_block_sizes_and_the_first_tree_that_does_not_fit(capi, oracle_mod, gpu, n_be, n_gates):
+    # 56 KB, 113 KB and 227 KB of words (4, 2 and 1 blocks an SM), and past them
+    g = synth.generate(synth.TreeSpec(n_be=n_be, n_gates=n_gates, mix={AND: 0.5, OR: 0.5}, p_range=(0.05, 0.5),
+                                      seed=5, share_be_frac=0.2))
+    _check(capi, oracle_mod, g.with_tallies(np.arange(n_be, g.n_nodes)), 333)
+
+
+@pytest.mark.gpu
+def test_event_tallies_without_gates_and_repeated_nodes(capi, oracle_mod, gpu):
+    g = synth.config1()
+    _check(capi, oracle_mod, g.with_tallies([3, 5, 3, 199]), 70)
+    _check(capi, oracle_mod, g.with_tallies([g.root, 4, g.root, g.n_be + 10]), 70)
+    _check(capi, oracle_mod, g.with_tallies(list(range(g.n_nodes)) * 40), 70)  # more counters than shared memory holds
