@@ -116,6 +116,31 @@ void save_file_locked() {
     if (!ok || std::rename(tmp.c_str(), path.c_str()) != 0) std::remove(tmp.c_str());
 }
 
+// A device's name and size, asked for once per process and device (the
+// properties take milliseconds a call).
+struct Device {
+    bool known = false;
+    std::string name;
+    int sms = 0, major = 0, minor = 0;
+};
+
+Device device_identity(int device) {
+    static std::mutex mu;
+    static std::unordered_map<int, Device> seen;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = seen.find(device);
+    if (it != seen.end()) return it->second;
+    Device d;
+    cudaDeviceProp prop;
+    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) {
+        cudaGetLastError();
+        return d;
+    }
+    d = Device{true, prop.name, prop.multiProcessorCount, prop.major, prop.minor};
+    seen[device] = d;
+    return d;
+}
+
 // Structure statistics and device identity that make up the shape key.
 mcg_status shape_key(const mcg_graph_desc &g, int device, uint64_t pass_words, uint64_t *key) {
     const uint64_t nn = (uint64_t)g.n_be + g.n_gates;
@@ -160,14 +185,13 @@ mcg_status shape_key(const mcg_graph_desc &g, int device, uint64_t pass_words, u
     h.add(per_op, sizeof per_op);
     h.add(info.max_live);
     h.add(pw_log2);
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) {
-        h.add(prop.name, std::strlen(prop.name));
-        h.add(prop.multiProcessorCount);
-        h.add(prop.major);
-        h.add(prop.minor);
+    const Device dev = device_identity(device);
+    if (dev.known) {
+        h.add(dev.name.data(), dev.name.size());
+        h.add(dev.sms);
+        h.add(dev.major);
+        h.add(dev.minor);
     } else {
-        cudaGetLastError();
         h.add("no-device", 9);
     }
     *key = h.h;

@@ -126,8 +126,8 @@ void release(mcg_batch *b) {
 
 mcg_status setup(mcg_batch *b, const mcg_run_desc &run) {
     MCG_CUDA(cudaSetDevice(b->device));
-    cudaDeviceProp prop;
-    MCG_CUDA(cudaGetDeviceProperties(&prop, b->device));
+    mcg::DeviceShape prop;
+    MCG_CUDA(mcg::device_shape(&prop, b->device));
     b->ctas_per_sm = run.ctas_per_sm ? run.ctas_per_sm : 4u;
     if (b->ctas_per_sm < 2 || b->ctas_per_sm > 4) return mcg::fail(MCG_ERR_INVALID, "ctas_per_sm must be 2..4");
     b->share = kShare;

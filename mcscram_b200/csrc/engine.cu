@@ -354,8 +354,8 @@ FusedKernel fused_kernel(uint32_t ctas_per_sm) {
 
 // Host-only compilation of the fused program (launch shape from the options).
 mcg_status compile_fused(mcg_engine *e, const mcg_run_desc &run) {
-    cudaDeviceProp prop;
-    MCG_CUDA(cudaGetDeviceProperties(&prop, e->device));
+    mcg::DeviceShape prop;
+    MCG_CUDA(mcg::device_shape(&prop, e->device));
     if (run.block_threads != 0 && run.block_threads != kFusedThreads)
         return mcg::fail(MCG_ERR_INVALID, "block_threads must be 0 or 256");
     e->nt = kFusedThreads;
@@ -482,11 +482,8 @@ mcg_status upload_tile(mcg_engine *e, const T **dptr, const std::vector<T> &v) {
 // shared memory (about 880 nodes on a B200): e->tile, or not.
 mcg_status setup_tile(mcg_engine *e) {
     const mcg::Graph &g = e->graph;
-    int optin = 0, per_sm = 0, reserved = 0, sms = 0;
-    MCG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, e->device));
-    MCG_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, e->device));
-    MCG_CUDA(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, e->device));
-    MCG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, e->device));
+    mcg::DeviceShape dev;
+    MCG_CUDA(mcg::device_shape(&dev, e->device));
     const TilePlan t = plan_tile(g);
     const uint64_t words = (uint64_t)t.slots() * mcg::dev::kTileLanes * sizeof(uint64_t);
     if (!t.fits) return MCG_OK;
@@ -497,7 +494,8 @@ mcg_status setup_tile(mcg_engine *e) {
     uint64_t room = 0;
     for (uint32_t nt : {256u, 512u, 1024u}) {
         const uint64_t own = (nt / 32u) * (mcg::dev::kEventTableStride + 1) * sizeof(uint2);
-        const uint64_t most = std::min<uint64_t>(optin, per_sm / (1024u / nt) - reserved);
+        const uint64_t most = std::min<uint64_t>(dev.sharedMemPerBlockOptin, dev.sharedMemPerMultiprocessor / (1024u / nt) -
+                                                                                 dev.reservedSharedMemPerBlock);
         if (words + own > most) continue;
         threads = nt;
         room = most - own;
@@ -509,7 +507,8 @@ mcg_status setup_tile(mcg_engine *e) {
     a = mcg::dev::TileArgs{};
     a.tally_in_smem = words + counters <= room ? 1u : 0u;
     e->tile_smem = (uint32_t)(words + (a.tally_in_smem ? counters : 0));
-    mcg_status st = mcg::set_smem_limit(tile_kernel(threads), e->tile_smem);
+    mcg_status st = MCG_OK;
+    for (uint32_t nt = threads; nt <= 1024u && st == MCG_OK; nt *= 2) st = mcg::set_smem_limit(tile_kernel(nt), e->tile_smem);
     if (st != MCG_OK) return st;
     std::vector<uint4> be(t.event.size());
     for (size_t i = 0; i < be.size(); ++i) {
@@ -528,7 +527,7 @@ mcg_status setup_tile(mcg_engine *e) {
     a.n_be_tally = (uint32_t)t.be_tally.size();
     a.n_tally = (uint32_t)g.tally_nodes.size();
     e->tile_threads = threads;
-    e->tile_grid = (uint32_t)sms * (1024u / threads);
+    e->tile_sms = (uint32_t)dev.multiProcessorCount;
     e->tile = true;
     return MCG_OK;
 }
@@ -541,8 +540,10 @@ mcg_status launch_tile(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t
     a.word_count = count;
     a.ones = e->d_tally;
     const uint64_t tiles = (count + mcg::dev::kTileLanes - 1) / mcg::dev::kTileLanes;
-    const uint32_t grid = (uint32_t)std::min<uint64_t>(e->tile_grid, std::max<uint64_t>(tiles, 1));
-    tile_kernel(e->tile_threads)<<<grid, e->tile_threads, e->tile_smem, e->stream>>>(a);
+    const uint32_t threads = e->tile_threads;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)e->tile_sms * (1024u / threads),
+                                                       std::max<uint64_t>(tiles, 1));
+    tile_kernel(threads)<<<grid, threads, e->tile_smem, e->stream>>>(a);
     ++e->launches;
     MCG_CUDA(cudaGetLastError());
     return MCG_OK;
@@ -594,8 +595,8 @@ mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
                         std::max<uint64_t>(e->graph.n_be, 1) * mcg::dev::kEventTableStride * sizeof(uint2)));
     // Cap the resident sampler blocks per SM through their shared-memory
     // footprint, so gate-phase blocks (memory bound) can run next to them.
-    cudaDeviceProp prop;
-    MCG_CUDA(cudaGetDeviceProperties(&prop, e->device));
+    mcg::DeviceShape prop;
+    MCG_CUDA(mcg::device_shape(&prop, e->device));
     const uint32_t blocks = run.sampler_blocks_per_sm ? run.sampler_blocks_per_sm : 8u;
     if (blocks < 1 || blocks > 8) return mcg::fail(MCG_ERR_INVALID, "sampler_blocks_per_sm must be 1..8");
     e->sampler_smem = blocks >= 8 ? 0u : (uint32_t)(prop.sharedMemPerMultiprocessor / blocks - 2048);
@@ -628,8 +629,8 @@ StripKernel strip_kernel(uint32_t blocks_per_sm) {
 
 mcg_status setup_strip(mcg_engine *e, const mcg_run_desc &run) {
     const mcg::Graph &g = e->graph;
-    cudaDeviceProp prop;
-    MCG_CUDA(cudaGetDeviceProperties(&prop, e->device));
+    mcg::DeviceShape prop;
+    MCG_CUDA(mcg::device_shape(&prop, e->device));
     const uint32_t target = run.ctas_per_sm ? run.ctas_per_sm : kStripBlocksPerSm;
     if (target < 4 || target > 6) return mcg::fail(MCG_ERR_INVALID, "strip mode: ctas_per_sm must be 0 or 4..6");
     e->strip_blocks = target;

@@ -43,7 +43,7 @@ struct mcg_engine {
     bool tile = false;
     mcg::dev::TileArgs tile_args{};        // device pointers and sizes; the pass is filled in per launch
     std::vector<void *> tile_tables;
-    uint32_t tile_threads = 0, tile_smem = 0, tile_grid = 0;
+    uint32_t tile_threads = 0, tile_smem = 0, tile_sms = 0;
 
     // tallies
     unsigned long long *d_tally = nullptr;

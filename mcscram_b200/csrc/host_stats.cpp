@@ -140,16 +140,28 @@ double gamma_p(double a, double x) {
     return 1.0 - std::exp(-x + a * std::log(x) - lg) * h;
 }
 
+// Newton's method on P(a, x) = q inside a shrinking bracket (bisecting where a
+// step leaves it), from the Wilson-Hilferty approximation, or the leading term
+// of P near 0: about six evaluations of P where bisection alone takes 53.
 double gamma_quantile(double a, double q) {
     double lo = 0.0, hi = std::max(1.0, a);
     while (gamma_p(a, hi) < q) hi *= 2.0;
+    const double lg = std::lgamma(a);
+    const double z = (q < 0.5 ? -1.0 : 1.0) * normal_quantile_two_sided(std::fabs(2.0 * q - 1.0));
+    const double wh = 1.0 - 1.0 / (9.0 * a) + z / (3.0 * std::sqrt(a));
+    double x = wh > 0.0 ? a * wh * wh * wh : 0.0;
+    if (!(x > 0.1 * a)) x = std::exp((std::log(q) + std::lgamma(a + 1.0)) / a);
+    if (!(x > lo && x < hi)) x = 0.5 * (lo + hi);
     for (int i = 0; i < 200; ++i) {
-        const double mid = 0.5 * (lo + hi);
-        if (gamma_p(a, mid) < q) lo = mid;
-        else hi = mid;
-        if (hi - lo <= 1e-15 * hi) break;
+        const double d = gamma_p(a, x) - q;
+        if (d < 0.0) lo = x;
+        else hi = x;
+        double next = x - d * std::exp(x - (a - 1.0) * std::log(x) + lg);
+        if (!(next > lo && next < hi)) next = 0.5 * (lo + hi);
+        if (std::fabs(next - x) <= 1e-15 * x || hi - lo <= 1e-15 * hi) return next;
+        x = next;
     }
-    return 0.5 * (lo + hi);
+    return x;
 }
 
 }  // namespace

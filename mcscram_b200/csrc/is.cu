@@ -1011,8 +1011,8 @@ mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in
     if (st != MCG_OK) return st;
     mcg_engine *e = is->engine;
     const uint32_t nb = e->graph.n_be;
-    cudaDeviceProp prop;
-    MCG_CUDA(cudaGetDeviceProperties(&prop, e->device));
+    mcg::DeviceShape prop;
+    MCG_CUDA(mcg::device_shape(&prop, e->device));
     if (2ull * std::max<uint32_t>(nb, 1) * sizeof(double) > prop.sharedMemPerBlockOptin) {
         // the documented limit of this entry point (larger trees: mcg_is_batch_create with one tree)
         mcg_destroy(e);

@@ -41,4 +41,28 @@ inline mcg_status set_smem_limit(F func, size_t need) {
     return MCG_OK;
 }
 
+// What the launch shapes need of a device, by attribute: cudaGetDeviceProperties
+// fills a hundred fields and took 2.4 to 12 ms a call, most of an engine's
+// creation.
+struct DeviceShape {
+    int multiProcessorCount = 0;
+    size_t sharedMemPerBlockOptin = 0, sharedMemPerMultiprocessor = 0, reservedSharedMemPerBlock = 0;
+};
+
+inline cudaError_t device_shape(DeviceShape *d, int device) {
+    int v[4] = {0, 0, 0, 0};
+    const cudaDeviceAttr attr[4] = {cudaDevAttrMultiProcessorCount, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+                                    cudaDevAttrMaxSharedMemoryPerMultiprocessor,
+                                    cudaDevAttrReservedSharedMemoryPerBlock};
+    for (int i = 0; i < 4; ++i) {
+        const cudaError_t err = cudaDeviceGetAttribute(&v[i], attr[i], device);
+        if (err != cudaSuccess) return err;
+    }
+    d->multiProcessorCount = v[0];
+    d->sharedMemPerBlockOptin = (size_t)v[1];
+    d->sharedMemPerMultiprocessor = (size_t)v[2];
+    d->reservedSharedMemPerBlock = (size_t)v[3];
+    return cudaSuccess;
+}
+
 }  // namespace mcg
