@@ -32,7 +32,9 @@ typedef struct mcg_batch_info {
     uint64_t total_ops;
     uint64_t launches;         /* kernel launches so far (graph replays count once each) */
     double last_kernel_ms;     /* duration of the last batched launch (CUDA events) */
-    uint32_t instances_per_item; /* instances of one tree evaluated together, sharing their
+    uint32_t instances_per_item; /* of the interpreter (run with smem_slots or ctas_per_sm given, or where
+                                  * the tile kernel's rows do not fit; tiles take up to 16): instances
+                                  * of one tree evaluated together, sharing their
                                   * Philox calls (4; 1 when a tree has an ATLEAST gate of
                                   * more than 15 inputs) */
 } mcg_batch_info;

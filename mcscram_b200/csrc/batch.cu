@@ -7,12 +7,14 @@
 #include <string>
 #include <vector>
 
+#include "batch_tile.cuh"
 #include "error.hpp"
 #include "graph.hpp"
 #include "kernels.cuh"
 #include "mcg_batch.h"
 #include "program.hpp"
 #include "smem_limit.hpp"
+#include "tile_plan.hpp"
 
 namespace {
 
@@ -96,6 +98,17 @@ struct mcg_batch {
     uint32_t *d_group_first = nullptr, *d_group_size = nullptr;
     uint64_t cap_grp = 0, cap_grp2 = 0;
     uint32_t n_groups = 0;
+    // tiles (the default shape): all trees' tables, and per run the groups and their event records
+    bool tile = false;
+    std::vector<mcg::dev::BatchTileTree> tile_trees;
+    mcg::dev::BatchTileArgs tile_args{};
+    std::vector<void *> tile_tables;
+    const uint2 *d_event = nullptr;
+    const uint32_t *d_event_node = nullptr, *d_event_off = nullptr;
+    mcg::dev::BatchTileGroup *d_tile_groups = nullptr;
+    uint4 *d_tile_recs = nullptr;
+    uint64_t cap_tile_groups = 0, cap_tile_recs = 0;
+    uint32_t n_tile_groups = 0, tile_most_events = 0;
     // graph
     cudaGraphExec_t graph = nullptr;
     uint32_t g_instances = 0, g_iteration = 0;
@@ -109,6 +122,9 @@ namespace {
 
 void release(mcg_batch *b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
+    for (void *p : b->tile_tables) cudaFree(p);
+    cudaFree(b->d_tile_groups);
+    cudaFree(b->d_tile_recs);
     cudaFree(b->d_ops);
     cudaFree(b->d_tree_off);
     cudaFree(b->d_scratch);
@@ -122,6 +138,82 @@ void release(mcg_batch *b) {
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
+}
+
+template <typename T>
+mcg_status upload_table(mcg_batch *b, const T **dptr, const std::vector<T> &v) {
+    void *p = nullptr;
+    MCG_CUDA(cudaMalloc(&p, std::max<size_t>(v.size(), 1) * sizeof(T)));
+    b->tile_tables.push_back(p);
+    if (!v.empty()) MCG_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+    *dptr = (const T *)p;
+    return MCG_OK;
+}
+
+// The tile kernel's scratch: a row of 4 KB per slot of the largest tree and
+// per SM (one block each).  Above this the interpreter's slots are smaller.
+constexpr uint64_t kTileScratchMost = 16ull << 30;
+
+// Tables of k_batch_tile; leaves b->tile false where the interpreter has to
+// take the batch (rows too large, or no memory for them).
+mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
+    using namespace mcg::dev;
+    std::vector<uint4> gates;
+    std::vector<uint32_t> in, layer, event_node, event_off;
+    std::vector<uint2> event, be_tally;
+    uint64_t most_slots = 0;
+    for (const auto &g : b->trees) {
+        const mcg::TilePlan t = mcg::plan_tile(g);
+        if (!t.fits || in.size() + t.in.size() > 0xFFFFFFFFull) return MCG_OK;
+        most_slots = std::max<uint64_t>(most_slots, t.slots() + 1ull);
+        if (most_slots * kTileRow > 0xFFFFFFFFull) return MCG_OK;
+        BatchTileTree x{};
+        x.n_be = (uint32_t)t.event.size();
+        x.n_layers = (uint32_t)t.layer.size() - 1;
+        x.gate_off = (uint32_t)gates.size();
+        x.layer_off = (uint32_t)layer.size();
+        x.in_off = (uint32_t)in.size();
+        x.be_tally_off = (uint32_t)be_tally.size();
+        for (const uint2 &s : t.be_tally) {  // {slot, tallies}: the slot's tallies follow each other
+            if (be_tally.size() > x.be_tally_off && be_tally.back().x == s.x + 1u) ++be_tally.back().y;
+            else be_tally.push_back(make_uint2(s.x + 1u, 1u));
+        }
+        x.n_be_tally = (uint32_t)be_tally.size() - x.be_tally_off;
+        gates.insert(gates.end(), t.gates.begin(), t.gates.end());
+        layer.insert(layer.end(), t.layer.begin(), t.layer.end());
+        for (uint32_t rec : t.in) in.push_back(mcg::TilePlan::byte_record(rec, kTileRow, 1, 0));
+        event_off.push_back((uint32_t)event.size());
+        for (uint32_t e : t.event) {
+            event.push_back(make_uint2((uint32_t)g.be_pdag_idx[e] + 1u, g.be_event_idx[e] + 1u));
+            event_node.push_back(e);
+        }
+        b->tile_most_events = std::max(b->tile_most_events, x.n_be);
+        b->tile_trees.push_back(x);
+    }
+    const uint64_t stride = most_slots * kTileRow;
+    const uint64_t blocks = (uint64_t)prop.multiProcessorCount * kBatchTileBlocks;
+    if (stride * blocks > kTileScratchMost) return MCG_OK;
+    const cudaError_t err = cudaMalloc((void **)&b->d_scratch, stride * blocks);
+    if (err == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        b->d_scratch = nullptr;
+        return MCG_OK;
+    }
+    MCG_CUDA(err);
+    BatchTileArgs &a = b->tile_args;
+    mcg_status st;
+    if ((st = upload_table(b, &a.trees, b->tile_trees)) != MCG_OK || (st = upload_table(b, &a.gates, gates)) != MCG_OK ||
+        (st = upload_table(b, &a.in, in)) != MCG_OK || (st = upload_table(b, &a.layer, layer)) != MCG_OK ||
+        (st = upload_table(b, &a.be_tally, be_tally)) != MCG_OK || (st = upload_table(b, &b->d_event, event)) != MCG_OK ||
+        (st = upload_table(b, &b->d_event_node, event_node)) != MCG_OK ||
+        (st = upload_table(b, &b->d_event_off, event_off)) != MCG_OK)
+        return st;
+    st = mcg::set_smem_limit(k_batch_tile, (kBatchTileThreads / 32) * kBatchTileOut);
+    if (st != MCG_OK) return st;
+    a.scratch = reinterpret_cast<unsigned char *>(b->d_scratch);
+    a.scratch_stride = stride;
+    b->tile = true;
+    return MCG_OK;
 }
 
 mcg_status setup(mcg_batch *b, const mcg_run_desc &run) {
@@ -171,10 +263,14 @@ mcg_status setup(mcg_batch *b, const mcg_run_desc &run) {
     MCG_CUDA(cudaMalloc((void **)&b->d_tree_off, b->tree_op_offset.size() * sizeof(uint32_t)));
     MCG_CUDA(cudaMemcpy(b->d_tree_off, b->tree_op_offset.data(), b->tree_op_offset.size() * sizeof(uint32_t),
                         cudaMemcpyHostToDevice));
-    if (b->max_global)
+    if (!run.smem_slots && !run.ctas_per_sm) {  // the default shape
+        const mcg_status ts = setup_tile(b, prop);
+        if (ts != MCG_OK) return ts;
+    }
+    if (b->max_global && !b->tile)
         MCG_CUDA(cudaMalloc((void **)&b->d_scratch,
                             (size_t)b->max_global * b->share * b->scratch_stride * sizeof(uint64_t)));
-    MCG_CUDA(cudaMalloc((void **)&b->d_queue, sizeof(unsigned int)));
+    MCG_CUDA(cudaMalloc((void **)&b->d_queue, sizeof(unsigned long long)));
     const mcg_status lim = mcg::set_smem_limit(batch_kernel(b->ctas_per_sm, b->share, b->atleast), b->smem_bytes);
     if (lim != MCG_OK) return lim;
     if (run.stream) {
@@ -214,9 +310,27 @@ mcg_status capture(mcg_batch *b, uint32_t n_inst, uint32_t iteration, uint64_t w
     a.n_groups = b->n_groups;
     cudaGraph_t g = nullptr;
     MCG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned int), b->stream);
+    cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned long long), b->stream);
     cudaMemsetAsync(b->d_ones, 0, (size_t)n_inst * sizeof(unsigned long long), b->stream);
-    batch_kernel(b->ctas_per_sm, b->share, b->atleast)<<<b->grid, kThreads, b->smem_bytes, b->stream>>>(a);
+    if (b->tile) {
+        using namespace mcg::dev;
+        BatchTileArgs t = b->tile_args;
+        t.groups = b->d_tile_groups;
+        t.recs = b->d_tile_recs;
+        t.words = words;
+        t.tiles = (words + kTileLanes - 1) / kTileLanes;
+        t.items = t.tiles * b->n_tile_groups;
+        t.iteration = iteration;
+        t.queue = reinterpret_cast<unsigned long long *>(b->d_queue);
+        t.ones = b->d_ones;
+        const dim3 grid(b->n_tile_groups, std::min(64u, std::max(1u, (b->tile_most_events + 255u) / 256u)));
+        k_batch_records<<<grid, 256, 0, b->stream>>>(b->d_tile_groups, b->d_event, b->d_event_node, b->d_event_off,
+                                                     t.trees, b->d_thr_off, b->d_thr, b->d_tile_recs);
+        k_batch_tile<<<(uint32_t)std::min<uint64_t>((uint64_t)(b->grid / b->ctas_per_sm) * kBatchTileBlocks, t.items), kBatchTileThreads,
+                       (kBatchTileThreads / 32) * kBatchTileOut, b->stream>>>(t);
+    } else {
+        batch_kernel(b->ctas_per_sm, b->share, b->atleast)<<<b->grid, kThreads, b->smem_bytes, b->stream>>>(a);
+    }
     const cudaError_t launch_err = cudaGetLastError();
     const cudaError_t end_err = cudaStreamEndCapture(b->stream, &g);
     if (launch_err != cudaSuccess || end_err != cudaSuccess) {
@@ -294,11 +408,12 @@ mcg_status mcg_batch_run(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tre
     }
     for (uint64_t k = 0; k < n_thr; ++k)
         if (thresholds[k] > (1ull << 32)) return mcg::fail(MCG_ERR_INVALID, "threshold above 2^32");
-    // groups of up to `share` consecutive instances of one tree
+    // groups of up to `share` consecutive instances of one tree (up to 16 in tiles)
+    const uint32_t most = b->tile ? mcg::dev::kTileInstances : b->share;
     std::vector<uint32_t> gfirst, gsize;
     for (uint32_t i = 0; i < n_inst;) {
         uint32_t n = 1;
-        while (n < b->share && i + n < n_inst && inst_tree[i + n] == inst_tree[i]) ++n;
+        while (n < most && i + n < n_inst && inst_tree[i + n] == inst_tree[i]) ++n;
         gfirst.push_back(i);
         gsize.push_back(n);
         i += n;
@@ -314,10 +429,32 @@ mcg_status mcg_batch_run(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tre
     MCG_CUDA(ensure(&b->d_ones, b->cap_ones, n_inst));
     MCG_CUDA(ensure(&b->d_group_first, b->cap_grp, gfirst.size()));
     MCG_CUDA(ensure(&b->d_group_size, b->cap_grp2, gsize.size()));
-    const bool moved = old_tree != b->d_inst_tree || old_off != b->d_thr_off || old_thr != b->d_thr ||
+    bool moved = old_tree != b->d_inst_tree || old_off != b->d_thr_off || old_thr != b->d_thr ||
                        old_ones != b->d_ones || old_gf != b->d_group_first || old_gs != b->d_group_size ||
                        b->n_groups != (uint32_t)gfirst.size();
     b->n_groups = (uint32_t)gfirst.size();
+    std::vector<mcg::dev::BatchTileGroup> groups;
+    if (b->tile) {
+        // the costliest first (events, and about as much again for every 20
+        // instances), so that the last items of the queue are small
+        std::vector<uint32_t> order(gfirst.size());
+        for (uint32_t i = 0; i < (uint32_t)order.size(); ++i) order[i] = i;
+        auto cost = [&](uint32_t i) { return (uint64_t)b->tile_trees[inst_tree[gfirst[i]]].n_be * (20u + gsize[i]); };
+        std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return cost(x) > cost(y); });
+        uint64_t recs = 0;
+        for (uint32_t i : order) {
+            const uint32_t t = inst_tree[gfirst[i]];
+            groups.push_back({t, gfirst[i], gsize[i], 0u, recs});
+            recs += b->tile_trees[t].n_be;
+        }
+        const void *old_groups = b->d_tile_groups, *old_recs = b->d_tile_recs;
+        MCG_CUDA(ensure(&b->d_tile_groups, b->cap_tile_groups, groups.size()));
+        MCG_CUDA(ensure(&b->d_tile_recs, b->cap_tile_recs, std::max<uint64_t>(recs, 1) * mcg::dev::kTileRec));
+        moved = moved || old_groups != b->d_tile_groups || old_recs != b->d_tile_recs;
+        b->n_tile_groups = (uint32_t)groups.size();
+        MCG_CUDA(cudaMemcpyAsync(b->d_tile_groups, groups.data(), groups.size() * sizeof(groups[0]),
+                                 cudaMemcpyHostToDevice, b->stream));
+    }
     MCG_CUDA(cudaMemcpyAsync(b->d_group_first, gfirst.data(), gfirst.size() * sizeof(uint32_t),
                              cudaMemcpyHostToDevice, b->stream));
     MCG_CUDA(cudaMemcpyAsync(b->d_group_size, gsize.data(), gsize.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,

@@ -24,6 +24,7 @@
 #include "mcg_tune.h"
 #include "program.hpp"
 #include "smem_limit.hpp"
+#include "tile_plan.hpp"
 
 namespace {
 
@@ -392,83 +393,6 @@ TileKernel tile_kernel(uint32_t threads) {
     }
 }
 
-// The nodes some tally depends on, as slots of the tile kernel: events in
-// their order, then gates layer by layer.  NOT and NULL gates read their last
-// input only.
-struct TilePlan {
-    std::vector<uint32_t> event;                 // slot -> event
-    std::vector<uint4> gates;
-    std::vector<uint32_t> in, layer{0}, tally_list;
-    std::vector<uint2> be_tally;
-    uint32_t slots() const { return (uint32_t)(event.size() + gates.size()) + 1u; }  // and the empty input
-    bool fits = true;  // the records' fields
-};
-
-TilePlan plan_tile(const mcg::Graph &g) {
-    TilePlan t;
-    const uint32_t nb = g.n_be;
-    auto first_input = [&](uint32_t i) {
-        const bool last_only = (g.gate_op[i] == MCG_NOT || g.gate_op[i] == MCG_NULL) && g.gate_in_count[i] > 0;
-        return last_only ? g.gate_in_count[i] - 1 : 0u;
-    };
-    std::vector<uint32_t> slot(g.n_nodes(), 0), depth(g.n_gates, 0);
-    std::vector<char> needed(g.n_nodes(), 0);
-    for (uint32_t v : g.tally_nodes) needed[v] = 1;
-    for (uint32_t i = g.n_gates; i-- > 0;) {
-        if (!needed[nb + i]) continue;
-        for (uint32_t j = first_input(i); j < g.gate_in_count[i]; ++j) needed[g.inputs[g.gate_in_begin[i] + j]] = 1;
-    }
-    std::vector<std::vector<uint32_t>> layers, tallies(g.n_nodes());
-    for (uint32_t i = 0; i < g.n_gates; ++i) {
-        if (!needed[nb + i]) continue;
-        for (uint32_t j = first_input(i); j < g.gate_in_count[i]; ++j) {
-            const uint32_t c = g.inputs[g.gate_in_begin[i] + j];
-            if (c >= nb) depth[i] = std::max(depth[i], depth[c - nb] + 1);
-        }
-        if (layers.size() <= depth[i]) layers.resize(depth[i] + 1);
-        layers[depth[i]].push_back(i);
-    }
-    for (uint32_t k = 0; k < (uint32_t)g.tally_nodes.size(); ++k) tallies[g.tally_nodes[k]].push_back(k);
-    for (uint32_t e = 0; e < nb; ++e) {
-        if (!needed[e]) continue;
-        slot[e] = (uint32_t)t.event.size();
-        t.event.push_back(e);
-        for (uint32_t k : tallies[e]) t.be_tally.push_back(make_uint2(slot[e], k));
-    }
-    constexpr uint32_t kSlotBytes = mcg::dev::kTileLanes * sizeof(uint64_t);
-    uint32_t next = (uint32_t)t.event.size(), n_gates = 0;
-    for (const auto &layer : layers) n_gates += (uint32_t)layer.size();
-    const uint32_t empty = (next + n_gates) * kSlotBytes;
-    for (const auto &layer : layers) {
-        for (uint32_t i : layer) slot[nb + i] = next++;
-        for (uint32_t i : layer) {
-            const uint8_t op = g.gate_op[i];
-            const uint32_t n = g.gate_in_count[i], from = first_input(i);
-            const bool and_type = op == MCG_AND || op == MCG_NAND;  // AND = ~OR(~x), NAND = OR(~x)
-            const bool inverted = op == MCG_AND || op == MCG_NOR || op == MCG_NOT;
-            const uint32_t kind = op == MCG_ATLEAST ? mcg::dev::kTileAtleast
-                                  : op == MCG_XOR   ? mcg::dev::kTileXor
-                                                    : mcg::dev::kTileOr;
-            uint32_t nbits = 0;
-            while (nbits < 8 && (n >> nbits) != 0) ++nbits;
-            const std::vector<uint32_t> &mine = tallies[nb + i];
-            if (mine.size() > 0xFFFu) t.fits = false;
-            t.gates.push_back(make_uint4(kind | (inverted ? 4u : 0u) | ((g.gate_k[i] & 0xFFu) << 8) |
-                                             (std::max(nbits, 1u) << 16) | ((uint32_t)mine.size() << 20),
-                                         (uint32_t)t.in.size(), (n - from + 1) / 2,
-                                         mine.size() == 1 ? mine[0] : (uint32_t)t.tally_list.size()));
-            if (mine.size() > 1) t.tally_list.insert(t.tally_list.end(), mine.begin(), mine.end());
-            for (uint32_t j = from; j < n; ++j) {
-                const bool negated = j >= n - g.gate_neg_count[i];
-                t.in.push_back(slot[g.inputs[g.gate_in_begin[i] + j]] * kSlotBytes | (uint32_t)(negated != and_type));
-            }
-            if ((n - from) % 2) t.in.push_back(empty);
-        }
-        t.layer.push_back((uint32_t)t.gates.size());
-    }
-    return t;
-}
-
 template <typename T>
 mcg_status upload_tile(mcg_engine *e, const T **dptr, const std::vector<T> &v) {
     T *p = nullptr;
@@ -484,8 +408,10 @@ mcg_status setup_tile(mcg_engine *e) {
     const mcg::Graph &g = e->graph;
     mcg::DeviceShape dev;
     MCG_CUDA(mcg::device_shape(&dev, e->device));
-    const TilePlan t = plan_tile(g);
-    const uint64_t words = (uint64_t)t.slots() * mcg::dev::kTileLanes * sizeof(uint64_t);
+    constexpr uint32_t kSlotBytes = mcg::dev::kTileLanes * sizeof(uint64_t);
+    mcg::TilePlan t = mcg::plan_tile(g);
+    for (uint32_t &rec : t.in) rec = t.byte_record(rec, kSlotBytes, 0, t.slots());
+    const uint64_t words = (uint64_t)(t.slots() + 1) * mcg::dev::kTileLanes * sizeof(uint64_t);
     if (!t.fits) return MCG_OK;
     // the most, and so the smallest, blocks that share an SM's 1,024 threads
     // and its shared memory; the tally counters go to shared memory where
@@ -522,7 +448,7 @@ mcg_status setup_tile(mcg_engine *e) {
         (st = upload_tile(e, &a.be_tally, t.be_tally)) != MCG_OK)
         return st;
     a.n_be = (uint32_t)t.event.size();
-    a.n_slots = t.slots();
+    a.n_slots = t.slots() + 1;  // and the empty input
     a.n_layers = (uint32_t)t.layer.size() - 1;
     a.n_be_tally = (uint32_t)t.be_tally.size();
     a.n_tally = (uint32_t)g.tally_nodes.size();

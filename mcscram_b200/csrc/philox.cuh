@@ -269,6 +269,32 @@ __device__ __forceinline__ uint64_t be_word_tab(uint32_t x1, const WordCtx &ctx,
     }
 }
 
+// Half of a word's outputs: the eight calls whose table entries are tab(0..7)
+// (lo32 is lo(M0 * x0)), handed to sink(call, out0, out1, out2, out3).
+template <class Table, class Sink>
+__device__ __forceinline__ void half_word_outputs(uint32_t x1, const WordCtx &ctx, uint32_t lo32, Table &&tab,
+                                                  Sink &&sink) {
+    const uint32_t a0 = ctx.hb ^ x1 ^ RoundKey<0>::k0;
+    uint32_t hc, b3, hf, c1;
+    mul_hilo(kM0, a0, hc, b3);
+    mul_hilo(kM1, hc ^ lo32 ^ RoundKey<1>::k1, hf, c1);
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+        const uint2 d = tab(g);
+        uint32_t he, x3;
+        mul_hilo(kM0, d.x ^ ctx.lb ^ RoundKey<1>::k0, he, x3);
+        uint32_t x0 = hf ^ d.y ^ RoundKey<2>::k0, y1 = c1, x2 = he ^ b3 ^ RoundKey<2>::k1;
+        philox_round<3>(x0, y1, x2, x3);
+        philox_round<4>(x0, y1, x2, x3);
+        philox_round<5>(x0, y1, x2, x3);
+        philox_round<6>(x0, y1, x2, x3);
+        philox_round<7>(x0, y1, x2, x3);
+        philox_round<8>(x0, y1, x2, x3);
+        philox_round<9>(x0, y1, x2, x3);
+        sink(g, x0, y1, x2, x3);
+    }
+}
+
 // Entry access for a table in global memory.
 struct GlobalTable {
     const uint2 *__restrict__ tab;

@@ -72,3 +72,35 @@ def test_event_tallies_without_gates_and_repeated_nodes(capi, oracle_mod, gpu):
     _check(capi, oracle_mod, g.with_tallies([3, 5, 3, 199]), 70)
     _check(capi, oracle_mod, g.with_tallies([g.root, 4, g.root, g.n_be + 10]), 70)
     _check(capi, oracle_mod, g.with_tallies(list(range(g.n_nodes)) * 40), 70)  # more counters than shared memory holds
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("draws,words", [((1,), 1), ((4, 5), 31), ((8, 9), 32), ((16,), 33), ((17, 3), 64),
+                                         ((33, 1, 16), 100), ((2, 15), 2049)])
+def test_batched_instances_in_tiles(oracle_mod, gpu, draws, words):
+    """Group sizes around the kernel's 4, 8 and 16 thresholds at a time, passes
+    around a tile, every connective, wide ATLEAST gates, constant thresholds
+    inside a group, rare and near-certain events, tallied events and nodes
+    tallied twice: every instance equals the oracle at its own thresholds."""
+    from mcscram_b200.uncertainty import Batch
+    rng = np.random.default_rng(len(draws) * 1000 + words)
+    trees = [synth.config1().with_tallies([299]), _every_connective(np.random.default_rng(1)),
+             synth.small_tree(4).with_tallies([35, 2, 35, 2, 30])]
+    inst_tree, thr = [], []
+    for t, n in enumerate(draws):
+        for d in range(n):
+            p = 10.0 ** rng.uniform(-4, 0, trees[t].n_be) if d % 3 else rng.uniform(0.5, 1.0, trees[t].n_be)
+            th = np.minimum((p * 2.0**32).astype(np.uint64), np.uint64((1 << 32) - 1))
+            if d % 4 == 1:
+                th[:3] = [0, 1 << 32, (1 << 32) - 1]
+            if d % 5 == 4:
+                th[:] = np.where(rng.random(th.size) < 0.5, 0, 1 << 32)
+            inst_tree.append(t)
+            thr.append(th)
+    order = rng.permutation(len(inst_tree))  # runs of one tree, and groups of one
+    runs = list(range(len(inst_tree))) + [int(i) for i in order]
+    with Batch(trees) as b:
+        got = b.run([inst_tree[i] for i in runs], [thr[i] for i in runs], iteration=5, words_per_instance=words)
+    for i, o in zip(runs, got):
+        g = trees[inst_tree[i]].with_thresholds(thr[i])
+        assert int(o) == int(np.sum(oracle_mod.tallies(g, 5, 1, 0, words))), (i, inst_tree[i])
