@@ -7,10 +7,11 @@
 // tensor memory (TMEM); the output layer (64 -> 1), the sigmoid and the loss
 // are per-row work on the CUDA cores.
 //
-// A CTA of 128 threads works on tiles of 128 rows: TMEM lane r and thread r
-// hold row r, so a tcgen05.ld of an accumulator gives each thread its own
-// row and every row-wise step (bias, ReLU, output dot product, loss) stays
-// in one thread.  Feature rows arrive by bulk copies (cp.async.bulk with an
+// A CTA of 256 threads works on tiles of 128 rows: TMEM lane r holds row r, and
+// threads r and r + 128 (warps w and w + 4 read the same lanes) each take half
+// of its units.  Bias, ReLU and the ReLU's derivative are per thread; the
+// output dot product runs on from the first thread's half to the second's, in
+// the order of the units, and the second computes the row's loss.  Feature rows arrive by bulk copies (cp.async.bulk with an
 // mbarrier transaction count), the next tile's while the current one is
 // computed.  One elected thread issues the MMAs and commits them to an
 // mbarrier the others wait on (bounded waits: a wait that runs out sets an
@@ -67,14 +68,36 @@ static_assert(kParams == MCG_MLP_PARAMS, "parameter layout");
 
 typedef __nv_bfloat16 bf16;
 
-// Packed BF16 operands: W1t[64][16] and W2t[64][64] (output-major), W3[64].
-constexpr int kPackW1t = 0;
-constexpr int kPackW2t = kPackW1t + kHid * kIn;
-constexpr int kPackW3 = kPackW2t + kHid * kHid;
+// BF16 copies of the weights as the kernels' shared memory holds them (one bulk
+// copy brings W1 and W2 in): W1 [hidden][feature] and W2 [out][in] in the
+// operand layout below (8 x 8 blocks of 128 bytes), then W3[64].
+constexpr int kPackW1 = 0;
+constexpr int kPackW2 = kPackW1 + kHid * kIn;
+constexpr int kPackW3 = kPackW2 + kHid * kHid;
 constexpr int kPackSize = kPackW3 + kHid;
+constexpr uint32_t kPackBytes = (uint32_t)kPackW3 * 2u;  // of W1 and W2
 
-constexpr int kTile = 128;     // rows per tile: the MMA's M, TMEM lanes, threads
-constexpr int kThreads = 128;  // 4 warps; warp w reads TMEM lanes 32w .. 32w + 31
+// Element (row n, column k) of a packed operand with `cols` columns.
+__host__ __device__ constexpr int pack_at(int n, int k, int cols) {
+    return ((n >> 3) * (cols >> 3) + (k >> 3)) * 64 + (n & 7) * 8 + (k & 7);
+}
+
+// Place of parameter i's BF16 copy, or -1 (biases).
+__host__ __device__ constexpr int pack_index(int i) {
+    if (i < kOffB1) return kPackW1 + pack_at((i - kOffW1) % kHid, (i - kOffW1) / kHid, kIn);
+    if (i >= kOffW2 && i < kOffB2) return kPackW2 + pack_at((i - kOffW2) % kHid, (i - kOffW2) / kHid, kHid);
+    if (i >= kOffW3 && i < kOffB3) return kPackW3 + i - kOffW3;
+    return -1;
+}
+
+constexpr int kTile = 128;     // rows per tile: the MMA's M, TMEM lanes
+// 8 warps, warp w reading TMEM lanes 32 (w % 4) .. + 31.  The kernels are a chain of short steps per tile, bound by
+// its latency and by the instructions of the row-wise steps at two CTAs per SM (a tile takes about 7,000 clocks, of
+// which the tensor pipe is busy 700).  The gradient of 250,000 rows: 50.2 us with one thread per row; 45.8 with two;
+// 44.7 with the weight gradients issued by a second thread and waited for on barriers of their own; 35.4 with the
+// row-wise steps on BF16 pairs, one add per descriptor and the weights brought in by one bulk copy (2,001 rows, one
+// tile per CTA: 14.9 -> 8.0 us).
+constexpr int kThreads = 256;
 constexpr int kCtasPerSm = 2;  // two CTAs of 256 TMEM columns fill the SM's 512
 constexpr uint32_t kTmemCols = 256;
 // TMEM columns (FP32 accumulators, 128 lanes each)
@@ -96,11 +119,12 @@ struct alignas(128) TcSmem {
     bf16 x[2][kTile * kUnitsX];  // two X tiles: a tile's G2 product may still read one while the next is filled
     bf16 e[kTile * kUnitsE];
     bf16 c[kTile * kUnitsC];
-    bf16 w1[kHid * kIn];     // B of layer 1: N = hidden, K = feature (K-major)
-    bf16 w2[kHid * kHid];    // B of layer 2: N = out, K = in (K-major); of dH2 W2^T: N = in, K = out (MN-major)
+    alignas(128) bf16 w1[kHid * kIn];  // B of layer 1: N = hidden, K = feature (K-major)
+    bf16 w2[kHid * kHid];    // right behind w1; B of layer 2: N = out, K = in (K-major); of dH2 W2^T: N = in, K = out (MN-major)
     float b1[kHid], b2[kHid], w3[kHid], w3b[kHid];
-    float red[2][kThreads / 32];
-    unsigned long long bar_mma, bar_end, bar_rows;
+    float z[kTile], d[kTile];  // a row's half dot product, its dL/dz
+    float red[2][kTile / 32];
+    unsigned long long bar_mma, bar_end, bar_rows, bar_w, bar_g1, bar_g2, bar_abort[2];
     uint32_t tmem;
 };
 
@@ -153,10 +177,19 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
 }
 
 // Shared-memory matrix descriptor, no swizzle: lbo = bytes between core
-// matrices along K, sbo = bytes between core matrices along M/N.
-__device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);  // version 1 (sm_100)
+// matrices along K, sbo = bytes between core matrices along M/N.  The high
+// word is a constant of the operand, and the K steps of a product only move
+// the address field: one add each (made anew per step, the descriptors took
+// the issuing thread about 90 clocks per MMA).
+struct Desc {
+    uint32_t lo, hi;
+    __device__ __forceinline__ Desc step(uint32_t bytes) const { return Desc{lo + (bytes >> 4), hi}; }
+    __device__ __forceinline__ uint64_t bits() const { return ((uint64_t)hi << 32) | lo; }
+};
+
+__device__ __forceinline__ Desc sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return Desc{((addr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16),
+                ((sbo >> 4) & 0x3FFFu) | (1u << 14)};  // version 1 (sm_100)
 }
 
 // Instruction descriptor: BF16 A and B, FP32 accumulator, M = 128, N = n;
@@ -167,10 +200,10 @@ __host__ __device__ constexpr uint32_t idesc(int n, bool a_mn, bool b_mn) {
 }
 
 // D (+)= A B, issued by one thread.
-__device__ __forceinline__ void umma(uint32_t d, uint64_t a, uint64_t b, uint32_t id, bool accumulate) {
+__device__ __forceinline__ void umma(uint32_t d, Desc a, Desc b, uint32_t id, bool accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),
-        "l"(a), "l"(b), "r"(id), "r"((uint32_t)accumulate)
+        "l"(a.bits()), "l"(b.bits()), "r"(id), "r"((uint32_t)accumulate)
         : "memory");
 }
 
@@ -226,49 +259,34 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-__device__ __forceinline__ void unpack8(const uint4 &q, float (&f)[8]) {
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        f[2 * i] = __uint_as_float(w[i] << 16);
-        f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-    }
+// 0xFFFF in each half of a BF16 pair that is above 0.
+__device__ __forceinline__ uint32_t positive2(uint32_t h) {
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+    return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&h), zero);
 }
 
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
     return make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
 }
 
-__device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
 // --- shared steps of the forward and gradient kernels ---------------------
 
-// Weights into their operand layouts, biases and W3; the constant zero
-// units of the X and E tiles.  Called by all threads before the first barrier.
+// Biases and W3; the constant zero units of the X and E tiles.  Called by all
+// threads before the first barrier; W1 and W2 follow by bulk copy (load_weights).
 __device__ void setup_operands(TcSmem &s, const bf16 *__restrict__ pack, const float *__restrict__ params) {
-    const int tid = threadIdx.x;
-    unsigned char *w1 = reinterpret_cast<unsigned char *>(s.w1);
-    for (int i = tid; i < kHid * kIn; i += kThreads) {  // N = hidden h, K = feature f
-        const int h = i / kIn, f = i % kIn;
-        *reinterpret_cast<bf16 *>(w1 + (((h >> 3) * (kIn / 8) + (f >> 3)) << 7) + ((h & 7) << 4) + ((f & 7) << 1)) =
-            pack[kPackW1t + i];
-    }
-    unsigned char *w2 = reinterpret_cast<unsigned char *>(s.w2);
-    for (int i = tid; i < kHid * kHid; i += kThreads) {  // N = out o, K = in j
-        const int o = i / kHid, j = i % kHid;
-        *reinterpret_cast<bf16 *>(w2 + (((o >> 3) * (kHid / 8) + (j >> 3)) << 7) + ((o & 7) << 4) + ((j & 7) << 1)) =
-            pack[kPackW2t + i];
-    }
-    for (int i = tid; i < kHid; i += kThreads) {
-        s.b1[i] = params[kOffB1 + i];
-        s.b2[i] = params[kOffB2 + i];
-        s.w3[i] = params[kOffW3 + i];
-        s.w3b[i] = __bfloat162float(pack[kPackW3 + i]);
-    }
+    const int tid = threadIdx.x, i = tid % kHid;
+    if (tid < kHid) s.b1[i] = params[kOffB1 + i];
+    else if (tid < 2 * kHid) s.b2[i] = params[kOffB2 + i];
+    else if (tid < 3 * kHid) s.w3[i] = params[kOffW3 + i];
+    else s.w3b[i] = __bfloat162float(pack[kPackW3 + i]);
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    *chunk<kUnitsX>(s.x[0], tid, 3) = zero;  // units 24..31
-    *chunk<kUnitsX>(s.x[1], tid, 3) = zero;
-    *chunk<kUnitsE>(s.e, tid, 9) = zero;  // units 72..79
+    *chunk<kUnitsX>(s.x[tid / kTile], tid % kTile, 3) = zero;  // units 24..31
+    if (tid < kTile) *chunk<kUnitsE>(s.e, tid, 9) = zero;      // units 72..79
+}
+
+// Thread 0: W1 and W2, completing bar_w; it waits for them before its first MMA.
+__device__ __forceinline__ void load_weights(TcSmem &s, const bf16 *__restrict__ pack) {
+    bulk_load(s.w1, pack + kPackW1, kPackBytes, &s.bar_w);
 }
 
 // TMEM allocation (warp 0) and mbarriers (thread 0); returns after the
@@ -285,6 +303,11 @@ __device__ uint32_t setup_tmem_and_barriers(TcSmem &s) {
         mbar_init(&s.bar_mma, 1);
         mbar_init(&s.bar_end, 1);
         mbar_init(&s.bar_rows, 1);
+        mbar_init(&s.bar_w, 1);
+        mbar_init(&s.bar_abort[0], 1);
+        mbar_init(&s.bar_abort[1], 1);
+        mbar_init(&s.bar_g1, 1);
+        mbar_init(&s.bar_g2, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     fence_async_smem();
@@ -319,24 +342,15 @@ __device__ __forceinline__ void load_rows(TcSmem &s, const float *__restrict__ f
     bulk_load(s.stage, feat + (uint64_t)row0 * kIn, rows * kIn * (uint32_t)sizeof(float), &s.bar_rows);
 }
 
-// Row r of the staged features (zero past n) into X tile xb, with the ones unit.
-__device__ __forceinline__ void rows_to_x(TcSmem &s, int xb, bool valid) {
-    const int r = threadIdx.x;
-    const float4 *src = reinterpret_cast<const float4 *>(s.stage + r * kIn);
-    float f[16];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float4 q = valid ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        f[4 * i] = q.x;
-        f[4 * i + 1] = q.y;
-        f[4 * i + 2] = q.z;
-        f[4 * i + 3] = q.w;
-    }
+// Row r's eight features of `half` (zero past n) from the stage into X tile xb;
+// the first half also writes the ones unit.
+__device__ __forceinline__ void rows_to_x(TcSmem &s, int xb, int r, int half, bool valid) {
+    const float4 *src = reinterpret_cast<const float4 *>(s.stage + r * kIn + 8 * half);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 a = valid ? src[0] : zero, b = valid ? src[1] : zero;
     bf16 *x = s.x[xb];
-    *chunk<kUnitsX>(x, r, 0) = make_uint4(pack2(f[0], f[1]), pack2(f[2], f[3]), pack2(f[4], f[5]), pack2(f[6], f[7]));
-    *chunk<kUnitsX>(x, r, 1) =
-        make_uint4(pack2(f[8], f[9]), pack2(f[10], f[11]), pack2(f[12], f[13]), pack2(f[14], f[15]));
-    *chunk<kUnitsX>(x, r, 2) = make_uint4(valid ? 0x3F80u : 0u, 0u, 0u, 0u);  // unit 16 = 1.0 (BF16 0x3F80)
+    *chunk<kUnitsX>(x, r, half) = make_uint4(pack2(a.x, a.y), pack2(a.z, a.w), pack2(b.x, b.y), pack2(b.z, b.w));
+    if (half == 0) *chunk<kUnitsX>(x, r, 2) = make_uint4(valid ? 0x3F80u : 0u, 0u, 0u, 0u);  // unit 16 = 1.0
 }
 
 // Thread 0: D1 = X W1 (one K = 16 step) from X tile xb.
@@ -345,75 +359,99 @@ __device__ __forceinline__ void issue_layer1(TcSmem &s, uint32_t tmem, int xb) {
          idesc(kHid, false, false), false);
 }
 
-// Thread 0: G2 += [dH1 | dH2]^T [X | 1] for the tile whose X tile is xb and
-// whose dH1, dH2 are in the C tile (K = rows, both operands MN-major).
+// G2 += [dH1 | dH2]^T [X | 1] for the tile whose X tile is xb and whose dH1,
+// dH2 are in the C tile (K = rows, both operands MN-major).
 __device__ __forceinline__ void issue_g2(TcSmem &s, uint32_t tmem, int xb, bool accumulate) {
-    const uint32_t a_c = smem_addr(s.c), a_x = smem_addr(s.x[xb]);
+    const Desc a = sdesc(smem_addr(s.c), kRowBlockC, 128), b = sdesc(smem_addr(s.x[xb]), kRowBlockX, 128);
 #pragma unroll
     for (int k = 0; k < kTile / 16; ++k)
-        umma(tmem + kColG2, sdesc(a_c + 2 * kRowBlockC * k, kRowBlockC, 128),
-             sdesc(a_x + 2 * kRowBlockX * k, kRowBlockX, 128), idesc(32, true, true), accumulate || k > 0);
+        umma(tmem + kColG2, a.step(2 * kRowBlockC * k), b.step(2 * kRowBlockX * k), idesc(32, true, true),
+             accumulate || k > 0);
+}
+
+// G1 += [dH2 | H2]^T [H1 | 1 | d]: K = rows, both operands MN-major.
+__device__ __forceinline__ void issue_g1(TcSmem &s, uint32_t tmem, bool accumulate) {
+    const Desc a = sdesc(smem_addr(s.c) + 8 * 128, kRowBlockC, 128), b = sdesc(smem_addr(s.e), kRowBlockE, 128);
+#pragma unroll
+    for (int k = 0; k < kTile / 16; ++k)
+        umma(tmem + kColG1, a.step(2 * kRowBlockC * k), b.step(2 * kRowBlockE * k), idesc(80, true, true),
+             accumulate || k > 0);
+}
+
+// Thread 0: dH2 W2^T into D1's columns: A = dH2 (K-major, K = out), B = W2
+// read as N = in, K = out (MN-major).
+__device__ __forceinline__ void issue_dh1(TcSmem &s, uint32_t tmem) {
+    const Desc a = sdesc(smem_addr(s.c) + 8 * 128, 128, kRowBlockC), b = sdesc(smem_addr(s.w2), (kHid / 8) * 128, 128);
+#pragma unroll
+    for (int k = 0; k < kHid / 16; ++k)
+        umma(tmem + kColD1, a.step(256 * k), b.step(2 * (kHid / 8) * 128 * k), idesc(kHid, false, true), k > 0);
 }
 
 // Thread 0: D2 = H1 W2 (four K = 16 steps).
 __device__ __forceinline__ void issue_layer2(TcSmem &s, uint32_t tmem) {
+    const Desc a = sdesc(smem_addr(s.e), 128, kRowBlockE), b = sdesc(smem_addr(s.w2), 128, (kHid / 8) * 128);
 #pragma unroll
     for (int k = 0; k < kHid / 16; ++k)
-        umma(tmem + kColD2, sdesc(smem_addr(s.e) + 256 * k, 128, kRowBlockE),
-             sdesc(smem_addr(s.w2) + 256 * k, 128, (kHid / 8) * 128), idesc(kHid, false, false), k > 0);
+        umma(tmem + kColD2, a.step(256 * k), b.step(256 * k), idesc(kHid, false, false), k > 0);
 }
 
-// H1 = relu(D1 + b1) into units 0..63 of the E tile.
-__device__ __forceinline__ void epilogue_h1(TcSmem &s, uint32_t t_row) {
-    const int r = threadIdx.x;
+// H1 = relu(D1 + b1), units 32 half .. + 31 of row r, into the E tile.
+__device__ __forceinline__ void epilogue_h1(TcSmem &s, uint32_t t_row, int r, int half) {
+    float v[32];
+    tmem_ld32(t_row + kColD1 + 32 * half, v);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        float v[32];
-        tmem_ld32(t_row + kColD1 + 32 * half, v);
+    for (int g = 0; g < 4; ++g) {
+        float h[8];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            float h[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) h[j] = fmaxf(v[8 * g + j] + s.b1[32 * half + 8 * g + j], 0.f);
-            *chunk<kUnitsE>(s.e, r, 4 * half + g) = pack8(h);
-        }
+        for (int j = 0; j < 8; ++j) h[j] = fmaxf(v[8 * g + j] + s.b1[32 * half + 8 * g + j], 0.f);
+        *chunk<kUnitsE>(s.e, r, 4 * half + g) = pack8(h);
     }
 }
 
-// H2 = relu(D2 + b2) (BF16-rounded), optionally stored into units 128..191
-// of the C tile; returns z = H2 . W3 + b3 with BF16 W3 and FP32 sums.
+// H2 = relu(D2 + b2), units 32 half .. + 31 of row r, as BF16 pairs into h and,
+// with STORE, into the C tile; returns z = H2 . W3 + b3 (BF16 operands, FP32
+// sums in unit order) in the second half's threads.  All threads call it: the
+// first half's sums cross a barrier.
 template <bool STORE>
-__device__ __forceinline__ float epilogue_h2(TcSmem &s, uint32_t t_row, float b3) {
-    const int r = threadIdx.x;
-    float z = b3;
+__device__ __forceinline__ float epilogue_h2(TcSmem &s, uint32_t t_row, int r, int half, float b3, uint32_t (&h)[16]) {
+    float v[32];
+    tmem_ld32(t_row + kColD2 + 32 * half, v);
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        float v[32];
-        tmem_ld32(t_row + kColD2 + 32 * half, v);
+    for (int j = 0; j < 16; ++j)
+        h[j] = pack2(fmaxf(v[2 * j] + s.b2[32 * half + 2 * j], 0.f), fmaxf(v[2 * j + 1] + s.b2[32 * half + 2 * j + 1], 0.f));
+    auto dot = [&](float z, const float *w) {
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            float h[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int u = 32 * half + 8 * g + j;
-                h[j] = bf16_round(fmaxf(v[8 * g + j] + s.b2[u], 0.f));
-                z = fmaf(h[j], s.w3b[u], z);
-            }
-            if constexpr (STORE) *chunk<kUnitsC>(s.c, r, 16 + 4 * half + g) = pack8(h);
+        for (int j = 0; j < 16; ++j) {
+            z = fmaf(__uint_as_float(h[j] << 16), w[2 * j], z);
+            z = fmaf(__uint_as_float(h[j] & 0xFFFF0000u), w[2 * j + 1], z);
         }
+        return z;
+    };
+    float z = b3;
+    if (half == 0) {
+        z = dot(z, s.w3b);
+        s.z[r] = z;
     }
+    if constexpr (STORE) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+            *chunk<kUnitsC>(s.c, r, 16 + 4 * half + g) = make_uint4(h[4 * g], h[4 * g + 1], h[4 * g + 2], h[4 * g + 3]);
+    }
+    __syncthreads();
+    if (half == 1) z = dot(s.z[r], s.w3b + 32);
     return z;
 }
 
-// Error exit (a wait ran out), thread 0: record it, let the bulk copies
-// still in flight land (the CTA's tiles [waited, issued)) and let every MMA
-// it issued finish (commits_end arrivals were committed to bar_end before),
-// so that shared memory and TMEM are no longer in use when the CTA leaves.
-__device__ void on_timeout(TcSmem &s, int *err, uint32_t waited, uint32_t issued, uint32_t commits_end) {
+// Error exit (a wait ran out), the two threads that issue work: record it, let
+// the bulk copies still in flight land (thread 0's: the weights, and the CTA's
+// tiles [waited, issued)) and let every MMA the thread issued finish, so that shared memory
+// and TMEM are no longer in use when the CTA leaves.
+__device__ void on_timeout(TcSmem &s, int *err, int issuer, uint32_t waited, uint32_t issued) {
     atomicExch(err, 1);
+    if (issuer == 0) mbar_wait(&s.bar_w, 0);
     for (uint32_t j = waited; j < issued; ++j) mbar_wait(&s.bar_rows, j & 1);
-    umma_commit(&s.bar_end);
-    mbar_wait(&s.bar_end, commits_end & 1);
+    umma_commit(&s.bar_abort[issuer]);
+    mbar_wait(&s.bar_abort[issuer], 0);
 }
 
 // q = sigmoid(network(features)) for rows [0, n): persistent CTAs over 128-row tiles.
@@ -422,25 +460,27 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
                   uint32_t n, float *__restrict__ q, int *__restrict__ err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     TcSmem &s = *reinterpret_cast<TcSmem *>(smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = tid >> 5, r = tid % kTile, half = tid / kTile;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     const uint32_t my_tiles = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
     setup_operands(s, pack, params);
     const uint32_t tmem = setup_tmem_and_barriers(s);
-    const uint32_t t_row = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t t_row = tmem + ((uint32_t)(warp % 4 * 32) << 16);
     const float b3 = params[kOffB3];
     uint32_t issued = 0;  // bulk copies issued (thread 0)
-    if (tid == 0 && my_tiles > 0) {
-        load_rows(s, feat, n, blockIdx.x);
-        issued = 1;
-    }
     bool ok = true;
+    if (tid == 0) {
+        load_weights(s, pack);
+        if (my_tiles > 0) load_rows(s, feat, n, blockIdx.x);
+        issued = my_tiles > 0 ? 1 : 0;
+        ok = mbar_wait(&s.bar_w, 0);
+    }
     uint32_t ph = 0, i = 0;
     for (; i < my_tiles; ++i) {
         const uint32_t tile = blockIdx.x + i * gridDim.x;
-        const uint32_t row = tile * kTile + tid;
+        const uint32_t row = tile * kTile + r;
         ok = mbar_wait(&s.bar_rows, i & 1) && ok;
-        rows_to_x(s, 0, row < n);
+        rows_to_x(s, 0, r, half, row < n);
         fence_async_smem();
         tc_before_sync();
         MCG_SYNC_OR_BREAK();
@@ -456,7 +496,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         ok = mbar_wait(&s.bar_mma, ph) && ok;
         ph ^= 1;
         tc_after_sync();
-        epilogue_h1(s, t_row);
+        epilogue_h1(s, t_row, r, half);
         fence_async_smem();
         tc_before_sync();
         MCG_SYNC_OR_BREAK();
@@ -468,53 +508,58 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         ok = mbar_wait(&s.bar_mma, ph) && ok;
         ph ^= 1;
         tc_after_sync();
-        const float z = epilogue_h2<false>(s, t_row, b3);
-        if (ok && row < n) q[row] = 1.f / (1.f + __expf(-z));
+        uint32_t h[16];
+        const float z = epilogue_h2<false>(s, t_row, r, half, b3, h);
+        if (ok && half == 1 && row < n) q[row] = 1.f / (1.f + __expf(-z));
         tc_before_sync();  // the next tile's layer 2 overwrites D2 after the next barrier
     }
     ok = __syncthreads_and(ok) != 0;
-    if (!ok && tid == 0) on_timeout(s, err, i, issued, 0);
+    if (!ok && tid == 0) on_timeout(s, err, 0, i, issued);
     release_tmem(tmem);
 }
 
 // Weighted BCE gradient of rows [0, n): persistent CTAs, CTA b taking tiles
 // b, b + gridDim.x, ...; its gradient (kParams floats, then the loss) goes to
-// partial[b * (kParams + 1) ..], every entry written once.  A tile's G2
-// product is issued with the next tile's layer 1 (or after the last tile):
-// it reads that tile's X tile (two alternate) and the dH1, dH2 units of the
-// C tile, which the next tile overwrites only after layer 1's completion --
-// and a commit covers every MMA issued before it.
+// partial[b * (kParams + 1) ..], every entry written once.  Thread 0 issues the
+// products the tile's chain waits for, thread kTile (warp 4) the weight
+// gradients: a tile's G1 once dH2, H2, H1 and d are published, its G2 with the
+// next tile's layer 1 (or after the last tile).  Their commits go to barriers
+// of their own, waited for where the operands are written again: G1's (E, and
+// the H2 and dH2 units of C) before the next tile's H1, G2's (dH1 and dH2; its
+// X tile alternates) before the next tile's dH2.
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     k_mlp_grad(const bf16 *__restrict__ pack, const float *__restrict__ params, const float *__restrict__ feat,
-               const float *__restrict__ tgt, const float *__restrict__ wts, float inv_wsum, uint32_t n,
-               float *__restrict__ partial, int *__restrict__ err) {
+               const float *__restrict__ tgt, const float *__restrict__ wts, float inv_wsum_host,
+               const float *__restrict__ inv_wsum_dev, uint32_t n, float *__restrict__ partial, int *__restrict__ err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     TcSmem &s = *reinterpret_cast<TcSmem *>(smem_raw);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = tid % kTile, half = tid / kTile;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     const uint32_t my_tiles = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
     setup_operands(s, pack, params);
     const uint32_t tmem = setup_tmem_and_barriers(s);
-    const uint32_t t_row = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t t_row = tmem + ((uint32_t)(warp % 4 * 32) << 16);
     const float b3 = params[kOffB3];
-    const uint32_t a_e = smem_addr(s.e), a_c = smem_addr(s.c), a_w2 = smem_addr(s.w2);
-    uint32_t issued = 0, commits_end = 0;  // thread 0's bulk copies and bar_end commits
-    if (tid == 0 && my_tiles > 0) {
-        load_rows(s, feat, n, blockIdx.x);
-        issued = 1;
-    }
-    float loss = 0.f, gb3 = 0.f;
+    uint32_t issued = 0;  // bulk copies issued (thread 0)
     bool ok = true;
+    if (tid == 0) {
+        load_weights(s, pack);
+        if (my_tiles > 0) load_rows(s, feat, n, blockIdx.x);
+        issued = my_tiles > 0 ? 1 : 0;
+        ok = mbar_wait(&s.bar_w, 0);
+    }
+    const float inv_wsum = inv_wsum_dev ? *inv_wsum_dev : inv_wsum_host;
+    float loss = 0.f, gb3 = 0.f;
     uint32_t ph = 0, i = 0;
     for (; i < my_tiles; ++i) {
         const uint32_t tile = blockIdx.x + i * gridDim.x;
         const int xb = (int)(i & 1);
-        const uint32_t row = tile * kTile + tid;
+        const uint32_t row = tile * kTile + r;
         const bool valid = row < n;
         const float tv = valid ? tgt[row] : 0.f;
         const float wv = valid ? (wts ? wts[row] : 1.f) * inv_wsum : 0.f;
         ok = mbar_wait(&s.bar_rows, i & 1) && ok;
-        rows_to_x(s, xb, valid);  // the X tile tile i - 2 used: its G2 completed before tile i - 1's layer 1 did
+        rows_to_x(s, xb, r, half, valid);  // the X tile tile i - 2 used: its G2 completed before tile i - 1's layer 1 did
         fence_async_smem();
         tc_before_sync();
         MCG_SYNC_OR_BREAK();
@@ -524,14 +569,17 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
                 load_rows(s, feat, n, tile + gridDim.x);
                 ++issued;
             }
-            if (i > 0) issue_g2(s, tmem, xb ^ 1, i > 1);
             issue_layer1(s, tmem, xb);
-            umma_commit(&s.bar_mma);  // also covers the previous tile's G1 and G2
+            umma_commit(&s.bar_mma);
+        } else if (tid == kTile && i > 0) {
+            issue_g2(s, tmem, xb ^ 1, i > 1);
+            umma_commit(&s.bar_g2);
         }
         ok = mbar_wait(&s.bar_mma, ph) && ok;
+        if (i > 0) ok = mbar_wait(&s.bar_g1, (i - 1) & 1) && ok;
         ph ^= 1;
         tc_after_sync();
-        epilogue_h1(s, t_row);
+        epilogue_h1(s, t_row, r, half);
         fence_async_smem();
         tc_before_sync();
         MCG_SYNC_OR_BREAK();
@@ -543,59 +591,62 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         ok = mbar_wait(&s.bar_mma, ph) && ok;
         ph ^= 1;
         tc_after_sync();
-        const float z = epilogue_h2<true>(s, t_row, b3);
-        // dL/dz = w (q - t) / sum w
-        float d = 0.f;
-        if (valid) {
-            const float qv = 1.f / (1.f + __expf(-z));
-            d = wv * (qv - tv);
-            const float qc = fminf(fmaxf(qv, 1e-7f), 1.f - 1e-7f);
-            loss -= wv * (tv * __logf(qc) + (1.f - tv) * __logf(1.f - qc));
+        uint32_t h[16];
+        const float z = epilogue_h2<true>(s, t_row, r, half, b3, h);
+        // dL/dz = w (q - t) / sum w, by the row's second thread; [1, d] into units 64, 65 of E
+        float qv = 0.f;
+        if (half == 1) {
+            float d = 0.f;
+            if (valid) {
+                qv = 1.f / (1.f + __expf(-z));
+                d = wv * (qv - tv);
+            }
+            gb3 += d;
+            s.d[r] = d;
+            *chunk<kUnitsE>(s.e, r, 8) = make_uint4(pack2(valid ? 1.f : 0.f, d), 0u, 0u, 0u);
         }
-        gb3 += d;
-        // dH2 = d W3 where H2 > 0, into units 64..127 of C; [1, d] into units 64, 65 of E
+        __syncthreads();
+        // dH2 = d W3 where H2 > 0, into units 64..127 of C
+        if (i > 0) ok = mbar_wait(&s.bar_g2, (i - 1) & 1) && ok;
+        const float d = s.d[r];
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
-            float h[8], dh[8];
-            unpack8(*chunk<kUnitsC>(s.c, tid, 16 + g), h);
+        for (int g = 0; g < 4; ++g) {
+            uint32_t q[4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) dh[j] = h[j] > 0.f ? d * s.w3[8 * g + j] : 0.f;
-            *chunk<kUnitsC>(s.c, tid, 8 + g) = pack8(dh);
+            for (int j = 0; j < 4; ++j) {
+                const float *w = s.w3 + 32 * half + 8 * g + 2 * j;
+                q[j] = pack2(d * w[0], d * w[1]) & positive2(h[4 * g + j]);
+            }
+            *chunk<kUnitsC>(s.c, r, 8 + 4 * half + g) = make_uint4(q[0], q[1], q[2], q[3]);
         }
-        *chunk<kUnitsE>(s.e, tid, 8) = make_uint4(pack2(valid ? 1.f : 0.f, d), 0u, 0u, 0u);
         fence_async_smem();
         tc_before_sync();
         MCG_SYNC_OR_BREAK();
         tc_after_sync();
         if (tid == 0) {
-            // dH2 W2^T into D1's columns: A = dH2 (K-major, K = out), B = W2 read as N = in, K = out (MN-major)
-#pragma unroll
-            for (int k = 0; k < kHid / 16; ++k)
-                umma(tmem + kColD1, sdesc(a_c + 8 * 128 + 256 * k, 128, kRowBlockC),
-                     sdesc(a_w2 + 2 * (kHid / 8) * 128 * k, (kHid / 8) * 128, 128), idesc(kHid, false, true), k > 0);
+            issue_dh1(s, tmem);
             umma_commit(&s.bar_mma);
-            // G1 += [dH2 | H2]^T [H1 | 1 | d]: K = rows, both operands MN-major
-#pragma unroll
-            for (int k = 0; k < kTile / 16; ++k)
-                umma(tmem + kColG1, sdesc(a_c + 8 * 128 + 2 * kRowBlockC * k, kRowBlockC, 128),
-                     sdesc(a_e + 2 * kRowBlockE * k, kRowBlockE, 128), idesc(80, true, true), i > 0 || k > 0);
+        } else if (tid == kTile) {
+            issue_g1(s, tmem, i > 0);
+            umma_commit(&s.bar_g1);
+        }
+        if (half == 1 && valid) {  // the loss, while the product runs
+            const float qc = fminf(fmaxf(qv, 1e-7f), 1.f - 1e-7f);
+            loss -= wv * (tv * __logf(qc) + (1.f - tv) * __logf(1.f - qc));
         }
         ok = mbar_wait(&s.bar_mma, ph) && ok;
         ph ^= 1;
         tc_after_sync();
         // dH1 = D1 where H1 > 0, into units 0..63 of C
+        float v[32];
+        tmem_ld32(t_row + kColD1 + 32 * half, v);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            float v[32];
-            tmem_ld32(t_row + kColD1 + 32 * half, v);
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                float h[8], dh[8];
-                unpack8(*chunk<kUnitsE>(s.e, tid, 4 * half + g), h);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) dh[j] = h[j] > 0.f ? v[8 * g + j] : 0.f;
-                *chunk<kUnitsC>(s.c, tid, 4 * half + g) = pack8(dh);
-            }
+        for (int g = 0; g < 4; ++g) {
+            const uint4 h1 = *chunk<kUnitsE>(s.e, r, 4 * half + g);
+            *chunk<kUnitsC>(s.c, r, 4 * half + g) =
+                make_uint4(pack2(v[8 * g], v[8 * g + 1]) & positive2(h1.x), pack2(v[8 * g + 2], v[8 * g + 3]) & positive2(h1.y),
+                           pack2(v[8 * g + 4], v[8 * g + 5]) & positive2(h1.z),
+                           pack2(v[8 * g + 6], v[8 * g + 7]) & positive2(h1.w));
         }
         fence_async_smem();  // published by the next barrier, before this tile's G2 is issued
         tc_before_sync();
@@ -603,67 +654,58 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     ok = __syncthreads_and(ok) != 0;
     if (ok && i > 0) {
         tc_after_sync();
-        if (tid == 0) {
+        if (tid == kTile) {  // its commit covers every G1 and G2 before
             issue_g2(s, tmem, (int)((i - 1) & 1), i > 1);
             umma_commit(&s.bar_end);
-            commits_end = 1;
-            ok = mbar_wait(&s.bar_end, 0);
         }
+        ok = mbar_wait(&s.bar_end, 0);
         ok = __syncthreads_and(ok) != 0;
     }
     float *out = partial + (uint64_t)blockIdx.x * (kParams + 1);
     if (ok) {
         tc_after_sync();
-        float g1[80], g2[32];
-        {
-            float v[32];
-            tmem_ld32(t_row + kColG1, v);
+        // row tid of G1: out unit tid of dW2^T (tid < 64), or H2 unit tid - 64 against d; of G2: hidden unit tid of
+        // dW1^T.  With no tile the accumulators were never written.
+        if (tid < kTile) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) g1[j] = v[j];
-            tmem_ld32(t_row + kColG1 + 32, v);
+            for (int c = 0; c < 2; ++c) {
+                float v[32];
+                tmem_ld32(t_row + kColG1 + 32 * c, v);
+                if (tid < kHid)
 #pragma unroll
-            for (int j = 0; j < 32; ++j) g1[32 + j] = v[j];
-            float w[16];
+                    for (int j = 0; j < 32; ++j) out[kOffW2 + (32 * c + j) * kHid + tid] = i ? v[j] : 0.f;
+            }
+            float w[16], v[32];
             tmem_ld16(t_row + kColG1 + 64, w);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) g1[64 + j] = w[j];
             tmem_ld32(t_row + kColG2, v);
+            if (tid < kHid) {
+                out[kOffB2 + tid] = i ? w[0] : 0.f;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) g2[j] = v[j];
-        }
-        if (i == 0) {  // no tile: the accumulators were never written
-#pragma unroll
-            for (int j = 0; j < 80; ++j) g1[j] = 0.f;
-#pragma unroll
-            for (int j = 0; j < 32; ++j) g2[j] = 0.f;
-        }
-        if (tid < kHid) {  // row tid of G1: out unit tid of dW2^T; of G2: hidden unit tid of dW1^T
-#pragma unroll
-            for (int j = 0; j < kHid; ++j) out[kOffW2 + j * kHid + tid] = g1[j];
-            out[kOffB2 + tid] = g1[64];
-#pragma unroll
-            for (int f = 0; f < kIn; ++f) out[kOffW1 + f * kHid + tid] = g2[f];
-            out[kOffB1 + tid] = g2[16];
-        } else {  // row tid of G1: H2 unit tid - 64 against d
-            out[kOffW3 + tid - kHid] = g1[65];
+                for (int f = 0; f < kIn; ++f) out[kOffW1 + f * kHid + tid] = i ? v[f] : 0.f;
+                out[kOffB1 + tid] = i ? v[16] : 0.f;
+            } else {
+                out[kOffW3 + tid - kHid] = i ? w[1] : 0.f;
+            }
         }
     } else if (tid == 0) {
-        on_timeout(s, err, i, issued, commits_end);
+        on_timeout(s, err, 0, i, issued);
+    } else if (tid == kTile) {
+        on_timeout(s, err, 1, 0, 0);
     }
-    // loss and db3: sums over the CTA's threads
+    // loss and db3: sums over the rows' second threads
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
         gb3 += __shfl_xor_sync(0xFFFFFFFFu, gb3, o);
     }
-    if (lane == 0) {
-        s.red[0][warp] = loss;
-        s.red[1][warp] = gb3;
+    if (half == 1 && lane == 0) {
+        s.red[0][warp - kTile / 32] = loss;
+        s.red[1][warp - kTile / 32] = gb3;
     }
     __syncthreads();
     if (tid == 0) {
         float l = 0.f, g = 0.f;
-        for (int w = 0; w < kThreads / 32; ++w) {
+        for (int w = 0; w < kTile / 32; ++w) {
             l += s.red[0][w];
             g += s.red[1][w];
         }
@@ -673,58 +715,98 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     release_tmem(tmem);
 }
 
-// grad[i] = sum over the CTAs of partial[b][i] (i = kParams: the loss).  A
-// block of 256 threads takes 32 entries: thread (g, p) sums the partials
-// b = g, g + 8, ... of entry p, then the eight sums are added in g order --
-// a fixed order, so the same partials give the same gradient bit for bit.
-constexpr int kReduceCols = 32, kReduceGroups = 8;
-__global__ void __launch_bounds__(kReduceCols * kReduceGroups)
-    k_mlp_reduce(const float *__restrict__ partial, uint32_t blocks, float *__restrict__ grad,
-                 float *__restrict__ loss) {
+// Sum over the CTAs of partial[b][i] (i = kParams: the loss), in the block's
+// threads p < kReduceCols, entry blockIdx.x * kReduceCols + p.  A block of
+// 1,024 threads brings 32 entries of all partials into shared memory (ten
+// loads in flight per thread), then sums them in a fixed order -- group g's
+// partials b = g, g + 8, ..., and the eight sums in g order -- so the same
+// partials give the same gradient bit for bit.
+constexpr int kReduceCols = 32, kReduceGroups = 8, kReduceThreads = 1024;
+__device__ __forceinline__ float reduce_entry(const float *__restrict__ partial, uint32_t blocks) {
+    extern __shared__ float s_partial[];  // [blocks][kReduceCols]
     __shared__ float part[kReduceGroups][kReduceCols];
     const int p = threadIdx.x % kReduceCols, g = threadIdx.x / kReduceCols;
     const int i = blockIdx.x * kReduceCols + p;
-    float v = 0.f;
-    if (i <= kParams)
-        for (uint32_t b = g; b < blocks; b += kReduceGroups) v += partial[(uint64_t)b * (kParams + 1) + i];
-    part[g][p] = v;
+#pragma unroll 10
+    for (uint32_t b = g; b < blocks; b += kReduceThreads / kReduceCols)
+        s_partial[b * kReduceCols + p] = i <= kParams ? partial[(uint64_t)b * (kParams + 1) + i] : 0.f;
     __syncthreads();
-    if (g == 0 && i <= kParams) {
-        float t = 0.f;
+    if (g < kReduceGroups) {
+        float v = 0.f;
+        for (uint32_t b = g; b < blocks; b += kReduceGroups) v += s_partial[b * kReduceCols + p];
+        part[g][p] = v;
+    }
+    __syncthreads();
+    float t = 0.f;
 #pragma unroll
-        for (int k = 0; k < kReduceGroups; ++k) t += part[k][p];
-        if (i < kParams) grad[i] = t;
-        else *loss = t;
-    }
+    for (int k = 0; k < kReduceGroups; ++k) t += part[k][p];
+    return t;
 }
 
-// FP32 master weights -> BF16 operand copies.
-__global__ void k_mlp_pack(const float *__restrict__ p, bf16 *__restrict__ pack) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kPackSize; i += gridDim.x * blockDim.x) {
-        float v;
-        if (i < kPackW2t) {  // W1t[h][f] = W1[f][h]
-            const int h = i / kIn, f = i % kIn;
-            v = p[kOffW1 + f * kHid + h];
-        } else if (i < kPackW3) {  // W2t[o][in] = W2[in][o]
-            const int j = i - kPackW2t, o = j / kHid, in = j % kHid;
-            v = p[kOffW2 + in * kHid + o];
-        } else {
-            v = p[kOffW3 + (i - kPackW3)];
-        }
-        pack[i] = __float2bfloat16(v);
-    }
+// The gradient (kParams entries) and behind it the loss.
+__global__ void __launch_bounds__(kReduceThreads)
+    k_mlp_reduce(const float *__restrict__ partial, uint32_t blocks, float *__restrict__ grad) {
+    const float t = reduce_entry(partial, blocks);
+    const int i = blockIdx.x * kReduceCols + threadIdx.x;
+    if (threadIdx.x < kReduceCols && i <= kParams) grad[i] = t;
 }
 
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
-                       float lr, float b1c, float b2c) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kParams) return;
-    const float gi = g[i];
+// A training step behind the gradient kernel: the gradient's sum, Adam and the
+// BF16 operand copy of each parameter, entry by entry (one launch where the
+// sum, Adam and the copy were three: 13.1 -> 9.5 us of a step at 250,000 rows).
+__global__ void __launch_bounds__(kReduceThreads)
+    k_mlp_step(const float *__restrict__ partial, uint32_t blocks, float *__restrict__ p, float *__restrict__ m,
+               float *__restrict__ v, float lr, float b1c, float b2c, bf16 *__restrict__ pack, float *__restrict__ loss) {
+    const float gi = reduce_entry(partial, blocks);
+    const int i = blockIdx.x * kReduceCols + threadIdx.x;
+    if (threadIdx.x >= kReduceCols || i > kParams) return;
+    if (i == kParams) {
+        *loss = gi;
+        return;
+    }
     const float mi = 0.9f * m[i] + 0.1f * gi;
     const float vi = 0.999f * v[i] + 0.001f * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / b1c) / (sqrtf(vi / b2c) + 1e-8f);
+    const float pi = p[i] - lr * (mi / b1c) / (sqrtf(vi / b2c) + 1e-8f);
+    p[i] = pi;
+    const int at = pack_index(i);
+    if (at >= 0) pack[at] = __float2bfloat16(pi);
+}
+
+// 1 / sum of the row weights (FP64, fixed order): kSumBlocks partial sums, then
+// their sum.  On the device for many rows: the host's serial sum took 0.3 ms
+// of a call with 250,000.
+constexpr int kSumBlocks = 64, kSumThreads = 256;
+constexpr uint32_t kHostSumRows = 1u << 15;
+__global__ void __launch_bounds__(kSumThreads) k_weight_sum(const float *__restrict__ w, uint32_t n,
+                                                            double *__restrict__ part) {
+    __shared__ double s_part[kSumThreads / 32];
+    double t = 0.0;
+    for (uint64_t i = (uint64_t)blockIdx.x * kSumThreads + threadIdx.x; i < n; i += (uint64_t)kSumBlocks * kSumThreads)
+        t += w[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+    if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < kSumThreads / 32; ++k) t += s_part[k];
+        part[blockIdx.x] = t;
+    }
+}
+
+__global__ void k_weight_inverse(const double *__restrict__ part, float *__restrict__ inv) {
+    double t = 0.0;
+    for (int k = 0; k < kSumBlocks; ++k) t += part[k];
+    *inv = t > 0.0 ? (float)(1.0 / t) : 0.f;
+}
+
+// FP32 master weights -> BF16 operand copies.
+__global__ void k_mlp_pack(const float *__restrict__ p, bf16 *__restrict__ pack) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= kParams) return;
+    const int at = pack_index(i);
+    if (at >= 0) pack[at] = __float2bfloat16(p[i]);
 }
 
 }  // namespace
@@ -732,11 +814,17 @@ __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float
 struct mcg_mlp {
     int device = 0;
     cudaStream_t stream = nullptr;
-    float *d_params = nullptr, *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr, *d_loss = nullptr;
+    float *d_params = nullptr, *d_m = nullptr, *d_v = nullptr;
+    float *d_grad = nullptr, *d_loss = nullptr;  // the loss lies behind the gradient: read back in one copy
+    double *d_wpart = nullptr;   // k_weight_sum's partial sums
+    float *d_inv_wsum = nullptr; // 1 / sum of the call's row weights, or
+    float inv_wsum = 0.f;        // summed on the host
+    bool inv_on_device = false;
     bf16 *d_pack = nullptr;
     float *d_feat = nullptr, *d_tgt = nullptr, *d_w = nullptr, *d_q = nullptr;
     float *d_partial = nullptr;  // [ctas][kParams + 1] per-CTA gradients and losses
-    int *d_err = nullptr;        // set by a kernel whose tensor-core or copy wait ran out
+    int *err = nullptr;          // set by a kernel whose tensor-core or copy wait ran out: host memory the device
+    int *d_err = nullptr;        // writes to, so that a call neither clears it on the stream nor copies it back
     uint32_t ctas = 0;           // persistent CTAs of the forward and gradient kernels
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around the steps of the last mcg_mlp_train
     double train_ms = 0.0;
@@ -764,50 +852,55 @@ mcg_status ensure_rows(mcg_mlp *m, uint32_t n) {
 
 // After a synchronised call: did one of its kernels give up on a tensor-core or copy wait?
 mcg_status check_waits(mcg_mlp *m) {
-    int err = 0;
-    MCG_CUDA(cudaMemcpy(&err, m->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (err)
+    if (*(volatile int *)m->err)
         return mcg::fail(MCG_ERR_CUDA, "proposal network: a tensor-core or bulk-copy wait timed out (results invalid)");
     return MCG_OK;
 }
 
 mcg_status pack(mcg_mlp *m) {
-    k_mlp_pack<<<(kPackSize + 255) / 256, 256, 0, m->stream>>>(m->d_params, m->d_pack);
+    k_mlp_pack<<<(kParams + 255) / 256, 256, 0, m->stream>>>(m->d_params, m->d_pack);
     MCG_CUDA(cudaGetLastError());
     return MCG_OK;
 }
 
-// The gradient of the uploaded rows into d_grad and d_loss: the persistent
-// gradient kernel, then the reduction of its partials.
-mcg_status grad_pass(mcg_mlp *m, uint32_t n, float inv_wsum, bool has_w) {
+// The gradient kernel over the uploaded rows; returns its CTAs (partial gradients).
+mcg_status grad_partials(mcg_mlp *m, uint32_t n, bool has_w, uint32_t &blocks) {
     const uint32_t tiles = (n + kTile - 1) / kTile;
-    const uint32_t blocks = std::max<uint32_t>(1, std::min<uint32_t>(tiles, m->ctas));
+    blocks = std::max<uint32_t>(1, std::min<uint32_t>(tiles, m->ctas));
     k_mlp_grad<<<blocks, kThreads, sizeof(TcSmem), m->stream>>>(m->d_pack, m->d_params, m->d_feat, m->d_tgt,
-                                                               has_w ? m->d_w : nullptr, inv_wsum, n, m->d_partial,
-                                                               m->d_err);
-    MCG_CUDA(cudaGetLastError());
-    k_mlp_reduce<<<(kParams + 1 + kReduceCols - 1) / kReduceCols, kReduceCols * kReduceGroups, 0, m->stream>>>(
-        m->d_partial, blocks, m->d_grad, m->d_loss);
+                                                               has_w ? m->d_w : nullptr, m->inv_wsum,
+                                                               m->inv_on_device ? m->d_inv_wsum : nullptr, n,
+                                                               m->d_partial, m->d_err);
     MCG_CUDA(cudaGetLastError());
     return MCG_OK;
 }
 
-// The call's rows to the device; also clears the wait-timeout flag, so that
+constexpr uint32_t kReduceBlocks = (kParams + 1 + kReduceCols - 1) / kReduceCols;
+
+// The call's rows to the device, and 1 / sum of their weights; also clears the
+// wait-timeout flag (the handle's earlier work has been waited for), so that
 // check_waits reports this call's kernels only.
-mcg_status upload_rows(mcg_mlp *m, const float *feat, const float *tgt, const float *w, uint32_t n, float &inv_wsum) {
+mcg_status upload_rows(mcg_mlp *m, const float *feat, const float *tgt, const float *w, uint32_t n) {
     mcg_status st = ensure_rows(m, n);
     if (st != MCG_OK) return st;
-    MCG_CUDA(cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream));
+    *(volatile int *)m->err = 0;
     MCG_CUDA(cudaMemcpyAsync(m->d_feat, feat, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    if (tgt) MCG_CUDA(cudaMemcpyAsync(m->d_tgt, tgt, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    double ws = 0.0;
-    if (w) {
-        for (uint32_t i = 0; i < n; ++i) ws += w[i];
-        MCG_CUDA(cudaMemcpyAsync(m->d_w, w, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    } else {
-        ws = n;
+    if (!tgt) return MCG_OK;
+    MCG_CUDA(cudaMemcpyAsync(m->d_tgt, tgt, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+    if (w) MCG_CUDA(cudaMemcpyAsync(m->d_w, w, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+    m->inv_on_device = w && n >= kHostSumRows;
+    if (m->inv_on_device) {
+        k_weight_sum<<<kSumBlocks, kSumThreads, 0, m->stream>>>(m->d_w, n, m->d_wpart);
+        k_weight_inverse<<<1, 1, 0, m->stream>>>(m->d_wpart, m->d_inv_wsum);
+        MCG_CUDA(cudaGetLastError());
+        return MCG_OK;
     }
-    inv_wsum = ws > 0 ? (float)(1.0 / ws) : 0.f;
+    double ws = n;
+    if (w) {
+        ws = 0.0;
+        for (uint32_t i = 0; i < n; ++i) ws += w[i];
+    }
+    m->inv_wsum = ws > 0 ? (float)(1.0 / ws) : 0.f;
     return MCG_OK;
 }
 
@@ -829,10 +922,12 @@ mcg_status mcg_mlp_create(int32_t device, uint64_t seed, mcg_mlp **out) {
     MCG_CUDA(cudaSetDevice(device));
     MCG_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
     MCG_CUDA(cudaMalloc((void **)&m->d_params, kParams * sizeof(float)));
-    MCG_CUDA(cudaMalloc((void **)&m->d_grad, kParams * sizeof(float)));
+    MCG_CUDA(cudaMalloc((void **)&m->d_grad, (kParams + 1) * sizeof(float)));
+    m->d_loss = m->d_grad + kParams;
+    MCG_CUDA(cudaMalloc((void **)&m->d_wpart, kSumBlocks * sizeof(double)));
+    MCG_CUDA(cudaMalloc((void **)&m->d_inv_wsum, sizeof(float)));
     MCG_CUDA(cudaMalloc((void **)&m->d_m, kParams * sizeof(float)));
     MCG_CUDA(cudaMalloc((void **)&m->d_v, kParams * sizeof(float)));
-    MCG_CUDA(cudaMalloc((void **)&m->d_loss, sizeof(float)));
     MCG_CUDA(cudaMalloc((void **)&m->d_pack, kPackSize * sizeof(bf16)));
     MCG_CUDA(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem)));
     MCG_CUDA(cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem)));
@@ -847,9 +942,13 @@ mcg_status mcg_mlp_create(int32_t device, uint64_t seed, mcg_mlp **out) {
     // SM's 512 TMEM columns
     const int per_sm = smem_sm / (int)(sizeof(TcSmem) + reserved);
     m->ctas = (uint32_t)std::max(1, sms * std::min(std::max(per_sm, 1), kCtasPerSm));
+    // the reduction holds 32 entries of every CTA's partial gradient
+    const size_t most = (48u << 10) - sizeof(float) * kReduceGroups * kReduceCols;
+    m->ctas = std::min<uint32_t>(m->ctas, (uint32_t)(most / (kReduceCols * sizeof(float))));
     MCG_CUDA(cudaMalloc((void **)&m->d_partial, (size_t)m->ctas * (kParams + 1) * sizeof(float)));
-    MCG_CUDA(cudaMalloc((void **)&m->d_err, sizeof(int)));
-    MCG_CUDA(cudaMemset(m->d_err, 0, sizeof(int)));
+    MCG_CUDA(cudaHostAlloc((void **)&m->err, sizeof(int), cudaHostAllocMapped));
+    *m->err = 0;
+    MCG_CUDA(cudaHostGetDevicePointer((void **)&m->d_err, m->err, 0));
     MCG_CUDA(cudaEventCreate(&m->ev0));
     MCG_CUDA(cudaEventCreate(&m->ev1));
     // He-style initialisation from a seeded host generator
@@ -878,14 +977,15 @@ mcg_status mcg_mlp_destroy(mcg_mlp *m) {
     cudaFree(m->d_grad);
     cudaFree(m->d_m);
     cudaFree(m->d_v);
-    cudaFree(m->d_loss);
+    cudaFree(m->d_wpart);
+    cudaFree(m->d_inv_wsum);
     cudaFree(m->d_pack);
     cudaFree(m->d_feat);
     cudaFree(m->d_tgt);
     cudaFree(m->d_w);
     cudaFree(m->d_q);
     cudaFree(m->d_partial);
-    cudaFree(m->d_err);
+    if (m->err) cudaFreeHost(m->err);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
     cudaStreamDestroy(m->stream);
@@ -921,8 +1021,7 @@ mcg_status mcg_mlp_forward(mcg_mlp *m, const float *features, uint32_t n, float 
     if (!m || !features || !q_out) return mcg::fail(MCG_ERR_INVALID, "NULL argument");
     if (n == 0) return MCG_OK;
     MCG_CUDA(cudaSetDevice(m->device));
-    float inv = 0.f;
-    mcg_status st = upload_rows(m, features, nullptr, nullptr, n, inv);
+    mcg_status st = upload_rows(m, features, nullptr, nullptr, n);
     if (st != MCG_OK) return st;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     k_mlp_forward<<<std::min(tiles, m->ctas), kThreads, sizeof(TcSmem), m->stream>>>(m->d_pack, m->d_params,
@@ -939,15 +1038,18 @@ mcg_status mcg_mlp_grad(mcg_mlp *m, const float *features, const float *targets,
     if (!m || !features || !targets || !grad_out) return mcg::fail(MCG_ERR_INVALID, "NULL argument");
     if (n == 0) return mcg::fail(MCG_ERR_INVALID, "no rows");
     MCG_CUDA(cudaSetDevice(m->device));
-    float inv = 0.f;
-    mcg_status st = upload_rows(m, features, targets, weights, n, inv);
+    mcg_status st = upload_rows(m, features, targets, weights, n);
     if (st != MCG_OK) return st;
-    st = grad_pass(m, n, inv, weights != nullptr);
+    uint32_t blocks = 0;
+    st = grad_partials(m, n, weights != nullptr, blocks);
     if (st != MCG_OK) return st;
-    MCG_CUDA(cudaMemcpyAsync(grad_out, m->d_grad, kParams * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-    float loss = 0.f;
-    MCG_CUDA(cudaMemcpyAsync(&loss, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+    k_mlp_reduce<<<kReduceBlocks, kReduceThreads, blocks * kReduceCols * sizeof(float), m->stream>>>(m->d_partial, blocks, m->d_grad);
+    MCG_CUDA(cudaGetLastError());
+    float out[kParams + 1];
+    MCG_CUDA(cudaMemcpyAsync(out, m->d_grad, sizeof(out), cudaMemcpyDeviceToHost, m->stream));
     MCG_CUDA(cudaStreamSynchronize(m->stream));
+    std::memcpy(grad_out, out, kParams * sizeof(float));
+    const float loss = out[kParams];
     st = check_waits(m);
     if (st != MCG_OK) return st;
     if (loss_out) *loss_out = loss;
@@ -960,19 +1062,18 @@ mcg_status mcg_mlp_train(mcg_mlp *m, const float *features, const float *targets
     if (!m || !features || !targets) return mcg::fail(MCG_ERR_INVALID, "NULL argument");
     if (n == 0) return mcg::fail(MCG_ERR_INVALID, "no rows");
     MCG_CUDA(cudaSetDevice(m->device));
-    float inv = 0.f;
-    mcg_status st = upload_rows(m, features, targets, weights, n, inv);
+    mcg_status st = upload_rows(m, features, targets, weights, n);
     if (st != MCG_OK) return st;
     MCG_CUDA(cudaEventRecord(m->ev0, m->stream));
     for (uint32_t s = 0; s < steps; ++s) {
-        st = grad_pass(m, n, inv, weights != nullptr);
+        uint32_t blocks = 0;
+        st = grad_partials(m, n, weights != nullptr, blocks);
         if (st != MCG_OK) return st;
         ++m->adam_t;
         const float b1c = 1.f - std::pow(0.9f, (float)m->adam_t);
         const float b2c = 1.f - std::pow(0.999f, (float)m->adam_t);
-        k_adam<<<(kParams + 255) / 256, 256, 0, m->stream>>>(m->d_params, m->d_grad, m->d_m, m->d_v, lr, b1c, b2c);
-        st = pack(m);
-        if (st != MCG_OK) return st;
+        k_mlp_step<<<kReduceBlocks, kReduceThreads, blocks * kReduceCols * sizeof(float), m->stream>>>(
+            m->d_partial, blocks, m->d_params, m->d_m, m->d_v, lr, b1c, b2c, m->d_pack, m->d_loss);
     }
     MCG_CUDA(cudaGetLastError());
     MCG_CUDA(cudaEventRecord(m->ev1, m->stream));
