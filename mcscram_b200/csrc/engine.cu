@@ -257,15 +257,6 @@ mcg_status build_layered_tables(mcg_engine *e) {
     std::vector<uint32_t> order(g.n_gates);
     for (uint32_t i = 0; i < g.n_gates; ++i) order[cursor[layer[i] - 1]++] = i;
 
-    // staged-mode tables
-    std::vector<uint4> smeta(g.n_gates);
-    for (uint32_t i = 0; i < g.n_gates; ++i) {
-        uint32_t nbits = 0;
-        while (nbits < 8 && (g.gate_in_count[i] >> nbits) != 0) ++nbits;
-        if (nbits == 0) nbits = 1;
-        smeta[i] = make_uint4((uint32_t)g.gate_op[i] | ((g.gate_k[i] & 0xFFu) << 8) | (nbits << 16),
-                              g.gate_in_begin[i], g.gate_in_count[i], g.gate_neg_count[i]);
-    }
     std::vector<std::vector<uint32_t>> per_gate(g.n_gates);
     std::vector<uint32_t> be_nodes, be_idx;
     for (uint32_t t = 0; t < (uint32_t)g.tally_nodes.size(); ++t) {
@@ -287,10 +278,27 @@ mcg_status build_layered_tables(mcg_engine *e) {
     if (e->mode == MCG_MODE_STRIP) {
         mcg_status st = build_strip_groups(e, order, gate_tally);
         if (st != MCG_OK) return st;
+        std::vector<uint4> smeta(g.n_gates);
+        for (uint32_t i = 0; i < g.n_gates; ++i) {
+            uint32_t nbits = 0;
+            while (nbits < 8 && (g.gate_in_count[i] >> nbits) != 0) ++nbits;
+            if (nbits == 0) nbits = 1;
+            smeta[i] = make_uint4((uint32_t)g.gate_op[i] | ((g.gate_k[i] & 0xFFu) << 8) | (nbits << 16),
+                                  g.gate_in_begin[i], g.gate_in_count[i], g.gate_neg_count[i]);
+        }
+        MCG_CUDA(upload(&e->d_smeta, smeta));
+        MCG_CUDA(upload(&e->d_gate_tally_list, gate_tally_list));
+    } else if (e->mode == MCG_MODE_STAGED) {
+        const mcg::GatePlan plan = mcg::plan_gates(g, layer);
+        e->n_gate_parts = (uint32_t)plan.part.size() - 1;
+        e->gates_largest_part = plan.largest;
+        MCG_CUDA(upload(&e->d_gates, plan.gates));
+        MCG_CUDA(upload(&e->d_gate_in, plan.in));
+        MCG_CUDA(upload(&e->d_gate_tally, plan.tally));
+        MCG_CUDA(upload(&e->d_gate_tally_list, plan.tally_list));
+        MCG_CUDA(upload(&e->d_gate_part, plan.part));
+        MCG_CUDA(upload(&e->d_gate_layer, plan.layer));
     }
-    MCG_CUDA(upload(&e->d_smeta, smeta));
-    MCG_CUDA(upload(&e->d_gate_tally, gate_tally));
-    MCG_CUDA(upload(&e->d_gate_tally_list, gate_tally_list));
     MCG_CUDA(upload(&e->d_be_tally_nodes, be_nodes));
     MCG_CUDA(upload(&e->d_be_tally_idx, be_idx));
 
@@ -503,15 +511,17 @@ mcg_status setup_fused(mcg_engine *e, const mcg_run_desc &run) {
 }
 
 constexpr uint32_t kStageEventsPerThread = 4;
+// From this many words on (a block of 64 per SM), gate blocks take two words
+// per lane: half the loads and instructions per word.  Fewer words are one per
+// lane, for twice the blocks (32,768 words of the 5,000-event tree: 6.23 ms,
+// one word per lane 6.55; 2,048 words of a 500-event tree: no difference).
+constexpr uint64_t kWideGateWords = 148 * 64;
 constexpr uint32_t kStripBlocksPerSm = 6;
-// Gate-phase blocks are small (128 threads, 2 words each) so that they fit in
-// the registers and threads left next to the capped sampler blocks.
-constexpr int kStageGateThreads = 128;
-constexpr int kStageWordsPerThread = 2;
 
 mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
                         const std::function<uint64_t(uint64_t)> &extra_words) {
-    const uint64_t nn = std::max<uint64_t>(e->graph.n_nodes(), 1);
+    const mcg::Graph &g = e->graph;
+    const uint64_t nn = std::max<uint64_t>(g.n_nodes(), 1);
     // two chunk buffers, together at most ~48 GB by default
     uint64_t words = run.layered_max_words ? run.layered_max_words : (24ull << 30) / (nn * sizeof(uint64_t));
     words = std::max<uint64_t>(256, std::min<uint64_t>(words, 1ull << 20));
@@ -533,6 +543,15 @@ mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
     const mcg_status lim = mcg::set_smem_limit(mcg::dev::k_stage_be<kPackForm, kStageEventsPerThread>,
                                                e->sampler_smem);
     if (lim != MCG_OK) return lim;
+    // Gate blocks of a chunk that the next one is sampled beside: two per SM, as
+    // they would otherwise fill the SMs' registers and stop the sampling while
+    // they wait for memory.  300,001 words of a 1,003-event tree in three
+    // chunks: 11.12 ms with all blocks at once, 10.84 ms with 3 per SM, 10.79
+    // with 2 or 1.5, 10.94 with 1.  Trees with so many gates per event that the
+    // gate phase is the longer one get all blocks.
+    const uint64_t traffic = g.inputs.size() + g.n_gates;
+    e->gates_beside_sampler = traffic <= 8ull * g.n_be;
+    e->gate_sms = (uint32_t)prop.multiProcessorCount;
     // The gate phase of chunk k runs while chunk k+1 is sampled: giving its
     // stream the higher priority lets its (memory-bound) blocks be scheduled
     // in between the sampler's blocks instead of after all of them.
@@ -641,13 +660,16 @@ mcg_status run_strip(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t w
     return MCG_OK;
 }
 
-// One chunk: phase A (sampling) on s_a into buffer `set`, phase B (gate layers
-// and tallies) on s_b once A is done.  A reuses a buffer only after the B that
+// One chunk: phase A (sampling) on s_a into buffer `set`, phase B (gates and
+// tallies) on s_b once A is done; `last`: no chunk follows it.  A reuses a buffer only after the B that
 // read it (two chunks earlier) has finished.
-mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t word_begin, uint64_t W) {
+mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t word_begin, uint64_t W,
+                        bool last) {
     const mcg::Graph &g = e->graph;
     const int set = (int)(k & 1);
     uint64_t *buf = e->d_stage[set];
+    // rows of an even length take 16-byte loads; hooks read rows of W words
+    const uint64_t stride = e->chunk_hook || e->sample_hook ? W : (W + 1) / 2 * 2;
     if (k >= 2) MCG_CUDA(cudaStreamWaitEvent(e->s_a, e->ev_b[set], 0));
     const uint32_t t3 = (iteration + 1u) << 6;
     const uint4 *be_tab = e->d_be_sample ? e->d_be_sample : e->d_be;
@@ -676,7 +698,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         }
         mcg::dev::k_stage_be<kPackForm, kStageEventsPerThread>
             <<<rows_grid(W, groups, 256), 256, e->sampler_smem, e->s_a>>>(be_tab, e->d_event_table, g.n_be, W,
-                                                                          word_begin, buf);
+                                                                          stride, word_begin, buf);
         ++e->launches;
         if (p1) MCG_CUDA(cudaEventRecord(p1, e->s_a));
     }
@@ -686,21 +708,37 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
     }
     MCG_CUDA(cudaEventRecord(e->ev_a[set], e->s_a));
     MCG_CUDA(cudaStreamWaitEvent(e->s_b, e->ev_a[set], 0));
-    const uint64_t words_per_block = (uint64_t)kStageGateThreads * kStageWordsPerThread;
-    for (size_t l = 0; l + 1 < e->layer_offsets.size(); ++l) {
-        const uint32_t n = e->layer_offsets[l + 1] - e->layer_offsets[l];
-        if (n == 0) continue;
-        dim3 grid = rows_grid(1, n, 256);
-        grid.x = (uint32_t)((W + words_per_block - 1) / words_per_block);
-        mcg::dev::k_stage_gates<kStageGateThreads, kStageWordsPerThread><<<grid, kStageGateThreads, 0, e->s_b>>>(
-            e->d_smeta, e->d_inputs, e->d_layer_gates + e->layer_offsets[l], n, g.n_be, W, buf, e->d_gate_tally,
-            e->d_gate_tally_list, e->d_tally);
+    if (g.n_gates > 0) {
+        mcg::dev::StageGateArgs a{};
+        a.gates = e->d_gates;
+        a.in = e->d_gate_in;
+        a.tally = e->d_gate_tally;
+        a.tally_list = e->d_gate_tally_list;
+        a.part = e->d_gate_part;
+        a.layer = e->d_gate_layer;
+        a.words = W;
+        a.stride = stride;
+        a.buf = buf;
+        a.ones = e->d_tally;
+        const bool wide = stride % 2 == 0 && W >= kWideGateWords;
+        uint64_t tiles = (W + (wide ? 63 : 31)) / (wide ? 64 : 32);
+        // Warps per block: the fewer blocks share the chip, the more of a
+        // layer's gates a block takes at a time.  Blocks are counted at the
+        // largest part's gates, which a small part's blocks do not wait for.
+        // 16 trees of very different sizes on 1,434 words: 0.49 ms with 512
+        // threads, 0.90 with 256; 640 words of them: 0.25 ms with 1,024, 0.83
+        // with 256.  512 blocks (32,768 words of one tree): 0.65 ms with 256.
+        const uint64_t blocks = tiles * g.n_gates / std::max<uint32_t>(e->gates_largest_part, 1);
+        const uint32_t threads = blocks >= 3ull * e->gate_sms ? 256u : blocks >= 2ull * e->gate_sms ? 512u : 1024u;
+        if (!last && e->gates_beside_sampler) tiles = std::min<uint64_t>(tiles, 2ull * e->gate_sms);
+        (wide ? mcg::dev::k_stage_gates<2> : mcg::dev::k_stage_gates<1>)<<<
+            dim3((uint32_t)tiles, e->n_gate_parts), threads, 0, e->s_b>>>(a);
         ++e->launches;
     }
     if (e->n_be_tally) {
         dim3 grid = rows_grid(1, e->n_be_tally, 256);
         grid.x = (uint32_t)std::min<uint64_t>((W + 255) / 256, 64);
-        mcg::dev::k_layer_tally<<<grid, 256, 0, e->s_b>>>(e->d_be_tally_nodes, e->n_be_tally, W, buf, e->d_tally,
+        mcg::dev::k_layer_tally<<<grid, 256, 0, e->s_b>>>(e->d_be_tally_nodes, e->n_be_tally, W, stride, buf, e->d_tally,
                                                           e->d_be_tally_idx);
         ++e->launches;
     }
@@ -720,10 +758,12 @@ mcg_status run_staged_impl(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint
     MCG_CUDA(cudaStreamWaitEvent(e->s_b, e->ev_fork, 0));
     uint64_t k = 0;
     for (uint32_t it = 0; it < n_it; ++it) {
-        for (uint64_t off = 0; off < count; off += e->stage_words, ++k) {
+        for (uint64_t off = 0; off < count; ++k) {
             const uint64_t n = std::min<uint64_t>(e->stage_words, count - off);
-            const mcg_status st = staged_chunk(e, k, it_first + it, word_begin + off, n);
+            const mcg_status st = staged_chunk(e, k, it_first + it, word_begin + off, n,
+                                               it + 1 == n_it && off + n == count);
             if (st != MCG_OK) return st;
+            off += n;
         }
     }
     // join back into the engine stream
@@ -775,6 +815,10 @@ void release(mcg_engine *e) {
     cudaFree(e->d_buf);
     cudaFree(e->d_smeta);
     cudaFree(e->d_gate_tally);
+    cudaFree(e->d_gates);
+    cudaFree(e->d_gate_in);
+    cudaFree(e->d_gate_part);
+    cudaFree(e->d_gate_layer);
     cudaFree(e->d_gate_tally_list);
     cudaFree(e->d_be_tally_nodes);
     cudaFree(e->d_be_tally_idx);
@@ -952,7 +996,7 @@ mcg_status mcg_run(mcg_engine *e, uint32_t iteration_first, uint32_t n_iteration
                     const uint32_t bx = (uint32_t)std::min<uint64_t>((n + 255) / 256, 64);
                     dim3 grid = rows_grid(1, n_tally, 256);
                     grid.x = bx;
-                    mcg::dev::k_layer_tally<<<grid, 256, 0, e->stream>>>(e->d_tally_nodes, n_tally, n, e->d_buf,
+                    mcg::dev::k_layer_tally<<<grid, 256, 0, e->stream>>>(e->d_tally_nodes, n_tally, n, n, e->d_buf,
                                                                          e->d_tally, nullptr);
                     ++e->launches;
                     MCG_CUDA(cudaGetLastError());

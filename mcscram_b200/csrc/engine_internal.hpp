@@ -61,8 +61,15 @@ struct mcg_engine {
     uint64_t layered_max_words = 0;
 
     // staged
-    uint4 *d_smeta = nullptr;           // gate meta with counter bits for the bit-sliced ATLEAST
+    uint4 *d_gates = nullptr;           // the gate kernel's tables (gate_plan.hpp)
+    uint32_t *d_gate_in = nullptr;
     uint2 *d_gate_tally = nullptr;      // per gate {offset, count} into d_gate_tally_list
+    uint32_t *d_gate_part = nullptr;
+    uint2 *d_gate_layer = nullptr;
+    uint32_t n_gate_parts = 0;
+    uint32_t gates_largest_part = 0;    // gates
+    uint32_t gate_sms = 0;              // SMs of the device
+    bool gates_beside_sampler = false;  // few gate blocks while the next chunk is sampled
     uint32_t *d_gate_tally_list = nullptr;
     uint32_t *d_be_tally_nodes = nullptr;  // tallied basic events
     uint32_t *d_be_tally_idx = nullptr;
@@ -83,6 +90,7 @@ struct mcg_engine {
     cudaEvent_t ev_fork = nullptr, ev_a[2] = {nullptr, nullptr}, ev_b[2] = {nullptr, nullptr};
     cudaEvent_t ev_join_a = nullptr, ev_join_b = nullptr;
     // strip
+    uint4 *d_smeta = nullptr;              // gate meta with counter bits for the bit-sliced ATLEAST
     uint64_t *d_strip_scratch = nullptr;   // per warp n_nodes x 32 words
     unsigned long long *d_queue = nullptr; // strip counter
     uint4 *d_strip_groups = nullptr;       // strip mode: gate groups, one layer at a time

@@ -1,0 +1,130 @@
+// gate_plan.hpp -- a graph's gates as the staged pipeline's gate kernel
+// evaluates them (host side; no CUDA calls).
+#pragma once
+#include <algorithm>
+#include <cstdint>
+#include <numeric>
+#include <vector>
+
+#include <vector_types.h>
+
+#include "graph.hpp"
+#include "mcg.h"
+
+namespace mcg {
+
+// Gate kinds.  AND, NAND, OR, NOR, one-of-n and n-of-n gates are ORs of
+// complemented or plain inputs with a complemented or plain result (De
+// Morgan), NOT and NULL ORs of their last input.  k-of-n gates with k or
+// n - k + 1 at most 4 keep that many running "at least j" words (kGateChain);
+// the others count in bit slices.
+constexpr uint32_t kGateOr = 0, kGateXor = 1, kGateChain = 2, kGateCount = 3;
+constexpr uint32_t kGateFlip = 0x80000000u;  // input record: node | kGateFlip if it is read complemented
+constexpr uint32_t kGateParts = 64;
+
+struct GatePlan {
+    // Gates part by part, layer by layer, two records each:
+    // {kind | inverted << 2 | k << 8 | counter bits << 16, first further input, inputs, output node} and the
+    // first four inputs.  Inputs are padded to a multiple of 4 with copies of the last one.
+    std::vector<uint4> gates;
+    std::vector<uint32_t> in;        // inputs from the fifth on, 4-aligned per gate
+    std::vector<uint2> tally;        // per gate {its tally (of several: their offset in tally_list), count}
+    std::vector<uint32_t> tally_list;
+    // Parts: sets of gates that read no gate of another part.  Part p's layers
+    // are layer[part[p]] .. layer[part[p + 1] - 1], each a gate range
+    // [layer[l].x, layer[l].y).
+    std::vector<uint32_t> part;
+    std::vector<uint2> layer;
+    uint32_t largest = 0;            // gates of the largest part
+};
+
+// `depth`: each gate's layer, from 1 on.
+inline GatePlan plan_gates(const Graph &g, const std::vector<uint32_t> &depth) {
+    GatePlan t;
+    const uint32_t nb = g.n_be, ng = g.n_gates;
+    std::vector<uint32_t> root(ng);
+    std::iota(root.begin(), root.end(), 0u);
+    auto find = [&](uint32_t i) {
+        while (root[i] != i) i = root[i] = root[root[i]];
+        return i;
+    };
+    for (uint32_t i = 0; i < ng; ++i)
+        for (uint32_t j = 0; j < g.gate_in_count[i]; ++j) {
+            const uint32_t c = g.inputs[g.gate_in_begin[i] + j];
+            if (c >= nb) root[find(i)] = find(c - nb);
+        }
+    // components, the largest first, each to the part with the fewest gates
+    std::vector<uint32_t> size(ng, 0), comps, part_of(ng, 0);
+    for (uint32_t i = 0; i < ng; ++i) ++size[find(i)];
+    for (uint32_t i = 0; i < ng; ++i)
+        if (size[i]) comps.push_back(i);
+    std::stable_sort(comps.begin(), comps.end(), [&](uint32_t x, uint32_t y) { return size[x] > size[y]; });
+    const uint32_t n_parts = std::max<uint32_t>(1, std::min<uint32_t>(kGateParts, (uint32_t)comps.size()));
+    std::vector<uint64_t> load(n_parts, 0);
+    for (uint32_t c : comps) {
+        const uint32_t p = (uint32_t)(std::min_element(load.begin(), load.end()) - load.begin());
+        load[p] += size[c];
+        part_of[c] = p;
+    }
+    t.largest = (uint32_t)*std::max_element(load.begin(), load.end());
+    std::vector<uint32_t> order(ng);
+    std::iota(order.begin(), order.end(), 0u);
+    for (uint32_t i = 0; i < ng; ++i) part_of[i] = part_of[find(i)];
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
+        return part_of[x] != part_of[y] ? part_of[x] < part_of[y] : depth[x] < depth[y];
+    });
+    std::vector<std::vector<uint32_t>> tallies(ng);
+    for (uint32_t k = 0; k < (uint32_t)g.tally_nodes.size(); ++k)
+        if (g.tally_nodes[k] >= nb) tallies[g.tally_nodes[k] - nb].push_back(k);
+
+    std::vector<uint32_t> rec;
+    uint32_t at = 0;
+    for (uint32_t p = 0; p < n_parts; ++p) {
+        t.part.push_back((uint32_t)t.layer.size());
+        while (at < ng && part_of[order[at]] == p) {
+            const uint32_t first = at;
+            for (; at < ng && part_of[order[at]] == p && depth[order[at]] == depth[order[first]]; ++at) {
+                const uint32_t i = order[at];
+                const uint8_t op = g.gate_op[i];
+                const uint32_t n = g.gate_in_count[i], k = g.gate_k[i] & 0xFFu;
+                const bool last_only = (op == MCG_NOT || op == MCG_NULL) && n > 0;
+                bool and_type = op == MCG_AND || op == MCG_NAND;  // AND = ~OR(~x), NAND = OR(~x)
+                bool inverted = op == MCG_AND || op == MCG_NOR || op == MCG_NOT;
+                uint32_t kind = op == MCG_XOR ? kGateXor : kGateOr, kk = k, nbits = 0;
+                if (op == MCG_ATLEAST) {
+                    kind = kGateCount;
+                    if (n <= 255 && k >= 1 && k <= n) {
+                        // at least k of x = not (at least n - k + 1 of ~x)
+                        const uint32_t co = n - k + 1;
+                        and_type = inverted = co < k;
+                        kk = std::min(k, co);
+                        if (kk == 1) kind = kGateOr;
+                        else if (kk <= 4) kind = kGateChain;
+                        else and_type = inverted = false, kk = k;
+                    }
+                    while (nbits < 8 && (n >> nbits) != 0) ++nbits;
+                }
+                rec.clear();
+                for (uint32_t j = last_only ? n - 1 : 0u; j < n; ++j) {
+                    const bool negated = j >= n - g.gate_neg_count[i];
+                    rec.push_back(g.inputs[g.gate_in_begin[i] + j] | (negated != and_type ? kGateFlip : 0u));
+                }
+                const uint32_t count = (uint32_t)rec.size();
+                t.gates.push_back(make_uint4(kind | (inverted ? 4u : 0u) | (kk << 8) | (std::max(nbits, 1u) << 16),
+                                             (uint32_t)t.in.size(), count, nb + i));
+                while (rec.size() < 4 || rec.size() % 4) rec.push_back(count ? rec[count - 1] : 0u);
+                t.gates.push_back(make_uint4(rec[0], rec[1], rec[2], rec[3]));
+                t.in.insert(t.in.end(), rec.begin() + 4, rec.end());
+                const std::vector<uint32_t> &mine = tallies[i];
+                t.tally.push_back(make_uint2(mine.size() == 1 ? mine[0] : (uint32_t)t.tally_list.size(),
+                                             (uint32_t)mine.size()));
+                if (mine.size() > 1) t.tally_list.insert(t.tally_list.end(), mine.begin(), mine.end());
+            }
+            t.layer.push_back(make_uint2(first, at));
+        }
+    }
+    t.part.push_back((uint32_t)t.layer.size());
+    return t;
+}
+
+}  // namespace mcg

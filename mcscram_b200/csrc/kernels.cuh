@@ -17,6 +17,7 @@
 #pragma once
 #include <cstdint>
 
+#include "gate_plan.hpp"
 #include "mcg.h"
 #include "philox.cuh"
 #include "program_format.h"
@@ -507,14 +508,14 @@ static __global__ void __launch_bounds__(256) k_layer_gates(const uint4 *__restr
 // Tallies: popcount, block reduction, one atomic per block and node.
 // tally_idx (optional) maps row t of tally_nodes to its counter.
 static __global__ void __launch_bounds__(256) k_layer_tally(const uint32_t *__restrict__ tally_nodes, uint32_t n_tally,
-                                                     uint64_t W, const uint64_t *__restrict__ buf,
+                                                     uint64_t W, uint64_t stride, const uint64_t *__restrict__ buf,
                                                      unsigned long long *__restrict__ ones,
                                                      const uint32_t *__restrict__ tally_idx) {
     __shared__ uint32_t warp_sums[8];
     const uint32_t t = blockIdx.y + gridDim.y * blockIdx.z;
     if (t >= n_tally) return;
     uint32_t c = 0;
-    const uint64_t *row = buf + (uint64_t)tally_nodes[t] * W;
+    const uint64_t *row = buf + (uint64_t)tally_nodes[t] * stride;
     for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < W; w += (uint64_t)gridDim.x * blockDim.x)
         c += (uint32_t)__popcll(row[w]);
     c = __reduce_add_sync(0xFFFFFFFFu, c);
@@ -547,8 +548,8 @@ static __global__ void __launch_bounds__(256) k_event_table(const uint4 *__restr
 // only caps the blocks per SM, leaving room for gate-phase blocks.
 template <int PF, int EPT>
 __global__ void __launch_bounds__(256, 6) k_stage_be(const uint4 *__restrict__ be, const uint2 *__restrict__ table,
-                                                  uint32_t n_be, uint64_t W, uint64_t word_begin,
-                                                  uint64_t *__restrict__ buf) {
+                                                  uint32_t n_be, uint64_t W, uint64_t stride,
+                                                  uint64_t word_begin, uint64_t *__restrict__ buf) {
     const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t e0 = (blockIdx.y + gridDim.y * blockIdx.z) * EPT;
     if (w >= W || e0 >= n_be) return;
@@ -562,120 +563,214 @@ __global__ void __launch_bounds__(256, 6) k_stage_be(const uint4 *__restrict__ b
         if (r.w != 0) v = kAllOnes;           // threshold 2^32
         else if (r.z == 0) v = 0;             // threshold 0
         else v = be_word_tab<PF>(r.y, ctx, GlobalTable{table + (uint64_t)e * kEventTableStride}, r.z);
-        buf[(uint64_t)e * W + w] = v;
+        buf[(uint64_t)e * stride + w] = v;
     }
 }
 
-// Phase B: gate layer_gates[blockIdx.y] for words [blockIdx.x * NT * WPT, ...),
-// WPT words per thread at stride NT (coalesced).  meta[g] = {op | k << 8 |
-// nbits << 16, in_begin, in_count, neg_count}; gate_tally[g] = {offset, count}
-// into tally_list.  Each block adds its popcount once per tally entry.
-template <int NT, int WPT>
-__global__ void __launch_bounds__(NT) k_stage_gates(const uint4 *__restrict__ meta, const uint32_t *__restrict__ inputs,
-                                                     const uint32_t *__restrict__ layer_gates, uint32_t n_layer,
-                                                     uint32_t n_be, uint64_t W, uint64_t *__restrict__ buf,
-                                                     const uint2 *__restrict__ gate_tally,
-                                                     const uint32_t *__restrict__ tally_list,
-                                                     unsigned long long *__restrict__ ones) {
-    constexpr uint32_t kMaxIn = 8;  // inputs loaded up front (memory-level parallelism)
-    __shared__ uint32_t warp_sums[NT / 32];
-    const uint32_t li = blockIdx.y + gridDim.y * blockIdx.z;
-    if (li >= n_layer) return;
-    const uint32_t gi = layer_gates[li];
-    const uint4 m = meta[gi];
-    const uint32_t op = m.x & 0xFFu;
-    const uint32_t kk = (m.x >> 8) & 0xFFu;
-    const uint32_t nbits = (m.x >> 16) & 0xFu;
-    const uint32_t n = m.z;
-    const uint32_t off = n - m.w;
-    const uint32_t *in = inputs + m.y;
-    uint64_t *out = buf + (uint64_t)(n_be + gi) * W;
-    const uint64_t base = (uint64_t)blockIdx.x * NT * WPT + threadIdx.x;
-    uint64_t r[WPT];
-    if (n <= kMaxIn) {
-        uint64_t v[kMaxIn][WPT];
+// Phase B: every layer of gates in one launch.  A block takes 32 * WPL words
+// (lane = WPL neighbouring words, one load each of a row) of one part
+// (gate_plan.hpp); its warps share out the gates of a layer, and a block
+// barrier ends the layer.  A block's gates read rows that the block or phase A
+// wrote, so no layer waits for the whole chip, and a pass of few words has no
+// launch per layer.  Bound by memory (5.4 TB/s of rows read and written) where
+// it runs alone on many words, by the latency of a gate's rows on few; under
+// the sampling of the next chunk it costs the issue slots of 166 instructions
+// per gate and 64 words.  32,768 words of the 5,000-event tree (20 layers):
+// 0.65 ms, 0.96 with a launch per layer.
+constexpr int kGateThreadsMost = 1024;
+struct StageGateArgs {
+    const uint4 *gates;
+    const uint32_t *in;
+    const uint2 *tally;
+    const uint32_t *tally_list;
+    const uint32_t *part;
+    const uint2 *layer;
+    uint64_t words, stride;  // per row: words in use, words from row to row
+    uint64_t *buf;
+    unsigned long long *ones;
+};
+
+// WPL words of a row, in 32-bit halves.
+template <int WPL>
+struct GateRow {
+    uint32_t w[2 * WPL];
+};
+
+template <int WPL>
+__device__ __forceinline__ GateRow<WPL> gate_load(const char *col, uint32_t stride, uint32_t rec) {
+    const char *p = col + (uint64_t)(rec & ~kGateFlip) * stride;
+    GateRow<WPL> r;
+    if constexpr (WPL == 2) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(p);
+        r.w[0] = v.x, r.w[1] = v.y, r.w[2] = v.z, r.w[3] = v.w;
+    } else {
+        const uint2 v = *reinterpret_cast<const uint2 *>(p);
+        r.w[0] = v.x, r.w[1] = v.y;
+    }
+    return r;
+}
+
+// Calls f(half, value) for every input of a gate, U loads in flight.  The
+// records behind the last input repeat it: their value is the input's again
+// (PAD: 0).
+template <int WPL, int U, bool PAD, class F>
+__device__ __forceinline__ void gate_inputs(const char *col, uint32_t stride, uint32_t n, uint4 q, const uint4 *more,
+                                            F f) {
+#pragma unroll 1
+    for (uint32_t j = 0; j < n;) {
+        const uint32_t rec[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (uint32_t i = 0; i < kMaxIn; ++i) {
-            if (i < n) {
-                const uint64_t *row = buf + (uint64_t)in[i] * W;
+        for (uint32_t u0 = 0; u0 < 4; u0 += U) {
+            if (U < 4 && u0 && j + u0 >= n) break;
+            GateRow<WPL> x[U];
 #pragma unroll
-                for (int k = 0; k < WPT; ++k) {
-                    const uint64_t w = base + (uint64_t)k * NT;
-                    v[i][k] = (w < W) ? row[w] : 0ull;
-                }
+            for (uint32_t u = 0; u < U; ++u) x[u] = gate_load<WPL>(col, stride, rec[u0 + u]);
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t flip = (uint32_t)((int32_t)rec[u0 + u] >> 31);
+                const uint32_t keep = j + u0 + u < n ? 0xFFFFFFFFu : 0u;
+#pragma unroll
+                for (int h = 0; h < 2 * WPL; ++h) f(h, PAD ? (x[u].w[h] ^ flip) & keep : x[u].w[h] ^ flip);
             }
         }
+        j += 4;
+        if (j < n) q = *more++;
+    }
+}
+
+// A gate's words: m and q are its two records.
+template <int WPL>
+__device__ __forceinline__ GateRow<WPL> gate_words(const char *col, uint32_t stride, const uint4 &m, const uint4 &q,
+                                                   const uint32_t *in) {
+    constexpr int H = 2 * WPL;
+    GateRow<WPL> r;
 #pragma unroll
-        for (int k = 0; k < WPT; ++k) {
-            if (op == MCG_ATLEAST) {
-                SlicedCount cnt;
-                cnt.clear();
+    for (int h = 0; h < H; ++h) r.w[h] = 0;
+    const uint32_t kind = m.x & 3u, kk = (m.x >> 8) & 0xFFu;
+    const uint4 *more = reinterpret_cast<const uint4 *>(in + m.y);
+    if (kind == kGateOr && m.z == 2) {
+        const GateRow<WPL> x = gate_load<WPL>(col, stride, q.x), y = gate_load<WPL>(col, stride, q.y);
+        const uint32_t fx = (uint32_t)((int32_t)q.x >> 31), fy = (uint32_t)((int32_t)q.y >> 31);
 #pragma unroll
-                for (uint32_t i = 0; i < kMaxIn; ++i)
-                    if (i < n) cnt.add(i >= off ? ~v[i][k] : v[i][k], nbits);
-                r[k] = cnt.ge(kk);
-            } else {
-                uint64_t a = (op == MCG_AND || op == MCG_NAND) ? kAllOnes : 0ull;
+        for (int h = 0; h < H; ++h) r.w[h] = (x.w[h] ^ fx) | (y.w[h] ^ fy);
+    } else if (kind == kGateOr) {
+        gate_inputs<WPL, 4, false>(col, stride, m.z, q, more, [&](int h, uint32_t v) { r.w[h] |= v; });
+    } else if (kind == kGateXor) {
+        gate_inputs<WPL, 4, true>(col, stride, m.z, q, more, [&](int h, uint32_t v) { r.w[h] ^= v; });
+    } else if (kind == kGateChain) {
+        // c[j]: at least j + 1 so far; r: at least kk
+        uint32_t c[3][H] = {};
+        const uint32_t two = kk == 2 ? 0xFFFFFFFFu : 0u, three = kk == 3 ? 0xFFFFFFFFu : 0u;
+        gate_inputs<WPL, 2, true>(col, stride, m.z, q, more, [&](int h, uint32_t v) {
+            const uint32_t below = (c[0][h] & two) | (c[1][h] & three) | (c[2][h] & ~(two | three));
+            r.w[h] |= below & v;
+            c[2][h] |= c[1][h] & v;
+            c[1][h] |= c[0][h] & v;
+            c[0][h] |= v;
+        });
+    } else {
+        // bit slices, a half at a time: few gates come here, and their
+        // counters then take no more registers than the rows of the others
+        const uint32_t nbits = (m.x >> 16) & 0xFu;
 #pragma unroll
-                for (uint32_t i = 0; i < kMaxIn; ++i) {
-                    if (i < n) {
-                        const uint64_t x = i >= off ? ~v[i][k] : v[i][k];
-                        if (op == MCG_OR || op == MCG_NOR) a |= x;
-                        else if (op == MCG_AND || op == MCG_NAND) a &= x;
-                        else if (op == MCG_XOR) a ^= x;
-                        else a = x;
+        for (int h = 0; h < H; ++h) {
+            uint32_t c[8] = {};
+#pragma unroll 1
+            for (uint32_t j = 0; j < m.z; ++j) {
+                const uint32_t rec = j == 0 ? q.x : j == 1 ? q.y : j == 2 ? q.z : j == 3 ? q.w : in[m.y + j - 4];
+                uint32_t v = reinterpret_cast<const uint32_t *>(col + (uint64_t)(rec & ~kGateFlip) * stride)[h] ^
+                             (uint32_t)((int32_t)rec >> 31);
+#pragma unroll
+                for (uint32_t b = 0; b < 8; ++b) {
+                    if (b < nbits) {
+                        const uint32_t s = c[b] & v;
+                        c[b] ^= v;
+                        v = s;
                     }
                 }
-                r[k] = (op == MCG_NAND || op == MCG_NOR || op == MCG_NOT) ? ~a : a;
             }
-        }
-    } else {
+            uint32_t gt = 0, eq = 0xFFFFFFFFu;
 #pragma unroll
-        for (int k = 0; k < WPT; ++k) {
-            const uint64_t w = base + (uint64_t)k * NT;
-            r[k] = 0;
-            if (w >= W) continue;
-            if (op == MCG_ATLEAST) {
-                SlicedCount cnt;
-                cnt.clear();
-                for (uint32_t i = 0; i < n; ++i) {
-                    const uint64_t x = buf[(uint64_t)in[i] * W + w];
-                    cnt.add(i >= off ? ~x : x, nbits);
+            for (int b = 7; b >= 0; --b) {
+                if ((kk >> b) & 1u) {
+                    eq &= c[b];
+                } else {
+                    gt |= eq & c[b];
+                    eq &= ~c[b];
                 }
-                r[k] = cnt.ge(kk);
-            } else {
-                uint64_t a = (op == MCG_AND || op == MCG_NAND) ? kAllOnes : 0ull;
-                for (uint32_t i = 0; i < n; ++i) {
-                    uint64_t x = buf[(uint64_t)in[i] * W + w];
-                    if (i >= off) x = ~x;
-                    if (op == MCG_OR || op == MCG_NOR) a |= x;
-                    else if (op == MCG_AND || op == MCG_NAND) a &= x;
-                    else if (op == MCG_XOR) a ^= x;
-                    else a = x;
-                }
-                r[k] = (op == MCG_NAND || op == MCG_NOR || op == MCG_NOT) ? ~a : a;
             }
+            r.w[h] = gt | eq;
         }
     }
-    uint32_t count = 0;
+    const uint32_t inverted = (m.x & 4u) ? 0xFFFFFFFFu : 0u;
 #pragma unroll
-    for (int k = 0; k < WPT; ++k) {
-        const uint64_t w = base + (uint64_t)k * NT;
-        if (w < W) {
-            out[w] = r[k];
-            count += (uint32_t)__popcll(r[k]);
+    for (int h = 0; h < H; ++h) r.w[h] ^= inverted;
+    return r;
+}
+
+template <int WPL>
+__global__ void __launch_bounds__(kGateThreadsMost) k_stage_gates(const __grid_constant__ StageGateArgs a) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t warps = blockDim.x >> 5;
+    const uint32_t stride = (uint32_t)(a.stride * sizeof(uint64_t));
+    const uint32_t l_begin = a.part[blockIdx.y], l_end = a.part[blockIdx.y + 1];
+    if (l_begin == l_end) return;
+    const uint32_t tiles = (uint32_t)((a.words + 32 * WPL - 1) / (32 * WPL));
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint64_t w0 = ((uint64_t)tile * 32u + lane) * WPL;
+        const bool valid = w0 < a.words, both = w0 + (WPL - 1) < a.words;
+        const bool whole = ((uint64_t)tile + 1) * (32 * WPL) <= a.words;
+        // lanes behind the end read the row's first words and store nothing
+        char *col = reinterpret_cast<char *>(a.buf + (valid ? w0 : 0));
+        uint32_t l = l_begin;
+        uint2 range = a.layer[l];
+        uint32_t i = range.x + warp;
+        uint4 m{}, q{};
+        auto head = [&](uint32_t g) {
+            m = a.gates[2 * (uint64_t)g];
+            q = a.gates[2 * (uint64_t)g + 1];
+        };
+        if (i < range.y) head(i);
+        for (;;) {
+            // the warp's next gate, in this layer or the next: its records are
+            // loaded under this gate's rows
+            const bool mine = i < range.y, last = i + warps >= range.y;
+            const uint4 cm = m, cq = q;
+            const uint32_t gate = i;
+            i += warps;
+            if (last && ++l < l_end) {
+                range = a.layer[l];
+                i = range.x + warp;
+            }
+            if (i < range.y) head(i);
+            if (mine) {
+                const uint2 t = a.tally[gate];
+                const GateRow<WPL> r = gate_words<WPL>(col, stride, cm, cq, a.in);
+                char *out = col + (uint64_t)cm.w * stride;
+                if (valid) {
+                    if constexpr (WPL == 2)
+                        *reinterpret_cast<uint4 *>(out) = make_uint4(r.w[0], r.w[1], r.w[2], r.w[3]);
+                    else
+                        *reinterpret_cast<uint2 *>(out) = make_uint2(r.w[0], r.w[1]);
+                }
+                if (t.y) {
+                    uint32_t n = __popc(r.w[0]) + __popc(r.w[1]), n2 = 0;
+                    if constexpr (WPL == 2) n2 = __popc(r.w[2]) + __popc(r.w[3]);
+                    n = whole ? n + n2 : (valid ? n : 0u) + (both ? n2 : 0u);
+                    n = __reduce_add_sync(0xFFFFFFFFu, n);
+                    if (lane == 0 && n) {
+                        if (t.y == 1) atomicAdd(&a.ones[t.x], (unsigned long long)n);
+                        else
+                            for (uint32_t j = 0; j < t.y; ++j)
+                                atomicAdd(&a.ones[a.tally_list[t.x + j]], (unsigned long long)n);
+                    }
+                }
+            }
+            if (last) {
+                __syncthreads();
+                if (l == l_end) break;
+            }
         }
-    }
-    const uint2 t = gate_tally[gi];
-    if (t.y == 0) return;  // uniform per block
-    count = __reduce_add_sync(0xFFFFFFFFu, count);
-    if ((threadIdx.x & 31u) == 0) warp_sums[threadIdx.x >> 5] = count;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long s = 0;
-        for (uint32_t i = 0; i < NT / 32; ++i) s += warp_sums[i];
-        if (s)
-            for (uint32_t j = 0; j < t.y; ++j) atomicAdd(&ones[tally_list[t.x + j]], s);
     }
 }
 
