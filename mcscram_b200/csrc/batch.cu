@@ -159,17 +159,20 @@ constexpr uint64_t kTileScratchMost = 16ull << 30;
 mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
     using namespace mcg::dev;
     std::vector<uint4> gates;
-    std::vector<uint32_t> in, layer, event_node, event_off;
-    std::vector<uint2> event, be_tally;
+    std::vector<uint32_t> in, layer, event_node, event_off, event_slot;
+    std::vector<uint2> event, be_tally, segment;
     uint64_t most_slots = 0;
     for (const auto &g : b->trees) {
-        const mcg::TilePlan t = mcg::plan_tile(g);
+        const mcg::SegmentPlan plan = mcg::plan_segments(g);
+        const mcg::TilePlan &t = plan.tile;
         if (!t.fits || in.size() + t.in.size() > 0xFFFFFFFFull) return MCG_OK;
-        most_slots = std::max<uint64_t>(most_slots, t.slots() + 1ull);
+        most_slots = std::max<uint64_t>(most_slots, plan.slots + 1ull);
         if (most_slots * kTileRow > 0xFFFFFFFFull) return MCG_OK;
         BatchTileTree x{};
         x.n_be = (uint32_t)t.event.size();
-        x.n_layers = (uint32_t)t.layer.size() - 1;
+        x.n_segments = (uint32_t)plan.segment.size();
+        x.seg_off = (uint32_t)segment.size();
+        x.event_off = (uint32_t)event_slot.size();
         x.gate_off = (uint32_t)gates.size();
         x.layer_off = (uint32_t)layer.size();
         x.in_off = (uint32_t)in.size();
@@ -180,6 +183,9 @@ mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
         }
         x.n_be_tally = (uint32_t)be_tally.size() - x.be_tally_off;
         gates.insert(gates.end(), t.gates.begin(), t.gates.end());
+        for (size_t i = 0; i < t.gates.size(); ++i) gates[x.gate_off + i].w = plan.gate_slot[i] + 1u;
+        for (uint32_t v : plan.event_slot) event_slot.push_back(v + 1u);
+        segment.insert(segment.end(), plan.segment.begin(), plan.segment.end());
         layer.insert(layer.end(), t.layer.begin(), t.layer.end());
         for (uint32_t rec : t.in) in.push_back(mcg::TilePlan::byte_record(rec, kTileRow, 1, 0));
         event_off.push_back((uint32_t)event.size());
@@ -204,7 +210,8 @@ mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
     mcg_status st;
     if ((st = upload_table(b, &a.trees, b->tile_trees)) != MCG_OK || (st = upload_table(b, &a.gates, gates)) != MCG_OK ||
         (st = upload_table(b, &a.in, in)) != MCG_OK || (st = upload_table(b, &a.layer, layer)) != MCG_OK ||
-        (st = upload_table(b, &a.be_tally, be_tally)) != MCG_OK || (st = upload_table(b, &b->d_event, event)) != MCG_OK ||
+        (st = upload_table(b, &a.be_tally, be_tally)) != MCG_OK || (st = upload_table(b, &a.segment, segment)) != MCG_OK ||
+        (st = upload_table(b, &a.event_slot, event_slot)) != MCG_OK || (st = upload_table(b, &b->d_event, event)) != MCG_OK ||
         (st = upload_table(b, &b->d_event_node, event_node)) != MCG_OK ||
         (st = upload_table(b, &b->d_event_off, event_off)) != MCG_OK)
         return st;

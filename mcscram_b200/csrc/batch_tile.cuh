@@ -18,13 +18,16 @@ namespace dev {
 // thresholds; only those (a few per lane: probabilities are small) are
 // compared with every instance's threshold.  Comparing all outputs with every
 // threshold cost the interpreter half of its time at four instances.
-// 512 threads, two blocks per SM: one block's gates, whose rows come from HBM
-// on large trees, run under the sampling of the other (37.5 ms for 16 trees of
-// 32 to 6,909 events, 16 draws, 16,384 words, where one block of 1,024 threads
-// took 48.2 ms and the interpreter 120).  Bound by those rows (177 GB in
-// 37.5 ms, 0.72 of the measured copy rate) on large trees, by the generator
-// and the compares on small ones (101 instances of the 200-event tree, 4,096
-// words: 0.72 ms, the interpreter 2.06).
+// 512 threads, two blocks per SM: one block's gates run under the sampling of
+// the other (16 trees of 32 to 6,909 events, 16 draws, 16,384 words: 37.5 ms
+// where one block of 1,024 threads took 48.2 and the interpreter 120).  A tree
+// is taken in segments of about 96 events and their gates, and rows are used
+// again (plan_segments): 107 GB of rows to and from memory in that run and not
+// 177; segments of 64, 192 and 384 events are 0.5 to 5 % slower.  Bound by the
+// issue of the generator's and the compares' instructions (0.57 of the slots,
+// as the sampler alone): that run takes 35.4 ms, 101 instances of the
+// 200-event tree on 4,096 words 0.66 ms (0.73 before the segments and the
+// compares' adds; the interpreter 2.06).
 
 // Thread (event of a group): its record from the instances' tables.
 static __global__ void __launch_bounds__(256) k_batch_records(const BatchTileGroup *__restrict__ groups,
@@ -55,9 +58,10 @@ static __global__ void __launch_bounds__(256) k_batch_records(const BatchTileGro
     }
 }
 
-// acc[k] |= bit where v < t[k].
-__device__ __forceinline__ void or_if_below(uint32_t &acc, uint32_t v, uint32_t t, uint32_t bit) {
-    asm("{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %1, %2;\n\t@p or.b32 %0, %0, %3;\n\t}" : "+r"(acc) : "r"(v), "r"(t), "r"(bit));
+// acc gets the bit, which it does not hold yet, where v < t.  An add and not
+// an or: adds take half the issue time of logic operations.
+__device__ __forceinline__ void add_if_below(uint32_t &acc, uint32_t v, uint32_t t, uint32_t bit) {
+    asm("{\n\t.reg .pred p;\n\tsetp.lt.u32 p, %1, %2;\n\t@p add.u32 %0, %0, %3;\n\t}" : "+r"(acc) : "r"(v), "r"(t), "r"(bit));
 }
 
 // The marked outputs of a lane against the first KG thresholds of the record;
@@ -84,7 +88,7 @@ __device__ __forceinline__ void batch_compare(const uint4 *__restrict__ rec, uin
         marked ^= bit;
         const uint32_t v = out[((b & 28u) << 5) + (b & 3u)];
 #pragma unroll
-        for (int k = 0; k < KG; ++k) or_if_below(acc[k], v, t[k], bit);
+        for (int k = 0; k < KG; ++k) add_if_below(acc[k], v, t[k], bit);
     }
     if (all) {
 #pragma unroll
@@ -163,37 +167,6 @@ static __global__ void __launch_bounds__(kBatchTileThreads, kBatchTileBlocks) k_
         const BatchTileTree t = a.trees[g.tree];
         const uint64_t w0 = (item % a.tiles) * kTileLanes;
         const WordCtx ctx = make_word_ctx((uint32_t)(w0 + lane));
-#pragma unroll 1
-        for (uint32_t u = warp; u < 2 * t.n_be; u += kWarps) {
-            const uint32_t half = u & 1u;
-            const uint4 *rec = a.recs + (g.rec_off + (u >> 1)) * kTileRec;
-            const uint4 r = rec[4];
-            uint32_t marked = 0;
-            __syncwarp();  // the last pair's entries and outputs have been read
-            if (r.x) {
-                if (lane < 9) event_table_entry(r.z, t3, lane < 8 ? (int)(8 * half + lane) : 16, s_tab[warp][lane]);
-                __syncwarp();
-                uint32_t ge = 0;
-                half_word_outputs(
-                    r.w, ctx, s_tab[warp][8].x, [&](int c) { return s_tab[warp][c]; },
-                    [&](int c, uint32_t o0, uint32_t o1, uint32_t o2, uint32_t o3) {
-                        out[c * 32] = make_uint4(o0, o1, o2, o3);
-                        ge = shift_in_ge(ge, o3, r.x);
-                        ge = shift_in_ge(ge, o2, r.x);
-                        ge = shift_in_ge(ge, o1, r.x);
-                        ge = shift_in_ge(ge, o0, r.x);
-                    });
-                // call c is at nibble 7 - c: reverse the nibbles, and "below" is not ">="
-                ge = ((ge & 0x0F0F0F0Fu) << 4) | ((ge >> 4) & 0x0F0F0F0Fu);
-                marked = ~__byte_perm(ge, 0, 0x0123);
-            }
-            uint32_t *row = reinterpret_cast<uint32_t *>(rows + (uint64_t)((u >> 1) + 1) * kTileRow) + half * 32u + lane;
-            const uint32_t *mine = reinterpret_cast<const uint32_t *>(out);
-            if (g.size > 8) batch_compare<16>(rec, r.y, marked, mine, g.size, row);
-            else if (g.size > 4) batch_compare<8>(rec, r.y, marked, mine, g.size, row);
-            else batch_compare<4>(rec, r.y, marked, mine, g.size, row);
-        }
-        __syncthreads();
         // a lane's 16 bytes of a row: words (4 * lane) % 32 .. + 3 of one half of instance lane / 16
         const uint32_t wl = (4u * lane) & 31u;
         const uint32_t live = a.words - w0 > wl ? (uint32_t)min((unsigned long long)(a.words - w0 - wl), 4ull) : 0u;
@@ -206,63 +179,103 @@ static __global__ void __launch_bounds__(kBatchTileThreads, kBatchTileBlocks) k_
         };
         const uint32_t quads = (g.size + 3) / 4;
         unsigned char *lane_base = rows + lane * 16u;  // instance lane / 16, and + 512 bytes the two after it
+        // a warp's four instances of every gate it takes: from k on
+        const uint32_t quad_bits = quads > 2 ? 2u : quads - 1u, k = 4 * (warp & ((1u << quad_bits) - 1u));
+        unsigned char *src = lane_base + k * 256u;
+        const bool more = k + 2 < g.size;
+        uint32_t e_begin = 0, l_begin = 0;
+        for (uint32_t sg = 0; sg < t.n_segments; ++sg) {
+            const uint2 end = a.segment[t.seg_off + sg];
+#pragma unroll 1
+            for (uint32_t u = 2 * e_begin + warp; u < 2 * end.x; u += kWarps) {
+                const uint32_t half = u & 1u;
+                const uint4 *rec = a.recs + (g.rec_off + (u >> 1)) * kTileRec;
+                const uint4 r = rec[4];
+                uint32_t marked = 0;
+                __syncwarp();  // the last pair's entries and outputs have been read
+                if (r.x) {
+                    if (lane < 9) event_table_entry(r.z, t3, lane < 8 ? (int)(8 * half + lane) : 16, s_tab[warp][lane]);
+                    __syncwarp();
+                    uint32_t ge = 0;
+                    half_word_outputs(
+                        r.w, ctx, s_tab[warp][8].x, [&](int c) { return s_tab[warp][c]; },
+                        [&](int c, uint32_t o0, uint32_t o1, uint32_t o2, uint32_t o3) {
+                            out[c * 32] = make_uint4(o0, o1, o2, o3);
+                            ge = shift_in_ge(ge, o3, r.x);
+                            ge = shift_in_ge(ge, o2, r.x);
+                            ge = shift_in_ge(ge, o1, r.x);
+                            ge = shift_in_ge(ge, o0, r.x);
+                        });
+                    // call c is at nibble 7 - c: reverse the nibbles, and "below" is not ">="
+                    ge = ((ge & 0x0F0F0F0Fu) << 4) | ((ge >> 4) & 0x0F0F0F0Fu);
+                    marked = ~__byte_perm(ge, 0, 0x0123);
+                }
+                unsigned char *event_row = rows + (uint64_t)a.event_slot[t.event_off + (u >> 1)] * kTileRow;
+                uint32_t *row = reinterpret_cast<uint32_t *>(event_row) + half * 32u + lane;
+                const uint32_t *mine = reinterpret_cast<const uint32_t *>(out);
+                if (g.size > 8) batch_compare<16>(rec, r.y, marked, mine, g.size, row);
+                else if (g.size > 4) batch_compare<8>(rec, r.y, marked, mine, g.size, row);
+                else batch_compare<4>(rec, r.y, marked, mine, g.size, row);
+            }
+            __syncthreads();
+            for (uint32_t l = l_begin; l < end.y; ++l) {
+                const uint32_t begin = a.layer[t.layer_off + l];
+                const uint32_t gates_end = k < g.size ? a.layer[t.layer_off + l + 1] : 0u;
+                for (uint32_t i = begin + (warp >> quad_bits); i < gates_end; i += kWarps >> quad_bits) {
+                    const uint4 m = a.gates[t.gate_off + i];
+                    const uint2 *in = reinterpret_cast<const uint2 *>(a.in + t.in_off + m.y);
+                    unsigned char *dst = src + (uint64_t)m.w * kTileRow;
+                    uint4 r0 = make_uint4(0u, 0u, 0u, 0u), r1 = r0;
+                    if ((m.x & 3u) == kTileOr) {
+                        // both pairs of instances at once: eight loads in flight
+                        if (more) {
+#pragma unroll 2
+                            for (uint32_t j = 0; j < m.z; ++j) {
+                                const uint2 s = in[j];
+                                const uint4 *p = reinterpret_cast<const uint4 *>(src + (s.x & ~1u));
+                                const uint4 *q = reinterpret_cast<const uint4 *>(src + (s.y & ~1u));
+                                const uint4 p0 = p[0], p1 = p[32], q0 = q[0], q1 = q[32];
+                                const uint32_t fp = 0u - (s.x & 1u), fq = 0u - (s.y & 1u);
+                                tile_or4(r0, p0, fp);
+                                tile_or4(r1, p1, fp);
+                                tile_or4(r0, q0, fq);
+                                tile_or4(r1, q1, fq);
+                            }
+                        } else {
+#pragma unroll 2
+                            for (uint32_t j = 0; j < m.z; ++j) {
+                                const uint2 s = in[j];
+                                tile_or4(r0, tile_in4(src, s.x), 0u);
+                                tile_or4(r0, tile_in4(src, s.y), 0u);
+                            }
+                        }
+                    } else {
+                        r0 = tile_gate4(m, in, src);
+                        if (more) r1 = tile_gate4(m, in, src + 512);
+                    }
+                    if (m.x & 4u) {
+                        r0 = make_uint4(~r0.x, ~r0.y, ~r0.z, ~r0.w);
+                        r1 = make_uint4(~r1.x, ~r1.y, ~r1.z, ~r1.w);
+                    }
+                    *reinterpret_cast<uint4 *>(dst) = r0;
+                    if (more) *reinterpret_cast<uint4 *>(dst + 512) = r1;
+                    const uint32_t nt = m.x >> 20;
+                    if (nt) {
+                        count(r0, k + lane / 16u, nt);
+                        if (more) count(r1, k + 2 + lane / 16u, nt);
+                    }
+                }
+                __syncthreads();
+            }
+            e_begin = end.x;
+            l_begin = end.y;
+        }
         for (uint32_t u = warp; u < t.n_be_tally * quads; u += kWarps) {
             const uint2 x = a.be_tally[t.be_tally_off + u / quads];
             const uint32_t k = 4 * (u % quads);
             for (uint32_t p = 0; p < 2 && k + 2 * p < g.size; ++p)
                 count(*reinterpret_cast<const uint4 *>(lane_base + (uint64_t)x.x * kTileRow + (k + 2 * p) * 256u),
                       k + 2 * p + lane / 16u, x.y);
-        }
-        for (uint32_t l = 0; l < t.n_layers; ++l) {
-            const uint32_t begin = a.layer[t.layer_off + l], n = a.layer[t.layer_off + l + 1] - begin;
-            for (uint32_t u = warp; u < n * quads; u += kWarps) {
-                const uint32_t i = begin + u / quads, k = 4 * (u % quads);
-                const uint4 m = a.gates[t.gate_off + i];
-                const uint2 *in = reinterpret_cast<const uint2 *>(a.in + t.in_off + m.y);
-                unsigned char *dst = lane_base + (uint64_t)(t.n_be + 1 + i) * kTileRow + k * 256u;
-                const unsigned char *src = lane_base + k * 256u;
-                const bool more = k + 2 < g.size;
-                uint4 r0 = make_uint4(0u, 0u, 0u, 0u), r1 = r0;
-                if ((m.x & 3u) == kTileOr) {
-                    // both pairs of instances at once: eight loads in flight
-                    if (more) {
-#pragma unroll 2
-                        for (uint32_t j = 0; j < m.z; ++j) {
-                            const uint2 s = in[j];
-                            const uint4 *p = reinterpret_cast<const uint4 *>(src + (s.x & ~1u));
-                            const uint4 *q = reinterpret_cast<const uint4 *>(src + (s.y & ~1u));
-                            const uint4 p0 = p[0], p1 = p[32], q0 = q[0], q1 = q[32];
-                            const uint32_t fp = 0u - (s.x & 1u), fq = 0u - (s.y & 1u);
-                            tile_or4(r0, p0, fp);
-                            tile_or4(r1, p1, fp);
-                            tile_or4(r0, q0, fq);
-                            tile_or4(r1, q1, fq);
-                        }
-                    } else {
-#pragma unroll 2
-                        for (uint32_t j = 0; j < m.z; ++j) {
-                            const uint2 s = in[j];
-                            tile_or4(r0, tile_in4(src, s.x), 0u);
-                            tile_or4(r0, tile_in4(src, s.y), 0u);
-                        }
-                    }
-                } else {
-                    r0 = tile_gate4(m, in, src);
-                    if (more) r1 = tile_gate4(m, in, src + 512);
-                }
-                if (m.x & 4u) {
-                    r0 = make_uint4(~r0.x, ~r0.y, ~r0.z, ~r0.w);
-                    r1 = make_uint4(~r1.x, ~r1.y, ~r1.z, ~r1.w);
-                }
-                *reinterpret_cast<uint4 *>(dst) = r0;
-                if (more) *reinterpret_cast<uint4 *>(dst + 512) = r1;
-                const uint32_t nt = m.x >> 20;
-                if (nt) {
-                    count(r0, k + lane / 16u, nt);
-                    if (more) count(r1, k + 2 + lane / 16u, nt);
-                }
-            }
-            __syncthreads();
         }
     }
 }

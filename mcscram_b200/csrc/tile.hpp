@@ -27,8 +27,8 @@ constexpr uint32_t kTileOr = 0, kTileXor = 1, kTileAtleast = 2;  // gate kinds (
 
 // Batched instances in tiles (k_batch_tile): tables of all trees, concatenated.
 struct BatchTileTree {
-    uint32_t n_be, n_layers, n_be_tally;
-    uint32_t gate_off, layer_off, in_off, be_tally_off;
+    uint32_t n_be, n_segments, n_be_tally;
+    uint32_t gate_off, layer_off, in_off, be_tally_off, seg_off, event_off;
 };
 
 // Up to kTileInstances instances of one tree that follow each other.
@@ -49,8 +49,10 @@ struct BatchTileArgs {
     const BatchTileTree *trees;
     const BatchTileGroup *groups;
     const uint4 *recs;
-    const uint4 *gates;            // as TileArgs; slots start at 1, row 0 is the empty input
+    const uint4 *gates;            // as TileArgs but for the last field, the gate's slot; row 0 is the empty input
     const uint32_t *in, *layer;
+    const uint2 *segment;          // {events' end, layers' end}
+    const uint32_t *event_slot;
     const uint2 *be_tally;         // tallied events {slot, tallies}
     uint64_t tiles, words;         // per instance
     uint64_t items;

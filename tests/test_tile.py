@@ -104,3 +104,36 @@ def test_batched_instances_in_tiles(oracle_mod, gpu, draws, words):
     for i, o in zip(runs, got):
         g = trees[inst_tree[i]].with_thresholds(thr[i])
         assert int(o) == int(np.sum(oracle_mod.tallies(g, 5, 1, 0, words))), (i, inst_tree[i])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_be,n_gates,tallies", [(95, 60, "root"), (96, 60, "all"), (700, 420, "root"),
+                                                  (700, 420, "some"), (1200, 700, "all"), (250, 0, "all")])
+def test_batched_trees_in_segments(oracle_mod, gpu, n_be, n_gates, tallies):
+    """Trees of several segments, whose rows are used again: nodes read far from
+    where they are written, tallied events (their rows last), events no gate reads."""
+    from mcscram_b200.uncertainty import Batch
+    rng = np.random.default_rng(n_be + n_gates)
+    ops, ks, begin, count, neg, inputs = [], [], [], [], [], []
+    for j in range(n_gates):
+        op = int(rng.choice([AND, OR, ATLEAST, XOR, NOT, NAND, NOR, NULL]))
+        n = 1 if op in (NOT, NULL) else int(rng.integers(2, 7))
+        last = max(1, min(n_be, (j + 1) * n_be // n_gates))
+        pool = np.concatenate([rng.integers(0, last, n), n_be + rng.integers(max(0, j - 40), j, n)]) if j else \
+            rng.integers(0, last, n)
+        ops.append(op)
+        ks.append(int(rng.integers(1, n + 1)))
+        begin.append(len(inputs))
+        count.append(n)
+        neg.append(int(rng.integers(0, n + 1)))
+        inputs += [int(x) for x in rng.choice(pool, n)]
+    nodes = n_be + n_gates
+    tally = {"root": [nodes - 1], "all": np.arange(nodes), "some": rng.integers(0, nodes, 25)}[tallies]
+    g = G.FlatGraph(be_pdag_idx=np.arange(2, 2 + n_be), be_event_idx=rng.permutation(n_be),
+                    be_threshold=np.zeros(n_be, np.uint64), gate_op=ops, gate_k=ks, gate_in_begin=begin,
+                    gate_in_count=count, gate_neg_count=neg, inputs=inputs, tally_nodes=tally)
+    thr = [(10.0 ** rng.uniform(-3, 0, n_be) * 2.0**32).astype(np.uint64) for _ in range(6)]
+    with Batch([g]) as b:
+        got = b.run([0] * len(thr), thr, iteration=2, words_per_instance=70)
+    for t, o in zip(thr, got):
+        assert int(o) == int(np.sum(oracle_mod.tallies(g.with_thresholds(t), 2, 1, 0, 70)))
