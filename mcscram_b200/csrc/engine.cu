@@ -751,27 +751,45 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
     return MCG_OK;
 }
 
-mcg_status run_staged_impl(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {
-    // fork from the engine stream so the chunks follow earlier work on it
+// Forks the staged streams from the engine stream, so that the chunks follow
+// earlier work on it.
+mcg_status staged_fork(mcg_engine *e) {
     MCG_CUDA(cudaEventRecord(e->ev_fork, e->stream));
     MCG_CUDA(cudaStreamWaitEvent(e->s_a, e->ev_fork, 0));
     MCG_CUDA(cudaStreamWaitEvent(e->s_b, e->ev_fork, 0));
-    uint64_t k = 0;
+    return MCG_OK;
+}
+
+// Chunks of n_it passes; *chunk counts them from the fork on (0 there), since
+// a buffer waits for the gates of the chunk before last.  `more`: chunks of
+// another call follow before the join.
+mcg_status staged_chunks(mcg_engine *e, uint64_t *chunk, uint32_t it_first, uint32_t n_it, uint64_t word_begin,
+                         uint64_t count, bool more) {
     for (uint32_t it = 0; it < n_it; ++it) {
-        for (uint64_t off = 0; off < count; ++k) {
+        for (uint64_t off = 0; off < count; ++*chunk) {
             const uint64_t n = std::min<uint64_t>(e->stage_words, count - off);
-            const mcg_status st = staged_chunk(e, k, it_first + it, word_begin + off, n,
-                                               it + 1 == n_it && off + n == count);
+            const mcg_status st = staged_chunk(e, *chunk, it_first + it, word_begin + off, n,
+                                               !more && it + 1 == n_it && off + n == count);
             if (st != MCG_OK) return st;
             off += n;
         }
     }
-    // join back into the engine stream
+    return MCG_OK;
+}
+
+mcg_status staged_join(mcg_engine *e) {
     MCG_CUDA(cudaEventRecord(e->ev_join_a, e->s_a));
     MCG_CUDA(cudaEventRecord(e->ev_join_b, e->s_b));
     MCG_CUDA(cudaStreamWaitEvent(e->stream, e->ev_join_a, 0));
     MCG_CUDA(cudaStreamWaitEvent(e->stream, e->ev_join_b, 0));
     return MCG_OK;
+}
+
+mcg_status run_staged_impl(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {
+    uint64_t chunk = 0;
+    mcg_status st = staged_fork(e);
+    if (st == MCG_OK) st = staged_chunks(e, &chunk, it_first, n_it, word_begin, count, false);
+    return st == MCG_OK ? staged_join(e) : st;
 }
 
 mcg_status launch_fused(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {
@@ -848,6 +866,12 @@ namespace internal {
 mcg_status run_staged(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {
     return run_staged_impl(e, it_first, n_it, word_begin, count);
 }
+mcg_status fork_staged(mcg_engine *e) { return staged_fork(e); }
+mcg_status add_staged(mcg_engine *e, uint64_t *chunk, uint32_t iteration, uint64_t word_begin, uint64_t count,
+                      bool more) {
+    return staged_chunks(e, chunk, iteration, 1, word_begin, count, more);
+}
+mcg_status join_staged(mcg_engine *e) { return staged_join(e); }
 }  // namespace internal
 }  // namespace mcg
 

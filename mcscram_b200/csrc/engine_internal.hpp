@@ -126,5 +126,13 @@ mcg_status create_with_extra(const mcg_graph_desc *graph, const mcg_run_desc *ru
 // Staged pass over [word_begin, word_begin + count) for n_it passes (engine.cu).
 mcg_status run_staged(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count);
 
+// The same in parts: several word ranges, each with its own hooks and event
+// table, whose sampling runs under the gates and hooks of the range before.
+// *chunk is 0 at the fork; `more`: another range follows before the join.
+mcg_status fork_staged(mcg_engine *e);
+mcg_status add_staged(mcg_engine *e, uint64_t *chunk, uint32_t iteration, uint64_t word_begin, uint64_t count,
+                      bool more);
+mcg_status join_staged(mcg_engine *e);
+
 }  // namespace internal
 }  // namespace mcg

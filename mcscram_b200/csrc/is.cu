@@ -1709,8 +1709,15 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
         return MCG_OK;
     };
     MCG_CUDA(cudaEventRecord(b->ev0, e->stream));
-    // component c draws the next comp_words[c] words with its own sampler table
-    uint64_t off = 0;
+    // component c draws the next comp_words[c] words with its own sampler
+    // table; it is sampled (and forced) under the gates and weights of the
+    // component before it, which wait for memory for most of their time
+    // (16 trees, 2,048 words, two components: 6.82 -> 6.45 ms)
+    uint64_t off = 0, chunk = 0;
+    uint32_t last_comp = 0;
+    for (uint32_t c = 0; c < nc; ++c)
+        if (comp_words[c]) last_comp = c;
+    st = mcg::internal::fork_staged(e);
     for (uint32_t c = 0; c < nc && st == MCG_OK; ++c) {
         if (!comp_words[c]) continue;
         e->d_be_sample = b->d_be_q + c * nb;
@@ -1751,10 +1758,11 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
                 return MCG_OK;
             };
         }
-        st = mcg::internal::run_staged(e, iteration, 1, word_begin + off, comp_words[c]);
+        st = mcg::internal::add_staged(e, &chunk, iteration, word_begin + off, comp_words[c], c != last_comp);
         e->sample_hook = nullptr;
         off += comp_words[c];
     }
+    if (st == MCG_OK) st = mcg::internal::join_staged(e);
     e->chunk_hook = nullptr;
     e->sample_hook = nullptr;
     e->d_be_sample = nullptr;
