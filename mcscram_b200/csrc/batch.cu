@@ -163,7 +163,7 @@ mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
     std::vector<uint2> event, be_tally, segment;
     uint64_t most_slots = 0;
     for (const auto &g : b->trees) {
-        const mcg::SegmentPlan plan = mcg::plan_segments(g);
+        const mcg::SegmentPlan plan = mcg::plan_segments(g, mcg::kSegmentEvents, true);
         const mcg::TilePlan &t = plan.tile;
         if (!t.fits || in.size() + t.in.size() > 0xFFFFFFFFull) return MCG_OK;
         most_slots = std::max<uint64_t>(most_slots, plan.slots + 1ull);

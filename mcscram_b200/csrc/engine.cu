@@ -147,82 +147,179 @@ extern "C" mcg_status mcg_trim_memory(int device) {
 
 namespace {
 
-// Strip mode's gate program: the gates of each layer in groups of up to
-// kStripGroup that the kernel evaluates together (no gate of a group reads
-// another, so all their input loads can be in flight at once).  AND, OR,
-// NAND and NOR gates of at most kStripGroupMaxIn inputs and one-input NOT and
-// NULL gates take the OR form r = outinv ^ OR_i (x_i ^ flip_i) (De Morgan:
-// AND = ~OR(~x), NAND = OR(~x)); flip_i also carries the input's negation.
-// Within a layer they are sorted by fan-in so a group's slots are mostly
-// full.  Every other gate (XOR, ATLEAST, NOT/NULL of other fan-in, wider
-// gates) is a group of one evaluated by strip_gate.  Each group is two
-// uint4 records: its header and the output nodes of its gates.
-mcg_status build_strip_groups(mcg_engine *e, const std::vector<uint32_t> &order,
-                              const std::vector<uint2> &gate_tally) {
+// Strip mode's program: segments of events and gates (plan_segments), the
+// gates of each in groups of up to kStripGroup that the kernel evaluates
+// together (no gate of a group reads another, so all their input loads can be
+// in flight at once).  AND, OR, NAND and NOR gates of at most
+// kStripGroupMaxIn inputs, one-of-n and n-of-n among them, and NOT and NULL
+// gates (of their last input) take the OR form r = outinv ^ OR_i (x_i ^
+// flip_i) (De Morgan: AND = ~OR(~x), NAND = OR(~x)); flip_i also carries the
+// input's negation.  A group is taken from the gates whose inputs are there,
+// four of one fan-in if there are so many, so that its slots are mostly full.
+// Every other gate (XOR, other ATLEAST, wider gates) is a group of one
+// evaluated by strip_gate.  Each group is two uint4 records: its header and
+// the output rows of its gates.
+//
+// 384 events per segment: the blocks of a launch start together, and where
+// all of them sampled all events and then evaluated all gates, the gates'
+// loads had little to hide under.  2^20 words of the 5,000-event tree: 190.8
+// ms; with one segment 197.7 (layer by layer 193.9), with 48 events per
+// segment, whose groups are less full, 197.1, with 96 to 768 190.7 to 191.
+constexpr uint32_t kStripSegmentEvents = 384;
+
+mcg_status build_strip_program(mcg_engine *e) {
     using mcg::dev::kStripGroup;
     using mcg::dev::kStripGroupMaxIn;
-    using mcg::dev::kStripNoInput;
     const mcg::Graph &g = e->graph;
-    if ((uint64_t)g.n_nodes() >= 0x7FFFFFFFull) return mcg::fail(MCG_ERR_INVALID, "strip mode: too many nodes");
-    std::vector<uint4> groups, ginfo;
-    std::vector<uint32_t> gin;
-    auto info = [&](uint32_t gi) { return make_uint4(g.n_be + gi, gate_tally[gi].x, gate_tally[gi].y, gi); };
-    auto or_form = [&](uint32_t gi) {
-        const uint8_t op = g.gate_op[gi];
-        const uint32_t n = g.gate_in_count[gi];
-        if (op == MCG_AND || op == MCG_OR || op == MCG_NAND || op == MCG_NOR) return n <= kStripGroupMaxIn;
-        return (op == MCG_NOT || op == MCG_NULL) && n == 1;
+    constexpr uint32_t kRowBytes = mcg::dev::kStripLanes * (uint32_t)sizeof(uint64_t);
+    const mcg::SegmentPlan plan = mcg::plan_segments(g, kStripSegmentEvents, false);
+    if ((uint64_t)plan.slots + 1 > 0xFFFFFFFFull / kRowBytes)
+        return mcg::fail(MCG_ERR_INVALID, "strip mode: too many nodes");
+    e->strip_rows = plan.slots + 1;
+    const uint32_t empty = plan.slots * kRowBytes;
+    const uint32_t nb = g.n_be;
+    std::vector<uint4> be, tab_be, groups, ginfo, single;
+    std::vector<uint2> segment, be_tally;
+    std::vector<uint32_t> gin, inputs, tally_list;
+    for (size_t i = 0; i < plan.tile.event.size(); ++i) {
+        const uint32_t v = plan.tile.event[i];
+        const uint4 r = make_uint4((uint32_t)g.be_pdag_idx[v] + 1u, g.be_event_idx[v] + 1u,
+                                   (uint32_t)g.be_threshold[v], (uint32_t)(g.be_threshold[v] >> 32));
+        tab_be.push_back(r);
+        be.push_back(make_uint4(plan.event_slot[i] * kRowBytes, r.y, r.z, r.w));
+    }
+    for (const uint2 &t : plan.tile.be_tally) be_tally.push_back(make_uint2(t.x * kRowBytes, t.y));
+    std::vector<std::vector<uint32_t>> tallies(g.n_gates);
+    for (uint32_t t = 0; t < (uint32_t)g.tally_nodes.size(); ++t)
+        if (g.tally_nodes[t] >= nb) tallies[g.tally_nodes[t] - nb].push_back(t);
+    // A row is used again by later segments, so the rows of a gate's inputs
+    // are those of its segment: kept per node as the segments go by.
+    std::vector<uint32_t> row(g.n_nodes(), 0);
+    std::vector<uint32_t> waiting(g.n_gates, 0);  // inputs of the gate that this segment still has to evaluate
+    std::vector<std::vector<uint32_t>> readers(g.n_gates);
+    std::vector<char> here(g.n_gates, 0);
+    auto last_only = [&](uint32_t i) { return g.gate_op[i] == MCG_NOT || g.gate_op[i] == MCG_NULL; };
+    auto first = [&](uint32_t i) { return last_only(i) && g.gate_in_count[i] ? g.gate_in_count[i] - 1 : 0u; };
+    auto fan_in = [&](uint32_t i) { return g.gate_in_count[i] - first(i); };
+    // 0: a group of its own, 1: OR form of the inputs, 2: of their complements
+    auto or_form = [&](uint32_t i) -> int {
+        const uint8_t op = g.gate_op[i];
+        const uint32_t n = g.gate_in_count[i], k = g.gate_k[i] & 0xFFu;
+        if (last_only(i)) return 1;
+        if (n > kStripGroupMaxIn) return 0;
+        if (op == MCG_OR || op == MCG_NOR || (op == MCG_ATLEAST && k == 1 && n >= 1)) return 1;
+        if (op == MCG_AND || op == MCG_NAND || (op == MCG_ATLEAST && k == n && n >= 1)) return 2;
+        return 0;
     };
-    std::vector<uint32_t> eligible;
-    for (size_t l = 0; l + 1 < e->layer_offsets.size(); ++l) {
-        eligible.clear();
-        for (uint32_t q = e->layer_offsets[l]; q < e->layer_offsets[l + 1]; ++q) {
-            const uint32_t gi = order[q];
-            if (or_form(gi)) {
-                eligible.push_back(gi);
-            } else {
-                groups.push_back(make_uint4(1u | (1u << 24), 0u, (uint32_t)ginfo.size(), 0u));
-                groups.push_back(make_uint4(g.n_be + gi, 0u, 0u, 0u));
-                ginfo.push_back(info(gi));
-            }
+    auto inverted = [&](uint32_t i) {  // of the OR form
+        const uint8_t op = g.gate_op[i];
+        return op == MCG_AND || op == MCG_NOR || op == MCG_NOT || (op == MCG_ATLEAST && or_form(i) == 2);
+    };
+    auto info = [&](uint32_t i, uint32_t own) {
+        ginfo.push_back(make_uint4(row[nb + i], (uint32_t)tally_list.size(), (uint32_t)tallies[i].size(), own));
+        tally_list.insert(tally_list.end(), tallies[i].begin(), tallies[i].end());
+    };
+    uint32_t ev = 0, layer = 0;
+    for (const uint2 &seg : plan.segment) {
+        for (; ev < seg.x; ++ev) row[plan.tile.event[ev]] = plan.event_slot[ev] * kRowBytes;
+        const uint32_t q0 = plan.tile.layer[layer], q1 = plan.tile.layer[seg.y];
+        layer = seg.y;
+        std::vector<uint32_t> ready[kStripGroupMaxIn + 1], own;  // by fan-in; groups of one
+        auto offer = [&](uint32_t i) { (or_form(i) ? ready[fan_in(i)] : own).push_back(i); };
+        for (uint32_t q = q0; q < q1; ++q) {
+            const uint32_t i = plan.gate[q];
+            here[i] = 1;
+            row[nb + i] = plan.gate_slot[q] * kRowBytes;
         }
-        std::stable_sort(eligible.begin(), eligible.end(),
-                         [&](uint32_t x, uint32_t y) { return g.gate_in_count[x] < g.gate_in_count[y]; });
-        for (size_t b = 0; b < eligible.size(); b += kStripGroup) {
-            const uint32_t cnt = (uint32_t)std::min<size_t>(kStripGroup, eligible.size() - b);
-            uint32_t maxn = 0, outinv = 0;
+        for (uint32_t q = q0; q < q1; ++q) {
+            const uint32_t i = plan.gate[q];
+            for (uint32_t j = first(i); j < g.gate_in_count[i]; ++j) {
+                const uint32_t c = g.inputs[g.gate_in_begin[i] + j];
+                if (c >= nb && here[c - nb]) {
+                    ++waiting[i];
+                    readers[c - nb].push_back(i);
+                }
+            }
+            if (!waiting[i]) offer(i);
+        }
+        auto done = [&](uint32_t i) {
+            for (uint32_t r : readers[i])
+                if (--waiting[r] == 0) offer(r);
+        };
+        for (uint32_t left = q1 - q0; left;) {
+            if (!own.empty()) {
+                const uint32_t i = own.back();
+                own.pop_back();
+                groups.push_back(make_uint4(1u | (1u << 24), 0u, (uint32_t)ginfo.size(), 0u));
+                groups.push_back(make_uint4(row[nb + i], 0u, 0u, 0u));
+                info(i, (uint32_t)single.size());
+                const uint32_t n = g.gate_in_count[i];
+                uint32_t nbits = 0;
+                while (nbits < 8 && (n >> nbits) != 0) ++nbits;
+                single.push_back(make_uint4((uint32_t)g.gate_op[i] | ((g.gate_k[i] & 0xFFu) << 8) |
+                                                (std::max(nbits, 1u) << 16),
+                                            (uint32_t)inputs.size(), n, g.gate_neg_count[i]));
+                for (uint32_t j = 0; j < n; ++j) inputs.push_back(row[g.inputs[g.gate_in_begin[i] + j]]);
+                done(i);
+                --left;
+                continue;
+            }
+            uint32_t most = 0;  // the fan-in of most ready gates
+            for (uint32_t f = 1; f <= kStripGroupMaxIn; ++f)
+                if (ready[f].size() > ready[most].size()) most = f;
+            std::vector<uint32_t> pick;
+            auto take = [&](std::vector<uint32_t> &from) {
+                while (pick.size() < kStripGroup && !from.empty()) {
+                    pick.push_back(from.back());
+                    from.pop_back();
+                }
+            };
+            if (ready[most].size() >= kStripGroup) take(ready[most]);
+            else
+                for (uint32_t f = kStripGroupMaxIn + 1; f-- > 0;) take(ready[f]);
+            const uint32_t cnt = (uint32_t)pick.size();
+            uint32_t maxn = 0, outinv = 0, outs[kStripGroup] = {0u, 0u, 0u, 0u};
             for (uint32_t j = 0; j < cnt; ++j) {
-                const uint32_t gi = eligible[b + j];
-                const uint8_t op = g.gate_op[gi];
-                maxn = std::max(maxn, g.gate_in_count[gi]);
-                if (op == MCG_AND || op == MCG_NOR || op == MCG_NOT) outinv |= 1u << j;
+                maxn = std::max(maxn, fan_in(pick[j]));
+                if (inverted(pick[j])) outinv |= 1u << j;
+                outs[j] = row[nb + pick[j]];
             }
             groups.push_back(make_uint4(cnt | (maxn << 8), (uint32_t)gin.size(), (uint32_t)ginfo.size(), outinv));
-            uint32_t outs[kStripGroup] = {0u, 0u, 0u, 0u};
-            for (uint32_t j = 0; j < cnt; ++j) outs[j] = g.n_be + eligible[b + j];
             groups.push_back(make_uint4(outs[0], outs[1], outs[2], outs[3]));
             for (uint32_t s = 0; s < maxn; ++s) {
                 for (uint32_t j = 0; j < kStripGroup; ++j) {
-                    uint32_t rec = kStripNoInput;
-                    if (j < cnt) {
-                        const uint32_t gi = eligible[b + j];
-                        const uint32_t n = g.gate_in_count[gi];
-                        if (s < n) {
-                            const bool negated = s >= n - g.gate_neg_count[gi];
-                            const bool and_type = g.gate_op[gi] == MCG_AND || g.gate_op[gi] == MCG_NAND;
-                            rec = (g.inputs[g.gate_in_begin[gi] + s] << 1) | (uint32_t)(negated != and_type);
-                        }
+                    uint32_t rec = empty;
+                    if (j < cnt && s < fan_in(pick[j])) {
+                        const uint32_t i = pick[j], at = first(i) + s, n = g.gate_in_count[i];
+                        const bool negated = at >= n - g.gate_neg_count[i];
+                        rec = row[g.inputs[g.gate_in_begin[i] + at]] | (uint32_t)(negated != (or_form(i) == 2));
                     }
                     gin.push_back(rec);
                 }
             }
-            for (uint32_t j = 0; j < cnt; ++j) ginfo.push_back(info(eligible[b + j]));
+            for (uint32_t i : pick) info(i, 0u);
+            for (uint32_t i : pick) done(i);
+            left -= cnt;
         }
+        for (uint32_t q = q0; q < q1; ++q) {
+            here[plan.gate[q]] = 0;
+            readers[plan.gate[q]].clear();
+        }
+        segment.push_back(make_uint2(ev, (uint32_t)groups.size() / 2));
     }
-    e->n_strip_groups = (uint32_t)(groups.size() / 2);
+    e->n_strip_be = (uint32_t)be.size();
+    e->n_strip_segments = (uint32_t)segment.size();
+    e->n_strip_be_tally = (uint32_t)be_tally.size();
+    MCG_CUDA(upload(&e->d_strip_be, be));
+    MCG_CUDA(upload(&e->d_strip_table_be, tab_be));
+    MCG_CUDA(upload(&e->d_strip_segment, segment));
+    MCG_CUDA(upload(&e->d_strip_single, single));
+    MCG_CUDA(upload(&e->d_strip_inputs, inputs));
     MCG_CUDA(upload(&e->d_strip_groups, groups));
     MCG_CUDA(upload(&e->d_strip_gin, gin));
     MCG_CUDA(upload(&e->d_strip_ginfo, ginfo));
+    MCG_CUDA(upload(&e->d_strip_be_tally, be_tally));
+    MCG_CUDA(upload(&e->d_gate_tally_list, tally_list));
     return MCG_OK;
 }
 
@@ -257,37 +354,17 @@ mcg_status build_layered_tables(mcg_engine *e) {
     std::vector<uint32_t> order(g.n_gates);
     for (uint32_t i = 0; i < g.n_gates; ++i) order[cursor[layer[i] - 1]++] = i;
 
-    std::vector<std::vector<uint32_t>> per_gate(g.n_gates);
     std::vector<uint32_t> be_nodes, be_idx;
     for (uint32_t t = 0; t < (uint32_t)g.tally_nodes.size(); ++t) {
-        const uint32_t v = g.tally_nodes[t];
-        if (v < g.n_be) {
-            be_nodes.push_back(v);
+        if (g.tally_nodes[t] < g.n_be) {
+            be_nodes.push_back(g.tally_nodes[t]);
             be_idx.push_back(t);
-        } else {
-            per_gate[v - g.n_be].push_back(t);
         }
-    }
-    std::vector<uint2> gate_tally(g.n_gates);
-    std::vector<uint32_t> gate_tally_list;
-    for (uint32_t i = 0; i < g.n_gates; ++i) {
-        gate_tally[i] = make_uint2((uint32_t)gate_tally_list.size(), (uint32_t)per_gate[i].size());
-        gate_tally_list.insert(gate_tally_list.end(), per_gate[i].begin(), per_gate[i].end());
     }
     e->n_be_tally = (uint32_t)be_nodes.size();
     if (e->mode == MCG_MODE_STRIP) {
-        mcg_status st = build_strip_groups(e, order, gate_tally);
+        mcg_status st = build_strip_program(e);
         if (st != MCG_OK) return st;
-        std::vector<uint4> smeta(g.n_gates);
-        for (uint32_t i = 0; i < g.n_gates; ++i) {
-            uint32_t nbits = 0;
-            while (nbits < 8 && (g.gate_in_count[i] >> nbits) != 0) ++nbits;
-            if (nbits == 0) nbits = 1;
-            smeta[i] = make_uint4((uint32_t)g.gate_op[i] | ((g.gate_k[i] & 0xFFu) << 8) | (nbits << 16),
-                                  g.gate_in_begin[i], g.gate_in_count[i], g.gate_neg_count[i]);
-        }
-        MCG_CUDA(upload(&e->d_smeta, smeta));
-        MCG_CUDA(upload(&e->d_gate_tally_list, gate_tally_list));
     } else if (e->mode == MCG_MODE_STAGED) {
         const mcg::GatePlan plan = mcg::plan_gates(g, layer);
         e->n_gate_parts = (uint32_t)plan.part.size() - 1;
@@ -596,7 +673,7 @@ mcg_status setup_strip(mcg_engine *e, const mcg_run_desc &run) {
     if (per_sm < 1) return mcg::fail(MCG_ERR_INVALID, "strip kernel does not fit on an SM");
     e->strip_grid = (uint32_t)(prop.multiProcessorCount * per_sm);
     const uint64_t warps = (uint64_t)e->strip_grid * (mcg::dev::kStripThreads / 32);
-    const uint64_t bytes = warps * std::max<uint64_t>(g.n_nodes(), 1) * mcg::dev::kStripLanes * sizeof(uint64_t);
+    const uint64_t bytes = warps * e->strip_rows * mcg::dev::kStripLanes * sizeof(uint64_t);
     MCG_CUDA(work_alloc(e, (void **)&e->d_strip_scratch, bytes));
     MCG_CUDA(cudaMalloc((void **)&e->d_queue, sizeof(unsigned long long)));
     MCG_CUDA(cudaMalloc((void **)&e->d_event_table,
@@ -608,20 +685,19 @@ mcg_status setup_strip(mcg_engine *e, const mcg_run_desc &run) {
 mcg_status run_strip(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {
     const mcg::Graph &g = e->graph;
     mcg::dev::StripArgs a{};
-    a.be = e->d_be;
+    a.be = e->d_strip_be;
     a.table = e->d_event_table;
-    a.n_be = g.n_be;
-    a.n_nodes = g.n_nodes();
-    a.smeta = e->d_smeta;
-    a.inputs = e->d_inputs;
+    a.segment = e->d_strip_segment;
+    a.n_segments = e->n_strip_segments;
+    a.rows = e->strip_rows;
+    a.single = e->d_strip_single;
+    a.inputs = e->d_strip_inputs;
     a.groups = e->d_strip_groups;
-    a.n_groups = e->n_strip_groups;
     a.gin = e->d_strip_gin;
     a.ginfo = e->d_strip_ginfo;
     a.tally_list = e->d_gate_tally_list;
-    a.be_tally_nodes = e->d_be_tally_nodes;
-    a.be_tally_idx = e->d_be_tally_idx;
-    a.n_be_tally = e->n_be_tally;
+    a.be_tally = e->d_strip_be_tally;
+    a.n_be_tally = e->n_strip_be_tally;
     a.n_tally = (uint32_t)g.tally_nodes.size();
     a.tally_in_smem = e->strip_smem ? 1u : 0u;
     a.ones = e->d_tally;
@@ -631,10 +707,10 @@ mcg_status run_strip(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t w
     a.queue = e->d_queue;
     for (uint32_t it = 0; it < n_it; ++it) {
         const uint32_t iteration = it_first + it;
-        if (g.n_be > 0 && e->table_iteration != iteration) {
-            const uint64_t n = (uint64_t)g.n_be * mcg::dev::kEventTableStride;
+        if (e->n_strip_be > 0 && e->table_iteration != iteration) {
+            const uint64_t n = (uint64_t)e->n_strip_be * mcg::dev::kEventTableStride;
             mcg::dev::k_event_table<<<(uint32_t)((n + 255) / 256), 256, 0, e->stream>>>(
-                e->d_be, g.n_be, (iteration + 1u) << 6, e->d_event_table);
+                e->d_strip_table_be, e->n_strip_be, (iteration + 1u) << 6, e->d_event_table);
             ++e->launches;
             e->table_iteration = iteration;
         }
@@ -831,7 +907,12 @@ void release(mcg_engine *e) {
     cudaFree(e->d_tally_nodes);
     cudaFree(e->d_layer_gates);
     cudaFree(e->d_buf);
-    cudaFree(e->d_smeta);
+    cudaFree(e->d_strip_be);
+    cudaFree(e->d_strip_table_be);
+    cudaFree(e->d_strip_segment);
+    cudaFree(e->d_strip_single);
+    cudaFree(e->d_strip_inputs);
+    cudaFree(e->d_strip_be_tally);
     cudaFree(e->d_gate_tally);
     cudaFree(e->d_gates);
     cudaFree(e->d_gate_in);

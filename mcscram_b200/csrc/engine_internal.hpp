@@ -90,13 +90,14 @@ struct mcg_engine {
     cudaEvent_t ev_fork = nullptr, ev_a[2] = {nullptr, nullptr}, ev_b[2] = {nullptr, nullptr};
     cudaEvent_t ev_join_a = nullptr, ev_join_b = nullptr;
     // strip
-    uint4 *d_smeta = nullptr;              // gate meta with counter bits for the bit-sliced ATLEAST
-    uint64_t *d_strip_scratch = nullptr;   // per warp n_nodes x 32 words
+    uint64_t *d_strip_scratch = nullptr;   // per warp strip_rows x 32 words
     unsigned long long *d_queue = nullptr; // strip counter
-    uint4 *d_strip_groups = nullptr;       // strip mode: gate groups, one layer at a time
-    uint32_t *d_strip_gin = nullptr;       // their inputs, slot-major, four records per slot
-    uint4 *d_strip_ginfo = nullptr;        // per grouped gate: output node, tally offset / count, gate id
-    uint32_t n_strip_groups = 0;
+    // its program (build_strip_program), as StripArgs has it
+    uint4 *d_strip_be = nullptr, *d_strip_table_be = nullptr;
+    uint2 *d_strip_segment = nullptr, *d_strip_be_tally = nullptr;
+    uint4 *d_strip_single = nullptr, *d_strip_groups = nullptr, *d_strip_ginfo = nullptr;
+    uint32_t *d_strip_inputs = nullptr, *d_strip_gin = nullptr;
+    uint32_t n_strip_be = 0, n_strip_segments = 0, n_strip_be_tally = 0, strip_rows = 1;
     uint32_t strip_grid = 0;
     uint32_t strip_smem = 0;               // tally counters in shared memory (0: global atomics)
     uint32_t strip_blocks = 6;             // resident blocks per SM the kernel is built for

@@ -776,36 +776,40 @@ __global__ void __launch_bounds__(kGateThreadsMost) k_stage_gates(const __grid_c
 
 // Strip mode: one persistent kernel per pass.  A block takes strips of 256
 // consecutive words from a queue; warp w owns words [32 w, 32 w + 32) of
-// the strip and a private scratch block of n_nodes rows x 32 words.  Lane l
-// first samples its word of every basic event (one Philox word per event,
-// event table of the pass), then evaluates every gate in layer order for the
-// same word, and adds the popcounts of tallied nodes into the block's
-// shared-memory counters.  A lane only reads the column it wrote, so the
-// only barrier is the strip hand-out: the eight warps of a block walk the
-// events together (the table rows they read stay in L1), while the blocks
-// on an SM drift apart, so the memory-bound gate work of some blocks runs
-// under the multiply-bound sampling of the others.
+// the strip and a private scratch block of rows of 32 words.  Lane l samples
+// its word of a segment's events (one Philox word per event, event table of
+// the pass), evaluates the segment's gates for the same word, adds the
+// popcounts of tallied nodes into the block's shared-memory counters, and goes
+// on to the next segment; rows are used again (build_strip_program).  A lane
+// only reads the column it wrote, so the only barrier is the strip hand-out:
+// the eight warps of a block walk the events together (the table rows they
+// read stay in L1), while the blocks on an SM drift apart, so the
+// memory-bound gate work of some blocks runs under the multiply-bound
+// sampling of the others.  Bound by the issue of the sampler's instructions
+// (711 per event and warp) and the gates' (46): 2^20 words of the 5,000-event
+// tree take 190.8 ms, where all events before all gates took 193.9.
 constexpr int kStripLanes = 32;
 constexpr int kStripThreads = 256;
 
 struct StripArgs {
-    const uint4 *be;              // {pdag + 1, event + 1, thr lo, thr hi}
-    const uint2 *table;           // event table of the pass
-    uint32_t n_be, n_nodes;
-    const uint4 *smeta;           // per gate: op | k << 8 | nbits << 16, in_begin, in_count, neg_count
-    const uint32_t *inputs;
+    const uint4 *be;              // in segment order: {row, event + 1, thr lo, thr hi}
+    const uint2 *table;           // event table of the pass, in the same order
+    const uint2 *segment;         // {events' end, groups' end}
+    uint32_t n_segments;
+    uint32_t rows;                // of a warp's scratch block; the last one holds zeros
+    const uint4 *single;          // gates of their own: op | k << 8 | nbits << 16, in_begin, in_count, neg_count
+    const uint32_t *inputs;       // their inputs: rows
     const uint4 *groups;          // per group two records: {count | fan-in << 8 | single << 24, gin offset,
-                                  // ginfo offset, outinv} and the output nodes of its gates
-    uint32_t n_groups;
-    const uint32_t *gin;          // group inputs, slot-major, kStripGroup records per slot: node << 1 | flip
-    const uint4 *ginfo;           // per grouped gate: {output node, tally offset, tally count, gate id}
+                                  // ginfo offset, outinv} and the output rows of its gates
+    const uint32_t *gin;          // group inputs, slot-major, kStripGroup records per slot: row | flip
+    const uint4 *ginfo;           // per grouped gate: {output row, tally offset, tally count, single gate}
     const uint32_t *tally_list;
-    const uint32_t *be_tally_nodes, *be_tally_idx;
+    const uint2 *be_tally;        // tallied events {row, tally index}
     uint32_t n_be_tally;
     uint32_t n_tally;
     uint32_t tally_in_smem;
     unsigned long long *ones;
-    uint64_t *scratch;            // per warp: n_nodes x 32 words
+    uint64_t *scratch;            // per warp: rows x 32 words
     uint64_t word_begin, word_count;
     unsigned long long *queue;
 };
@@ -816,21 +820,21 @@ __device__ __forceinline__ void strip_tally(const StripArgs &a, unsigned long lo
     else atomicAdd(&a.ones[idx], (unsigned long long)c);
 }
 
-// Gate groups of the strip kernel: up to kStripGroup gates of one layer
-// evaluated together in the OR form r = outinv ^ OR_i (x_i ^ flip_i); an
-// input record is node << 1 | flip, kStripNoInput an empty slot.
+// Gate groups of the strip kernel: up to kStripGroup gates that read none of
+// each other, evaluated together in the OR form
+// r = outinv ^ OR_i (x_i ^ flip_i).  A row is its byte offset in the warp's
+// scratch block; an input record is the row | flip, an empty slot the row of
+// zeros.
 constexpr uint32_t kStripGroup = 4;
 constexpr uint32_t kStripGroupMaxIn = 8;
-constexpr uint32_t kStripNoInput = 0xFFFFFFFFu;
 static_assert(kStripGroup == 4, "k_strip's group loop packs four gates' tallies into two reductions");
 
+__device__ __forceinline__ uint64_t &strip_row(const uint64_t *col, uint32_t row) {
+    return *reinterpret_cast<uint64_t *>(reinterpret_cast<unsigned char *>(const_cast<uint64_t *>(col)) + row);
+}
+
 __device__ __forceinline__ uint64_t strip_in(const uint64_t *col, uint32_t rec) {
-    uint64_t x = 0;
-    if (rec != kStripNoInput) {
-        x = col[(uint64_t)(rec >> 1) * kStripLanes];
-        if (rec & 1u) x = ~x;
-    }
-    return x;
+    return strip_row(col, rec & ~1u) ^ (uint64_t)(-(int64_t)(rec & 1u));
 }
 
 // Tally of one gate word column: warp sum of the valid lanes' popcounts,
@@ -850,7 +854,7 @@ __device__ __forceinline__ void strip_gate_tally(const StripArgs &a, unsigned lo
 // 36 bytes instead of 376 at 40 registers.
 static __device__ __noinline__ uint64_t strip_gate(const StripArgs &a, const uint64_t *col, uint32_t gi) {
     constexpr uint32_t kMaxIn = 8;
-    const uint4 m = a.smeta[gi];
+    const uint4 m = a.single[gi];
     const uint32_t op = m.x & 0xFFu, kk = (m.x >> 8) & 0xFFu, nbits = (m.x >> 16) & 0xFu;
     const uint32_t n = m.z, off = n - m.w;
     const uint32_t *in = a.inputs + m.y;
@@ -863,7 +867,7 @@ static __device__ __noinline__ uint64_t strip_gate(const StripArgs &a, const uin
                 uint64_t v[4];
 #pragma unroll
                 for (uint32_t j = 0; j < 4; ++j)
-                    if (i0 + j < n) v[j] = col[(uint64_t)in[i0 + j] * kStripLanes];
+                    if (i0 + j < n) v[j] = strip_row(col, in[i0 + j]);
 #pragma unroll
                 for (uint32_t j = 0; j < 4; ++j)
                     if (i0 + j < n) cnt.add(i0 + j >= off ? ~v[j] : v[j]);
@@ -873,7 +877,7 @@ static __device__ __noinline__ uint64_t strip_gate(const StripArgs &a, const uin
         SlicedCount cnt;
         cnt.clear();
         for (uint32_t i = 0; i < n; ++i) {
-            const uint64_t x = col[(uint64_t)in[i] * kStripLanes];
+            const uint64_t x = strip_row(col, in[i]);
             cnt.add(i >= off ? ~x : x, nbits);
         }
         return cnt.ge(kk);
@@ -885,7 +889,7 @@ static __device__ __noinline__ uint64_t strip_gate(const StripArgs &a, const uin
             uint64_t v[4];
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j)
-                if (i0 + j < n) v[j] = col[(uint64_t)in[i0 + j] * kStripLanes];
+                if (i0 + j < n) v[j] = strip_row(col, in[i0 + j]);
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) {
                 if (i0 + j < n) {
@@ -899,7 +903,7 @@ static __device__ __noinline__ uint64_t strip_gate(const StripArgs &a, const uin
         }
     } else {
         for (uint32_t i = 0; i < n; ++i) {
-            uint64_t x = col[(uint64_t)in[i] * kStripLanes];
+            uint64_t x = strip_row(col, in[i]);
             if (i >= off) x = ~x;
             if (op == MCG_OR || op == MCG_NOR) acc |= x;
             else if (op == MCG_AND || op == MCG_NAND) acc &= x;
@@ -918,7 +922,8 @@ __global__ void __launch_bounds__(kStripThreads, MINB) k_strip(StripArgs a) {
     if (a.tally_in_smem)
         for (uint32_t i = threadIdx.x; i < a.n_tally; i += blockDim.x) s_ones[i] = 0;
     const uint64_t gwarp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    uint64_t *col = a.scratch + gwarp * (uint64_t)a.n_nodes * kStripLanes + lane;
+    uint64_t *col = a.scratch + gwarp * (uint64_t)a.rows * kStripLanes + lane;
+    col[(uint64_t)(a.rows - 1) * kStripLanes] = 0;
     const uint64_t n_strips = (a.word_count + kStripThreads - 1) / kStripThreads;
     for (;;) {
         __syncthreads();  // s_strip is free again (and the tally counters are zeroed)
@@ -929,63 +934,67 @@ __global__ void __launch_bounds__(kStripThreads, MINB) k_strip(StripArgs a) {
         const uint64_t wl = strip * kStripThreads + threadIdx.x;
         const bool valid = wl < a.word_count;
         const WordCtx ctx = make_word_ctx((uint32_t)(a.word_begin + wl));
+        uint32_t e = 0, gq = 0;
 #pragma unroll 1
-        for (uint32_t e = 0; e < a.n_be; ++e) {
-            const uint4 r = a.be[e];
-            uint64_t v;
-            if (r.w != 0) v = kAllOnes;
-            else if (r.z == 0) v = 0;
-            else v = be_word_tab<PF>(r.y, ctx, GlobalTable{a.table + (uint64_t)e * kEventTableStride}, r.z);
-            col[(uint64_t)e * kStripLanes] = v;
+        for (uint32_t sg = 0; sg < a.n_segments; ++sg) {
+            const uint2 end = a.segment[sg];
+#pragma unroll 1
+            for (; e < end.x; ++e) {
+                const uint4 r = a.be[e];
+                uint64_t v;
+                if (r.w != 0) v = kAllOnes;
+                else if (r.z == 0) v = 0;
+                else v = be_word_tab<PF>(r.y, ctx, GlobalTable{a.table + (uint64_t)e * kEventTableStride}, r.z);
+                strip_row(col, r.x) = v;
+            }
+            // no gate of a group reads another, so the loads of a whole group
+            // are in flight together and its outputs are stored after them
+#pragma unroll 1
+            for (; gq < end.y; ++gq) {
+                const uint4 h = a.groups[2 * gq];
+                if (h.x >> 24) {
+                    const uint4 f = a.ginfo[h.z];
+                    const uint64_t r = strip_gate(a, col, f.w);
+                    strip_row(col, f.x) = r;
+                    strip_gate_tally(a, s_ones, f, r, valid, lane);
+                    continue;
+                }
+                const uint32_t cnt = h.x & 0xFFu, maxn = (h.x >> 8) & 0xFFFFu;
+                const uint4 *rec = reinterpret_cast<const uint4 *>(a.gin + h.y);
+                uint64_t acc[kStripGroup] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll 2
+                for (uint32_t sl = 0; sl < maxn; ++sl) {
+                    const uint4 rr = rec[sl];
+                    acc[0] |= strip_in(col, rr.x);
+                    acc[1] |= strip_in(col, rr.y);
+                    acc[2] |= strip_in(col, rr.z);
+                    acc[3] |= strip_in(col, rr.w);
+                }
+                const uint4 out = a.groups[2 * gq + 1];
+                uint32_t pc[kStripGroup];
+#pragma unroll
+                for (uint32_t j = 0; j < kStripGroup; ++j) {
+                    const uint64_t r = ((h.w >> j) & 1u) ? ~acc[j] : acc[j];
+                    pc[j] = valid && j < cnt ? (uint32_t)__popcll(r) : 0u;
+                    const uint32_t node = j == 0 ? out.x : j == 1 ? out.y : j == 2 ? out.z : out.w;
+                    if (j < cnt) strip_row(col, node) = r;
+                }
+                // tallies: two gates' warp sums (at most 32 x 64 each) per 32-bit
+                // reduction, then lane j adds gate j's sum to its tally slots
+                const uint32_t s01 = __reduce_add_sync(0xFFFFFFFFu, pc[0] | (pc[1] << 16));
+                const uint32_t s23 = __reduce_add_sync(0xFFFFFFFFu, pc[2] | (pc[3] << 16));
+                if (lane < cnt) {
+                    const uint4 f = a.ginfo[h.z + lane];
+                    const uint32_t c = ((lane < 2 ? s01 : s23) >> (16 * (lane & 1u))) & 0xFFFFu;
+                    if (f.z && c)
+                        for (uint32_t t = 0; t < f.z; ++t) strip_tally(a, s_ones, a.tally_list[f.y + t], c);
+                }
+            }
         }
         for (uint32_t j = 0; j < a.n_be_tally; ++j) {
-            const uint64_t v = col[(uint64_t)a.be_tally_nodes[j] * kStripLanes];
-            const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, valid ? (uint32_t)__popcll(v) : 0u);
-            if (lane == 0 && c) strip_tally(a, s_ones, a.be_tally_idx[j], c);
-        }
-        // gates, layer by layer, a group at a time: no gate of a group reads
-        // another, so the loads of a whole group are in flight together and
-        // its outputs are stored after them
-#pragma unroll 1
-        for (uint32_t gq = 0; gq < a.n_groups; ++gq) {
-            const uint4 h = a.groups[2 * gq];
-            if (h.x >> 24) {
-                const uint4 f = a.ginfo[h.z];
-                const uint64_t r = strip_gate(a, col, f.w);
-                col[(uint64_t)f.x * kStripLanes] = r;
-                strip_gate_tally(a, s_ones, f, r, valid, lane);
-                continue;
-            }
-            const uint32_t cnt = h.x & 0xFFu, maxn = (h.x >> 8) & 0xFFFFu;
-            const uint4 *rec = reinterpret_cast<const uint4 *>(a.gin + h.y);
-            uint64_t acc[kStripGroup] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll 2
-            for (uint32_t sl = 0; sl < maxn; ++sl) {
-                const uint4 rr = rec[sl];
-                acc[0] |= strip_in(col, rr.x);
-                acc[1] |= strip_in(col, rr.y);
-                acc[2] |= strip_in(col, rr.z);
-                acc[3] |= strip_in(col, rr.w);
-            }
-            const uint4 out = a.groups[2 * gq + 1];
-            uint32_t pc[kStripGroup];
-#pragma unroll
-            for (uint32_t j = 0; j < kStripGroup; ++j) {
-                const uint64_t r = ((h.w >> j) & 1u) ? ~acc[j] : acc[j];
-                pc[j] = valid && j < cnt ? (uint32_t)__popcll(r) : 0u;
-                const uint32_t node = j == 0 ? out.x : j == 1 ? out.y : j == 2 ? out.z : out.w;
-                if (j < cnt) col[(uint64_t)node * kStripLanes] = r;
-            }
-            // tallies: two gates' warp sums (at most 32 x 64 each) per 32-bit
-            // reduction, then lane j adds gate j's sum to its tally slots
-            const uint32_t s01 = __reduce_add_sync(0xFFFFFFFFu, pc[0] | (pc[1] << 16));
-            const uint32_t s23 = __reduce_add_sync(0xFFFFFFFFu, pc[2] | (pc[3] << 16));
-            if (lane < cnt) {
-                const uint4 f = a.ginfo[h.z + lane];
-                const uint32_t c = ((lane < 2 ? s01 : s23) >> (16 * (lane & 1u))) & 0xFFFFu;
-                if (f.z && c)
-                    for (uint32_t t = 0; t < f.z; ++t) strip_tally(a, s_ones, a.tally_list[f.y + t], c);
-            }
+            const uint2 t = a.be_tally[j];
+            const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, valid ? (uint32_t)__popcll(strip_row(col, t.x)) : 0u);
+            if (lane == 0 && c) strip_tally(a, s_ones, t.y, c);
         }
     }
     __syncthreads();

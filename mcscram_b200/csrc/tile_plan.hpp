@@ -103,21 +103,24 @@ inline TilePlan plan_tile(const Graph &g) {
     return t;
 }
 
-// The plan of the batch tile kernel, whose rows lie in memory: the gates in
-// depth-first postorder, cut into segments that each sample their own new
-// events (kSegmentEvents of them, if so many are left) and then evaluate their
-// gates by layers.  A node's row is free again after the layer that reads it
-// last and is the next one to be written, so that rows mostly stay in the L2
-// from writer to reader and their memory is mostly never written back.
+// The plan of the kernels whose rows lie in memory (the batch tile kernel and
+// the strip kernel): the gates in depth-first postorder, cut into segments
+// that each sample their own new events (`events` of them, if so many are
+// left) and then evaluate their gates.  A node's row is free again after the
+// layer that reads it last (by_layer; else after the segment, whose gates may
+// then be taken in any order that respects their inputs) and is the next one
+// to be written, so that rows mostly stay in the L2 from writer to reader and
+// their memory is mostly never written back.
 constexpr uint32_t kSegmentEvents = 96;
 struct SegmentPlan {
     TilePlan tile;                    // tile.layer over all segments; slots from 0
     std::vector<uint2> segment;       // per segment: its events' and its layers' end
     std::vector<uint32_t> event_slot, gate_slot;
+    std::vector<uint32_t> gate;       // gate ids, in tile.gates' order
     uint32_t slots = 0;
 };
 
-inline SegmentPlan plan_segments(const Graph &g) {
+inline SegmentPlan plan_segments(const Graph &g, uint32_t events, bool by_layer) {
     SegmentPlan p;
     TilePlan &t = p.tile;
     const uint32_t nb = g.n_be;
@@ -164,7 +167,7 @@ inline SegmentPlan plan_segments(const Graph &g) {
     std::vector<char> sampled(nb, 0);
     std::vector<uint32_t> seg_of(g.n_gates, 0), depth(g.n_gates, 0);
     for (uint32_t i : order) {
-        if (segs.back().events.size() >= kSegmentEvents) segs.emplace_back();
+        if (segs.back().events.size() >= events) segs.emplace_back();
         Segment &s = segs.back();
         seg_of[i] = (uint32_t)segs.size();
         for (uint32_t j = needs.first_input(i); j < g.gate_in_count[i]; ++j) {
@@ -203,9 +206,9 @@ inline SegmentPlan plan_segments(const Graph &g) {
             p.event_slot.push_back(slot[e]);
         }
         for (const auto &layer : s.layers) {
-            dead.clear();
             for (uint32_t i : layer) {
                 take(nb + i);
+                p.gate.push_back(i);
                 p.gate_slot.push_back(slot[nb + i]);
                 needs.emit(t, i, slot);
             }
@@ -214,9 +217,14 @@ inline SegmentPlan plan_segments(const Graph &g) {
                     if (--reads[needs.input(i, j)] == 0) dead.push_back(slot[needs.input(i, j)]);
                 if (reads[nb + i] == 0) dead.push_back(slot[nb + i]);
             }
-            free_slots.insert(free_slots.end(), dead.begin(), dead.end());
+            if (by_layer) {
+                free_slots.insert(free_slots.end(), dead.begin(), dead.end());
+                dead.clear();
+            }
             t.layer.push_back((uint32_t)t.gates.size());
         }
+        free_slots.insert(free_slots.end(), dead.begin(), dead.end());
+        dead.clear();
         p.segment.push_back(make_uint2((uint32_t)t.event.size(), (uint32_t)t.layer.size() - 1));
     }
     for (uint32_t e = 0; e < nb; ++e)

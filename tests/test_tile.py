@@ -106,14 +106,8 @@ def test_batched_instances_in_tiles(oracle_mod, gpu, draws, words):
         assert int(o) == int(np.sum(oracle_mod.tallies(g, 5, 1, 0, words))), (i, inst_tree[i])
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("n_be,n_gates,tallies", [(95, 60, "root"), (96, 60, "all"), (700, 420, "root"),
-                                                  (700, 420, "some"), (1200, 700, "all"), (250, 0, "all")])
-def test_batched_trees_in_segments(oracle_mod, gpu, n_be, n_gates, tallies):
-    """Trees of several segments, whose rows are used again: nodes read far from
-    where they are written, tallied events (their rows last), events no gate reads."""
-    from mcscram_b200.uncertainty import Batch
-    rng = np.random.default_rng(n_be + n_gates)
+def _far_reads(rng, n_be, n_gates, tallies):
+    """Gates that read the last 40 gates and any event up to their share of them."""
     ops, ks, begin, count, neg, inputs = [], [], [], [], [], []
     for j in range(n_gates):
         op = int(rng.choice([AND, OR, ATLEAST, XOR, NOT, NAND, NOR, NULL]))
@@ -129,11 +123,39 @@ def test_batched_trees_in_segments(oracle_mod, gpu, n_be, n_gates, tallies):
         inputs += [int(x) for x in rng.choice(pool, n)]
     nodes = n_be + n_gates
     tally = {"root": [nodes - 1], "all": np.arange(nodes), "some": rng.integers(0, nodes, 25)}[tallies]
-    g = G.FlatGraph(be_pdag_idx=np.arange(2, 2 + n_be), be_event_idx=rng.permutation(n_be),
-                    be_threshold=np.zeros(n_be, np.uint64), gate_op=ops, gate_k=ks, gate_in_begin=begin,
-                    gate_in_count=count, gate_neg_count=neg, inputs=inputs, tally_nodes=tally)
+    return G.FlatGraph(be_pdag_idx=np.arange(2, 2 + n_be), be_event_idx=rng.permutation(n_be),
+                       be_threshold=(10.0 ** rng.uniform(-3, 0, n_be) * 2.0**32).astype(np.uint64), gate_op=ops,
+                       gate_k=ks, gate_in_begin=begin, gate_in_count=count, gate_neg_count=neg, inputs=inputs,
+                       tally_nodes=tally)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_be,n_gates,tallies", [(95, 60, "root"), (96, 60, "all"), (700, 420, "root"),
+                                                  (700, 420, "some"), (1200, 700, "all"), (250, 0, "all")])
+def test_batched_trees_in_segments(oracle_mod, gpu, n_be, n_gates, tallies):
+    """Trees of several segments, whose rows are used again: nodes read far from
+    where they are written, tallied events (their rows last), events no gate reads."""
+    from mcscram_b200.uncertainty import Batch
+    rng = np.random.default_rng(n_be + n_gates)
+    g = _far_reads(rng, n_be, n_gates, tallies)
     thr = [(10.0 ** rng.uniform(-3, 0, n_be) * 2.0**32).astype(np.uint64) for _ in range(6)]
     with Batch([g]) as b:
         got = b.run([0] * len(thr), thr, iteration=2, words_per_instance=70)
     for t, o in zip(thr, got):
         assert int(o) == int(np.sum(oracle_mod.tallies(g.with_thresholds(t), 2, 1, 0, 70)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_be,n_gates,tallies", [(383, 200, "all"), (385, 300, "some"), (1600, 1000, "all"),
+                                                  (1600, 1000, "root"), (900, 0, "all")])
+def test_strip_segments(capi, oracle_mod, gpu, n_be, n_gates, tallies):
+    """The strip mode's segments and reused rows on the same graphs, and on one of
+    every connective with empty and wide gates."""
+    g = _far_reads(np.random.default_rng(n_be + n_gates), n_be, n_gates, tallies)
+    for h in (g, _every_connective(np.random.default_rng(n_be))):
+        with capi.Engine(h, mode=capi.MODE_STRIP) as e:
+            e.run(4, 2, 3, 300)
+            ones, total = e.tallies()
+        want = sum(_popcounts(oracle_mod.eval_words(h, 4 + i, 3, 300)[h.tally_nodes]) for i in range(2))
+        assert total == 2 * 300 * 64
+        assert np.array_equal(ones, want)
