@@ -504,7 +504,7 @@ mcg_status setup_tile(mcg_engine *e) {
     uint32_t threads = 0;
     uint64_t room = 0;
     for (uint32_t nt : {256u, 512u, 1024u}) {
-        const uint64_t own = (nt / 32u) * (mcg::dev::kEventTableStride + 1) * sizeof(uint2);
+        const uint64_t own = (nt / 32u) * mcg::dev::kEventTableStride * sizeof(uint2);
         const uint64_t most = std::min<uint64_t>(dev.sharedMemPerBlockOptin, dev.sharedMemPerMultiprocessor / (1024u / nt) -
                                                                                  dev.reservedSharedMemPerBlock);
         if (words + own > most) continue;

@@ -787,7 +787,8 @@ __global__ void __launch_bounds__(kGateThreadsMost) k_stage_gates(const __grid_c
 // memory-bound gate work of some blocks runs under the multiply-bound
 // sampling of the others.  Bound by the issue of the sampler's instructions
 // (711 per event and warp) and the gates' (46): 2^20 words of the 5,000-event
-// tree take 190.8 ms, where all events before all gates took 193.9.
+// tree take 188.0 ms; 193.9 with all events before all gates and 8-byte table
+// loads.
 constexpr int kStripLanes = 32;
 constexpr int kStripThreads = 256;
 
@@ -1036,7 +1037,7 @@ template <int NT, int PF>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_tile(const __grid_constant__ TileArgs a) {
     constexpr uint32_t kWarps = NT / 32;
     extern __shared__ __align__(16) uint64_t smem[];
-    __shared__ uint4 s_tab[kWarps][(kEventTableStride + 1) / 2];
+    __shared__ uint4 s_tab[kWarps][kEventTableStride / 2];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint64_t *col = smem + lane;
     unsigned long long *s_ones = reinterpret_cast<unsigned long long *>(smem + (size_t)a.n_slots * kTileLanes);
