@@ -587,7 +587,6 @@ mcg_status setup_fused(mcg_engine *e, const mcg_run_desc &run) {
     return MCG_OK;
 }
 
-constexpr uint32_t kStageEventsPerThread = 4;
 // From this many words on (a block of 64 per SM), gate blocks take two words
 // per lane: half the loads and instructions per word.  Fewer words are one per
 // lane, for twice the blocks (32,768 words of the 5,000-event tree: 6.23 ms,
@@ -617,7 +616,7 @@ mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
     const uint32_t blocks = run.sampler_blocks_per_sm ? run.sampler_blocks_per_sm : 8u;
     if (blocks < 1 || blocks > 8) return mcg::fail(MCG_ERR_INVALID, "sampler_blocks_per_sm must be 1..8");
     e->sampler_smem = blocks >= 8 ? 0u : (uint32_t)(prop.sharedMemPerMultiprocessor / blocks - 2048);
-    const mcg_status lim = mcg::set_smem_limit(mcg::dev::k_stage_be<kPackForm, kStageEventsPerThread>,
+    const mcg_status lim = mcg::set_smem_limit(mcg::dev::k_stage_be<kPackForm>,
                                                e->sampler_smem);
     if (lim != MCG_OK) return lim;
     // Gate blocks of a chunk that the next one is sampled beside: two per SM, as
@@ -758,7 +757,11 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         e->table_iteration = iteration;
     }
     if (g.n_be > 0) {
-        const uint32_t groups = (g.n_be + kStageEventsPerThread - 1) / kStageEventsPerThread;
+        // events per thread: fewer where the last wave of blocks would leave much
+        // of the chip idle (2,048 words of 500 events: 185 us for the call, 188 with 4)
+        const uint64_t waves = (uint64_t)g.n_be * ((W + 511) / 512) / (4ull * e->gate_sms);
+        const uint32_t ept = waves >= 32 ? 4u : waves >= 16 ? 2u : 1u;
+        const uint32_t groups = (g.n_be + ept - 1) / ept;
         cudaEvent_t p0 = nullptr, p1 = nullptr;
         if (e->profile_a) {
             if (e->prof_used == e->prof_events.size()) {
@@ -772,9 +775,8 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
             ++e->prof_used;
             MCG_CUDA(cudaEventRecord(p0, e->s_a));
         }
-        mcg::dev::k_stage_be<kPackForm, kStageEventsPerThread>
-            <<<rows_grid(W, groups, 256), 256, e->sampler_smem, e->s_a>>>(be_tab, e->d_event_table, g.n_be, W,
-                                                                          stride, word_begin, buf);
+        mcg::dev::k_stage_be<kPackForm><<<rows_grid((W + 1) / 2, groups, 256), 256, e->sampler_smem, e->s_a>>>(
+            be_tab, e->d_event_table, g.n_be, ept, W, stride, word_begin, buf);
         ++e->launches;
         if (p1) MCG_CUDA(cudaEventRecord(p1, e->s_a));
     }

@@ -543,27 +543,37 @@ static __global__ void __launch_bounds__(256) k_event_table(const uint4 *__restr
     event_table_entry(be[e].x, t3, g, table[i]);
 }
 
-// Phase A: thread (w, group) samples word w of events [group * EPT, +EPT)
-// using the pass's event table.  Launched with dynamic shared memory that
-// only caps the blocks per SM, leaving room for gate-phase blocks.
-template <int PF, int EPT>
-__global__ void __launch_bounds__(256, 6) k_stage_be(const uint4 *__restrict__ be, const uint2 *__restrict__ table,
-                                                  uint32_t n_be, uint64_t W, uint64_t stride,
-                                                  uint64_t word_begin, uint64_t *__restrict__ buf) {
-    const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t e0 = (blockIdx.y + gridDim.y * blockIdx.z) * EPT;
+// Phase A: thread (w, group) samples words 2 w and 2 w + 1 of events
+// [group * ept, + ept) using the pass's event table.  Launched with dynamic
+// shared memory that only caps the blocks per SM, leaving room for gate-phase
+// blocks.  Bound by the sampler's instructions: two words per thread share the
+// table's loads and leave 64 registers to a thread, in four blocks per SM
+// (300,001 words of the 1,003-event tree with its gates: 10.48 ms; one word per
+// thread in six blocks of 40 registers 10.72, two in three or five blocks
+// 10.63, four in two or three 10.61 and 10.65).
+template <int PF>
+__global__ void __launch_bounds__(256, 4) k_stage_be(const uint4 *__restrict__ be, const uint2 *__restrict__ table,
+                                                     uint32_t n_be, uint32_t ept, uint64_t W, uint64_t stride,
+                                                     uint64_t word_begin, uint64_t *__restrict__ buf) {
+    const uint64_t w = 2 * ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    const uint32_t e0 = (blockIdx.y + gridDim.y * blockIdx.z) * ept;
     if (w >= W || e0 >= n_be) return;
-    const WordCtx ctx = make_word_ctx((uint32_t)(word_begin + w));
+    const WordCtx ctx[2] = {make_word_ctx((uint32_t)(word_begin + w)), make_word_ctx((uint32_t)(word_begin + w + 1))};
+    const uint32_t end = min(e0 + ept, n_be);
 #pragma unroll 1
-    for (uint32_t i = 0; i < EPT; ++i) {
-        const uint32_t e = e0 + i;
-        if (e >= n_be) break;
+    for (uint32_t e = e0; e < end; ++e) {
         const uint4 r = be[e];
-        uint64_t v;
-        if (r.w != 0) v = kAllOnes;           // threshold 2^32
-        else if (r.z == 0) v = 0;             // threshold 0
-        else v = be_word_tab<PF>(r.y, ctx, GlobalTable{table + (uint64_t)e * kEventTableStride}, r.z);
-        buf[(uint64_t)e * stride + w] = v;
+        uint64_t v[2];
+        if (r.w != 0) v[0] = v[1] = kAllOnes;           // threshold 2^32
+        else if (r.z == 0) v[0] = v[1] = 0;             // threshold 0
+        else be_words_tab<PF, 2>(r.y, ctx, GlobalTable{table + (uint64_t)e * kEventTableStride}, r.z, v);
+        uint64_t *out = buf + (uint64_t)e * stride + w;
+        if (stride % 2 == 0) {  // the row has room for an even number of words
+            *reinterpret_cast<ulonglong2 *>(out) = make_ulonglong2(v[0], v[1]);
+        } else {
+            out[0] = v[0];
+            if (w + 1 < W) out[1] = v[1];
+        }
     }
 }
 

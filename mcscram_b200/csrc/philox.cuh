@@ -194,7 +194,7 @@ __device__ __forceinline__ uint64_t be_word(uint32_t x0, uint32_t x1, const Word
 // g = 0..15, [16] = {lo(M0 * x0), hi(M0 * x0)}.
 // Rows are 18 entries long, for two entries to a 16-byte load: nine loads per
 // word and not 17.  2^20 words of the 5,000-event tree 190.8 -> 188.0 ms in
-// strips; 32,768 words of it, staged, 6.22 -> 6.19 ms.
+// strips; 32,768 words of it, staged, one word per thread, 6.22 -> 6.19 ms.
 constexpr int kEventTableStride = 18;
 
 __device__ __forceinline__ void event_table_entry(uint32_t x0, uint32_t t3, int g, uint2 &out) {
@@ -210,66 +210,70 @@ __device__ __forceinline__ void event_table_entry(uint32_t x0, uint32_t t3, int 
     }
 }
 
-// be_word with the per-pass event table (same result as be_word); tab(g) gives
-// entry g.
-template <int PackForm, class Table>
-__device__ __forceinline__ uint64_t be_word_tab(uint32_t x1, const WordCtx &ctx, Table &&tab, uint32_t thr) {
-    const uint32_t a0 = ctx.hb ^ x1 ^ RoundKey<0>::k0;
-    const uint32_t a1 = ctx.lb;
+// K words of one event with the per-pass event table (be_word's results); tab(g)
+// gives entry g.  The entries are read once for all K words, whose chains of
+// multiplies are in flight together.
+template <int PackForm, int K, class Table>
+__device__ __forceinline__ void be_words_tab(uint32_t x1, const WordCtx (&ctx)[K], Table &&tab, uint32_t thr,
+                                             uint64_t (&out)[K]) {
     const uint32_t a3 = tab(16).x;
-    uint32_t hc, lc;
-    mul_hilo(kM0, a0, hc, lc);
-    const uint32_t b2 = hc ^ a3 ^ RoundKey<1>::k1;
-    const uint32_t b3 = lc;
-    uint32_t hf, lf;
-    mul_hilo(kM1, b2, hf, lf);
-    const uint32_t c1 = lf;
-    uint32_t lo = 0, hi = 0;
+    uint32_t hf[K], c1[K], b3[K], lo[K] = {}, hi[K] = {};
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        uint32_t hc;
+        mul_hilo(kM0, ctx[k].hb ^ x1 ^ RoundKey<0>::k0, hc, b3[k]);
+        mul_hilo(kM1, hc ^ a3 ^ RoundKey<1>::k1, hf[k], c1[k]);
+    }
 #pragma unroll
     for (int g = 0; g < 16; ++g) {
         const uint2 d = tab(g);
-        const uint32_t b0 = d.x ^ a1 ^ RoundKey<1>::k0;
-        const uint32_t b1 = d.y;
-        uint32_t he, le;
-        mul_hilo(kM0, b0, he, le);
-        uint32_t x0r = hf ^ b1 ^ RoundKey<2>::k0;
-        uint32_t x1r = c1;
-        uint32_t x2r = he ^ b3 ^ RoundKey<2>::k1;
-        uint32_t x3r = le;
-        philox_round<3>(x0r, x1r, x2r, x3r);
-        philox_round<4>(x0r, x1r, x2r, x3r);
-        philox_round<5>(x0r, x1r, x2r, x3r);
-        philox_round<6>(x0r, x1r, x2r, x3r);
-        philox_round<7>(x0r, x1r, x2r, x3r);
-        philox_round<8>(x0r, x1r, x2r, x3r);
-        philox_round<9>(x0r, x1r, x2r, x3r);
-        if constexpr (PackForm == 0) {
-            const uint32_t nib = nibble_lt(x0r, x1r, x2r, x3r, thr);
-            if (g < 8) lo |= nib << (4 * g);
-            else hi |= nib << (4 * (g - 8));
-        } else {
-            if (g < 8) {
-                lo = shift_in_ge(lo, x3r, thr);
-                lo = shift_in_ge(lo, x2r, thr);
-                lo = shift_in_ge(lo, x1r, thr);
-                lo = shift_in_ge(lo, x0r, thr);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const uint32_t b0 = d.x ^ ctx[k].lb ^ RoundKey<1>::k0;
+            uint32_t he, le;
+            mul_hilo(kM0, b0, he, le);
+            uint32_t x0r = hf[k] ^ d.y ^ RoundKey<2>::k0;
+            uint32_t x1r = c1[k];
+            uint32_t x2r = he ^ b3[k] ^ RoundKey<2>::k1;
+            uint32_t x3r = le;
+            philox_round<3>(x0r, x1r, x2r, x3r);
+            philox_round<4>(x0r, x1r, x2r, x3r);
+            philox_round<5>(x0r, x1r, x2r, x3r);
+            philox_round<6>(x0r, x1r, x2r, x3r);
+            philox_round<7>(x0r, x1r, x2r, x3r);
+            philox_round<8>(x0r, x1r, x2r, x3r);
+            philox_round<9>(x0r, x1r, x2r, x3r);
+            uint32_t &half = g < 8 ? lo[k] : hi[k];
+            if constexpr (PackForm == 0) {
+                half |= nibble_lt(x0r, x1r, x2r, x3r, thr) << (4 * (g & 7));
             } else {
-                hi = shift_in_ge(hi, x3r, thr);
-                hi = shift_in_ge(hi, x2r, thr);
-                hi = shift_in_ge(hi, x1r, thr);
-                hi = shift_in_ge(hi, x0r, thr);
+                half = shift_in_ge(half, x3r, thr);
+                half = shift_in_ge(half, x2r, thr);
+                half = shift_in_ge(half, x1r, thr);
+                half = shift_in_ge(half, x0r, thr);
             }
         }
     }
-    if constexpr (PackForm == 0) {
-        return ((uint64_t)hi << 32) | (uint64_t)lo;
-    } else {
-        auto rev_nibbles = [](uint32_t v) -> uint32_t {
-            v = ((v & 0x0F0F0F0Fu) << 4) | ((v >> 4) & 0x0F0F0F0Fu);
-            return __byte_perm(v, 0, 0x0123);
-        };
-        return ((uint64_t)(~rev_nibbles(hi)) << 32) | (uint64_t)(~rev_nibbles(lo));
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        if constexpr (PackForm == 0) {
+            out[k] = ((uint64_t)hi[k] << 32) | (uint64_t)lo[k];
+        } else {
+            auto rev_nibbles = [](uint32_t v) -> uint32_t {
+                v = ((v & 0x0F0F0F0Fu) << 4) | ((v >> 4) & 0x0F0F0F0Fu);
+                return __byte_perm(v, 0, 0x0123);
+            };
+            out[k] = ((uint64_t)(~rev_nibbles(hi[k])) << 32) | (uint64_t)(~rev_nibbles(lo[k]));
+        }
     }
+}
+
+template <int PackForm, class Table>
+__device__ __forceinline__ uint64_t be_word_tab(uint32_t x1, const WordCtx &ctx, Table &&tab, uint32_t thr) {
+    const WordCtx c[1] = {ctx};
+    uint64_t out[1];
+    be_words_tab<PackForm, 1>(x1, c, tab, thr, out);
+    return out[0];
 }
 
 // Half of a word's outputs: the eight calls whose table entries are tab(0..7)
