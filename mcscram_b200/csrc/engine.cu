@@ -487,32 +487,59 @@ mcg_status upload_tile(mcg_engine *e, const T **dptr, const std::vector<T> &v) {
     return MCG_OK;
 }
 
-// Fused mode's default shape where every needed node has room for 32 words in
-// shared memory (about 880 nodes on a B200): e->tile, or not.
+// Fused mode's default shape where 32 words of every needed node (about 880 on
+// a B200), or of every one that is live at a time in segments, have room in
+// shared memory: e->tile, or not.  233,937
+// words, all gates tallied: 1,030 events in segments 9.1 ms, the interpreter
+// 13.9; 2,500 events 23.5 and 36.3; 4,096 words of them 0.22 and 2.75, 0.50 and
+// 7.3 ms.
 mcg_status setup_tile(mcg_engine *e) {
     const mcg::Graph &g = e->graph;
     mcg::DeviceShape dev;
     MCG_CUDA(mcg::device_shape(&dev, e->device));
     constexpr uint32_t kSlotBytes = mcg::dev::kTileLanes * sizeof(uint64_t);
-    mcg::TilePlan t = mcg::plan_tile(g);
-    for (uint32_t &rec : t.in) rec = t.byte_record(rec, kSlotBytes, 0, t.slots());
-    const uint64_t words = (uint64_t)(t.slots() + 1) * mcg::dev::kTileLanes * sizeof(uint64_t);
-    if (!t.fits) return MCG_OK;
     // the most, and so the smallest, blocks that share an SM's 1,024 threads
     // and its shared memory; the tally counters go to shared memory where
     // they fit as well
     uint32_t threads = 0;
-    uint64_t room = 0;
-    for (uint32_t nt : {256u, 512u, 1024u}) {
-        const uint64_t own = (nt / 32u) * mcg::dev::kEventTableStride * sizeof(uint2);
-        const uint64_t most = std::min<uint64_t>(dev.sharedMemPerBlockOptin, dev.sharedMemPerMultiprocessor / (1024u / nt) -
-                                                                                 dev.reservedSharedMemPerBlock);
-        if (words + own > most) continue;
-        threads = nt;
-        room = most - own;
-        break;
+    uint64_t room = 0, words = 0;
+    auto fit = [&](uint64_t slots) {
+        words = (slots + 1) * kSlotBytes;  // and the empty input
+        for (uint32_t nt : {256u, 512u, 1024u}) {
+            const uint64_t own = (nt / 32u) * mcg::dev::kEventTableStride * sizeof(uint2);
+            const uint64_t most = std::min<uint64_t>(
+                dev.sharedMemPerBlockOptin, dev.sharedMemPerMultiprocessor / (1024u / nt) - dev.reservedSharedMemPerBlock);
+            if (words + own > most) continue;
+            threads = nt;
+            room = most - own;
+            return true;
+        }
+        return false;
+    };
+    mcg::TilePlan t = mcg::plan_tile(g);
+    uint32_t slots = t.slots();
+    std::vector<uint32_t> event_slot(t.event.size()), gate_slot(t.gates.size());
+    std::vector<uint2> segment{make_uint2((uint32_t)t.event.size(), (uint32_t)t.layer.size() - 1)};
+    for (uint32_t i = 0; i < slots; ++i) (i < t.event.size() ? event_slot[i] : gate_slot[i - t.event.size()]) = i;
+    if (!fit(slots)) {
+        // segments: as long as their rows fit, since each has its own layers to wait for
+        for (uint32_t events : {256u, 96u}) {
+            mcg::SegmentPlan p = mcg::plan_segments(g, events, true, 32);
+            slots = p.slots;
+            if (!fit(slots)) continue;
+            t = std::move(p.tile);
+            segment = std::move(p.segment);
+            event_slot = std::move(p.event_slot);
+            gate_slot = std::move(p.gate_slot);
+            break;
+        }
     }
-    if (!threads) return MCG_OK;
+    if (!threads || !t.fits) return MCG_OK;
+    for (uint32_t &rec : t.in) rec = t.byte_record(rec, kSlotBytes, 0, slots);
+    for (size_t i = 0; i < t.gates.size(); ++i) {
+        if (t.gates[i].z > 0xFFFFu) return MCG_OK;
+        t.gates[i].z |= gate_slot[i] * mcg::dev::kTileLanes << 16;
+    }
     const uint64_t counters = g.tally_nodes.size() * sizeof(unsigned long long);
     mcg::dev::TileArgs &a = e->tile_args;
     a = mcg::dev::TileArgs{};
@@ -525,16 +552,16 @@ mcg_status setup_tile(mcg_engine *e) {
     for (size_t i = 0; i < be.size(); ++i) {
         const uint32_t v = t.event[i];
         be[i] = make_uint4((uint32_t)g.be_pdag_idx[v] + 1u, g.be_event_idx[v] + 1u, (uint32_t)g.be_threshold[v],
-                           (uint32_t)(g.be_threshold[v] >> 32));
+                           (uint32_t)(g.be_threshold[v] >> 32) | event_slot[i] * mcg::dev::kTileLanes << 1);
     }
     if ((st = upload_tile(e, &a.be, be)) != MCG_OK || (st = upload_tile(e, &a.gates, t.gates)) != MCG_OK ||
         (st = upload_tile(e, &a.in, t.in)) != MCG_OK || (st = upload_tile(e, &a.layer, t.layer)) != MCG_OK ||
         (st = upload_tile(e, &a.tally_list, t.tally_list)) != MCG_OK ||
-        (st = upload_tile(e, &a.be_tally, t.be_tally)) != MCG_OK)
+        (st = upload_tile(e, &a.be_tally, t.be_tally)) != MCG_OK ||
+        (st = upload_tile(e, &a.segment, segment)) != MCG_OK)
         return st;
-    a.n_be = (uint32_t)t.event.size();
-    a.n_slots = t.slots() + 1;  // and the empty input
-    a.n_layers = (uint32_t)t.layer.size() - 1;
+    a.n_slots = slots + 1;
+    a.n_segments = (uint32_t)segment.size();
     a.n_be_tally = (uint32_t)t.be_tally.size();
     a.n_tally = (uint32_t)g.tally_nodes.size();
     e->tile_threads = threads;

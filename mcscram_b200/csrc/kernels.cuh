@@ -1067,84 +1067,90 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_tile(const __grid_constant__ 
             const uint64_t wl = tile * kTileLanes + lane;
             const bool valid = wl < a.word_count;
             const WordCtx ctx = make_word_ctx((uint32_t)(a.word_begin + wl));
+            uint32_t e_begin = 0, l = 0;
+            for (uint32_t sg = 0; sg < a.n_segments; ++sg) {
+                const uint2 end = a.segment[sg];
 #pragma unroll 1
-            for (uint32_t e = warp; e < a.n_be; e += kWarps) {
-                const uint4 r = a.be[e];
-                uint64_t v;
-                if (r.w != 0) {
-                    v = kAllOnes;
-                } else if (r.z == 0) {
-                    v = 0;
-                } else {
-                    __syncwarp();  // the last event's entries have been read
-                    if (lane < (uint32_t)kEventTableStride)
-                        event_table_entry(r.x, t3, (int)lane, reinterpret_cast<uint2 *>(s_tab[warp])[lane]);
-                    __syncwarp();
-                    v = be_word_tab<PF>(r.y, ctx, SharedTable{s_tab[warp]}, r.z);
+                for (uint32_t e = e_begin + warp; e < end.x; e += kWarps) {
+                    const uint4 r = a.be[e];
+                    uint64_t v;
+                    if (r.w & 1u) {
+                        v = kAllOnes;
+                    } else if (r.z == 0) {
+                        v = 0;
+                    } else {
+                        __syncwarp();  // the last event's entries have been read
+                        if (lane < (uint32_t)kEventTableStride)
+                            event_table_entry(r.x, t3, (int)lane, reinterpret_cast<uint2 *>(s_tab[warp])[lane]);
+                        __syncwarp();
+                        v = be_word_tab<PF>(r.y, ctx, SharedTable{s_tab[warp]}, r.z);
+                    }
+                    col[r.w >> 1] = v;
                 }
-                col[e * kTileLanes] = v;
+                __syncthreads();
+                for (; l < end.y; ++l) {
+                    const uint32_t gates_end = a.layer[l + 1];
+                    for (uint32_t i = a.layer[l] + warp; i < gates_end; i += kWarps) {
+                        const uint4 m = a.gates[i];
+                        const uint32_t kind = m.x & 3u;
+                        const uint2 *in = reinterpret_cast<const uint2 *>(a.in + m.y);
+                        const uint32_t pairs = m.z & 0xFFFFu;
+                        uint64_t r = 0;
+                        if (kind == kTileOr) {
+#pragma unroll 2
+                            for (uint32_t j = 0; j < pairs; ++j) {
+                                const uint2 s = in[j];
+                                r |= tile_in(col, s.x) | tile_in(col, s.y);
+                            }
+                        } else if (kind == kTileXor) {
+                            for (uint32_t j = 0; j < pairs; ++j) {
+                                const uint2 s = in[j];
+                                r ^= tile_in(col, s.x) ^ tile_in(col, s.y);
+                            }
+                        } else {
+                            const uint32_t kk = (m.x >> 8) & 0xFFu, nbits = (m.x >> 16) & 0xFu;
+                            if (nbits <= 4) {  // at most 15 inputs
+                                SlicedCount4 cnt;
+                                for (uint32_t j = 0; j < pairs; ++j) {
+                                    const uint2 s = in[j];
+                                    cnt.add(tile_in(col, s.x));
+                                    cnt.add(tile_in(col, s.y));
+                                }
+                                r = kk > 15 ? 0ull : cnt.ge(kk);
+                            } else {
+                                SlicedCount cnt;
+                                cnt.clear();
+                                for (uint32_t j = 0; j < pairs; ++j) {
+                                    const uint2 s = in[j];
+                                    cnt.add(tile_in(col, s.x), nbits);
+                                    cnt.add(tile_in(col, s.y), nbits);
+                                }
+                                r = cnt.ge(kk);
+                            }
+                        }
+                        if (m.x & 4u) r = ~r;
+                        col[m.z >> 16] = r;
+                        const uint32_t nt = m.x >> 20;  // tallies of the gate: one (its index), or a list
+                        if (nt) {
+                            const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, valid ? (uint32_t)__popcll(r) : 0u);
+                            if (lane == 0 && c) {
+                                if (nt == 1) add(m.w, c);
+                                else
+                                    for (uint32_t j = 0; j < nt; ++j) add(a.tally_list[m.w + j], c);
+                            }
+                        }
+                    }
+                    __syncthreads();
+                }
+                e_begin = end.x;
             }
-            __syncthreads();
             for (uint32_t j = warp; j < a.n_be_tally; j += kWarps) {
                 const uint2 t = a.be_tally[j];
                 const uint32_t c =
                     __reduce_add_sync(0xFFFFFFFFu, valid ? (uint32_t)__popcll(col[t.x * kTileLanes]) : 0u);
                 if (lane == 0 && c) add(t.y, c);
             }
-            for (uint32_t l = 0; l < a.n_layers; ++l) {
-                const uint32_t end = a.layer[l + 1];
-                for (uint32_t i = a.layer[l] + warp; i < end; i += kWarps) {
-                    const uint4 m = a.gates[i];
-                    const uint32_t kind = m.x & 3u;
-                    const uint2 *in = reinterpret_cast<const uint2 *>(a.in + m.y);
-                    uint64_t r = 0;
-                    if (kind == kTileOr) {
-#pragma unroll 2
-                        for (uint32_t j = 0; j < m.z; ++j) {
-                            const uint2 s = in[j];
-                            r |= tile_in(col, s.x) | tile_in(col, s.y);
-                        }
-                    } else if (kind == kTileXor) {
-                        for (uint32_t j = 0; j < m.z; ++j) {
-                            const uint2 s = in[j];
-                            r ^= tile_in(col, s.x) ^ tile_in(col, s.y);
-                        }
-                    } else {
-                        const uint32_t kk = (m.x >> 8) & 0xFFu, nbits = (m.x >> 16) & 0xFu;
-                        if (nbits <= 4) {  // at most 15 inputs
-                            SlicedCount4 cnt;
-                            for (uint32_t j = 0; j < m.z; ++j) {
-                                const uint2 s = in[j];
-                                cnt.add(tile_in(col, s.x));
-                                cnt.add(tile_in(col, s.y));
-                            }
-                            r = kk > 15 ? 0ull : cnt.ge(kk);
-                        } else {
-                            SlicedCount cnt;
-                            cnt.clear();
-                            for (uint32_t j = 0; j < m.z; ++j) {
-                                const uint2 s = in[j];
-                                cnt.add(tile_in(col, s.x), nbits);
-                                cnt.add(tile_in(col, s.y), nbits);
-                            }
-                            r = cnt.ge(kk);
-                        }
-                    }
-                    if (m.x & 4u) r = ~r;
-                    col[(a.n_be + i) * kTileLanes] = r;
-                    const uint32_t nt = m.x >> 20;  // tallies of the gate: one (its index), or a list
-                    if (nt) {
-                        const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, valid ? (uint32_t)__popcll(r) : 0u);
-                        if (lane == 0 && c) {
-                            if (nt == 1) add(m.w, c);
-                            else
-                                for (uint32_t j = 0; j < nt; ++j) add(a.tally_list[m.w + j], c);
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-            if (a.n_layers == 0) __syncthreads();  // the words are free again
+            if (a.n_be_tally) __syncthreads();  // the words are free again
         }
     }
     __syncthreads();

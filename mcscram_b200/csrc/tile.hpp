@@ -8,15 +8,18 @@ namespace mcg {
 namespace dev {
 
 struct TileArgs {
-    const uint4 *be;               // needed events {pdag + 1, event + 1, thr lo, thr hi}: node slots [0, n_be)
-    const uint4 *gates;            // gate i (slot n_be + i), layer by layer: kind | inverted << 2 | k << 8 | counter
-                                   // bits << 16 | tallies << 20, in_begin, input pairs, tally index (or list offset)
+    const uint4 *be;               // needed events, segment by segment: {pdag + 1, event + 1, thr lo,
+                                   // thr hi | first word of the slot << 1}
+    const uint4 *gates;            // gates, layer by layer: kind | inverted << 2 | k << 8 | counter
+                                   // bits << 16 | tallies << 20, in_begin, input pairs | first word of the slot << 16,
+                                   // tally index (or list offset)
     const uint32_t *in;            // inputs, an even number per gate: the slot's byte offset | complemented;
                                    // the last slot is the empty input (zeros)
-    const uint32_t *layer;         // n_layers + 1 gate indices
+    const uint32_t *layer;         // gate indices
+    const uint2 *segment;          // {events' end, layers' end}
     const uint32_t *tally_list;
     const uint2 *be_tally;         // tallied events {slot, tally index}
-    uint32_t n_be, n_slots, n_layers, n_be_tally, n_tally, tally_in_smem;
+    uint32_t n_slots, n_segments, n_be_tally, n_tally, tally_in_smem;
     uint32_t iteration_first, n_iterations;
     uint64_t word_begin, word_count;
     unsigned long long *ones;
@@ -49,7 +52,8 @@ struct BatchTileArgs {
     const BatchTileTree *trees;
     const BatchTileGroup *groups;
     const uint4 *recs;
-    const uint4 *gates;            // as TileArgs but for the last field, the gate's slot; row 0 is the empty input
+    const uint4 *gates;            // as TileArgs but for the last two fields, input pairs and the gate's slot; row 0
+                                   // is the empty input
     const uint32_t *in, *layer;
     const uint2 *segment;          // {events' end, layers' end}
     const uint32_t *event_slot;

@@ -103,8 +103,8 @@ inline TilePlan plan_tile(const Graph &g) {
     return t;
 }
 
-// The plan of the kernels whose rows lie in memory (the batch tile kernel and
-// the strip kernel): the gates in depth-first postorder, cut into segments
+// The plan of the kernels whose rows are used again (the batch tile kernel, the
+// strip kernel, the tile kernel on large trees): the gates in depth-first postorder, cut into segments
 // that each sample their own new events (`events` of them, if so many are
 // left) and then evaluate their gates.  A node's row is free again after the
 // layer that reads it last (by_layer; else after the segment, whose gates may
@@ -120,7 +120,9 @@ struct SegmentPlan {
     uint32_t slots = 0;
 };
 
-inline SegmentPlan plan_segments(const Graph &g, uint32_t events, bool by_layer) {
+// `round`: segments are filled up to whole multiples of so many events with the
+// next one's first.
+inline SegmentPlan plan_segments(const Graph &g, uint32_t events, bool by_layer, uint32_t round = 1) {
     SegmentPlan p;
     TilePlan &t = p.tile;
     const uint32_t nb = g.n_be;
@@ -184,6 +186,12 @@ inline SegmentPlan plan_segments(const Graph &g, uint32_t events, bool by_layer)
     }
     for (uint32_t e = 0; e < nb; ++e)
         if (needs.needed[e] && !sampled[e]) segs.back().events.push_back(e);
+    for (size_t k = 0; k + 1 < segs.size(); ++k) {
+        std::vector<uint32_t> &to = segs[k].events, &from = segs[k + 1].events;
+        const size_t n = std::min<size_t>((round - to.size() % round) % round, from.size());
+        to.insert(to.end(), from.begin(), from.begin() + (std::ptrdiff_t)n);
+        from.erase(from.begin(), from.begin() + (std::ptrdiff_t)n);
+    }
     // reads left of each node; tallied events keep their rows (counted at the end)
     std::vector<uint32_t> reads(g.n_nodes(), 0);
     for (uint32_t i : order)

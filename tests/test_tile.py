@@ -159,3 +159,14 @@ def test_strip_segments(capi, oracle_mod, gpu, n_be, n_gates, tallies):
         want = sum(_popcounts(oracle_mod.eval_words(h, 4 + i, 3, 300)[h.tally_nodes]) for i in range(2))
         assert total == 2 * 300 * 64
         assert np.array_equal(ones, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_be,n_gates,tallies,words", [(600, 400, "all", 40), (900, 700, "root", 33),
+                                                        (1600, 1000, "some", 64), (1600, 1000, "all", 5000),
+                                                        (3000, 300, "root", 100), (900, 0, "all", 70)])
+def test_tile_segments(capi, oracle_mod, gpu, n_be, n_gates, tallies, words):
+    """The fused mode's default shape on trees beyond the tile: in segments, or by
+    the interpreter where too many nodes are live at a time."""
+    g = _far_reads(np.random.default_rng(n_be * 3 + n_gates), n_be, n_gates, tallies)
+    _check(capi, oracle_mod, g, words, 9, passes=2)
