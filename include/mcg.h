@@ -49,16 +49,16 @@ enum mcg_mode {
                              (include/mcg_tune.h): strip, staged or fused, with its CTAs per SM */
     MCG_MODE_LAYERED = 1, /* reference dataflow: materialised node words, one launch per layer */
     MCG_MODE_STAGED = 2,  /* two-phase pipeline: a pure sampler kernel writes basic-event words to
-                             HBM, per-layer gate kernels with fused tallies read them; chunks are
-                             double buffered on two streams so the phases overlap */
+                             HBM, a gate kernel with fused tallies reads them; chunks are double
+                             buffered on two streams so the phases overlap */
     MCG_MODE_STRIP = 3,   /* one persistent kernel per pass: each block takes 256-word strips, its
-                             threads sample every event of their word and then evaluate every gate
-                             for it from scratch rows of their own (n_nodes x 32 words per warp);
-                             sampling and gate work of different blocks overlap on every SM */
+                             threads sample a segment of events for their word and evaluate the gates
+                             it completes, from scratch rows of their own (32 words per warp and live
+                             node); sampling and gate work of different blocks overlap on every SM */
     MCG_MODE_FUSED = 4    /* one persistent kernel per launch chunk: sample, gates, tallies fused; in its
-                             default shape a tree whose node words fit in shared memory (about 880
-                             nodes) is evaluated in tiles of 32 words per block, others (and other
-                             shapes) by an interpreter of the compiled program */
+                             default shape a tree whose live node words fit in shared memory (about
+                             880 at a time) is evaluated in tiles of 32 words per block, others (and
+                             other shapes) by an interpreter of the compiled program */
 };
 
 /* Flattened PDAG handed to the engine.  All arrays are host memory, copied

@@ -1014,20 +1014,22 @@ __global__ void __launch_bounds__(kStripThreads, MINB) k_strip(StripArgs a) {
             if (s_ones[i]) atomicAdd(&a.ones[i], s_ones[i]);
 }
 
-// Tile kernel (fused mode, trees whose node words fit in shared memory): a
+// Tile kernel (fused mode, trees whose live node words fit in shared memory): a
 // block evaluates 32 sample words (lane = word) of every needed node at a
-// time, the whole pass in one launch.  Its warps share the events out, then
-// the gates of each layer.  Nothing but the counters leaves the SM, an event's
-// table entries are made by the warp that samples it (17 lanes, one product
+// time, the whole pass in one launch.  Its warps share out the events of a
+// segment (small trees: of the tree), then the gates of each of its layers.
+// Nothing but the counters leaves the SM, an event's
+// table entries are made by the warp that samples it (18 lanes, one product
 // each: 1.5 % of the sampling), and a pass spreads over events x words, so
 // that 4,096 words of a small tree already keep every SM busy where the
 // interpreter had 16 blocks.  1,024 threads per SM in all (64 registers each),
 // in as many blocks as the tile's size allows: one block's layers run under
 // the sampling of another.  Bound by the sampler's multiplies (0.86 of the
 // register-only sampler; the rest is gate work and the last, partly filled
-// round of events).  262,221 words of the 200-event tree: 1.98 ms, the
-// interpreter 2.67 ms; 4,096 words of a 60-event tree: 23 us of kernel where
-// the staged pipeline ran nine launches.
+// round of events).  262,221 words of the 200-event tree: 2.00 ms, the
+// interpreter 2.67 ms; 233,937 words of a 1,030-event tree in segments 9.1 ms
+// and 13.9; 4,096 words of a 60-event tree: 18 us of kernel where the
+// staged pipeline ran nine launches.
 // An input record's word: x, or its complement.
 __device__ __forceinline__ uint64_t tile_in(const uint64_t *col, uint32_t rec) {
     const uint64_t x = *reinterpret_cast<const uint64_t *>(reinterpret_cast<const unsigned char *>(col) + (rec & ~1u));
