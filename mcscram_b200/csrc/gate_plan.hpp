@@ -67,15 +67,28 @@ inline GatePlan plan_gates(const Graph &g, const std::vector<uint32_t> &depth) {
         part_of[c] = p;
     }
     t.largest = (uint32_t)*std::max_element(load.begin(), load.end());
+    for (uint32_t i = 0; i < ng; ++i) part_of[i] = part_of[find(i)];
+    // by part, in a part by layer: two counting sorts
+    auto sorted = [&](const std::vector<uint32_t> &from, const std::vector<uint32_t> &key) {
+        std::vector<uint32_t> at(*std::max_element(key.begin(), key.end()) + 2, 0), to(ng);
+        for (uint32_t k : key) ++at[k + 1];
+        std::partial_sum(at.begin(), at.end(), at.begin());
+        for (uint32_t i : from) to[at[key[i]]++] = i;
+        return to;
+    };
     std::vector<uint32_t> order(ng);
     std::iota(order.begin(), order.end(), 0u);
-    for (uint32_t i = 0; i < ng; ++i) part_of[i] = part_of[find(i)];
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) {
-        return part_of[x] != part_of[y] ? part_of[x] < part_of[y] : depth[x] < depth[y];
-    });
-    std::vector<std::vector<uint32_t>> tallies(ng);
+    if (ng) order = sorted(sorted(order, depth), part_of);
+    // the gates' tallies: gate i's are tally[tally_at[i]] .. tally[tally_at[i + 1] - 1]
+    std::vector<uint32_t> tally_at(ng + 1, 0), tally(g.tally_nodes.size());
+    for (uint32_t v : g.tally_nodes)
+        if (v >= nb) ++tally_at[v - nb + 1];
+    std::partial_sum(tally_at.begin(), tally_at.end(), tally_at.begin());
+    std::vector<uint32_t> next(tally_at);
     for (uint32_t k = 0; k < (uint32_t)g.tally_nodes.size(); ++k)
-        if (g.tally_nodes[k] >= nb) tallies[g.tally_nodes[k] - nb].push_back(k);
+        if (g.tally_nodes[k] >= nb) tally[next[g.tally_nodes[k] - nb]++] = k;
+    t.gates.reserve(2 * (size_t)ng);
+    t.tally.reserve(ng);
 
     std::vector<uint32_t> rec;
     uint32_t at = 0;
@@ -115,10 +128,9 @@ inline GatePlan plan_gates(const Graph &g, const std::vector<uint32_t> &depth) {
                 while (rec.size() < 4 || rec.size() % 4) rec.push_back(count ? rec[count - 1] : 0u);
                 t.gates.push_back(make_uint4(rec[0], rec[1], rec[2], rec[3]));
                 t.in.insert(t.in.end(), rec.begin() + 4, rec.end());
-                const std::vector<uint32_t> &mine = tallies[i];
-                t.tally.push_back(make_uint2(mine.size() == 1 ? mine[0] : (uint32_t)t.tally_list.size(),
-                                             (uint32_t)mine.size()));
-                if (mine.size() > 1) t.tally_list.insert(t.tally_list.end(), mine.begin(), mine.end());
+                const uint32_t *mine = tally.data() + tally_at[i], n_mine = tally_at[i + 1] - tally_at[i];
+                t.tally.push_back(make_uint2(n_mine == 1 ? mine[0] : (uint32_t)t.tally_list.size(), n_mine));
+                if (n_mine > 1) t.tally_list.insert(t.tally_list.end(), mine, mine + n_mine);
             }
             t.layer.push_back(make_uint2(first, at));
         }
