@@ -619,7 +619,7 @@ mcg_status setup_fused(mcg_engine *e, const mcg_run_desc &run) {
 // lane, for twice the blocks (32,768 words of the 5,000-event tree: 6.23 ms,
 // one word per lane 6.55; 2,048 words of a 500-event tree: no difference).
 constexpr uint64_t kWideGateWords = 148 * 64;
-constexpr uint32_t kStripBlocksPerSm = 6;
+constexpr uint32_t kStripBlocksPerSm = 6, kStripFewBlocks = 4;
 
 mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
                         const std::function<uint64_t(uint64_t)> &extra_words) {
@@ -698,6 +698,11 @@ mcg_status setup_strip(mcg_engine *e, const mcg_run_desc &run) {
     MCG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, mcg::dev::kStripThreads, e->strip_smem));
     if (per_sm < 1) return mcg::fail(MCG_ERR_INVALID, "strip kernel does not fit on an SM");
     e->strip_grid = (uint32_t)(prop.multiProcessorCount * per_sm);
+    if (!run.ctas_per_sm) {
+        const mcg_status few = mcg::set_smem_limit(strip_kernel(kStripFewBlocks), e->strip_smem);
+        if (few != MCG_OK) return few;
+        e->strip_few = kStripFewBlocks * (uint64_t)prop.multiProcessorCount;
+    }
     const uint64_t warps = (uint64_t)e->strip_grid * (mcg::dev::kStripThreads / 32);
     const uint64_t bytes = warps * e->strip_rows * mcg::dev::kStripLanes * sizeof(uint64_t);
     MCG_CUDA(work_alloc(e, (void **)&e->d_strip_scratch, bytes));
@@ -731,6 +736,14 @@ mcg_status run_strip(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t w
     a.word_begin = word_begin;
     a.word_count = count;
     a.queue = e->d_queue;
+    // No more blocks than strips: they then lie one to an SM, two to an SM and so
+    // on, where of a full grid any blocks take the strips.  At up to four strips
+    // per SM the kernel for four blocks, whose threads have 64 registers, is the
+    // faster one.  958 events, 27,987 words: 1.95 ms (five blocks 2.07, full grid
+    // 5.4); 151,552 words: 5.38 (five blocks 5.53, full grid of six 7.9).
+    const uint64_t strips = (count + mcg::dev::kStripThreads - 1) / mcg::dev::kStripThreads;
+    const uint32_t blocks = strips <= e->strip_few ? kStripFewBlocks : e->strip_blocks;
+    const uint32_t grid = (uint32_t)std::min<uint64_t>(e->strip_grid, std::max<uint64_t>(strips, 1));
     for (uint32_t it = 0; it < n_it; ++it) {
         const uint32_t iteration = it_first + it;
         if (e->n_strip_be > 0 && e->table_iteration != iteration) {
@@ -754,7 +767,7 @@ mcg_status run_strip(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t w
             ++e->prof_used;
             MCG_CUDA(cudaEventRecord(p0, e->stream));
         }
-        strip_kernel(e->strip_blocks)<<<e->strip_grid, mcg::dev::kStripThreads, e->strip_smem, e->stream>>>(a);
+        strip_kernel(blocks)<<<grid, mcg::dev::kStripThreads, e->strip_smem, e->stream>>>(a);
         ++e->launches;
         if (p1) MCG_CUDA(cudaEventRecord(p1, e->stream));
         MCG_CUDA(cudaGetLastError());

@@ -99,6 +99,7 @@ struct mcg_engine {
     uint32_t *d_strip_inputs = nullptr, *d_strip_gin = nullptr;
     uint32_t n_strip_be = 0, n_strip_segments = 0, n_strip_be_tally = 0, strip_rows = 1;
     uint32_t strip_grid = 0;
+    uint64_t strip_few = 0;                // up to so many strips the four-block kernel runs
     uint32_t strip_smem = 0;               // tally counters in shared memory (0: global atomics)
     uint32_t strip_blocks = 6;             // resident blocks per SM the kernel is built for
 

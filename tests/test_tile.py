@@ -170,3 +170,16 @@ def test_tile_segments(capi, oracle_mod, gpu, n_be, n_gates, tallies, words):
     the interpreter where too many nodes are live at a time."""
     g = _far_reads(np.random.default_rng(n_be * 3 + n_gates), n_be, n_gates, tallies)
     _check(capi, oracle_mod, g, words, 9, passes=2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("words", [1, 256, 257, 4 * 148 * 256, 4 * 148 * 256 + 1])
+def test_strip_grid(capi, oracle_mod, gpu, words):
+    """Strip passes of fewer strips than blocks, and both sides of the line between the kernels."""
+    g = synth.small_tree(4)
+    g = g.with_tallies(np.arange(g.n_nodes))
+    with capi.Engine(g, mode=capi.MODE_STRIP) as e:
+        e.run(2, 1, 11, words)
+        ones, total = e.tallies()
+    assert total == words * 64
+    assert np.array_equal(ones, _popcounts(oracle_mod.eval_words(g, 2, 11, words)[g.tally_nodes]))
