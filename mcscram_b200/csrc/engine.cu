@@ -24,6 +24,7 @@
 #include "mcg_tune.h"
 #include "program.hpp"
 #include "smem_limit.hpp"
+#include "staged_run.hpp"
 #include "tile_plan.hpp"
 
 namespace {
@@ -905,9 +906,9 @@ mcg_status staged_join(mcg_engine *e) {
 
 mcg_status run_staged_impl(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {
     uint64_t chunk = 0;
-    mcg_status st = staged_fork(e);
-    if (st == MCG_OK) st = staged_chunks(e, &chunk, it_first, n_it, word_begin, count, false);
-    return st == MCG_OK ? staged_join(e) : st;
+    return mcg::forked_run([&] { return staged_fork(e); },
+                           [&] { return staged_chunks(e, &chunk, it_first, n_it, word_begin, count, false); },
+                           [&] { return staged_join(e); });
 }
 
 mcg_status launch_fused(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -16,6 +17,7 @@
 #include "error.hpp"
 #include "mcg_is.h"
 #include "smem_limit.hpp"
+#include "staged_run.hpp"
 
 namespace {
 
@@ -968,6 +970,14 @@ mcg_status check_thresholds(const mcg::Graph &g, const uint64_t *q_thr) {
                                           " must lie in [1, 2^32 - 1] (or equal a constant nominal one)");
 }
 
+// The engine as it is outside of a run: no hooks, its own event table.
+void plain_sampling(mcg_engine *e) {
+    e->chunk_hook = nullptr;
+    e->sample_hook = nullptr;
+    e->d_be_sample = nullptr;
+    e->table_iteration = 0xFFFFFFFFu;
+}
+
 }  // namespace
 
 struct mcg_is {
@@ -1066,6 +1076,7 @@ mcg_status mcg_is_run(mcg_is *is, const uint64_t *q_thr, uint32_t iteration, uin
     MCG_CUDA(cudaSetDevice(e->device));
     MCG_CUDA(cudaMemcpyAsync(is->d_q, q_thr, nb * sizeof(uint64_t), cudaMemcpyHostToDevice, e->stream));
     const bool want_ce = ce_num != nullptr;
+    const mcg::AtExit plain_again([e] { plain_sampling(e); });
     e->d_be_sample = is->d_be_q;
     e->table_iteration = 0xFFFFFFFFu;  // the sampler table follows the proposal
     int sms = 148;
@@ -1105,10 +1116,7 @@ mcg_status mcg_is_run(mcg_is *is, const uint64_t *q_thr, uint32_t iteration, uin
         return MCG_OK;
     };
     MCG_CUDA(cudaEventRecord(is->ev0, e->stream));
-    mcg_status st = mcg::internal::run_staged(e, iteration, 1, word_begin, word_count);
-    e->chunk_hook = nullptr;
-    e->d_be_sample = nullptr;
-    e->table_iteration = 0xFFFFFFFFu;
+    const mcg_status st = mcg::internal::run_staged(e, iteration, 1, word_begin, word_count);
     if (st != MCG_OK) return st;
     MCG_CUDA(cudaEventRecord(is->ev1, e->stream));
     std::vector<double> sums(4ull + (want_ce ? nb : 0));
@@ -1699,6 +1707,7 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
     args.n_be_nodes = g.n_be;
     args.error = b->d_cut_error;
     if (cut_comp >= 0) MCG_CUDA(cudaMemsetAsync(b->d_cut_error, 0, sizeof(unsigned int), e->stream));
+    const mcg::AtExit plain_again([e] { plain_sampling(e); });
     e->chunk_hook = [=](cudaStream_t s, const uint64_t *buf, uint64_t W) -> mcg_status {
         IsBatchArgs p = args;
         p.buf = buf;
@@ -1717,56 +1726,58 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
     uint32_t last_comp = 0;
     for (uint32_t c = 0; c < nc; ++c)
         if (comp_words[c]) last_comp = c;
-    st = mcg::internal::fork_staged(e);
-    for (uint32_t c = 0; c < nc && st == MCG_OK; ++c) {
-        if (!comp_words[c]) continue;
-        e->d_be_sample = b->d_be_q + c * nb;
-        e->table_iteration = 0xFFFFFFFFu;  // the sampler table follows the component
-        if ((int)c == cut_comp) {
-            CutArgs ca{};
-            ca.n_inst = n_inst;
-            ca.n_be = g.n_be;
-            ca.root_row = b->d_root;
-            ca.gate = b->d_cut_gate;
-            ca.inputs = e->d_inputs;
-            ca.S = b->d_cut_S;
-            ca.tab = b->d_cut_tab;
-            ca.tree_ok = b->d_tree_ok;
-            ca.shared = b->d_shared;
-            ca.gate_occ = b->d_gate_occ;
-            ca.z_begin = b->d_z_begin;
-            ca.z_event = b->d_z_event;
-            ca.q = b->d_q + (uint64_t)cut_comp * nb;
-            ca.z_occ_begin = b->d_z_occ_begin;
-            ca.z_occ = b->d_z_occ;
-            ca.seed = mix64_host(((uint64_t)iteration << 32) ^ 0x5bd1e995u);
-            ca.error = b->d_cut_error;
-            const uint32_t n_z = (uint32_t)b->z_event.size();
-            e->sample_hook = [=](cudaStream_t s, uint64_t *buf, uint64_t W, uint64_t wb) -> mcg_status {
-                CutArgs x = ca;
-                x.buf = buf;
-                x.W = W;
-                x.word_begin = wb;
-                const uint64_t threads = (uint64_t)x.n_inst * W * 64;
-                if (n_z) {
-                    const dim3 grid((n_z + kDrawEvents - 1) / kDrawEvents, (uint32_t)((W + kDrawWords - 1) / kDrawWords));
-                    k_cut_draw<<<grid, 256, 0, s>>>(x, n_z);
-                }
-                k_cut_force<<<(uint32_t)((threads + 255) / 256), 256, 0, s>>>(x);
-                const cudaError_t err = cudaGetLastError();
-                if (err != cudaSuccess) return mcg::fail(MCG_ERR_CUDA, std::string("k_cut_force: ") + cudaGetErrorString(err));
-                return MCG_OK;
-            };
-        }
-        st = mcg::internal::add_staged(e, &chunk, iteration, word_begin + off, comp_words[c], c != last_comp);
-        e->sample_hook = nullptr;
-        off += comp_words[c];
+    std::function<mcg_status(cudaStream_t, uint64_t *, uint64_t, uint64_t)> cut_hook;
+    if (cut_comp >= 0) {
+        CutArgs ca{};
+        ca.n_inst = n_inst;
+        ca.n_be = g.n_be;
+        ca.root_row = b->d_root;
+        ca.gate = b->d_cut_gate;
+        ca.inputs = e->d_inputs;
+        ca.S = b->d_cut_S;
+        ca.tab = b->d_cut_tab;
+        ca.tree_ok = b->d_tree_ok;
+        ca.shared = b->d_shared;
+        ca.gate_occ = b->d_gate_occ;
+        ca.z_begin = b->d_z_begin;
+        ca.z_event = b->d_z_event;
+        ca.q = b->d_q + (uint64_t)cut_comp * nb;
+        ca.z_occ_begin = b->d_z_occ_begin;
+        ca.z_occ = b->d_z_occ;
+        ca.seed = mix64_host(((uint64_t)iteration << 32) ^ 0x5bd1e995u);
+        ca.error = b->d_cut_error;
+        const uint32_t n_z = (uint32_t)b->z_event.size();
+        cut_hook = [=](cudaStream_t s, uint64_t *buf, uint64_t W, uint64_t wb) -> mcg_status {
+            CutArgs x = ca;
+            x.buf = buf;
+            x.W = W;
+            x.word_begin = wb;
+            const uint64_t threads = (uint64_t)x.n_inst * W * 64;
+            if (n_z) {
+                const dim3 grid((n_z + kDrawEvents - 1) / kDrawEvents, (uint32_t)((W + kDrawWords - 1) / kDrawWords));
+                k_cut_draw<<<grid, 256, 0, s>>>(x, n_z);
+            }
+            k_cut_force<<<(uint32_t)((threads + 255) / 256), 256, 0, s>>>(x);
+            const cudaError_t err = cudaGetLastError();
+            if (err != cudaSuccess) return mcg::fail(MCG_ERR_CUDA, std::string("k_cut_force: ") + cudaGetErrorString(err));
+            return MCG_OK;
+        };
     }
-    if (st == MCG_OK) st = mcg::internal::join_staged(e);
-    e->chunk_hook = nullptr;
-    e->sample_hook = nullptr;
-    e->d_be_sample = nullptr;
-    e->table_iteration = 0xFFFFFFFFu;
+    auto add_components = [&]() -> mcg_status {
+        for (uint32_t c = 0; c < nc; ++c) {
+            if (!comp_words[c]) continue;
+            e->d_be_sample = b->d_be_q + c * nb;
+            e->table_iteration = 0xFFFFFFFFu;  // the sampler table follows the component
+            e->sample_hook = (int)c == cut_comp ? cut_hook : nullptr;
+            const mcg_status added =
+                mcg::internal::add_staged(e, &chunk, iteration, word_begin + off, comp_words[c], c != last_comp);
+            if (added != MCG_OK) return added;
+            off += comp_words[c];
+        }
+        return MCG_OK;
+    };
+    st = mcg::forked_run([&] { return mcg::internal::fork_staged(e); }, add_components,
+                         [&] { return mcg::internal::join_staged(e); });
     if (st != MCG_OK) return st;
     MCG_CUDA(cudaEventRecord(b->ev1, e->stream));
     MCG_CUDA(cudaMemcpyAsync(tree_sums, b->d_sums, 4ull * n_inst * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
