@@ -40,7 +40,10 @@ typedef struct mcg_is_result {
 
 /* Engine over a flattened graph whose tally list holds exactly the top
  * event.  Nominal thresholds come from graph->be_threshold.  Uses the
- * staged kernels (layered_max_words = words per chunk). */
+ * staged kernels (layered_max_words = words per chunk).  Takes as many basic
+ * events as two doubles each fit in a block's shared memory (14,528 on a
+ * B200) and refuses more with MCG_ERR_INVALID before it allocates anything;
+ * mcg_is_batch_create with one tree has no such limit. */
 mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run, mcg_is **out);
 mcg_status mcg_is_destroy(mcg_is *is);
 

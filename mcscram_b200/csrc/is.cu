@@ -1004,6 +1004,26 @@ static void default_chunk(const mcg_graph_desc &graph, mcg_run_desc &run) {
     run.layered_max_words = std::min<uint64_t>(1ull << 17, std::max<uint64_t>(256, (24ull << 30) / (nn * 8)));
 }
 
+// Frees everything; keeps the error message a failed create has just set.
+static void release_is(mcg_is *is) {
+    const std::string keep = mcg::last_error();
+    if (is->engine) {
+        cudaSetDevice(is->engine->device);
+        cudaStreamSynchronize(is->engine->stream);
+    }
+    cudaFree(is->d_be_q);
+    cudaFree(is->d_q);
+    cudaFree(is->d_a);
+    cudaFree(is->d_sums);
+    cudaFree(is->d_C);
+    cudaFree(is->d_tree);
+    if (is->ev0) cudaEventDestroy(is->ev0);
+    if (is->ev1) cudaEventDestroy(is->ev1);
+    if (is->engine) mcg_destroy(is->engine);
+    delete is;
+    mcg::last_error() = keep;
+}
+
 extern "C" {
 
 mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in, mcg_is **out) {
@@ -1015,19 +1035,19 @@ mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in
     if (run_in) run = *run_in;
     run.mode = MCG_MODE_STAGED;
     default_chunk(*graph, run);
-    auto is = std::make_unique<mcg_is>();
+    // the entry point's limit, before any of the engine's buffers is taken (a
+    // device that does not exist is refused by the engine's creation)
+    mcg::DeviceShape prop;
+    if (mcg::device_shape(&prop, run.device) != cudaSuccess) cudaGetLastError();
+    else if (2ull * graph->n_be * sizeof(double) > prop.sharedMemPerBlockOptin)
+        return mcg::fail(MCG_ERR_INVALID, "too many basic events for a single-tree handle (mcg_is_batch_create with one "
+                                          "tree takes them)");
+    auto is = std::unique_ptr<mcg_is, void (*)(mcg_is *)>(new mcg_is, release_is);
     mcg_status st = mcg::internal::create_with_extra(
         graph, &run, [](uint64_t words) { return hit_weight_words(1, words); }, &is->engine);
     if (st != MCG_OK) return st;
     mcg_engine *e = is->engine;
     const uint32_t nb = e->graph.n_be;
-    mcg::DeviceShape prop;
-    MCG_CUDA(mcg::device_shape(&prop, e->device));
-    if (2ull * std::max<uint32_t>(nb, 1) * sizeof(double) > prop.sharedMemPerBlockOptin) {
-        // the documented limit of this entry point (larger trees: mcg_is_batch_create with one tree)
-        mcg_destroy(e);
-        return mcg::fail(MCG_ERR_INVALID, "too many basic events for the weights kernel's shared memory");
-    }
     MCG_CUDA(cudaMalloc((void **)&is->d_be_q, std::max<uint32_t>(nb, 1) * sizeof(uint4)));
     MCG_CUDA(cudaMalloc((void **)&is->d_a, std::max<uint32_t>(nb, 1) * sizeof(double)));
     MCG_CUDA(cudaMalloc((void **)&is->d_q, std::max<uint32_t>(nb, 1) * sizeof(uint64_t)));
@@ -1045,21 +1065,7 @@ mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in
 
 mcg_status mcg_is_destroy(mcg_is *is) {
     mcg::clear_error();
-    if (!is) return MCG_OK;
-    if (is->engine) {
-        cudaSetDevice(is->engine->device);
-        cudaStreamSynchronize(is->engine->stream);
-    }
-    cudaFree(is->d_be_q);
-    cudaFree(is->d_q);
-    cudaFree(is->d_a);
-    cudaFree(is->d_sums);
-    cudaFree(is->d_C);
-    cudaFree(is->d_tree);
-    if (is->ev0) cudaEventDestroy(is->ev0);
-    if (is->ev1) cudaEventDestroy(is->ev1);
-    if (is->engine) mcg_destroy(is->engine);
-    delete is;
+    if (is) release_is(is);
     return MCG_OK;
 }
 
