@@ -120,14 +120,38 @@ struct mcg_batch {
 
 namespace {
 
-void release(mcg_batch *b) {
+void drop_graph(mcg_batch *b) {
     if (b->graph) cudaGraphExecDestroy(b->graph);
+    b->graph = nullptr;
+}
+
+// Gives all of the tile kernel's memory back.
+void drop_tile(mcg_batch *b) {
+    drop_graph(b);
     for (void *p : b->tile_tables) cudaFree(p);
+    b->tile_tables.clear();
     cudaFree(b->d_tile_groups);
     cudaFree(b->d_tile_recs);
+    cudaFree(b->d_scratch);
+    b->d_tile_groups = nullptr;
+    b->d_tile_recs = nullptr;
+    b->d_scratch = nullptr;
+    b->cap_tile_groups = b->cap_tile_recs = 0;
+    b->tile = false;
+}
+
+// A per-run buffer of n elements; the captured graph goes with a buffer it reads.
+template <typename T>
+cudaError_t grow(mcg_batch *b, T **p, uint64_t &cap, uint64_t n) {
+    if (n <= cap && *p) return cudaSuccess;
+    drop_graph(b);
+    return ensure(p, cap, n);
+}
+
+void release(mcg_batch *b) {
+    drop_tile(b);
     cudaFree(b->d_ops);
     cudaFree(b->d_tree_off);
-    cudaFree(b->d_scratch);
     cudaFree(b->d_queue);
     cudaFree(b->d_inst_tree);
     cudaFree(b->d_thr_off);
@@ -155,7 +179,7 @@ mcg_status upload_table(mcg_batch *b, const T **dptr, const std::vector<T> &v) {
 constexpr uint64_t kTileScratchMost = 16ull << 30;
 
 // Tables of k_batch_tile; leaves b->tile false where the interpreter has to
-// take the batch (rows too large, or no memory for them).
+// take the batch (rows too large).  Out of memory is the caller's to handle.
 mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
     using namespace mcg::dev;
     std::vector<uint4> gates;
@@ -199,13 +223,7 @@ mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
     const uint64_t stride = most_slots * kTileRow;
     const uint64_t blocks = (uint64_t)prop.multiProcessorCount * kBatchTileBlocks;
     if (stride * blocks > kTileScratchMost) return MCG_OK;
-    const cudaError_t err = cudaMalloc((void **)&b->d_scratch, stride * blocks);
-    if (err == cudaErrorMemoryAllocation) {
-        cudaGetLastError();
-        b->d_scratch = nullptr;
-        return MCG_OK;
-    }
-    MCG_CUDA(err);
+    MCG_CUDA(cudaMalloc((void **)&b->d_scratch, stride * blocks));
     BatchTileArgs &a = b->tile_args;
     mcg_status st;
     if ((st = upload_table(b, &a.trees, b->tile_trees)) != MCG_OK || (st = upload_table(b, &a.gates, gates)) != MCG_OK ||
@@ -221,6 +239,24 @@ mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
     a.scratch_stride = stride;
     b->tile = true;
     return MCG_OK;
+}
+
+// The interpreter's scratch, where it runs the batch and has none yet.
+mcg_status interpreter_scratch(mcg_batch *b) {
+    if (b->tile || !b->max_global || b->d_scratch) return MCG_OK;
+    void *p = nullptr;
+    MCG_CUDA(cudaMalloc(&p, (size_t)b->max_global * b->share * b->scratch_stride * sizeof(uint64_t)));
+    b->d_scratch = static_cast<uint64_t *>(p);
+    return MCG_OK;
+}
+
+// From here on the interpreter runs the batch: it needs less memory where few
+// values are live, and no records per group.
+mcg_status use_interpreter(mcg_batch *b) {
+    cudaGetLastError();
+    mcg::clear_error();
+    drop_tile(b);
+    return interpreter_scratch(b);
 }
 
 mcg_status setup(mcg_batch *b, const mcg_run_desc &run) {
@@ -270,14 +306,11 @@ mcg_status setup(mcg_batch *b, const mcg_run_desc &run) {
     MCG_CUDA(cudaMalloc((void **)&b->d_tree_off, b->tree_op_offset.size() * sizeof(uint32_t)));
     MCG_CUDA(cudaMemcpy(b->d_tree_off, b->tree_op_offset.data(), b->tree_op_offset.size() * sizeof(uint32_t),
                         cudaMemcpyHostToDevice));
-    if (!run.smem_slots && !run.ctas_per_sm) {  // the default shape
-        const mcg_status ts = setup_tile(b, prop);
-        if (ts != MCG_OK) return ts;
-    }
-    if (b->max_global && !b->tile)
-        MCG_CUDA(cudaMalloc((void **)&b->d_scratch,
-                            (size_t)b->max_global * b->share * b->scratch_stride * sizeof(uint64_t)));
     MCG_CUDA(cudaMalloc((void **)&b->d_queue, sizeof(unsigned long long)));
+    mcg_status ts = MCG_OK;
+    if (!run.smem_slots && !run.ctas_per_sm) ts = setup_tile(b, prop);  // the default shape
+    if (ts == MCG_ERR_OOM || (ts == MCG_OK && !b->tile)) ts = use_interpreter(b);
+    if (ts != MCG_OK) return ts;
     const mcg_status lim = mcg::set_smem_limit(batch_kernel(b->ctas_per_sm, b->share, b->atleast), b->smem_bytes);
     if (lim != MCG_OK) return lim;
     if (run.stream) {
@@ -293,10 +326,7 @@ mcg_status setup(mcg_batch *b, const mcg_run_desc &run) {
 
 // Captures [zero queue, zero ones, persistent launch] for the current shapes.
 mcg_status capture(mcg_batch *b, uint32_t n_inst, uint32_t iteration, uint64_t words) {
-    if (b->graph) {
-        cudaGraphExecDestroy(b->graph);
-        b->graph = nullptr;
-    }
+    drop_graph(b);
     mcg::dev::BatchArgs a;
     a.ops = b->d_ops;
     a.tree_op_offset = b->d_tree_off;
@@ -351,6 +381,73 @@ mcg_status capture(mcg_batch *b, uint32_t n_inst, uint32_t iteration, uint64_t w
     b->g_instances = n_inst;
     b->g_iteration = iteration;
     b->g_words = words;
+    return MCG_OK;
+}
+
+// A validated run, from its groups to its results on the host.
+mcg_status run_instances(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tree, const uint64_t *thr_offset,
+                         const uint64_t *thresholds, uint64_t n_thr, uint32_t iteration, uint64_t words,
+                         uint64_t *ones) {
+    const mcg_status scratch = interpreter_scratch(b);
+    if (scratch != MCG_OK) return scratch;
+    // groups of up to `share` consecutive instances of one tree (up to 16 in tiles)
+    const uint32_t most = b->tile ? mcg::dev::kTileInstances : b->share;
+    std::vector<uint32_t> gfirst, gsize;
+    for (uint32_t i = 0; i < n_inst;) {
+        uint32_t n = 1;
+        while (n < most && i + n < n_inst && inst_tree[i + n] == inst_tree[i]) ++n;
+        gfirst.push_back(i);
+        gsize.push_back(n);
+        i += n;
+    }
+    MCG_CUDA(grow(b, &b->d_inst_tree, b->cap_inst, n_inst));
+    MCG_CUDA(grow(b, &b->d_thr_off, b->cap_inst2, n_inst));
+    MCG_CUDA(grow(b, &b->d_thr, b->cap_thr, n_thr));
+    MCG_CUDA(grow(b, &b->d_ones, b->cap_ones, n_inst));
+    MCG_CUDA(grow(b, &b->d_group_first, b->cap_grp, gfirst.size()));
+    MCG_CUDA(grow(b, &b->d_group_size, b->cap_grp2, gsize.size()));
+    if (b->n_groups != (uint32_t)gfirst.size()) drop_graph(b);
+    b->n_groups = (uint32_t)gfirst.size();
+    std::vector<mcg::dev::BatchTileGroup> groups;
+    if (b->tile) {
+        // the costliest first (events, and about as much again for every 20
+        // instances), so that the last items of the queue are small
+        std::vector<uint32_t> order(gfirst.size());
+        for (uint32_t i = 0; i < (uint32_t)order.size(); ++i) order[i] = i;
+        auto cost = [&](uint32_t i) { return (uint64_t)b->tile_trees[inst_tree[gfirst[i]]].n_be * (20u + gsize[i]); };
+        std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return cost(x) > cost(y); });
+        uint64_t recs = 0;
+        for (uint32_t i : order) {
+            const uint32_t t = inst_tree[gfirst[i]];
+            groups.push_back({t, gfirst[i], gsize[i], 0u, recs});
+            recs += b->tile_trees[t].n_be;
+        }
+        MCG_CUDA(grow(b, &b->d_tile_groups, b->cap_tile_groups, groups.size()));
+        MCG_CUDA(grow(b, &b->d_tile_recs, b->cap_tile_recs, std::max<uint64_t>(recs, 1) * mcg::dev::kTileRec));
+        b->n_tile_groups = (uint32_t)groups.size();
+        MCG_CUDA(cudaMemcpyAsync(b->d_tile_groups, groups.data(), groups.size() * sizeof(groups[0]),
+                                 cudaMemcpyHostToDevice, b->stream));
+    }
+    MCG_CUDA(cudaMemcpyAsync(b->d_group_first, gfirst.data(), gfirst.size() * sizeof(uint32_t),
+                             cudaMemcpyHostToDevice, b->stream));
+    MCG_CUDA(cudaMemcpyAsync(b->d_group_size, gsize.data(), gsize.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                             b->stream));
+    MCG_CUDA(cudaMemcpyAsync(b->d_inst_tree, inst_tree, n_inst * sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream));
+    MCG_CUDA(cudaMemcpyAsync(b->d_thr_off, thr_offset, n_inst * sizeof(uint64_t), cudaMemcpyHostToDevice, b->stream));
+    MCG_CUDA(cudaMemcpyAsync(b->d_thr, thresholds, n_thr * sizeof(uint64_t), cudaMemcpyHostToDevice, b->stream));
+    if (!b->graph || b->g_instances != n_inst || b->g_iteration != iteration || b->g_words != words) {
+        const mcg_status st = capture(b, n_inst, iteration, words);
+        if (st != MCG_OK) return st;
+    }
+    MCG_CUDA(cudaEventRecord(b->ev0, b->stream));
+    MCG_CUDA(cudaGraphLaunch(b->graph, b->stream));
+    MCG_CUDA(cudaEventRecord(b->ev1, b->stream));
+    ++b->launches;
+    MCG_CUDA(cudaMemcpyAsync(ones, b->d_ones, n_inst * sizeof(uint64_t), cudaMemcpyDeviceToHost, b->stream));
+    MCG_CUDA(cudaStreamSynchronize(b->stream));
+    float ms = 0;
+    MCG_CUDA(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
+    b->last_ms = ms;
     return MCG_OK;
 }
 
@@ -415,74 +512,14 @@ mcg_status mcg_batch_run(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tre
     }
     for (uint64_t k = 0; k < n_thr; ++k)
         if (thresholds[k] > (1ull << 32)) return mcg::fail(MCG_ERR_INVALID, "threshold above 2^32");
-    // groups of up to `share` consecutive instances of one tree (up to 16 in tiles)
-    const uint32_t most = b->tile ? mcg::dev::kTileInstances : b->share;
-    std::vector<uint32_t> gfirst, gsize;
-    for (uint32_t i = 0; i < n_inst;) {
-        uint32_t n = 1;
-        while (n < most && i + n < n_inst && inst_tree[i + n] == inst_tree[i]) ++n;
-        gfirst.push_back(i);
-        gsize.push_back(n);
-        i += n;
-    }
-    if ((uint64_t)gfirst.size() * slabs >= 0xFFFFFFFFull) return mcg::fail(MCG_ERR_INVALID, "too many work items");
     MCG_CUDA(cudaSetDevice(b->device));
-    const uint32_t *old_tree = b->d_inst_tree, *old_gf = b->d_group_first, *old_gs = b->d_group_size;
-    const uint64_t *old_off = b->d_thr_off, *old_thr = b->d_thr;
-    const unsigned long long *old_ones = b->d_ones;
-    MCG_CUDA(ensure(&b->d_inst_tree, b->cap_inst, n_inst));
-    MCG_CUDA(ensure(&b->d_thr_off, b->cap_inst2, n_inst));
-    MCG_CUDA(ensure(&b->d_thr, b->cap_thr, n_thr));
-    MCG_CUDA(ensure(&b->d_ones, b->cap_ones, n_inst));
-    MCG_CUDA(ensure(&b->d_group_first, b->cap_grp, gfirst.size()));
-    MCG_CUDA(ensure(&b->d_group_size, b->cap_grp2, gsize.size()));
-    bool moved = old_tree != b->d_inst_tree || old_off != b->d_thr_off || old_thr != b->d_thr ||
-                       old_ones != b->d_ones || old_gf != b->d_group_first || old_gs != b->d_group_size ||
-                       b->n_groups != (uint32_t)gfirst.size();
-    b->n_groups = (uint32_t)gfirst.size();
-    std::vector<mcg::dev::BatchTileGroup> groups;
-    if (b->tile) {
-        // the costliest first (events, and about as much again for every 20
-        // instances), so that the last items of the queue are small
-        std::vector<uint32_t> order(gfirst.size());
-        for (uint32_t i = 0; i < (uint32_t)order.size(); ++i) order[i] = i;
-        auto cost = [&](uint32_t i) { return (uint64_t)b->tile_trees[inst_tree[gfirst[i]]].n_be * (20u + gsize[i]); };
-        std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return cost(x) > cost(y); });
-        uint64_t recs = 0;
-        for (uint32_t i : order) {
-            const uint32_t t = inst_tree[gfirst[i]];
-            groups.push_back({t, gfirst[i], gsize[i], 0u, recs});
-            recs += b->tile_trees[t].n_be;
-        }
-        const void *old_groups = b->d_tile_groups, *old_recs = b->d_tile_recs;
-        MCG_CUDA(ensure(&b->d_tile_groups, b->cap_tile_groups, groups.size()));
-        MCG_CUDA(ensure(&b->d_tile_recs, b->cap_tile_recs, std::max<uint64_t>(recs, 1) * mcg::dev::kTileRec));
-        moved = moved || old_groups != b->d_tile_groups || old_recs != b->d_tile_recs;
-        b->n_tile_groups = (uint32_t)groups.size();
-        MCG_CUDA(cudaMemcpyAsync(b->d_tile_groups, groups.data(), groups.size() * sizeof(groups[0]),
-                                 cudaMemcpyHostToDevice, b->stream));
+    mcg_status st = run_instances(b, n_inst, inst_tree, thr_offset, thresholds, n_thr, iteration, words, ones);
+    if (st == MCG_ERR_OOM && b->tile) {  // a buffer did not fit next to the tile kernel's memory
+        st = use_interpreter(b);
+        if (st == MCG_OK)
+            st = run_instances(b, n_inst, inst_tree, thr_offset, thresholds, n_thr, iteration, words, ones);
     }
-    MCG_CUDA(cudaMemcpyAsync(b->d_group_first, gfirst.data(), gfirst.size() * sizeof(uint32_t),
-                             cudaMemcpyHostToDevice, b->stream));
-    MCG_CUDA(cudaMemcpyAsync(b->d_group_size, gsize.data(), gsize.size() * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                             b->stream));
-    MCG_CUDA(cudaMemcpyAsync(b->d_inst_tree, inst_tree, n_inst * sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream));
-    MCG_CUDA(cudaMemcpyAsync(b->d_thr_off, thr_offset, n_inst * sizeof(uint64_t), cudaMemcpyHostToDevice, b->stream));
-    MCG_CUDA(cudaMemcpyAsync(b->d_thr, thresholds, n_thr * sizeof(uint64_t), cudaMemcpyHostToDevice, b->stream));
-    if (!b->graph || moved || b->g_instances != n_inst || b->g_iteration != iteration || b->g_words != words) {
-        const mcg_status st = capture(b, n_inst, iteration, words);
-        if (st != MCG_OK) return st;
-    }
-    MCG_CUDA(cudaEventRecord(b->ev0, b->stream));
-    MCG_CUDA(cudaGraphLaunch(b->graph, b->stream));
-    MCG_CUDA(cudaEventRecord(b->ev1, b->stream));
-    ++b->launches;
-    MCG_CUDA(cudaMemcpyAsync(ones, b->d_ones, n_inst * sizeof(uint64_t), cudaMemcpyDeviceToHost, b->stream));
-    MCG_CUDA(cudaStreamSynchronize(b->stream));
-    float ms = 0;
-    MCG_CUDA(cudaEventElapsedTime(&ms, b->ev0, b->ev1));
-    b->last_ms = ms;
-    return MCG_OK;
+    return st;
 }
 
 mcg_status mcg_batch_info_get(mcg_batch *b, mcg_batch_info *info) {
