@@ -60,7 +60,7 @@ cudaError_t upload(T **dptr, const std::vector<T> &v) {
 // kKeptBytes bytes are kept per device, and a failed allocation first
 // frees the kept ones.  mcg_trim_memory frees them all.
 constexpr size_t kKeptBuffers = 2;
-constexpr size_t kKeptBytes = 32ull << 30;
+constexpr size_t kKeptBytes = 33ull << 30;  // two chunk buffers of 16 GiB, with 1 GiB of hit weights behind one
 
 struct KeptBuffer {
     void *ptr;
