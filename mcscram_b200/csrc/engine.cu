@@ -632,6 +632,7 @@ mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
     words = (words + 255) / 256 * 256;
     e->stage_words = words;
     const uint64_t extra = extra_words ? extra_words(words) : 0;
+    e->stage_extra_words = extra;
     MCG_CUDA(work_alloc(e, (void **)&e->d_stage[0], (nn * words + extra) * sizeof(uint64_t)));
     MCG_CUDA(work_alloc(e, (void **)&e->d_stage[1], nn * words * sizeof(uint64_t)));
     if (extra) e->d_stage_extra = e->d_stage[0] + nn * words;

@@ -86,6 +86,7 @@ struct mcg_engine {
     uint32_t sampler_smem = 0;          // dynamic smem that caps sampler blocks per SM
     uint64_t stage_words = 0;           // words per chunk the stage buffers hold
     uint64_t *d_stage_extra = nullptr;  // extra words the creator asked for, behind the first stage buffer
+    uint64_t stage_extra_words = 0;
     cudaStream_t s_a = nullptr, s_b = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_a[2] = {nullptr, nullptr}, ev_b[2] = {nullptr, nullptr};
     cudaEvent_t ev_join_a = nullptr, ev_join_b = nullptr;

@@ -857,11 +857,22 @@ __global__ void __launch_bounds__(kWeightThreads) k_is_ce(const __grid_constant_
 }
 
 // Size of the buffer between the two kernels (behind the engine's first stage
-// buffer), for chunks of `words` words: 64 weights per tree and word, at most
-// 1 GiB; longer chunks are taken in several launches.
-uint64_t hit_weight_words(uint32_t n_inst, uint64_t words) {
-    const uint64_t most = std::max<uint64_t>(32, (1ull << 27) / (64ull * n_inst));
-    return 64ull * n_inst * std::min<uint64_t>(words, most);
+// buffer), for chunks of `words` words: 64 weights per tree and word, `most` in
+// all or those of 32 words; longer chunks are taken in several launches.
+constexpr uint64_t kHitWeights = 1ull << 27;  // 1 GiB
+uint64_t hit_weight_words(uint32_t n_inst, uint64_t words, uint64_t most) {
+    return 64ull * n_inst * std::min<uint64_t>(words, std::max<uint64_t>(32, most / (64ull * n_inst)));
+}
+
+// create(most): a handle with so many hit weights; with the least of them, and
+// without the buffers kept on the device, where there is no room for that.
+template <class Create>
+mcg_status create_with_room(int device, Create create) {
+    const mcg_status st = create(kHitWeights);
+    if (st != MCG_ERR_OOM) return st;
+    cudaGetLastError();
+    mcg_trim_memory(device);
+    return create(0);
 }
 
 // Queues both kernels for one chunk of W words.
@@ -1024,6 +1035,29 @@ static void release_is(mcg_is *is) {
     mcg::last_error() = keep;
 }
 
+// A single-tree handle with so many hit weights (hit_weight_words).
+static mcg_status create_is(const mcg_graph_desc *graph, const mcg_run_desc &run, uint64_t most, mcg_is **out) {
+    auto is = std::unique_ptr<mcg_is, void (*)(mcg_is *)>(new mcg_is, release_is);
+    mcg_status st = mcg::internal::create_with_extra(
+        graph, &run, [most](uint64_t words) { return hit_weight_words(1, words, most); }, &is->engine);
+    if (st != MCG_OK) return st;
+    mcg_engine *e = is->engine;
+    const uint32_t nb = e->graph.n_be;
+    MCG_CUDA(cudaMalloc((void **)&is->d_be_q, std::max<uint32_t>(nb, 1) * sizeof(uint4)));
+    MCG_CUDA(cudaMalloc((void **)&is->d_a, std::max<uint32_t>(nb, 1) * sizeof(double)));
+    MCG_CUDA(cudaMalloc((void **)&is->d_q, std::max<uint32_t>(nb, 1) * sizeof(uint64_t)));
+    MCG_CUDA(cudaMalloc((void **)&is->d_sums, (4ull + nb) * sizeof(double)));
+    is->d_ce = is->d_sums + 4;
+    MCG_CUDA(cudaMalloc((void **)&is->d_C, sizeof(double)));
+    MCG_CUDA(cudaMalloc((void **)&is->d_tree, 3 * sizeof(uint32_t)));
+    const uint32_t tree[3] = {0u, nb, e->graph.tally_nodes[0]};
+    MCG_CUDA(cudaMemcpy(is->d_tree, tree, sizeof(tree), cudaMemcpyHostToDevice));
+    MCG_CUDA(cudaEventCreate(&is->ev0));
+    MCG_CUDA(cudaEventCreate(&is->ev1));
+    *out = is.release();
+    return MCG_OK;
+}
+
 extern "C" {
 
 mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in, mcg_is **out) {
@@ -1042,25 +1076,7 @@ mcg_status mcg_is_create(const mcg_graph_desc *graph, const mcg_run_desc *run_in
     else if (2ull * graph->n_be * sizeof(double) > prop.sharedMemPerBlockOptin)
         return mcg::fail(MCG_ERR_INVALID, "too many basic events for a single-tree handle (mcg_is_batch_create with one "
                                           "tree takes them)");
-    auto is = std::unique_ptr<mcg_is, void (*)(mcg_is *)>(new mcg_is, release_is);
-    mcg_status st = mcg::internal::create_with_extra(
-        graph, &run, [](uint64_t words) { return hit_weight_words(1, words); }, &is->engine);
-    if (st != MCG_OK) return st;
-    mcg_engine *e = is->engine;
-    const uint32_t nb = e->graph.n_be;
-    MCG_CUDA(cudaMalloc((void **)&is->d_be_q, std::max<uint32_t>(nb, 1) * sizeof(uint4)));
-    MCG_CUDA(cudaMalloc((void **)&is->d_a, std::max<uint32_t>(nb, 1) * sizeof(double)));
-    MCG_CUDA(cudaMalloc((void **)&is->d_q, std::max<uint32_t>(nb, 1) * sizeof(uint64_t)));
-    MCG_CUDA(cudaMalloc((void **)&is->d_sums, (4ull + nb) * sizeof(double)));
-    is->d_ce = is->d_sums + 4;
-    MCG_CUDA(cudaMalloc((void **)&is->d_C, sizeof(double)));
-    MCG_CUDA(cudaMalloc((void **)&is->d_tree, 3 * sizeof(uint32_t)));
-    const uint32_t tree[3] = {0u, nb, e->graph.tally_nodes[0]};
-    MCG_CUDA(cudaMemcpy(is->d_tree, tree, sizeof(tree), cudaMemcpyHostToDevice));
-    MCG_CUDA(cudaEventCreate(&is->ev0));
-    MCG_CUDA(cudaEventCreate(&is->ev1));
-    *out = is.release();
-    return MCG_OK;
+    return create_with_room(run.device, [&](uint64_t most) { return create_is(graph, run, most, out); });
 }
 
 mcg_status mcg_is_destroy(mcg_is *is) {
@@ -1112,7 +1128,7 @@ mcg_status mcg_is_run(mcg_is *is, const uint64_t *q_thr, uint32_t iteration, uin
     args.sums = is->d_sums;
     args.weights = want_ce ? reinterpret_cast<double *>(e->d_stage_extra) : nullptr;
     args.ce = want_ce ? is->d_ce : nullptr;
-    const uint64_t weight_words = hit_weight_words(1, e->stage_words) / 64u;
+    const uint64_t weight_words = e->stage_extra_words / 64u;
     e->chunk_hook = [=](cudaStream_t s, const uint64_t *buf, uint64_t W) -> mcg_status {
         IsBatchArgs p = args;
         p.buf = buf;
@@ -1326,6 +1342,41 @@ bool add_companions(const mcg_graph_desc &d, uint32_t n_inst, const uint32_t *be
     return true;
 }
 
+// A handle over n_inst trees with so many hit weights (hit_weight_words).
+mcg_status create_is_batch(const mcg_graph_desc *graph, uint32_t n_inst, const uint32_t *be_begin,
+                           const mcg_run_desc &run, uint64_t most, mcg_is_batch **out) {
+    auto b = std::unique_ptr<mcg_is_batch, void (*)(mcg_is_batch *)>(new mcg_is_batch, [](mcg_is_batch *x) {
+        release_batch(x);
+        delete x;
+    });
+    b->n_inst = n_inst;
+    b->be_begin.assign(be_begin, be_begin + n_inst + 1);
+    b->n_gates_in = graph->n_gates;
+    Augmented aug;
+    b->companions = add_companions(*graph, n_inst, be_begin, aug);
+    b->companion = aug.companion;
+    b->tree_gates_ok = aug.tree_ok;
+    mcg_status st = mcg::internal::create_with_extra(
+        b->companions ? &aug.desc : graph, &run,
+        [n_inst, most](uint64_t words) { return hit_weight_words(n_inst, words, most); }, &b->engine);
+    if (st != MCG_OK) return st;
+    const mcg::Graph &g = b->engine->graph;
+    const std::string bad = check_partition(g, b->be_begin);
+    if (!bad.empty()) return mcg::fail(MCG_ERR_INVALID, bad);
+    const uint32_t nb = std::max<uint32_t>(g.n_be, 1);
+    MCG_CUDA(cudaSetDevice(b->engine->device));
+    MCG_CUDA(cudaMalloc((void **)&b->d_ce, nb * sizeof(double)));
+    MCG_CUDA(cudaMalloc((void **)&b->d_sums, 4ull * n_inst * sizeof(double)));
+    MCG_CUDA(cudaMalloc((void **)&b->d_be_begin, (n_inst + 1ull) * sizeof(uint32_t)));
+    MCG_CUDA(cudaMalloc((void **)&b->d_root, n_inst * sizeof(uint32_t)));
+    MCG_CUDA(cudaMemcpy(b->d_be_begin, be_begin, (n_inst + 1ull) * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    MCG_CUDA(cudaMemcpy(b->d_root, g.tally_nodes.data(), n_inst * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    MCG_CUDA(cudaEventCreate(&b->ev0));
+    MCG_CUDA(cudaEventCreate(&b->ev1));
+    *out = b.release();
+    return MCG_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1345,36 +1396,8 @@ mcg_status mcg_is_batch_create(const mcg_graph_desc *graph, uint32_t n_inst, con
     if (run_in) run = *run_in;
     run.mode = MCG_MODE_STAGED;
     default_chunk(*graph, run);
-    auto b = std::unique_ptr<mcg_is_batch, void (*)(mcg_is_batch *)>(new mcg_is_batch, [](mcg_is_batch *x) {
-        release_batch(x);
-        delete x;
-    });
-    b->n_inst = n_inst;
-    b->be_begin.assign(be_begin, be_begin + n_inst + 1);
-    b->n_gates_in = graph->n_gates;
-    Augmented aug;
-    b->companions = add_companions(*graph, n_inst, be_begin, aug);
-    b->companion = aug.companion;
-    b->tree_gates_ok = aug.tree_ok;
-    mcg_status st = mcg::internal::create_with_extra(
-        b->companions ? &aug.desc : graph, &run,
-        [n_inst](uint64_t words) { return hit_weight_words(n_inst, words); }, &b->engine);
-    if (st != MCG_OK) return st;
-    const mcg::Graph &g = b->engine->graph;
-    const std::string bad = check_partition(g, b->be_begin);
-    if (!bad.empty()) return mcg::fail(MCG_ERR_INVALID, bad);
-    const uint32_t nb = std::max<uint32_t>(g.n_be, 1);
-    MCG_CUDA(cudaSetDevice(b->engine->device));
-    MCG_CUDA(cudaMalloc((void **)&b->d_ce, nb * sizeof(double)));
-    MCG_CUDA(cudaMalloc((void **)&b->d_sums, 4ull * n_inst * sizeof(double)));
-    MCG_CUDA(cudaMalloc((void **)&b->d_be_begin, (n_inst + 1ull) * sizeof(uint32_t)));
-    MCG_CUDA(cudaMalloc((void **)&b->d_root, n_inst * sizeof(uint32_t)));
-    MCG_CUDA(cudaMemcpy(b->d_be_begin, be_begin, (n_inst + 1ull) * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    MCG_CUDA(cudaMemcpy(b->d_root, g.tally_nodes.data(), n_inst * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    MCG_CUDA(cudaEventCreate(&b->ev0));
-    MCG_CUDA(cudaEventCreate(&b->ev1));
-    *out = b.release();
-    return MCG_OK;
+    return create_with_room(run.device,
+                            [&](uint64_t most) { return create_is_batch(graph, n_inst, be_begin, run, most, out); });
 }
 
 mcg_status mcg_is_batch_destroy(mcg_is_batch *b) {
@@ -1701,7 +1724,7 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
     args.sums = b->d_sums;
     args.ce = ce_num ? b->d_ce : nullptr;
     args.weights = ce_num ? reinterpret_cast<double *>(e->d_stage_extra) : nullptr;
-    const uint64_t weight_words = hit_weight_words(n_inst, e->stage_words) / (64ull * n_inst);
+    const uint64_t weight_words = e->stage_extra_words / (64ull * n_inst);
     args.cut_comp = cut_comp;
     args.cut_logS = b->d_cut_logS;
     args.cut_gate = b->d_cut_gate;
