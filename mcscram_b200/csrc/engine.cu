@@ -38,6 +38,7 @@ using mcg::internal::kFusedThreads;
     do {                                                                                        \
         cudaError_t err_ = (call);                                                              \
         if (err_ != cudaSuccess) {                                                              \
+            cudaGetLastError(); /* reported here, and not by the next launch's check */         \
             return mcg::fail(err_ == cudaErrorMemoryAllocation ? MCG_ERR_OOM : MCG_ERR_CUDA,    \
                              std::string(#call) + ": " + cudaGetErrorString(err_));             \
         }                                                                                       \
@@ -1064,6 +1065,7 @@ mcg_status mcg::internal::create_with_extra(const mcg_graph_desc *graph, const m
         // the counters and, behind them, two snapshot slots (mcg_snapshot_tallies)
         if (cudaMalloc((void **)&e->d_tally, 3 * nt * sizeof(unsigned long long)) != cudaSuccess ||
             cudaMemset(e->d_tally, 0, nt * sizeof(unsigned long long)) != cudaSuccess) {
+            cudaGetLastError();
             st = mcg::fail(MCG_ERR_OOM, "tally allocation failed");
             break;
         }
@@ -1315,6 +1317,7 @@ mcg_status mcg_sampler_peak(int32_t device, uint64_t n_events, uint64_t n_words,
     uint2 *table = nullptr;
     MCG_CUDA(cudaMalloc((void **)&sink, n_words * sizeof(uint64_t)));
     if (cudaMalloc((void **)&table, n_events * mcg::dev::kEventTableStride * sizeof(uint2)) != cudaSuccess) {
+        cudaGetLastError();
         cudaFree(sink);
         return mcg::fail(MCG_ERR_OOM, "sampler table allocation failed");
     }

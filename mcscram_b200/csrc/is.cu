@@ -25,6 +25,7 @@ namespace {
     do {                                                                                        \
         cudaError_t err_ = (call);                                                              \
         if (err_ != cudaSuccess) {                                                              \
+            cudaGetLastError(); /* reported here, and not by the next launch's check */         \
             return mcg::fail(err_ == cudaErrorMemoryAllocation ? MCG_ERR_OOM : MCG_ERR_CUDA,    \
                              std::string(#call) + ": " + cudaGetErrorString(err_));             \
         }                                                                                       \
