@@ -371,6 +371,7 @@ mcg_status build_layered_tables(mcg_engine *e) {
         const mcg::GatePlan plan = mcg::plan_gates(g, layer);
         e->n_gate_parts = (uint32_t)plan.part.size() - 1;
         e->gates_largest_part = plan.largest;
+        e->gates_count = plan.counts;
         MCG_CUDA(upload(&e->d_gates, plan.gates));
         MCG_CUDA(upload(&e->d_gate_in, plan.in));
         MCG_CUDA(upload(&e->d_gate_tally, plan.tally));
@@ -778,6 +779,12 @@ mcg_status run_strip(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t w
     return MCG_OK;
 }
 
+using StageGatesKernel = void (*)(const mcg::dev::StageGateArgs);
+StageGatesKernel stage_gates_kernel(bool wide, bool count) {
+    if (wide) return count ? mcg::dev::k_stage_gates<2, true> : mcg::dev::k_stage_gates<2, false>;
+    return count ? mcg::dev::k_stage_gates<1, true> : mcg::dev::k_stage_gates<1, false>;
+}
+
 // One chunk: phase A (sampling) on s_a into buffer `set`, phase B (gates and
 // tallies) on s_b once A is done; `last`: no chunk follows it.  A reuses a buffer only after the B that
 // read it (two chunks earlier) has finished.
@@ -852,8 +859,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         const uint64_t blocks = tiles * g.n_gates / std::max<uint32_t>(e->gates_largest_part, 1);
         const uint32_t threads = blocks >= 3ull * e->gate_sms ? 256u : blocks >= 2ull * e->gate_sms ? 512u : 1024u;
         if (!last && e->gates_beside_sampler) tiles = std::min<uint64_t>(tiles, 2ull * e->gate_sms);
-        (wide ? mcg::dev::k_stage_gates<2> : mcg::dev::k_stage_gates<1>)<<<
-            dim3((uint32_t)tiles, e->n_gate_parts), threads, 0, e->s_b>>>(a);
+        stage_gates_kernel(wide, e->gates_count)<<<dim3((uint32_t)tiles, e->n_gate_parts), threads, 0, e->s_b>>>(a);
         ++e->launches;
     }
     if (e->n_be_tally) {

@@ -36,6 +36,7 @@ struct GatePlan {
     std::vector<uint32_t> part;
     std::vector<uint2> layer;
     uint32_t largest = 0;            // gates of the largest part
+    bool counts = false;             // some gate is a kGateCount
 };
 
 // `depth`: each gate's layer, from 1 on.
@@ -117,6 +118,7 @@ inline GatePlan plan_gates(const Graph &g, const std::vector<uint32_t> &depth) {
                     }
                     while (nbits < 8 && (n >> nbits) != 0) ++nbits;
                 }
+                t.counts |= kind == kGateCount;
                 rec.clear();
                 for (uint32_t j = last_only ? n - 1 : 0u; j < n; ++j) {
                     const bool negated = j >= n - g.gate_neg_count[i];
