@@ -369,8 +369,10 @@ mcg_status build_layered_tables(mcg_engine *e) {
         if (st != MCG_OK) return st;
     } else if (e->mode == MCG_MODE_STAGED) {
         const mcg::GatePlan plan = mcg::plan_gates(g, layer);
-        e->n_gate_parts = (uint32_t)plan.part.size() - 1;
+        e->n_gate_parts = plan.parts();
+        e->n_gate_layers = plan.part[plan.parts() + 1] - plan.part[plan.parts()];
         e->gates_largest_part = plan.largest;
+        e->gate_block_ns = plan.block_ns;
         e->gates_count = plan.counts;
         MCG_CUDA(upload(&e->d_gates, plan.gates));
         MCG_CUDA(upload(&e->d_gate_in, plan.in));
@@ -785,6 +787,26 @@ StageGatesKernel stage_gates_kernel(bool wide, bool count) {
     return count ? mcg::dev::k_stage_gates<1, true> : mcg::dev::k_stage_gates<1, false>;
 }
 
+// Blocks that share the gates of a layer and tile, a launch per layer; 0: every
+// layer in one launch, a block per tile and part.  The one launch leaves most of
+// the chip idle where a pass has few tiles, and its blocks walk all gates of a
+// part (gate_block_ns) where a launch per layer costs about 4 us, and more the
+// more tiles share the rows.  The line is where the two sides crossed for 50 to
+// 8,000 gates of 2 to 60 inputs in 2 to 50 layers: 64 words of 8,000 gates of 6
+// inputs in 5 layers 57 us by layers and 283 in one launch, 256 words of 3,000 of
+// 20 inputs 70 and 198, 2,048 words of 2,000 k-of-16 gates in 40 layers 378 and
+// 370; from 3,000 words on one launch is the faster one but for layers of
+// hundreds of gates.
+constexpr uint64_t kGateLaunchNs = 4000;
+uint32_t gate_splits(const mcg_engine *e, uint64_t tiles, uint64_t blocks) {
+    if (2 * blocks > e->gate_sms ||
+        e->gate_block_ns * e->gate_sms <= kGateLaunchNs * e->n_gate_layers * (e->gate_sms + 3 * blocks))
+        return 0;
+    const uint64_t wanted = (e->graph.n_gates / e->n_gate_layers + 7) / 8;  // a gate per warp of 256 threads
+    const uint64_t most = (8ull * e->gate_sms + tiles - 1) / tiles;
+    return (uint32_t)std::max<uint64_t>(1, std::min(wanted, most));
+}
+
 // One chunk: phase A (sampling) on s_a into buffer `set`, phase B (gates and
 // tallies) on s_b once A is done; `last`: no chunk follows it.  A reuses a buffer only after the B that
 // read it (two chunks earlier) has finished.
@@ -859,8 +881,19 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         const uint64_t blocks = tiles * g.n_gates / std::max<uint32_t>(e->gates_largest_part, 1);
         const uint32_t threads = blocks >= 3ull * e->gate_sms ? 256u : blocks >= 2ull * e->gate_sms ? 512u : 1024u;
         if (!last && e->gates_beside_sampler) tiles = std::min<uint64_t>(tiles, 2ull * e->gate_sms);
-        stage_gates_kernel(wide, e->gates_count)<<<dim3((uint32_t)tiles, e->n_gate_parts), threads, 0, e->s_b>>>(a);
-        ++e->launches;
+        const StageGatesKernel kern = stage_gates_kernel(wide, e->gates_count);
+        const uint32_t splits = gate_splits(e, tiles, blocks);
+        if (!splits) {
+            a.layers = e->n_gate_layers;
+            kern<<<dim3((uint32_t)tiles, e->n_gate_parts), threads, 0, e->s_b>>>(a);
+            ++e->launches;
+        } else {
+            a.part_first = e->n_gate_parts;  // all parts as one
+            for (a.layers = 1; a.first < e->n_gate_layers; ++a.first) {
+                kern<<<dim3((uint32_t)tiles, 1, splits), 256, 0, e->s_b>>>(a);
+                ++e->launches;
+            }
+        }
     }
     if (e->n_be_tally) {
         dim3 grid = rows_grid(1, e->n_be_tally, 256);

@@ -67,7 +67,9 @@ struct mcg_engine {
     uint32_t *d_gate_part = nullptr;
     uint2 *d_gate_layer = nullptr;
     uint32_t n_gate_parts = 0;
+    uint32_t n_gate_layers = 0;
     uint32_t gates_largest_part = 0;    // gates
+    uint64_t gate_block_ns = 0;         // a block's walk over the costliest part (gate_plan.hpp)
     bool gates_count = false;           // some gate counts in bit slices
     uint32_t gate_sms = 0;              // SMs of the device
     bool gates_beside_sampler = false;  // few gate blocks while the next chunk is sampled

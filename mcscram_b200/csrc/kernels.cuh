@@ -530,8 +530,7 @@ static __global__ void __launch_bounds__(256) k_layer_tally(const uint32_t *__re
 
 // ---------------------------------------------------------------------------
 // Staged pipeline.  Phase A samples basic-event words into buf rows
-// [0, n_be); phase B evaluates one layer of gates per launch into rows
-// n_be + g, with tallies fused.
+// [0, n_be); phase B evaluates the gates into rows n_be + g, with tallies fused.
 
 // Per-pass event table (philox.cuh): thread (e, g) fills entry g of event e.
 static __global__ void __launch_bounds__(256) k_event_table(const uint4 *__restrict__ be, uint32_t n_be, uint32_t t3,
@@ -577,7 +576,8 @@ __global__ void __launch_bounds__(256, 4) k_stage_be(const uint4 *__restrict__ b
     }
 }
 
-// Phase B: every layer of gates in one launch.  A block takes 32 * WPL words
+// Phase B: every layer of gates in one launch, or a launch per layer for few words
+// of many gates (gate_splits).  A block takes 32 * WPL words
 // (lane = WPL neighbouring words, one load each of a row) of one part
 // (gate_plan.hpp); its warps share out the gates of a layer, and a block
 // barrier ends the layer.  A block's gates read rows that the block or phase A
@@ -596,6 +596,8 @@ struct StageGateArgs {
     const uint32_t *part;
     const uint2 *layer;
     uint64_t words, stride;  // per row: words in use, words from row to row
+    uint32_t part_first;     // part of blockIdx.y = 0
+    uint32_t first, layers;  // the layers that the launch takes of every part
     uint64_t *buf;
     unsigned long long *ones;
 };
@@ -756,8 +758,11 @@ __global__ void __launch_bounds__(kGateThreadsMost) k_stage_gates(const __grid_c
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t warps = blockDim.x >> 5;
     const uint32_t stride = (uint32_t)(a.stride * sizeof(uint64_t));
-    const uint32_t l_begin = a.part[blockIdx.y], l_end = a.part[blockIdx.y + 1];
-    if (l_begin == l_end) return;
+    // more than one block of a part (blockIdx.z) only where the launch takes one layer
+    const uint32_t step = warps * gridDim.z, mine0 = blockIdx.z * warps + warp;
+    const uint32_t *part = a.part + a.part_first + blockIdx.y;
+    const uint32_t l_begin = part[0] + a.first, l_end = min(l_begin + a.layers, part[1]);
+    if (l_begin >= l_end) return;
     const uint32_t tiles = (uint32_t)((a.words + 32 * WPL - 1) / (32 * WPL));
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const uint64_t w0 = ((uint64_t)tile * 32u + lane) * WPL;
@@ -767,7 +772,7 @@ __global__ void __launch_bounds__(kGateThreadsMost) k_stage_gates(const __grid_c
         char *col = reinterpret_cast<char *>(a.buf + (valid ? w0 : 0));
         uint32_t l = l_begin;
         uint2 range = a.layer[l];
-        uint32_t i = range.x + warp;
+        uint32_t i = range.x + mine0;
         uint4 m{}, q{};
         auto head = [&](uint32_t g) {
             m = a.gates[2 * (uint64_t)g];
@@ -777,13 +782,13 @@ __global__ void __launch_bounds__(kGateThreadsMost) k_stage_gates(const __grid_c
         for (;;) {
             // the warp's next gate, in this layer or the next: its records are
             // loaded under this gate's rows
-            const bool mine = i < range.y, last = i + warps >= range.y;
+            const bool mine = i < range.y, last = i + step >= range.y;
             const uint4 cm = m, cq = q;
             const uint32_t gate = i;
-            i += warps;
+            i += step;
             if (last && ++l < l_end) {
                 range = a.layer[l];
-                i = range.x + warp;
+                i = range.x + mine0;
             }
             if (i < range.y) head(i);
             if (mine) {
