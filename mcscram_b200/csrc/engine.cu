@@ -619,11 +619,11 @@ mcg_status setup_fused(mcg_engine *e, const mcg_run_desc &run) {
     return MCG_OK;
 }
 
-// From this many words on (a block of 64 per SM), gate blocks take two words
-// per lane: half the loads and instructions per word.  Fewer words are one per
-// lane, for twice the blocks (32,768 words of the 5,000-event tree: 6.23 ms,
-// one word per lane 6.55; 2,048 words of a 500-event tree: no difference).
-constexpr uint64_t kWideGateWords = 148 * 64;
+// From a block of so many words per SM on, gate blocks take two words per lane:
+// half the loads and instructions per word.  Fewer words are one per lane, for
+// twice the blocks (32,768 words of the 5,000-event tree: 6.23 ms, one word per
+// lane 6.55; 2,048 words of a 500-event tree: no difference).
+constexpr uint64_t kWideGateWords = 64;
 constexpr uint32_t kStripBlocksPerSm = 6, kStripFewBlocks = 4;
 
 mcg_status setup_staged(mcg_engine *e, const mcg_run_desc &run,
@@ -870,7 +870,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         a.stride = stride;
         a.buf = buf;
         a.ones = e->d_tally;
-        const bool wide = stride % 2 == 0 && W >= kWideGateWords;
+        const bool wide = stride % 2 == 0 && W >= kWideGateWords * e->gate_sms;
         uint64_t tiles = (W + (wide ? 63 : 31)) / (wide ? 64 : 32);
         // Warps per block: the fewer blocks share the chip, the more of a
         // layer's gates a block takes at a time.  Blocks are counted at the
