@@ -804,9 +804,11 @@ __global__ void __launch_bounds__(kWeightThreads, NC <= 2 ? 8 : 4) k_is_weights(
 // share of the words, reading the weights k_is_weights left of the samples
 // where the event and the top event fired, and one reduction per warp (inside
 // the weights kernel it was one per event and 32 words, with an FP64 atomic
-// each: 5.4 ms of the 20).  Shares of at most 256 words: the events whose
-// proposal is near 1/2 read every word and would be a long tail (0.31 ms on
-// the set above; 0.75 ms with 1,024 words).
+// each: 5.4 ms of the 20).  32 U words at a time; bound by the latency of the
+// weights, so the words an event fires in often are read four at a time, and few
+// events' words are shared out to more warps (launch_weights): 4,096 words of 60
+// events at 0.3 take 21 us, 131 a word at a time in shares of 256.
+template <int U>
 __global__ void __launch_bounds__(kWeightThreads) k_is_ce(const __grid_constant__ IsBatchArgs p, uint32_t n_events) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t e = blockIdx.x * kWeightWarps + (threadIdx.x >> 5);
@@ -821,16 +823,16 @@ __global__ void __launch_bounds__(kWeightThreads) k_is_ce(const __grid_constant_
     const uint64_t *top = p.buf + (uint64_t)p.root_row[lo] * p.W + p.w_begin;
     const double *weights = p.weights + (uint64_t)lo * p.w_count * 64u;
     double c = 0.0;
-    const uint64_t step = 128ull * gridDim.y;
-    for (uint64_t w0 = 128ull * blockIdx.y; w0 < p.w_count; w0 += step) {
-        uint64_t x[4];
+    const uint64_t step = 32ull * U * gridDim.y;
+    for (uint64_t w0 = 32ull * U * blockIdx.y; w0 < p.w_count; w0 += step) {
+        uint64_t x[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             const uint64_t w = w0 + 32u * u + lane;
             x[u] = w < p.w_count ? row[w] : 0ull;
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             const uint64_t w = w0 + 32u * u + lane;
             if (x[u]) x[u] &= top[w];
             // a word with few samples is its lane's; a dense one (an event whose proposal is near 1/2) is read by
@@ -840,12 +842,22 @@ __global__ void __launch_bounds__(kWeightThreads) k_is_ce(const __grid_constant_
             if (!dense)
                 for (uint64_t b = x[u]; b; b &= b - 1)
                     c += weights[w * 64u + (uint32_t)__ffsll((long long)b) - 1u];
-            for (; m; m &= m - 1) {
-                const int src = __ffs((int)m) - 1;
-                const uint64_t xe = __shfl_sync(0xFFFFFFFFu, x[u], src);
-                const double *ww = weights + (w0 + 32u * u + (uint32_t)src) * 64u + lane;
-                if ((xe >> lane) & 1ull) c += ww[0];
-                if ((xe >> (lane + 32u)) & 1ull) c += ww[32];
+            while (m) {
+                double v[4][2];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {  // past the last dense word: lane 0's, with no sample
+                    const int src = m ? __ffs((int)m) - 1 : 0;
+                    const uint64_t xe = __shfl_sync(0xFFFFFFFFu, x[u], src) & (m ? ~0ull : 0ull);
+                    m &= m - 1;
+                    const double *ww = weights + (w0 + 32u * u + (uint32_t)src) * 64u + lane;
+                    v[k][0] = (xe >> lane) & 1ull ? ww[0] : 0.0;
+                    v[k][1] = (xe >> (lane + 32u)) & 1ull ? ww[32] : 0.0;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    c += v[k][0];
+                    c += v[k][1];
+                }
             }
         }
     }
@@ -894,9 +906,14 @@ cudaError_t launch_weights(IsBatchArgs p, uint32_t n_events, uint64_t weight_wor
         else k_is_weights<kMaxComponents><<<blocks, kWeightThreads, 0, s>>>(p);
         if (p.ce && n_events) {
             const uint32_t eb = (n_events + kWeightWarps - 1) / kWeightWarps;
+            // shares of at most 256 words: the events whose proposal is near 1/2 read every word and would be a
+            // long tail (16 trees of 55 to 9,956 events, 2,048 words: 0.31 ms, 0.75 with 1,024 words); of as few as
+            // 32 where the events do not give every SM 16 warps
             uint32_t split = 1;
-            while (p.w_count / split > 256) split *= 2;
-            k_is_ce<<<dim3(eb, split), kWeightThreads, 0, s>>>(p, n_events);
+            while (p.w_count / split > 256 ||
+                   (p.w_count / split > 32 && (uint64_t)n_events * split < 16ull * (uint64_t)sms))
+                split *= 2;
+            (p.w_count / split < 128 ? k_is_ce<1> : k_is_ce<4>)<<<dim3(eb, split), kWeightThreads, 0, s>>>(p, n_events);
         }
         const cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) return err;
