@@ -194,6 +194,13 @@ mcg_status mcg_program_info_get(mcg_engine *engine, mcg_program_info *info);
 mcg_status mcg_compile(const mcg_graph_desc *graph, uint32_t smem_slot_budget, uint32_t flags,
                        mcg_program_info *info, uint32_t *ops, uint64_t ops_capacity);
 
+/* The kernel that a pass of word_count words takes on a fused-mode engine (by
+ * the tree and the pass; the results are the same): *tile_threads is the block
+ * size of the tile kernel or 0 for the interpreter, *segments the parts in which
+ * the tile kernel takes the tree (0: it does not fit).  NULL pointers are
+ * skipped; other modes return MCG_ERR_STATE. */
+mcg_status mcg_fused_kernel(mcg_engine *e, uint64_t word_count, uint32_t *tile_threads, uint32_t *segments);
+
 /* Number of fused/layered kernel launches the engine has issued so far. */
 mcg_status mcg_launch_count(mcg_engine *engine, uint64_t *launches);
 

@@ -147,6 +147,7 @@ _SIGNATURES = {
     "mcg_tune_set_cache_file": (C.c_int, [C.c_char_p]),
     "mcg_tune_forget": (C.c_int, []),
     "mcg_engine_launch_shape": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint32), C.POINTER(C.c_uint32)]),
+    "mcg_fused_kernel": (C.c_int, [C.c_void_p, C.c_uint64, C.POINTER(C.c_uint32), C.POINTER(C.c_uint32)]),
     "mcg_last_error": (C.c_char_p, []),
     "mcg_version": (C.c_char_p, []),
 }
@@ -320,6 +321,12 @@ class Engine:
         mode, ctas = C.c_uint32(), C.c_uint32()
         check(self.lib.mcg_engine_launch_shape(self.handle, C.byref(mode), C.byref(ctas)))
         return int(mode.value), int(ctas.value)
+
+    def fused_kernel(self, word_count: int):
+        """(block size of the tile kernel or 0 for the interpreter, segments of the tile plan) of a fused pass."""
+        threads, segments = C.c_uint32(), C.c_uint32()
+        check(self.lib.mcg_fused_kernel(self.handle, word_count, C.byref(threads), C.byref(segments)))
+        return int(threads.value), int(segments.value)
 
     def time_runs(self, iteration_first: int, word_begin: int, word_count: int, repeats: int) -> float:
         ms = C.c_double()

@@ -572,7 +572,26 @@ mcg_status setup_tile(mcg_engine *e) {
     e->tile_threads = threads;
     e->tile_sms = (uint32_t)dev.multiProcessorCount;
     e->tile = true;
+    e->tile_cost = mcg::TileCost(t.layer, t.gates, t.event.size(), t.in.size(), g.tally_nodes.size(), e->tile_sms, threads,
+                                 e->tile_smem + (threads / 32) * sizeof(uint2) * mcg::dev::kEventTableStride +
+                                     dev.reservedSharedMemPerBlock);
     return MCG_OK;
+}
+
+uint64_t tiles_of(uint64_t words) { return (words + mcg::dev::kTileLanes - 1) / mcg::dev::kTileLanes; }
+
+// Threads of the tile kernel's blocks in a pass: a pass with fewer tiles than
+// resident blocks gives each of them more warps (4,096 words of a 60-event tree
+// are 128 tiles: 18.2 us with 1,024 threads each, 23.3 us with 256).
+uint32_t tile_pass_threads(const mcg_engine *e, uint64_t words) {
+    uint32_t threads = e->tile_threads;
+    while (threads < 1024u && tiles_of(words) < (uint64_t)e->tile_sms * (1024u / threads)) threads *= 2;
+    return threads;
+}
+
+// Whether a launch over so many words of a fused-mode engine is the tile kernel's.
+bool takes_tile(const mcg_engine *e, uint64_t words) {
+    return e->tile && (!e->d_ops || !e->tile_cost.interpreter_is_faster(words));
 }
 
 mcg_status launch_tile(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t word_begin, uint64_t count) {
@@ -582,12 +601,8 @@ mcg_status launch_tile(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t
     a.word_begin = word_begin;
     a.word_count = count;
     a.ones = e->d_tally;
-    const uint64_t tiles = (count + mcg::dev::kTileLanes - 1) / mcg::dev::kTileLanes;
-    // a pass with fewer tiles than resident blocks gives each of them more
-    // warps (4,096 words of a 60-event tree are 128 tiles: 18.2 us with 1,024
-    // threads each, 23.3 us with 256)
-    uint32_t threads = e->tile_threads;
-    while (threads < 1024u && tiles < (uint64_t)e->tile_sms * (1024u / threads)) threads *= 2;
+    const uint64_t tiles = tiles_of(count);
+    const uint32_t threads = tile_pass_threads(e, count);
     const uint32_t grid = (uint32_t)std::min<uint64_t>((uint64_t)e->tile_sms * (1024u / threads),
                                                        std::max<uint64_t>(tiles, 1));
     tile_kernel(threads)<<<grid, threads, e->tile_smem, e->stream>>>(a);
@@ -596,26 +611,32 @@ mcg_status launch_tile(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t
     return MCG_OK;
 }
 
+mcg_status setup_interpreter(mcg_engine *e, const mcg_run_desc &run) {
+    mcg_status st = compile_fused(e, run);
+    if (st != MCG_OK) return st;
+    st = mcg::set_smem_limit(fused_kernel(e->ctas_per_sm), e->smem_bytes);
+    if (st != MCG_OK) return st;
+    if (e->prog.global_slots)
+        MCG_CUDA(work_alloc(e, (void **)&e->d_scratch,
+                            (size_t)e->prog.global_slots * e->scratch_stride * sizeof(uint64_t)));
+    MCG_CUDA(upload(reinterpret_cast<mcg::Op **>(&e->d_ops), e->prog.ops));
+    return MCG_OK;
+}
+
 mcg_status setup_fused(mcg_engine *e, const mcg_run_desc &run) {
     // the default shape (no slot count, block size or residency of its own)
     if (!run.smem_slots && !run.block_threads && (!run.ctas_per_sm || run.ctas_per_sm == 4)) {
         const mcg_status ts = setup_tile(e);
         if (ts != MCG_OK) return ts;
-        if (e->tile) {
-            e->ctas_per_sm = 4;
-            e->chunk_words = run.chunk_words ? run.chunk_words : kDefaultChunkWords;
-            return MCG_OK;
-        }
     }
-    mcg_status st = compile_fused(e, run);
-    if (st != MCG_OK) return st;
-    st = mcg::set_smem_limit(fused_kernel(e->ctas_per_sm), e->smem_bytes);
-    if (st != MCG_OK) return st;
-    MCG_CUDA(upload(reinterpret_cast<mcg::Op **>(&e->d_ops), e->prog.ops));
-    if (e->prog.global_slots && e->mode == MCG_MODE_FUSED) {
-        MCG_CUDA(work_alloc(e, (void **)&e->d_scratch,
-                            (size_t)e->prog.global_slots * e->scratch_stride * sizeof(uint64_t)));
-    }
+    if (!e->tile) return setup_interpreter(e, run);
+    e->ctas_per_sm = 4;
+    e->chunk_words = run.chunk_words ? run.chunk_words : kDefaultChunkWords;
+    // next to the tile kernel where some passes are the interpreter's, and where there is room for it
+    if (!e->tile_cost.interpreter_may_be_faster()) return MCG_OK;
+    const mcg_status st = setup_interpreter(e, run);
+    if (st != MCG_ERR_OOM) return st;
+    mcg::clear_error();
     return MCG_OK;
 }
 
@@ -1139,6 +1160,16 @@ mcg_status mcg_engine_launch_shape(mcg_engine *e, uint32_t *mode, uint32_t *ctas
     return MCG_OK;
 }
 
+mcg_status mcg_fused_kernel(mcg_engine *e, uint64_t word_count, uint32_t *tile_threads, uint32_t *segments) {
+    mcg::clear_error();
+    if (!e) return mcg::fail(MCG_ERR_INVALID, "engine is NULL");
+    if (e->mode != MCG_MODE_FUSED) return mcg::fail(MCG_ERR_STATE, "not a fused-mode engine");
+    const bool tile = takes_tile(e, std::min<uint64_t>(word_count, e->chunk_words));
+    if (tile_threads) *tile_threads = tile ? tile_pass_threads(e, std::min<uint64_t>(word_count, e->chunk_words)) : 0u;
+    if (segments) *segments = e->tile ? e->tile_args.n_segments : 0u;
+    return MCG_OK;
+}
+
 mcg_status mcg_destroy(mcg_engine *e) {
     mcg::clear_error();
     if (!e) return MCG_OK;
@@ -1168,8 +1199,8 @@ mcg_status mcg_run(mcg_engine *e, uint32_t iteration_first, uint32_t n_iteration
     } else if (e->mode == MCG_MODE_FUSED) {
         for (uint64_t off = 0; off < word_count; off += e->chunk_words) {
             const uint64_t n = std::min<uint64_t>(e->chunk_words, word_count - off);
-            const mcg_status st = (e->tile ? launch_tile : launch_fused)(e, iteration_first, n_iterations,
-                                                                         word_begin + off, n);
+            const mcg_status st = (takes_tile(e, n) ? launch_tile : launch_fused)(e, iteration_first, n_iterations,
+                                                                                  word_begin + off, n);
             if (st != MCG_OK) return st;
         }
     } else {

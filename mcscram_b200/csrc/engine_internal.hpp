@@ -10,6 +10,7 @@
 #include "graph.hpp"
 #include "mcg.h"
 #include "program.hpp"
+#include "tile_cost.hpp"
 #include "tile.hpp"
 
 namespace mcg {
@@ -44,6 +45,7 @@ struct mcg_engine {
     mcg::dev::TileArgs tile_args{};        // device pointers and sizes; the pass is filled in per launch
     std::vector<void *> tile_tables;
     uint32_t tile_threads = 0, tile_smem = 0, tile_sms = 0;
+    mcg::TileCost tile_cost;               // its and the interpreter's time for a pass (tile_plan.hpp)
 
     // tallies
     unsigned long long *d_tally = nullptr;

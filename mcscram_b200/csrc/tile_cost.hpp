@@ -1,0 +1,56 @@
+// tile_cost.hpp -- the fused mode's choice between the tile kernel and the
+// interpreter for a pass (host side; no CUDA calls).
+#pragma once
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+#include <vector_types.h>
+
+namespace mcg {
+
+// SM clocks of a pass.  The tile kernel's layers each cost a block a barrier and
+// a chain of table loads, however few gates they have, and the blocks of an SM
+// come to them together; the interpreter has no barrier, but every warp walks
+// every op.  So deep graphs of few events are the interpreter's where the words
+// are many: 800 gates in a chain over 60 events on 262,144 words take 15.4 ms in
+// tiles and 2.6 there; 2,048 words 0.37 and 0.90.  The coefficients are fitted to
+// both kernels on 2 to 13,000 ops, 5 to 800 layers, fan-ins of 2 to 9 and 2,048
+// to 262,144 words (within 12 % for eight of ten).
+struct TileCost {
+    uint64_t sms = 1, blocks = 1;      // blocks: per SM, in long passes
+    uint64_t events = 0, inputs = 0;   // inputs: records of all gates
+    uint64_t rounds = 0, pairs = 0;    // over the layers: gates per warp of the one with most, input pairs of the widest gate
+    uint64_t ops = 0;                  // of the interpreter's program, about
+    bool l1 = true;                    // the blocks leave the SM some L1 for the tables
+
+    // layer: gate indices; gates: .z's low half the input pairs; block_bytes: shared memory of a block
+    TileCost() = default;
+    TileCost(const std::vector<uint32_t> &layer, const std::vector<uint4> &gates, size_t n_events, size_t n_inputs,
+             size_t n_tally, uint32_t n_sms, uint32_t threads, size_t block_bytes)
+        : sms(n_sms), blocks(1024 / threads), events(n_events), inputs(n_inputs),
+          ops(n_inputs + 2 * gates.size() + n_tally), l1(blocks * block_bytes <= (200u << 10)) {
+        const uint32_t warps = threads / 32;
+        for (size_t l = 0; l + 1 < layer.size(); ++l) {
+            uint32_t widest = 0;
+            for (uint32_t i = layer[l]; i < layer[l + 1]; ++i) widest = std::max(widest, gates[i].z & 0xFFFFu);
+            pairs += widest;
+            rounds += (layer[l + 1] - layer[l] + warps - 1) / warps;
+        }
+    }
+    uint64_t tile(uint64_t words) const {
+        const uint64_t tiles = (words + 31) / 32;
+        uint64_t b = blocks;
+        while (b > 1 && tiles < sms * b) b /= 2;
+        return (tiles + sms * b - 1) / (sms * b) * (b * (318 * events + 3 * inputs) + 580 * rounds + (l1 ? 55 : 111) * pairs);
+    }
+    uint64_t interpreter(uint64_t words) const {
+        const uint64_t warps = (words + 256 * sms - 1) / (256 * sms) * 8;  // blocks of eight warps
+        return std::max(warps * (413 * events + 19 * ops), 3900 * events + 500 * ops - 120 * inputs);
+    }
+    bool interpreter_is_faster(uint64_t words) const { return interpreter(words) < tile(words); }
+    bool interpreter_may_be_faster() const { return interpreter_is_faster(1ull << 32); }
+};
+
+}  // namespace mcg
