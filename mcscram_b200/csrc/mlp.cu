@@ -816,46 +816,71 @@ struct mcg_mlp {
     int device = 0;
     cudaStream_t stream = nullptr;
     float *d_params = nullptr, *d_m = nullptr, *d_v = nullptr;
-    float *d_grad = nullptr, *d_loss = nullptr;  // the loss lies behind the gradient: read back in one copy
+    // results, in one buffer so that a call reads its own and the flag back in one copy: the gradient, the loss,
+    // the flag that a kernel sets whose tensor-core or copy wait ran out, the forward pass's q
+    float *d_grad = nullptr, *d_loss = nullptr, *d_q = nullptr;
+    int *d_err = nullptr;        // 0 but between a kernel that gave up and the end of its call (check_waits)
+    std::vector<float> host_q;   // flag and q of a short forward pass
     double *d_wpart = nullptr;   // k_weight_sum's partial sums
     float *d_inv_wsum = nullptr; // 1 / sum of the call's row weights, or
     float inv_wsum = 0.f;        // summed on the host
     bool inv_on_device = false;
     bf16 *d_pack = nullptr;
-    float *d_feat = nullptr, *d_tgt = nullptr, *d_w = nullptr, *d_q = nullptr;
+    float *d_feat = nullptr, *d_tgt = nullptr, *d_w = nullptr;
     float *d_partial = nullptr;  // [ctas][kParams + 1] per-CTA gradients and losses
-    int *err = nullptr;          // set by a kernel whose tensor-core or copy wait ran out: host memory the device
-    int *d_err = nullptr;        // writes to, so that a call neither clears it on the stream nor copies it back
     uint32_t ctas = 0;           // persistent CTAs of the forward and gradient kernels
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around the steps of the last mcg_mlp_train
     double train_ms = 0.0;
-    uint32_t cap = 0;
+    uint32_t cap = 0, cap_q = 0;
     uint64_t adam_t = 0;
 };
 
 namespace {
+
+// Up to so many rows a forward pass reads the flag and q in one copy through the
+// host; a second copy costs about as much as moving so many values there.
+constexpr uint32_t kStagedRows = 1u << 15;
+
+// The results' buffer for n rows; its flag is 0.
+mcg_status ensure_results(mcg_mlp *m, uint32_t n) {
+    if (n <= m->cap_q) return MCG_OK;
+    m->cap_q = 0;
+    cudaFree(m->d_grad);
+    m->d_grad = m->d_loss = m->d_q = nullptr;
+    m->d_err = nullptr;
+    float *p = nullptr;
+    MCG_CUDA(cudaMalloc((void **)&p, (kParams + 2ull + n) * sizeof(float)));
+    m->d_grad = p;
+    m->d_loss = p + kParams;
+    m->d_err = reinterpret_cast<int *>(m->d_loss + 1);
+    m->d_q = m->d_loss + 2;
+    MCG_CUDA(cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream));
+    m->cap_q = n;
+    return MCG_OK;
+}
 
 mcg_status ensure_rows(mcg_mlp *m, uint32_t n) {
     if (n <= m->cap) return MCG_OK;
     cudaFree(m->d_feat);
     cudaFree(m->d_tgt);
     cudaFree(m->d_w);
-    cudaFree(m->d_q);
-    m->d_feat = m->d_tgt = m->d_w = m->d_q = nullptr;
+    m->d_feat = m->d_tgt = m->d_w = nullptr;
     m->cap = 0;
     MCG_CUDA(cudaMalloc((void **)&m->d_feat, (size_t)n * kIn * sizeof(float)));
     MCG_CUDA(cudaMalloc((void **)&m->d_tgt, (size_t)n * sizeof(float)));
     MCG_CUDA(cudaMalloc((void **)&m->d_w, (size_t)n * sizeof(float)));
-    MCG_CUDA(cudaMalloc((void **)&m->d_q, (size_t)n * sizeof(float)));
+    const mcg_status st = ensure_results(m, n);
+    if (st != MCG_OK) return st;
     m->cap = n;
     return MCG_OK;
 }
 
-// After a synchronised call: did one of its kernels give up on a tensor-core or copy wait?
-mcg_status check_waits(mcg_mlp *m) {
-    if (*(volatile int *)m->err)
-        return mcg::fail(MCG_ERR_CUDA, "proposal network: a tensor-core or bulk-copy wait timed out (results invalid)");
-    return MCG_OK;
+// After a synchronised call that read the flag `err`: did one of its kernels
+// give up on a tensor-core or copy wait?  The flag is cleared for the next call.
+mcg_status check_waits(mcg_mlp *m, int err) {
+    if (!err) return MCG_OK;
+    MCG_CUDA(cudaMemsetAsync(m->d_err, 0, sizeof(int), m->stream));
+    return mcg::fail(MCG_ERR_CUDA, "proposal network: a tensor-core or bulk-copy wait timed out (results invalid)");
 }
 
 mcg_status pack(mcg_mlp *m) {
@@ -878,13 +903,10 @@ mcg_status grad_partials(mcg_mlp *m, uint32_t n, bool has_w, uint32_t &blocks) {
 
 constexpr uint32_t kReduceBlocks = (kParams + 1 + kReduceCols - 1) / kReduceCols;
 
-// The call's rows to the device, and 1 / sum of their weights; also clears the
-// wait-timeout flag (the handle's earlier work has been waited for), so that
-// check_waits reports this call's kernels only.
+// The call's rows to the device, and 1 / sum of their weights.
 mcg_status upload_rows(mcg_mlp *m, const float *feat, const float *tgt, const float *w, uint32_t n) {
     mcg_status st = ensure_rows(m, n);
     if (st != MCG_OK) return st;
-    *(volatile int *)m->err = 0;
     MCG_CUDA(cudaMemcpyAsync(m->d_feat, feat, (size_t)n * kIn * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     if (!tgt) return MCG_OK;
     MCG_CUDA(cudaMemcpyAsync(m->d_tgt, tgt, (size_t)n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
@@ -923,8 +945,6 @@ mcg_status mcg_mlp_create(int32_t device, uint64_t seed, mcg_mlp **out) {
     MCG_CUDA(cudaSetDevice(device));
     MCG_CUDA(cudaStreamCreateWithFlags(&m->stream, cudaStreamNonBlocking));
     MCG_CUDA(cudaMalloc((void **)&m->d_params, kParams * sizeof(float)));
-    MCG_CUDA(cudaMalloc((void **)&m->d_grad, (kParams + 1) * sizeof(float)));
-    m->d_loss = m->d_grad + kParams;
     MCG_CUDA(cudaMalloc((void **)&m->d_wpart, kSumBlocks * sizeof(double)));
     MCG_CUDA(cudaMalloc((void **)&m->d_inv_wsum, sizeof(float)));
     MCG_CUDA(cudaMalloc((void **)&m->d_m, kParams * sizeof(float)));
@@ -947,9 +967,8 @@ mcg_status mcg_mlp_create(int32_t device, uint64_t seed, mcg_mlp **out) {
     const size_t most = (48u << 10) - sizeof(float) * kReduceGroups * kReduceCols;
     m->ctas = std::min<uint32_t>(m->ctas, (uint32_t)(most / (kReduceCols * sizeof(float))));
     MCG_CUDA(cudaMalloc((void **)&m->d_partial, (size_t)m->ctas * (kParams + 1) * sizeof(float)));
-    MCG_CUDA(cudaHostAlloc((void **)&m->err, sizeof(int), cudaHostAllocMapped));
-    *m->err = 0;
-    MCG_CUDA(cudaHostGetDevicePointer((void **)&m->d_err, m->err, 0));
+    mcg_status st = ensure_results(m.get(), kStagedRows);
+    if (st != MCG_OK) return st;
     MCG_CUDA(cudaEventCreate(&m->ev0));
     MCG_CUDA(cudaEventCreate(&m->ev1));
     // He-style initialisation from a seeded host generator
@@ -962,7 +981,7 @@ mcg_status mcg_mlp_create(int32_t device, uint64_t seed, mcg_mlp **out) {
     MCG_CUDA(cudaMemcpy(m->d_params, p.data(), kParams * sizeof(float), cudaMemcpyHostToDevice));
     MCG_CUDA(cudaMemset(m->d_m, 0, kParams * sizeof(float)));
     MCG_CUDA(cudaMemset(m->d_v, 0, kParams * sizeof(float)));
-    mcg_status st = pack(m.get());
+    st = pack(m.get());
     if (st != MCG_OK) return st;
     MCG_CUDA(cudaStreamSynchronize(m->stream));
     *out = m.release();
@@ -984,9 +1003,7 @@ mcg_status mcg_mlp_destroy(mcg_mlp *m) {
     cudaFree(m->d_feat);
     cudaFree(m->d_tgt);
     cudaFree(m->d_w);
-    cudaFree(m->d_q);
     cudaFree(m->d_partial);
-    if (m->err) cudaFreeHost(m->err);
     if (m->ev0) cudaEventDestroy(m->ev0);
     if (m->ev1) cudaEventDestroy(m->ev1);
     cudaStreamDestroy(m->stream);
@@ -1028,9 +1045,20 @@ mcg_status mcg_mlp_forward(mcg_mlp *m, const float *features, uint32_t n, float 
     k_mlp_forward<<<std::min(tiles, m->ctas), kThreads, sizeof(TcSmem), m->stream>>>(m->d_pack, m->d_params,
                                                                                      m->d_feat, n, m->d_q, m->d_err);
     MCG_CUDA(cudaGetLastError());
+    if (n <= kStagedRows) {
+        m->host_q.resize(n + 1u);
+        MCG_CUDA(cudaMemcpyAsync(m->host_q.data(), m->d_err, (n + 1u) * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+        MCG_CUDA(cudaStreamSynchronize(m->stream));
+        int err;
+        std::memcpy(&err, m->host_q.data(), sizeof(err));
+        std::memcpy(q_out, m->host_q.data() + 1, (size_t)n * sizeof(float));
+        return check_waits(m, err);
+    }
+    int err = 0;
     MCG_CUDA(cudaMemcpyAsync(q_out, m->d_q, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+    MCG_CUDA(cudaMemcpyAsync(&err, m->d_err, sizeof(err), cudaMemcpyDeviceToHost, m->stream));
     MCG_CUDA(cudaStreamSynchronize(m->stream));
-    return check_waits(m);
+    return check_waits(m, err);
 }
 
 mcg_status mcg_mlp_grad(mcg_mlp *m, const float *features, const float *targets, const float *weights, uint32_t n,
@@ -1046,12 +1074,14 @@ mcg_status mcg_mlp_grad(mcg_mlp *m, const float *features, const float *targets,
     if (st != MCG_OK) return st;
     k_mlp_reduce<<<kReduceBlocks, kReduceThreads, blocks * kReduceCols * sizeof(float), m->stream>>>(m->d_partial, blocks, m->d_grad);
     MCG_CUDA(cudaGetLastError());
-    float out[kParams + 1];
+    float out[kParams + 2];  // gradient, loss, flag
     MCG_CUDA(cudaMemcpyAsync(out, m->d_grad, sizeof(out), cudaMemcpyDeviceToHost, m->stream));
     MCG_CUDA(cudaStreamSynchronize(m->stream));
     std::memcpy(grad_out, out, kParams * sizeof(float));
     const float loss = out[kParams];
-    st = check_waits(m);
+    int err;
+    std::memcpy(&err, out + kParams + 1, sizeof(err));
+    st = check_waits(m, err);
     if (st != MCG_OK) return st;
     if (loss_out) *loss_out = loss;
     return MCG_OK;
@@ -1078,15 +1108,17 @@ mcg_status mcg_mlp_train(mcg_mlp *m, const float *features, const float *targets
     }
     MCG_CUDA(cudaGetLastError());
     MCG_CUDA(cudaEventRecord(m->ev1, m->stream));
-    float loss = 0.f;
-    MCG_CUDA(cudaMemcpyAsync(&loss, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+    float out[2];  // loss, flag
+    MCG_CUDA(cudaMemcpyAsync(out, m->d_loss, sizeof(out), cudaMemcpyDeviceToHost, m->stream));
     MCG_CUDA(cudaStreamSynchronize(m->stream));
     float ms = 0.f;
     MCG_CUDA(cudaEventElapsedTime(&ms, m->ev0, m->ev1));
     m->train_ms = ms;
-    st = check_waits(m);
+    int err;
+    std::memcpy(&err, out + 1, sizeof(err));
+    st = check_waits(m, err);
     if (st != MCG_OK) return st;
-    if (loss_out) *loss_out = loss;
+    if (loss_out) *loss_out = out[0];
     return MCG_OK;
 }
 
