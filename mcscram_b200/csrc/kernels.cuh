@@ -107,7 +107,7 @@ __device__ __forceinline__ void store_slot(uint32_t ref, uint64_t v, uint64_t *m
 // basic-event ops carry an index into thr (a per-instance uint64 threshold
 // table) instead of the threshold itself.  tally(index, count) is called by
 // lane 0 of each warp with the warp's popcount sum for a TALLY op.
-template <int NT, int PF, bool THR_TABLE, class Tally>
+template <int NT, int PF, bool THR_TABLE, bool SPLIT, class Tally>
 __device__ __forceinline__ void interpret(const uint4 *__restrict__ ops, const WordCtx &ctx, uint32_t t3, bool valid,
                                           uint64_t *my_slots, uint64_t *my_scratch, uint64_t stride,
                                           const uint64_t *__restrict__ thr, Tally &&tally) {
@@ -130,9 +130,9 @@ __device__ __forceinline__ void interpret(const uint4 *__restrict__ ops, const W
                 const uint64_t t = thr[op.z];
                 if (t >= (1ull << 32)) v = kAllOnes;
                 else if (t == 0) v = 0;
-                else v = be_word<PF>(op.y, op.w, ctx, t3, (uint32_t)t);
+                else v = be_word<PF, SPLIT>(op.y, op.w, ctx, t3, (uint32_t)t);
             } else {
-                v = be_word<PF>(op.y, op.w, ctx, t3, op.z);
+                v = be_word<PF, SPLIT>(op.y, op.w, ctx, t3, op.z);
             }
         } else if (code == kOpInSlot) {
             v = load_slot(op.y, my_slots, my_scratch, NT, stride);
@@ -207,8 +207,8 @@ __global__ void __launch_bounds__(NT, MINB) k_fused(FusedArgs a) {
         for (uint64_t base = 0; base < a.word_count; base += total_threads) {
             const uint64_t j = base + gtid;
             const WordCtx ctx = make_word_ctx((uint32_t)(a.word_begin + j));
-            interpret<NT, PF, false>(a.ops, ctx, t3, j < a.word_count, my_slots, my_scratch, a.scratch_stride,
-                                         nullptr, add);
+            interpret<NT, PF, false, MINB == 4>(a.ops, ctx, t3, j < a.word_count, my_slots, my_scratch,
+                                                a.scratch_stride, nullptr, add);
         }
     }
     if (a.tally_in_smem) {
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(NT, MINB) k_fused_batch(BatchArgs a) {
         const WordCtx ctx = make_word_ctx((uint32_t)j);
         unsigned long long *ones = a.inst_ones + inst;
         auto add = [ones](uint32_t, uint32_t c) { atomicAdd(ones, (unsigned long long)c); };
-        interpret<NT, PF, true>(a.ops + a.tree_op_offset[a.inst_tree[inst]], ctx, t3, j < a.words_per_instance,
+        interpret<NT, PF, true, false>(a.ops + a.tree_op_offset[a.inst_tree[inst]], ctx, t3, j < a.words_per_instance,
                                     my_slots, my_scratch, a.scratch_stride, a.thr + a.inst_thr_offset[inst], add);
     }
 }

@@ -38,19 +38,28 @@ struct RoundKey {
 // through 64-bit operations (0.82 of the rate in the strip kernel), written as
 // a high and a low multiply it adds 30 register moves per word on the multiply
 // pipe (30.1 against 30.8 G words/s register-only, 198.0 against 194.3 ms for
-// 2^20 words of the 5,000-event tree).
+// 2^20 words of the 5,000-event tree).  SPLIT takes those two all the same: the
+// interpreter in four blocks per SM, whose 64 registers do not hold the pairs of
+// a wide product, is the faster for it (2,048 words of 3,000 events 6.72 and 6.90
+// ms; in three blocks 6.66 and 6.38).
+template <bool SPLIT = false>
 __device__ __forceinline__ void mul_hilo(uint32_t a, uint32_t b, uint32_t &hi, uint32_t &lo) {
+    if constexpr (SPLIT) {
+        hi = __umulhi(a, b);
+        lo = a * b;
+        return;
+    }
     asm("{\n\t.reg .u64 p;\n\tmul.wide.u32 p, %2, %3;\n\tmov.b64 {%1, %0}, p;\n\t}"
         : "=r"(hi), "=r"(lo)
         : "r"(a), "r"(b));
 }
 
 // Standard round r on the full state (rounds 4..10 of every call).
-template <int R>
+template <int R, bool SPLIT = false>
 __device__ __forceinline__ void philox_round(uint32_t &x0, uint32_t &x1, uint32_t &x2, uint32_t &x3) {
     uint32_t ha, la, hb, lb;
-    mul_hilo(kM0, x0, ha, la);
-    mul_hilo(kM1, x2, hb, lb);
+    mul_hilo<SPLIT>(kM0, x0, ha, la);
+    mul_hilo<SPLIT>(kM1, x2, hb, lb);
     x0 = hb ^ x1 ^ RoundKey<R>::k0;
     x1 = lb;
     x2 = ha ^ x3 ^ RoundKey<R>::k1;
@@ -93,24 +102,24 @@ __device__ __forceinline__ uint32_t shift_in_ge(uint32_t acc, uint32_t o, uint32
 // the word be_word gives for that threshold.  Instances that share a counter
 // stream but not their thresholds (draws of one tree) pay for the 16 Philox
 // calls once.
-template <int PackForm, int K>
+template <int PackForm, int K, bool SPLIT = false>
 __device__ __forceinline__ void be_words(uint32_t x0, uint32_t x1, const WordCtx &ctx, uint32_t t3,
                                          const uint32_t (&thr)[K], uint64_t (&out)[K]) {
     // Round 1, shared by the 16 calls.
     uint32_t ha, la;
-    mul_hilo(kM0, x0, ha, la);
+    mul_hilo<SPLIT>(kM0, x0, ha, la);
     const uint32_t a0 = ctx.hb ^ x1 ^ RoundKey<0>::k0;
     const uint32_t a1 = ctx.lb;
     const uint32_t a2base = ha ^ t3 ^ RoundKey<0>::k1;  // x3 = t3 + g == t3 ^ g (g < 64)
     const uint32_t a3 = la;
     // Round 2: the M0 product is shared.
     uint32_t hc, lc;
-    mul_hilo(kM0, a0, hc, lc);
+    mul_hilo<SPLIT>(kM0, a0, hc, lc);
     const uint32_t b2 = hc ^ a3 ^ RoundKey<1>::k1;
     const uint32_t b3 = lc;
     // Round 3: the M1 product is shared.
     uint32_t hf, lf;
-    mul_hilo(kM1, b2, hf, lf);
+    mul_hilo<SPLIT>(kM1, b2, hf, lf);
     const uint32_t c1 = lf;
 
     uint32_t lo[K], hi[K];
@@ -120,23 +129,23 @@ __device__ __forceinline__ void be_words(uint32_t x0, uint32_t x1, const WordCtx
     for (int g = 0; g < 16; ++g) {
         // Round 2, per call.
         uint32_t hd, ld;
-        mul_hilo(kM1, a2base ^ (uint32_t)g, hd, ld);
+        mul_hilo<SPLIT>(kM1, a2base ^ (uint32_t)g, hd, ld);
         const uint32_t b0 = hd ^ a1 ^ RoundKey<1>::k0;
         const uint32_t b1 = ld;
         // Round 3, per call.
         uint32_t he, le;
-        mul_hilo(kM0, b0, he, le);
+        mul_hilo<SPLIT>(kM0, b0, he, le);
         uint32_t x0r = hf ^ b1 ^ RoundKey<2>::k0;
         uint32_t x1r = c1;
         uint32_t x2r = he ^ b3 ^ RoundKey<2>::k1;
         uint32_t x3r = le;
-        philox_round<3>(x0r, x1r, x2r, x3r);
-        philox_round<4>(x0r, x1r, x2r, x3r);
-        philox_round<5>(x0r, x1r, x2r, x3r);
-        philox_round<6>(x0r, x1r, x2r, x3r);
-        philox_round<7>(x0r, x1r, x2r, x3r);
-        philox_round<8>(x0r, x1r, x2r, x3r);
-        philox_round<9>(x0r, x1r, x2r, x3r);
+        philox_round<3, SPLIT>(x0r, x1r, x2r, x3r);
+        philox_round<4, SPLIT>(x0r, x1r, x2r, x3r);
+        philox_round<5, SPLIT>(x0r, x1r, x2r, x3r);
+        philox_round<6, SPLIT>(x0r, x1r, x2r, x3r);
+        philox_round<7, SPLIT>(x0r, x1r, x2r, x3r);
+        philox_round<8, SPLIT>(x0r, x1r, x2r, x3r);
+        philox_round<9, SPLIT>(x0r, x1r, x2r, x3r);
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             if constexpr (PackForm == 0) {
@@ -176,12 +185,12 @@ __device__ __forceinline__ void be_words(uint32_t x0, uint32_t x1, const WordCtx
     }
 }
 
-template <int PackForm>
+template <int PackForm, bool SPLIT = false>
 __device__ __forceinline__ uint64_t be_word(uint32_t x0, uint32_t x1, const WordCtx &ctx, uint32_t t3,
                                             uint32_t thr) {
     const uint32_t t[1] = {thr};
     uint64_t w[1];
-    be_words<PackForm, 1>(x0, x1, ctx, t3, t, w);
+    be_words<PackForm, 1, SPLIT>(x0, x1, ctx, t3, t, w);
     return w[0];
 }
 
