@@ -12,6 +12,7 @@ ROOT = Path(__file__).resolve().parent.parent
 SOURCE = r"""
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <random>
 #include <cuda_runtime.h>
 #include "gate_plan.hpp"
@@ -280,7 +281,34 @@ static void walk_parts(const Graph &g, const std::vector<uint64_t> &val) {
     }
 }
 
+// Parts of a plan over separate trees of so many gates (each a chain).
+static void parts_of(int n, char **sizes) {
+    Graph g;
+    g.n_be = 1;
+    g.be_pdag_idx = {2};
+    g.be_event_idx = {0};
+    g.be_threshold = {1};
+    std::vector<uint32_t> depth;
+    for (int t = 0; t < n; ++t)
+        for (int i = 0; i < std::atoi(sizes[t]); ++i) {
+            g.gate_op.push_back(MCG_NULL);
+            g.gate_k.push_back(0);
+            g.gate_in_begin.push_back((uint32_t)g.inputs.size());
+            g.gate_in_count.push_back(1);
+            g.gate_neg_count.push_back(0);
+            g.inputs.push_back(i ? g.n_gates : 0);
+            ++g.n_gates;
+            depth.push_back((uint32_t)i + 1);
+        }
+    const GatePlan t = plan_gates(g, depth);
+    std::printf("ok %u %u\n", t.parts(), t.largest);
+}
+
 int main(int argc, char **argv) {
+    if (!std::strcmp(argv[1], "parts")) {
+        parts_of(argc - 2, argv + 2);
+        return 0;
+    }
     const uint32_t n_be = (uint32_t)std::atoi(argv[1]), n_gates = (uint32_t)std::atoi(argv[2]);
     const uint32_t reach = (uint32_t)std::atoi(argv[3]);
     size_t most = 0;
@@ -317,3 +345,11 @@ def test_every_plan_gives_every_value(walker, n_be, n_gates, reach, segments):
     r = subprocess.run([str(walker), str(n_be), str(n_gates), str(reach)], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.startswith("ok"), r.stdout
     assert int(r.stdout.split()[1]) >= segments  # the most that a plan had, at 8 events each
+
+
+@pytest.mark.parametrize("sizes,parts,largest", [([7], 1, 7), ([5] * 16, 16, 5), ([5] * 200, 64, 20), ([1000] + [1] * 900, 2, 1000),
+                                                 ([60, 60, 1, 2, 3], 3, 60), ([40, 30, 20, 10], 3, 40)])
+def test_parts_are_evenly_loaded(walker, sizes, parts, largest):
+    """A part is a block per tile: trees of a few gates beside large ones share one."""
+    r = subprocess.run([str(walker), "parts", *map(str, sizes)], capture_output=True, text=True, check=True)
+    assert r.stdout.split() == ["ok", str(parts), str(largest)]
