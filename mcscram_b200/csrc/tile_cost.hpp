@@ -16,8 +16,9 @@ namespace mcg {
 // every op.  So deep graphs of few events are the interpreter's where the words
 // are many: 800 gates in a chain over 60 events on 262,144 words take 15.4 ms in
 // tiles and 2.6 there; 2,048 words 0.37 and 0.90.  The coefficients are fitted to
-// both kernels on 2 to 13,000 ops, 5 to 800 layers, fan-ins of 2 to 9 and 2,048
-// to 262,144 words (within 12 % for eight of ten).
+// both kernels on graphs of 4 to 2,000 events, 2 to 800 layers and fan-ins of 2
+// to 24, 2,048 to 2^20 words (within 12 % for eight of ten); over 1,833 passes of
+// 507 graphs the choice was more than 10 % behind the better kernel in 9.
 struct TileCost {
     uint64_t sms = 1, blocks = 1;      // blocks: per SM, in long passes
     uint64_t events = 0, inputs = 0;   // inputs: records of all gates
@@ -43,11 +44,11 @@ struct TileCost {
         const uint64_t tiles = (words + 31) / 32;
         uint64_t b = blocks;
         while (b > 1 && tiles < sms * b) b /= 2;
-        return (tiles + sms * b - 1) / (sms * b) * (b * (318 * events + 3 * inputs) + 580 * rounds + (l1 ? 55 : 111) * pairs);
+        return (tiles + sms * b - 1) / (sms * b) * (b * (318 * events + 3 * inputs) + 1500 + 580 * rounds + (l1 ? 55 : 111) * pairs);
     }
     uint64_t interpreter(uint64_t words) const {
         const uint64_t warps = (words + 256 * sms - 1) / (256 * sms) * 8;  // blocks of eight warps
-        return std::max(warps * (413 * events + 19 * ops), 3900 * events + 500 * ops - 120 * inputs);
+        return std::max(warps * (390 * events + 20 * ops), 3900 * events + 500 * ops - 120 * inputs);
     }
     bool interpreter_is_faster(uint64_t words) const { return interpreter(words) < tile(words); }
     bool interpreter_may_be_faster() const { return interpreter_is_faster(1ull << 32); }
