@@ -39,7 +39,9 @@ struct Candidate {
 };
 
 // Launch shapes measured on a miss: the strip kernel at each residency it is
-// built for, the staged pipeline, the fused interpreter at 4 and 2 CTAs per SM.
+// built for, the staged pipeline, the fused mode in its default shape (the tile
+// kernel, or the interpreter where the tree does not fit it) and the interpreter
+// at 2 CTAs per SM.
 constexpr Candidate kCandidates[] = {{MCG_MODE_STRIP, 6}, {MCG_MODE_STRIP, 5}, {MCG_MODE_STRIP, 4},
                                      {MCG_MODE_STAGED, 0}, {MCG_MODE_FUSED, 4}, {MCG_MODE_FUSED, 2}};
 

@@ -175,8 +175,10 @@ mcg_status upload_table(mcg_batch *b, const T **dptr, const std::vector<T> &v) {
     return MCG_OK;
 }
 
-// The tile kernel's scratch: a row of 4 KB per slot of the largest tree and
-// per SM (one block each).  Above this the interpreter's slots are smaller.
+// The tile kernel's scratch: a row of 4 KB per slot of the largest tree for each
+// of the two blocks of every SM, held as long as the batch (84 MB for trees of
+// 60 events, 0.4 GB for 2,000, 1.5 GB for the 5,000-event tree; the interpreter
+// 26 MB, 1.0 and 5.3 GB).  Above this much the interpreter takes the batch.
 constexpr uint64_t kTileScratchMost = 16ull << 30;
 
 // Tables of k_batch_tile; leaves b->tile false where the interpreter has to

@@ -836,8 +836,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
     const mcg::Graph &g = e->graph;
     const int set = (int)(k & 1);
     uint64_t *buf = e->d_stage[set];
-    // rows of an even length take 16-byte loads; hooks read rows of W words
-    const uint64_t stride = e->chunk_hook || e->sample_hook ? W : (W + 1) / 2 * 2;
+    const uint64_t stride = (W + 1) / 2 * 2;  // rows of an even length take 16-byte loads
     if (k >= 2) MCG_CUDA(cudaStreamWaitEvent(e->s_a, e->ev_b[set], 0));
     const uint32_t t3 = (iteration + 1u) << 6;
     const uint4 *be_tab = e->d_be_sample ? e->d_be_sample : e->d_be;
@@ -874,7 +873,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         if (p1) MCG_CUDA(cudaEventRecord(p1, e->s_a));
     }
     if (e->sample_hook) {
-        const mcg_status st = e->sample_hook(e->s_a, buf, W, word_begin);
+        const mcg_status st = e->sample_hook(e->s_a, buf, W, stride, word_begin);
         if (st != MCG_OK) return st;
     }
     MCG_CUDA(cudaEventRecord(e->ev_a[set], e->s_a));
@@ -891,7 +890,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         a.stride = stride;
         a.buf = buf;
         a.ones = e->d_tally;
-        const bool wide = stride % 2 == 0 && W >= kWideGateWords * e->gate_sms;
+        const bool wide = W >= kWideGateWords * e->gate_sms;
         uint64_t tiles = (W + (wide ? 63 : 31)) / (wide ? 64 : 32);
         // Warps per block: the fewer blocks share the chip, the more of a
         // layer's gates a block takes at a time.  Blocks are counted at the
@@ -924,7 +923,7 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         ++e->launches;
     }
     if (e->chunk_hook) {
-        const mcg_status st = e->chunk_hook(e->s_b, buf, W);
+        const mcg_status st = e->chunk_hook(e->s_b, buf, W, stride);
         if (st != MCG_OK) return st;
     }
     MCG_CUDA(cudaEventRecord(e->ev_b[set], e->s_b));

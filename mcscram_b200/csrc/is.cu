@@ -121,7 +121,7 @@ __device__ __forceinline__ double cut_uniform(uint64_t base, uint32_t draw) {
 
 struct CutArgs {
     uint64_t *buf;
-    uint64_t W, word_begin;
+    uint64_t W, stride, word_begin;  // words of the chunk, row stride of buf
     uint32_t n_inst, n_be;
     const uint32_t *root_row;      // per tree
     const uint4 *gate;             // per gate: op | k << 8, in_begin, in_count, table offset
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(256) k_cut_draw(const __grid_constant__ CutArg
     }
     __syncthreads();
     for (uint32_t j = j0 + warp; j < j1; j += 8)
-        if (w0 + lane < a.W) a.buf[(uint64_t)a.z_event[j] * a.W + w0 + lane] = s_word[j - j0][lane];
+        if (w0 + lane < a.W) a.buf[(uint64_t)a.z_event[j] * a.stride + w0 + lane] = s_word[j - j0][lane];
 }
 
 // One thread per (tree, word, sample): collects the sample's shared events
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256) k_cut_force(CutArgs a) {
     const uint32_t z0 = a.z_begin[k], z1 = a.z_begin[k + 1];
     for (uint32_t j0 = z0; j0 < z1; j0 += 32) {
         uint32_t x = 0;
-        if (j0 + lane < z1) x = (uint32_t)(a.buf[(uint64_t)a.z_event[j0 + lane] * a.W + w] >> half);
+        if (j0 + lane < z1) x = (uint32_t)(a.buf[(uint64_t)a.z_event[j0 + lane] * a.stride + w] >> half);
         for (uint32_t m = __ballot_sync(0xFFFFFFFFu, x != 0); m; m &= m - 1) {
             const int src = __ffs((int)m) - 1;
             if (!((__shfl_sync(0xFFFFFFFFu, x, src) >> lane) & 1u)) continue;
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(256) k_cut_force(CutArgs a) {
         return false;
     };
     auto leaf = [&](uint32_t x) -> double {
-        return a.shared[x] ? (double)((a.buf[(uint64_t)x * a.W + w] >> b) & 1ull) : a.S[x];
+        return a.shared[x] ? (double)((a.buf[(uint64_t)x * a.stride + w] >> b) & 1ull) : a.S[x];
     };
     auto s0 = [&](uint32_t x) -> double { return a.S[x]; };
     GateMemo memo;
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256) k_cut_force(CutArgs a) {
         const uint32_t node = stack[--sp];
         if (node < n_be) {
             if (!a.shared[node])
-                atomicOr(reinterpret_cast<unsigned long long *>(a.buf + (uint64_t)node * a.W + w), bit);
+                atomicOr(reinterpret_cast<unsigned long long *>(a.buf + (uint64_t)node * a.stride + w), bit);
             continue;
         }
         const uint4 g = a.gate[node - n_be];
@@ -889,8 +889,8 @@ mcg_status create_with_room(int device, Create create) {
 }
 
 // Queues both kernels for one chunk of W words.
-cudaError_t launch_weights(IsBatchArgs p, uint32_t n_events, uint64_t weight_words, int sms, cudaStream_t s) {
-    const uint64_t W = p.W;
+cudaError_t launch_weights(IsBatchArgs p, uint64_t W, uint32_t n_events, uint64_t weight_words, int sms,
+                           cudaStream_t s) {
     for (uint64_t at = 0; at < W; at += p.w_count) {
         p.w_begin = at;
         p.w_count = p.ce ? std::min<uint64_t>(W - at, weight_words) : W - at;
@@ -1147,11 +1147,11 @@ mcg_status mcg_is_run(mcg_is *is, const uint64_t *q_thr, uint32_t iteration, uin
     args.weights = want_ce ? reinterpret_cast<double *>(e->d_stage_extra) : nullptr;
     args.ce = want_ce ? is->d_ce : nullptr;
     const uint64_t weight_words = e->stage_extra_words / 64u;
-    e->chunk_hook = [=](cudaStream_t s, const uint64_t *buf, uint64_t W) -> mcg_status {
+    e->chunk_hook = [=](cudaStream_t s, const uint64_t *buf, uint64_t W, uint64_t stride) -> mcg_status {
         IsBatchArgs p = args;
         p.buf = buf;
-        p.W = W;
-        const cudaError_t err = launch_weights(p, nb, weight_words, sms, s);
+        p.W = stride;
+        const cudaError_t err = launch_weights(p, W, nb, weight_words, sms, s);
         if (err != cudaSuccess) return mcg::fail(MCG_ERR_CUDA, std::string("k_is_weights: ") + cudaGetErrorString(err));
         return MCG_OK;
     };
@@ -1755,11 +1755,11 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
     args.error = b->d_cut_error;
     if (cut_comp >= 0) MCG_CUDA(cudaMemsetAsync(b->d_cut_error, 0, sizeof(unsigned int), e->stream));
     const mcg::AtExit plain_again([e] { plain_sampling(e); });
-    e->chunk_hook = [=](cudaStream_t s, const uint64_t *buf, uint64_t W) -> mcg_status {
+    e->chunk_hook = [=](cudaStream_t s, const uint64_t *buf, uint64_t W, uint64_t stride) -> mcg_status {
         IsBatchArgs p = args;
         p.buf = buf;
-        p.W = W;
-        const cudaError_t err = launch_weights(p, (uint32_t)nb, weight_words, sms, s);
+        p.W = stride;
+        const cudaError_t err = launch_weights(p, W, (uint32_t)nb, weight_words, sms, s);
         if (err != cudaSuccess)
             return mcg::fail(MCG_ERR_CUDA, std::string("k_is_weights: ") + cudaGetErrorString(err));
         return MCG_OK;
@@ -1773,7 +1773,7 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
     uint32_t last_comp = 0;
     for (uint32_t c = 0; c < nc; ++c)
         if (comp_words[c]) last_comp = c;
-    std::function<mcg_status(cudaStream_t, uint64_t *, uint64_t, uint64_t)> cut_hook;
+    std::function<mcg_status(cudaStream_t, uint64_t *, uint64_t, uint64_t, uint64_t)> cut_hook;
     if (cut_comp >= 0) {
         CutArgs ca{};
         ca.n_inst = n_inst;
@@ -1794,10 +1794,11 @@ mcg_status mcg_is_batch_run(mcg_is_batch *b, const uint64_t *q_thr, uint32_t n_d
         ca.seed = mix64_host(((uint64_t)iteration << 32) ^ 0x5bd1e995u);
         ca.error = b->d_cut_error;
         const uint32_t n_z = (uint32_t)b->z_event.size();
-        cut_hook = [=](cudaStream_t s, uint64_t *buf, uint64_t W, uint64_t wb) -> mcg_status {
+        cut_hook = [=](cudaStream_t s, uint64_t *buf, uint64_t W, uint64_t stride, uint64_t wb) -> mcg_status {
             CutArgs x = ca;
             x.buf = buf;
             x.W = W;
+            x.stride = stride;
             x.word_begin = wb;
             const uint64_t threads = (uint64_t)x.n_inst * W * 64;
             if (n_z) {

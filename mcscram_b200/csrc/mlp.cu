@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
         const float tv = valid ? tgt[row] : 0.f;
         const float wv = valid ? (wts ? wts[row] : 1.f) * inv_wsum : 0.f;
         ok = mbar_wait(&s.bar_rows, i & 1) && ok;
-        rows_to_x(s, xb, r, half, valid);  // the X tile tile i - 2 used: its G2 completed before tile i - 1's layer 1 did
+        rows_to_x(s, xb, r, half, valid);  // the X tile tile i - 2 used: its G2 was waited for before tile i - 1's dH2
         fence_async_smem();
         tc_before_sync();
         MCG_SYNC_OR_BREAK();
