@@ -93,8 +93,8 @@ __host__ __device__ constexpr int pack_index(int i) {
 
 constexpr int kTile = 128;     // rows per tile: the MMA's M, TMEM lanes
 // 8 warps, warp w reading TMEM lanes 32 (w % 4) .. + 31.  The kernels are a chain of short steps per tile, bound by
-// its latency and by the instructions of the row-wise steps at two CTAs per SM (a tile takes about 7,000 clocks, of
-// which the tensor pipe is busy 700).  The gradient of 250,000 rows: 50.2 us with one thread per row; 45.8 with two;
+// its latency and by the instructions of the row-wise steps at two CTAs per SM (the tensor pipe is busy 18 % of its
+// active cycles).  The gradient of 250,000 rows: 50.2 us with one thread per row; 45.8 with two;
 // 44.7 with the weight gradients issued by a second thread and waited for on barriers of their own; 35.4 with the
 // row-wise steps on BF16 pairs, one add per descriptor and the weights brought in by one bulk copy (2,001 rows, one
 // tile per CTA: 14.9 -> 8.0 us).
