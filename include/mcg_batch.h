@@ -32,15 +32,19 @@ typedef struct mcg_batch_info {
     uint64_t total_ops;
     uint64_t launches;         /* kernel launches so far (graph replays count once each) */
     double last_kernel_ms;     /* duration of the last batched launch (CUDA events) */
-    uint32_t instances_per_item; /* of the interpreter (run with smem_slots or ctas_per_sm given, or where
-                                  * the tile kernel's rows do not fit; tiles take up to 16): instances
+    uint32_t instances_per_item; /* of the interpreter (run with smem_slots or ctas_per_sm given, where the
+                                  * tile kernel's rows do not fit, or where mcg_batch_kernel says so; tiles
+                                  * take up to 16): instances
                                   * of one tree evaluated together, sharing their
                                   * Philox calls (4; 1 when a tree has an ATLEAST gate of
                                   * more than 15 inputs) */
 } mcg_batch_info;
 
 /* Compiles every tree (a flattened graph whose tally_nodes are the nodes to
- * count, normally the root) for threshold tables supplied per instance. */
+ * count, normally the root) for threshold tables supplied per instance.  A
+ * batch holds device memory as long as it lives: the tile kernel's rows (4 KB
+ * per live node of the largest tree and block, two blocks per SM, at most 16
+ * GiB) and, from the first run that takes it, the interpreter's scratch. */
 mcg_status mcg_batch_create(const mcg_graph_desc *trees, uint32_t n_trees, const mcg_run_desc *run,
                             mcg_batch **out);
 mcg_status mcg_batch_destroy(mcg_batch *b);
@@ -56,6 +60,12 @@ mcg_status mcg_batch_run(mcg_batch *b, uint32_t n_instances, const uint32_t *ins
                          uint64_t words_per_instance, uint64_t *ones);
 
 mcg_status mcg_batch_info_get(mcg_batch *b, mcg_batch_info *info);
+
+/* The kernel that mcg_batch_run takes for these instances (by the trees, the
+ * instances of each that follow one another, and the words; the results are the
+ * same): *tiles is 1 for the tile kernel and 0 for the interpreter. */
+mcg_status mcg_batch_kernel(mcg_batch *b, uint32_t n_instances, const uint32_t *inst_tree,
+                            uint64_t words_per_instance, int32_t *tiles);
 
 #define MCG_UA_MEDIAN 0 /* base probability is the lognormal median */
 #define MCG_UA_MEAN 1   /* base probability is the lognormal mean (LognormalDeviate, src/expression/random_deviate.cc:101-109) */

@@ -14,6 +14,7 @@
 #include "mcg_batch.h"
 #include "program.hpp"
 #include "smem_limit.hpp"
+#include "tile_cost.hpp"
 #include "tile_plan.hpp"
 
 namespace {
@@ -87,7 +88,7 @@ struct mcg_batch {
     uint64_t total_ops = 0;
     uint4 *d_ops = nullptr;
     uint32_t *d_tree_off = nullptr;
-    uint64_t *d_scratch = nullptr;
+    uint64_t *d_scratch = nullptr;       // of the interpreter (interpreter_scratch)
     uint64_t scratch_stride = 0;
     unsigned int *d_queue = nullptr;
     // per-run buffers
@@ -101,7 +102,10 @@ struct mcg_batch {
     uint32_t n_groups = 0;
     // tiles (the default shape): all trees' tables, and per run the groups and their event records
     bool tile = false;
+    unsigned char *d_tile_rows = nullptr;
+    uint32_t tile_blocks = 0;
     std::vector<mcg::dev::BatchTileTree> tile_trees;
+    std::vector<mcg::BatchTreeCost> cost;  // per tree
     mcg::dev::BatchTileArgs tile_args{};
     std::vector<void *> tile_tables;
     const uint2 *d_event = nullptr;
@@ -112,6 +116,7 @@ struct mcg_batch {
     uint32_t n_tile_groups = 0, tile_most_events = 0;
     // graph
     cudaGraphExec_t graph = nullptr;
+    bool g_tile = false;
     uint32_t g_instances = 0, g_iteration = 0;
     uint64_t g_words = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -133,10 +138,10 @@ void drop_tile(mcg_batch *b) {
     b->tile_tables.clear();
     cudaFree(b->d_tile_groups);
     cudaFree(b->d_tile_recs);
-    cudaFree(b->d_scratch);
+    cudaFree(b->d_tile_rows);
     b->d_tile_groups = nullptr;
     b->d_tile_recs = nullptr;
-    b->d_scratch = nullptr;
+    b->d_tile_rows = nullptr;
     b->cap_tile_groups = b->cap_tile_recs = 0;
     b->tile = false;
 }
@@ -153,6 +158,7 @@ void release(mcg_batch *b) {
     drop_tile(b);
     cudaFree(b->d_ops);
     cudaFree(b->d_tree_off);
+    cudaFree(b->d_scratch);
     cudaFree(b->d_queue);
     cudaFree(b->d_inst_tree);
     cudaFree(b->d_thr_off);
@@ -222,11 +228,15 @@ mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
         }
         b->tile_most_events = std::max(b->tile_most_events, x.n_be);
         b->tile_trees.push_back(x);
+        const size_t k = b->cost.size(), ops_end = k + 1 < b->trees.size() ? b->tree_op_offset[k + 1] : b->total_ops;
+        b->cost.emplace_back(t.layer, t.gates, t.event.size(), plan.segment.size(), t.in.size(),
+                             ops_end - b->tree_op_offset[k]);
     }
     const uint64_t stride = most_slots * kTileRow;
     const uint64_t blocks = (uint64_t)prop.multiProcessorCount * kBatchTileBlocks;
     if (stride * blocks > kTileScratchMost) return MCG_OK;
-    MCG_CUDA(cudaMalloc((void **)&b->d_scratch, stride * blocks));
+    MCG_CUDA(cudaMalloc((void **)&b->d_tile_rows, stride * blocks));
+    b->tile_blocks = (uint32_t)blocks;
     BatchTileArgs &a = b->tile_args;
     mcg_status st;
     if ((st = upload_table(b, &a.trees, b->tile_trees)) != MCG_OK || (st = upload_table(b, &a.gates, gates)) != MCG_OK ||
@@ -238,15 +248,15 @@ mcg_status setup_tile(mcg_batch *b, const mcg::DeviceShape &prop) {
         return st;
     st = mcg::set_smem_limit(k_batch_tile, (kBatchTileThreads / 32) * kBatchTileOut);
     if (st != MCG_OK) return st;
-    a.scratch = reinterpret_cast<unsigned char *>(b->d_scratch);
+    a.scratch = b->d_tile_rows;
     a.scratch_stride = stride;
     b->tile = true;
     return MCG_OK;
 }
 
-// The interpreter's scratch, where it runs the batch and has none yet.
+// The interpreter's scratch, from its first run on.
 mcg_status interpreter_scratch(mcg_batch *b) {
-    if (b->tile || !b->max_global || b->d_scratch) return MCG_OK;
+    if (!b->max_global || b->d_scratch) return MCG_OK;
     void *p = nullptr;
     MCG_CUDA(cudaMalloc(&p, (size_t)b->max_global * b->share * b->scratch_stride * sizeof(uint64_t)));
     b->d_scratch = static_cast<uint64_t *>(p);
@@ -260,6 +270,28 @@ mcg_status use_interpreter(mcg_batch *b) {
     mcg::clear_error();
     drop_tile(b);
     return interpreter_scratch(b);
+}
+
+// Whether the interpreter is the faster one for a run (tile_cost.hpp).
+bool interpreter_is_faster(const mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tree, uint64_t words) {
+    const uint64_t tiles = (words + mcg::dev::kTileLanes - 1) / mcg::dev::kTileLanes;
+    const uint64_t slabs = (words + kThreads - 1) / kThreads, sms = b->tile_blocks / mcg::dev::kBatchTileBlocks;
+    uint64_t tile = 0, tile_least = 0, interp = 0, interp_least = 0;
+    for (uint32_t i = 0; i < n_inst;) {
+        const mcg::BatchTreeCost &c = b->cost[inst_tree[i]];
+        uint32_t n = 1;
+        while (i + n < n_inst && inst_tree[i + n] == inst_tree[i]) ++n;
+        i += n;
+        interp += (n + b->share - 1) / b->share * slabs * (kThreads / 32) * c.interpreter(b->share);
+        interp_least = std::max(interp_least, c.interpreter_alone(b->share));
+        for (uint32_t left = n; left;) {
+            const uint32_t size = std::min(left, mcg::dev::kTileInstances);
+            left -= size;
+            tile += tiles * c.tile(size);
+            tile_least = std::max(tile_least, c.tile(size) / 2);  // alone on its SM
+        }
+    }
+    return std::max(interp / sms, interp_least) < std::max(tile / b->tile_blocks, tile_least);
 }
 
 mcg_status setup(mcg_batch *b, const mcg_run_desc &run) {
@@ -328,7 +360,7 @@ mcg_status setup(mcg_batch *b, const mcg_run_desc &run) {
 }
 
 // Captures [zero queue, zero ones, persistent launch] for the current shapes.
-mcg_status capture(mcg_batch *b, uint32_t n_inst, uint32_t iteration, uint64_t words) {
+mcg_status capture(mcg_batch *b, bool tile, uint32_t n_inst, uint32_t iteration, uint64_t words) {
     drop_graph(b);
     mcg::dev::BatchArgs a;
     a.ops = b->d_ops;
@@ -352,7 +384,7 @@ mcg_status capture(mcg_batch *b, uint32_t n_inst, uint32_t iteration, uint64_t w
     MCG_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(b->d_queue, 0, sizeof(unsigned long long), b->stream);
     cudaMemsetAsync(b->d_ones, 0, (size_t)n_inst * sizeof(unsigned long long), b->stream);
-    if (b->tile) {
+    if (tile) {
         using namespace mcg::dev;
         BatchTileArgs t = b->tile_args;
         t.groups = b->d_tile_groups;
@@ -366,7 +398,7 @@ mcg_status capture(mcg_batch *b, uint32_t n_inst, uint32_t iteration, uint64_t w
         const dim3 grid(b->n_tile_groups, std::min(64u, std::max(1u, (b->tile_most_events + 255u) / 256u)));
         k_batch_records<<<grid, 256, 0, b->stream>>>(b->d_tile_groups, b->d_event, b->d_event_node, b->d_event_off,
                                                      t.trees, b->d_thr_off, b->d_thr, b->d_tile_recs);
-        k_batch_tile<<<(uint32_t)std::min<uint64_t>((uint64_t)(b->grid / b->ctas_per_sm) * kBatchTileBlocks, t.items), kBatchTileThreads,
+        k_batch_tile<<<(uint32_t)std::min<uint64_t>(b->tile_blocks, t.items), kBatchTileThreads,
                        (kBatchTileThreads / 32) * kBatchTileOut, b->stream>>>(t);
     } else {
         batch_kernel(b->ctas_per_sm, b->share, b->atleast)<<<b->grid, kThreads, b->smem_bytes, b->stream>>>(a);
@@ -381,20 +413,20 @@ mcg_status capture(mcg_batch *b, uint32_t n_inst, uint32_t iteration, uint64_t w
     const cudaError_t inst_err = cudaGraphInstantiate(&b->graph, g, 0);
     cudaGraphDestroy(g);
     if (inst_err != cudaSuccess) return mcg::fail(MCG_ERR_CUDA, cudaGetErrorString(inst_err));
+    b->g_tile = tile;
     b->g_instances = n_inst;
     b->g_iteration = iteration;
     b->g_words = words;
     return MCG_OK;
 }
 
-// A validated run, from its groups to its results on the host.
-mcg_status run_instances(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tree, const uint64_t *thr_offset,
+// A validated run in tiles or by the interpreter, from its groups to its results
+// on the host.
+mcg_status run_instances(mcg_batch *b, bool tile, uint32_t n_inst, const uint32_t *inst_tree, const uint64_t *thr_offset,
                          const uint64_t *thresholds, uint64_t n_thr, uint32_t iteration, uint64_t words,
                          uint64_t *ones) {
-    const mcg_status scratch = interpreter_scratch(b);
-    if (scratch != MCG_OK) return scratch;
     // groups of up to `share` consecutive instances of one tree (up to 16 in tiles)
-    const uint32_t most = b->tile ? mcg::dev::kTileInstances : b->share;
+    const uint32_t most = tile ? mcg::dev::kTileInstances : b->share;
     std::vector<uint32_t> gfirst, gsize;
     for (uint32_t i = 0; i < n_inst;) {
         uint32_t n = 1;
@@ -412,7 +444,7 @@ mcg_status run_instances(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tre
     if (b->n_groups != (uint32_t)gfirst.size()) drop_graph(b);
     b->n_groups = (uint32_t)gfirst.size();
     std::vector<mcg::dev::BatchTileGroup> groups;
-    if (b->tile) {
+    if (tile) {
         // the costliest first (events, and about as much again for every 20
         // instances), so that the last items of the queue are small
         std::vector<uint32_t> order(gfirst.size());
@@ -438,8 +470,8 @@ mcg_status run_instances(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tre
     MCG_CUDA(cudaMemcpyAsync(b->d_inst_tree, inst_tree, n_inst * sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream));
     MCG_CUDA(cudaMemcpyAsync(b->d_thr_off, thr_offset, n_inst * sizeof(uint64_t), cudaMemcpyHostToDevice, b->stream));
     MCG_CUDA(cudaMemcpyAsync(b->d_thr, thresholds, n_thr * sizeof(uint64_t), cudaMemcpyHostToDevice, b->stream));
-    if (!b->graph || b->g_instances != n_inst || b->g_iteration != iteration || b->g_words != words) {
-        const mcg_status st = capture(b, n_inst, iteration, words);
+    if (!b->graph || b->g_tile != tile || b->g_instances != n_inst || b->g_iteration != iteration || b->g_words != words) {
+        const mcg_status st = capture(b, tile, n_inst, iteration, words);
         if (st != MCG_OK) return st;
     }
     MCG_CUDA(cudaEventRecord(b->ev0, b->stream));
@@ -516,13 +548,30 @@ mcg_status mcg_batch_run(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tre
     for (uint64_t k = 0; k < n_thr; ++k)
         if (thresholds[k] > (1ull << 32)) return mcg::fail(MCG_ERR_INVALID, "threshold above 2^32");
     MCG_CUDA(cudaSetDevice(b->device));
-    mcg_status st = run_instances(b, n_inst, inst_tree, thr_offset, thresholds, n_thr, iteration, words, ones);
-    if (st == MCG_ERR_OOM && b->tile) {  // a buffer did not fit next to the tile kernel's memory
+    bool tile = b->tile && !interpreter_is_faster(b, n_inst, inst_tree, words);
+    mcg_status st = tile ? MCG_OK : interpreter_scratch(b);
+    if (st == MCG_ERR_OOM && b->tile) {  // no room for the interpreter next to the tile kernel's memory
+        mcg::clear_error();
+        tile = true;
+        st = MCG_OK;
+    }
+    if (st != MCG_OK) return st;
+    st = run_instances(b, tile, n_inst, inst_tree, thr_offset, thresholds, n_thr, iteration, words, ones);
+    if (st == MCG_ERR_OOM && tile) {  // a buffer did not fit there
         st = use_interpreter(b);
         if (st == MCG_OK)
-            st = run_instances(b, n_inst, inst_tree, thr_offset, thresholds, n_thr, iteration, words, ones);
+            st = run_instances(b, false, n_inst, inst_tree, thr_offset, thresholds, n_thr, iteration, words, ones);
     }
     return st;
+}
+
+mcg_status mcg_batch_kernel(mcg_batch *b, uint32_t n_inst, const uint32_t *inst_tree, uint64_t words, int32_t *tiles) {
+    mcg::clear_error();
+    if (!b || !inst_tree || !tiles) return mcg::fail(MCG_ERR_INVALID, "NULL argument");
+    for (uint32_t i = 0; i < n_inst; ++i)
+        if (inst_tree[i] >= b->trees.size()) return mcg::fail(MCG_ERR_INVALID, "instance tree out of range");
+    *tiles = b->tile && !interpreter_is_faster(b, n_inst, inst_tree, words) ? 1 : 0;
+    return MCG_OK;
 }
 
 mcg_status mcg_batch_info_get(mcg_batch *b, mcg_batch_info *info) {

@@ -1,5 +1,6 @@
-// tile_cost.hpp -- the fused mode's choice between the tile kernel and the
-// interpreter for a pass (host side; no CUDA calls).
+// tile_cost.hpp -- the choice between the tile kernels and the interpreters, for a
+// pass of the fused mode and for a run of batched instances (host side; no CUDA
+// calls).
 #pragma once
 #include <algorithm>
 #include <cstddef>
@@ -7,6 +8,8 @@
 #include <vector>
 
 #include <vector_types.h>
+
+#include "tile.hpp"
 
 namespace mcg {
 
@@ -52,6 +55,58 @@ struct TileCost {
     }
     bool interpreter_is_faster(uint64_t words) const { return interpreter(words) < tile(words); }
     bool interpreter_may_be_faster() const { return interpreter_is_faster(1ull << 32); }
+};
+
+// The same for batched instances, per tree.  The batch tile kernel shares an
+// event's generator calls between up to 16 instances and the interpreter between
+// four, but each of its layers is a barrier and a walk through rows in the L2, so
+// that few instances of deep trees on many words are the interpreter's: two
+// instances of a chain of 522 gates over 360 events on 204,067 words take 11.7 ms
+// in tiles and 6.5 there, one of 200 events on 4,096 words 0.14 and 1.6.
+// Coefficients fitted to both on 60 graphs of 10 to 3,000 events, 1 to 32
+// instances and 2,048 to 131,072 words: of 1,428 runs 36 are more than 4 % behind
+// the better kernel, 11 more than 15 %.
+struct BatchTreeCost {
+    uint64_t events = 0, segments = 0, inputs = 0, ops = 0;
+    uint64_t rounds[3] = {0, 0, 0};        // over the layers: gates per warp, with 1, 2 and 4 quads of instances a gate
+    uint64_t pairs = 0;                    // over the layers: input pairs of the widest gate
+    uint64_t counts = 0, widest_count = 0; // of k-of-n gates: input pairs times counter bits, of all and of the layers' widest
+
+    BatchTreeCost() = default;
+    // layer: gate indices; gates: their records (.x: kind and counter bits, .z: input pairs)
+    BatchTreeCost(const std::vector<uint32_t> &layer, const std::vector<uint4> &gates, size_t n_events, size_t n_segments,
+                  size_t n_inputs, size_t n_ops)
+        : events(n_events), segments(n_segments), inputs(n_inputs), ops(n_ops) {
+        constexpr uint32_t warps = dev::kBatchTileThreads / 32;
+        for (size_t l = 0; l + 1 < layer.size(); ++l) {
+            uint64_t widest = 0, widest_k = 0;
+            for (uint32_t i = layer[l]; i < layer[l + 1]; ++i) {
+                const uint64_t n = gates[i].z;
+                if ((gates[i].x & 3u) == dev::kTileAtleast) {
+                    widest_k = std::max(widest_k, n * ((gates[i].x >> 16) & 0xFu));
+                    counts += n * ((gates[i].x >> 16) & 0xFu);
+                } else {
+                    widest = std::max(widest, n);
+                }
+            }
+            pairs += widest;
+            widest_count += widest_k;
+            for (uint32_t q = 0; q < 3; ++q) rounds[q] += (layer[l + 1] - layer[l] + (warps >> q) - 1) / (warps >> q);
+        }
+    }
+    // Clocks of a block for 32 words of `size` instances, two blocks on its SM.
+    uint64_t tile(uint32_t size) const {
+        const uint64_t quads = (size + 3) / 4;
+        return (size > 8 ? 1315 : size > 4 ? 1037 : 835) * events + 1450 * rounds[quads > 2 ? 2 : quads - 1] + 110 * pairs +
+               30 * inputs * quads + 4590 * segments + 55 * widest_count + 157 * counts * quads;
+    }
+    // Clocks of an SM for a warp's 32 words of `share` instances (4 or 1), and of such a warp on its own.
+    uint64_t interpreter(uint32_t share) const {
+        return share > 1 ? 455 * events + 42 * ops + 65 * counts : 303 * events + 19 * ops + 14 * counts;
+    }
+    uint64_t interpreter_alone(uint32_t share) const {
+        return share > 1 ? 14200 * events + 1325 * ops : 7900 * events + 730 * ops;
+    }
 };
 
 }  // namespace mcg

@@ -55,6 +55,7 @@ _capi.register_signatures({
     "mcg_batch_destroy": (C.c_int, [_vp]),
     "mcg_batch_run": (C.c_int, [_vp, C.c_uint32, _u32p, _u64p, _u64p, C.c_uint64, C.c_uint32, C.c_uint64, _u64p]),
     "mcg_batch_info_get": (C.c_int, [_vp, C.POINTER(BatchInfo)]),
+    "mcg_batch_kernel": (C.c_int, [_vp, C.c_uint32, _u32p, C.c_uint64, C.POINTER(C.c_int32)]),
     "mcg_ua_run": (C.c_int, [_vp, C.POINTER(UaDesc), _dp, C.POINTER(UaStats), _u64p, _dp]),
 })
 
@@ -103,6 +104,14 @@ class Batch:
                                            p(thr, C.c_uint64), thr.size, iteration, words_per_instance,
                                            p(ones, C.c_uint64)))
         return ones
+
+    def takes_tiles(self, inst_tree: Sequence[int], words_per_instance: int) -> bool:
+        """Whether run takes the tile kernel for these instances (else the interpreter)."""
+        inst_tree = np.ascontiguousarray(inst_tree, dtype=np.uint32)
+        tiles = C.c_int32()
+        _capi.check(self.lib.mcg_batch_kernel(self.h, len(inst_tree), inst_tree.ctypes.data_as(_u32p), words_per_instance,
+                                              C.byref(tiles)))
+        return bool(tiles.value)
 
     def info(self) -> dict:
         i = BatchInfo()
