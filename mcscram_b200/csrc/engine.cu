@@ -803,9 +803,11 @@ mcg_status run_strip(mcg_engine *e, uint32_t it_first, uint32_t n_it, uint64_t w
 }
 
 using StageGatesKernel = void (*)(const mcg::dev::StageGateArgs);
-StageGatesKernel stage_gates_kernel(bool wide, bool count) {
-    if (wide) return count ? mcg::dev::k_stage_gates<2, true> : mcg::dev::k_stage_gates<2, false>;
-    return count ? mcg::dev::k_stage_gates<1, true> : mcg::dev::k_stage_gates<1, false>;
+StageGatesKernel stage_gates_kernel(bool wide, bool count, bool split) {
+    using mcg::dev::k_stage_gates;
+    if (split) return count ? k_stage_gates<1, true, true> : k_stage_gates<1, false, true>;
+    if (wide) return count ? k_stage_gates<2, true, false> : k_stage_gates<2, false, false>;
+    return count ? k_stage_gates<1, true, false> : k_stage_gates<1, false, false>;
 }
 
 // Blocks that share the gates of a layer and tile, a launch per layer; 0: every
@@ -901,8 +903,8 @@ mcg_status staged_chunk(mcg_engine *e, uint64_t k, uint32_t iteration, uint64_t 
         const uint64_t blocks = tiles * g.n_gates / std::max<uint32_t>(e->gates_largest_part, 1);
         const uint32_t threads = blocks >= 3ull * e->gate_sms ? 256u : blocks >= 2ull * e->gate_sms ? 512u : 1024u;
         if (!last && e->gates_beside_sampler) tiles = std::min<uint64_t>(tiles, 2ull * e->gate_sms);
-        const StageGatesKernel kern = stage_gates_kernel(wide, e->gates_count);
         const uint32_t splits = gate_splits(e, tiles, blocks);
+        const StageGatesKernel kern = stage_gates_kernel(wide, e->gates_count, splits > 0);
         if (!splits) {
             a.layers = e->n_gate_layers;
             kern<<<dim3((uint32_t)tiles, e->n_gate_parts), threads, 0, e->s_b>>>(a);
