@@ -58,7 +58,8 @@ enum mcg_mode {
     MCG_MODE_FUSED = 4    /* one persistent kernel per launch chunk: sample, gates, tallies fused; in its
                              default shape a tree whose live node words fit in shared memory (about
                              880 at a time) is evaluated in tiles of 32 words per block, others (and
-                             other shapes) by an interpreter of the compiled program */
+                             other shapes, and deep graphs of few events on many words) by an
+                             interpreter of the compiled program (mcg_fused_kernel) */
 };
 
 /* Flattened PDAG handed to the engine.  All arrays are host memory, copied

@@ -7,22 +7,22 @@ import pytest
 from mcscram_b200 import synth
 
 
-def _median_ms(f, n=15):
+def _least_ms(f, n=30):
     t = []
-    for _ in range(n + 3):
+    for _ in range(n):
         a = time.perf_counter()
         f()
         t.append((time.perf_counter() - a) * 1e3)
-    return float(np.median(t[3:]))
+    return min(t)
 
 
 @pytest.mark.gpu
 def test_creation_takes_about_as_long_as_a_plain_engine(capi, gpu):
     """Device buffers, a stream and two events either way: 1.5 ms next to 0.9 for
-    an engine of the layered mode (3.2 to 4.8 with a page of mapped host memory)."""
+    an engine of the layered mode (2.8 to 4.8 with a page of mapped host memory)."""
     from mcscram_b200.importance import ProposalMLP
     g = synth.config1()
-    assert _median_ms(lambda: ProposalMLP().close()) <= 2.5 * _median_ms(
+    assert _least_ms(lambda: ProposalMLP().close()) <= 2.5 * _least_ms(
         lambda: capi.Engine(g, mode=capi.MODES["layered"]).close())
 
 
